@@ -545,30 +545,66 @@ __global__ void __launch_bounds__(kBtThreads, kBtBlocksPerSm) bt_update_kernel(f
   if (threadIdx.x < 32) partial[blockIdx.x * 32 + lane] = v[0];
 }
 
-// One warp: chain lane.  mode 0: start norms -> s_in = 1/||raw||, c2 = 0.
-// mode 1: dot partials <W_k, H W_k> -> z = s_in^2 <W_k, H W_k>, alpha_k, c1 = z * s_in.  mode 2: norm partials -> beta_k, next
-// s_in = 1/beta_k, c2 = beta_k * s_in (old), breakdown bookkeeping.
-__global__ void bt_scalar_kernel(const double* __restrict__ partial, int nblocks, int mode, int k,
-                                 double* __restrict__ st, double* __restrict__ alpha, double* __restrict__ beta,
-                                 int* __restrict__ used) {
-  const int lane = threadIdx.x;
-  if (lane >= 32) return;
-  if (mode == 1) {
-    Neu sr, si;
-    for (int b = 0; b < nblocks; ++b) {
-      sr.add(partial[(b * 32 + lane) * 2]);
-      si.add(partial[(b * 32 + lane) * 2 + 1]);
+// Per-chain totals of the nblocks partial sums of a step, then the recurrence's scalars.  One block, lane = chain:
+// each of the 32 warps adds every 32nd block's partials and warp 0 adds the warps' sums in order, both compensated
+// (fixed order: bitwise repeatable).  The kernel is a serial chain of additions, so its time is the number of
+// additions in series, 740 / 32 + 32 here; with all 740 in one warp it took 88 us, a large part of every step below
+// a million states (4x3 (6,6): 2 x 89 of 1260 us), now about 5 us.
+// mode 0: start norms -> s_in = 1/||raw||, c2 = 0.
+// mode 1: dot partials <W_k, H W_k> -> z = s_in^2 <W_k, H W_k>, alpha_k, c1 = z * s_in; clears the next vector's flag.
+// mode 2: norm partials -> beta_k, next s_in = 1/beta_k, c2 = beta_k * s_in (old), breakdown bookkeeping.
+constexpr int kScalarWarps = 32;
+
+template <int kVals>
+__device__ __forceinline__ void chain_totals(const double* __restrict__ partial, int nblocks, Neu (&tot)[kVals]) {
+  __shared__ double sh[2 * kVals][kScalarWarps][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  Neu acc[kVals];
+#pragma unroll 4
+  for (int b = warp; b < nblocks; b += kScalarWarps) {
+#pragma unroll
+    for (int v = 0; v < kVals; ++v) acc[v].add(partial[(b * 32 + lane) * kVals + v]);
+  }
+#pragma unroll
+  for (int v = 0; v < kVals; ++v) {
+    sh[2 * v][warp][lane] = acc[v].s;
+    sh[2 * v + 1][warp][lane] = acc[v].c;
+  }
+  __syncthreads();
+  if (warp == 0) {
+#pragma unroll 4
+    for (int w = 0; w < kScalarWarps; ++w) {
+#pragma unroll
+      for (int v = 0; v < kVals; ++v) {
+        tot[v].add(sh[2 * v][w][lane]);
+        tot[v].c += sh[2 * v + 1][w][lane];
+      }
     }
+  }
+}
+
+__global__ void __launch_bounds__(32 * kScalarWarps) bt_scalar_kernel(const double* __restrict__ partial, int nblocks,
+                                                                      int mode, int k, double* __restrict__ st,
+                                                                      double* __restrict__ alpha,
+                                                                      double* __restrict__ beta, int* __restrict__ used,
+                                                                      int* __restrict__ clear) {
+  const int lane = threadIdx.x & 31;
+  if (mode == 1) {
+    Neu z[2];
+    chain_totals<2>(partial, nblocks, z);
+    if (threadIdx.x >= 32) return;
     const double s_in = st[kBtSin * 32 + lane];
-    const double zr = sr.value() * s_in * s_in, zi = si.value() * s_in * s_in;
+    const double zr = z[0].value() * s_in * s_in, zi = z[1].value() * s_in * s_in;
     st[kBtC1r * 32 + lane] = zr * s_in;
     st[kBtC1i * 32 + lane] = zi * s_in;
     if (st[kBtActive * 32 + lane] != 0.0) alpha[k * 32 + lane] = zr;
+    if (lane == 0) *clear = 0;
     return;
   }
-  Neu s;
-  for (int b = 0; b < nblocks; ++b) s.add(partial[b * 32 + lane]);
-  const double n2 = s.value();
+  Neu s[1];
+  chain_totals<1>(partial, nblocks, s);
+  if (threadIdx.x >= 32) return;
+  const double n2 = s[0].value();
   if (mode == 0) {
     const double n0 = sqrt(n2);
     st[kBtSin * 32 + lane] = (n0 < 1e-18) ? 0.0 : 1.0 / n0;
@@ -745,22 +781,20 @@ cudaError_t bt_start(float2* W, int64_t dim, unsigned seed, double* st, double* 
   if (e != cudaSuccess) return e;
   bt_start_kernel<<<kBtBlocks, kBtThreads, 0, s>>>(W, dim, seed, partial, flags, gauge ? gauge->umask : nullptr,
                                                    gauge ? gauge->dmask : nullptr, gauge ? gauge->Dd : 1);
-  bt_scalar_kernel<<<1, 32, 0, s>>>(partial, kBtBlocks, 0, 0, st, nullptr, nullptr, used);
+  bt_scalar_kernel<<<1, 32 * kScalarWarps, 0, s>>>(partial, kBtBlocks, 0, 0, st, nullptr, nullptr, used, nullptr);
   return cudaGetLastError();
 }
 
 cudaError_t bt_step(const DevSector& S, const float2* Wk, const float2* Wkm1, float2* Y, int k, double* st,
                     double* partial, double* alpha, double* beta, int* used, int* flags, cudaStream_t s) {
-  // flags[k % 2]: written vector W_k has a tiny non-zero entry; flags[(k+1) % 2] is cleared for W_{k+1}.
+  // flags[k % 2]: written vector W_k has a tiny non-zero entry; flags[(k+1) % 2] is cleared for W_{k+1} by the alpha scalars' kernel.
   int* fin = flags + (k & 1);
   int* fout = flags + ((k + 1) & 1);
-  cudaError_t e = cudaMemsetAsync(fout, 0, sizeof(int), s);
-  if (e != cudaSuccess) return e;
   launch_bt_rows(S, Wk, Y, fin, s);
   launch_bt_cols(S.bt_cols, S, Wk, Y, partial, fin, s);
-  bt_scalar_kernel<<<1, 32, 0, s>>>(partial, kBtBlocks, 1, k, st, alpha, beta, used);
+  bt_scalar_kernel<<<1, 32 * kScalarWarps, 0, s>>>(partial, kBtBlocks, 1, k, st, alpha, beta, used, fout);
   bt_update_kernel<<<kBtBlocks, kBtThreads, 0, s>>>(Y, Wk, Wkm1, S.dim, st, k > 0, partial, fout);
-  bt_scalar_kernel<<<1, 32, 0, s>>>(partial, kBtBlocks, 2, k, st, alpha, beta, used);
+  bt_scalar_kernel<<<1, 32 * kScalarWarps, 0, s>>>(partial, kBtBlocks, 2, k, st, alpha, beta, used, nullptr);
   return cudaGetLastError();
 }
 
@@ -768,12 +802,10 @@ cudaError_t bt_orbit_step(const OrbitApplyDev& A, const float2* Wk, const float2
                           double* partial, double* alpha, double* beta, int* used, int* flags, cudaStream_t s) {
   int* fin = flags + (k & 1);
   int* fout = flags + ((k + 1) & 1);
-  cudaError_t e = cudaMemsetAsync(fout, 0, sizeof(int), s);
-  if (e != cudaSuccess) return e;
   bt_orbit_kernel<<<kBtBlocks, kBtThreads, 0, s>>>(A, Wk, Y, st, partial, fin);
-  bt_scalar_kernel<<<1, 32, 0, s>>>(partial, kBtBlocks, 1, k, st, alpha, beta, used);
+  bt_scalar_kernel<<<1, 32 * kScalarWarps, 0, s>>>(partial, kBtBlocks, 1, k, st, alpha, beta, used, fout);
   bt_update_kernel<<<kBtBlocks, kBtThreads, 0, s>>>(Y, Wk, Wkm1, A.dk, st, k > 0, partial, fout);
-  bt_scalar_kernel<<<1, 32, 0, s>>>(partial, kBtBlocks, 2, k, st, alpha, beta, used);
+  bt_scalar_kernel<<<1, 32 * kScalarWarps, 0, s>>>(partial, kBtBlocks, 2, k, st, alpha, beta, used, nullptr);
   return cudaGetLastError();
 }
 

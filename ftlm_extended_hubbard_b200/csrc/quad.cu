@@ -1,6 +1,6 @@
 // Tridiagonal quadrature on the GPU, FP64 (reference src/ftlm_thermo.cpp:17-146, 150-256):
 //   quad_jacobi   the reference's classical Jacobi (largest |off-diagonal| first, row-major
-//                 first occurrence on ties), one CTA per chain, the dense n x n matrix in shared
+//                 first occurrence on ties), one warp per chain, the upper triangle in shared
 //                 memory, only row 0 of the eigenvector matrix carried (rows of V never mix).
 //                 Rotation arithmetic uses explicit round-to-nearest operations in the
 //                 reference's evaluation order (no contraction), so results follow the
@@ -18,29 +18,60 @@ namespace ftlm_b200 {
 
 namespace {
 
-constexpr int kJacThreads = 256;
-
 __device__ __forceinline__ double mul(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ double add(double a, double b) { return __dadd_rn(a, b); }
 __device__ __forceinline__ double sub(double a, double b) { return __dsub_rn(a, b); }
 
-__global__ void __launch_bounds__(kJacThreads) jacobi_kernel(const double* __restrict__ alpha,
-                                                             const double* __restrict__ beta,
-                                                             const int* __restrict__ nv, int ld, int max_rot_in,
-                                                             double tol, double* __restrict__ lam,
-                                                             double* __restrict__ w0, int* __restrict__ bad) {
+// One warp per chain.  The strict upper triangle is packed (row i: A_ij, j > i, at tri_row(i) + j), the diagonal and
+// row 0 of V apart.  The pivot comes from a maximum kept per row (lane k % 32 owns row k): a rotation (p, q) rewrites
+// rows p and q, whose maxima are reduced as they are written, and the two entries (k, p), (k, q) of each row k above
+// them.  Where the entry that was a row's maximum shrinks, the old value stays as an upper bound without a column,
+// and the row is searched only when that bound is the largest of all (one rotation in three).  So the pivots, and
+// with them every rotation, are those of a full search.
+// The kernel is a serial chain of rotations (atan2, sincos, the row updates, the maxima), bound by its latency; the
+// rows per lane are a template parameter so that nothing is spent on rows that are not there.  n = 60, 4 chains:
+// 15.4 ms with a full search by 256 threads and four block barriers a rotation, 5.5 ms here (0.84 us a rotation, 0.37 of it
+// the trigonometry); 1600 chains: 48 ms, here 8.1, since the packed triangle
+// also lets 15 instead of 7 chains of n = 60 share an SM.
+constexpr int kJacMaxRows = 5;       // rows per lane: n <= 160
+constexpr unsigned kNoCol = 255u;    // the row's value is an upper bound, its column unknown
+
+__device__ __forceinline__ int tri_row(int i, int n) { return i * n - (i * (i + 1)) / 2 - i - 1; }
+
+// |v| as an ordered integer, 0 for NaN (which the strict > of a full search never takes either).
+__device__ __forceinline__ unsigned long long jac_key(double v) {
+  const unsigned long long k = static_cast<unsigned long long>(__double_as_longlong(v)) & 0x7fffffffffffffffull;
+  return k > 0x7ff0000000000000ull ? 0ull : k;
+}
+
+// The lane that holds the warp's largest key, the smallest id among equals.  The upper halves decide unless two
+// lanes share the largest one.
+__device__ __forceinline__ int warp_top(unsigned long long key, unsigned id, unsigned mhi) {
+  const unsigned hi = static_cast<unsigned>(key >> 32);
+  unsigned m = __ballot_sync(0xffffffffu, hi == mhi);
+  if (m & (m - 1u)) {
+    const unsigned lo = static_cast<unsigned>(key);
+    const unsigned mlo = __reduce_max_sync(0xffffffffu, hi == mhi ? lo : 0u);
+    const bool top = hi == mhi && lo == mlo;
+    const unsigned least = __reduce_min_sync(0xffffffffu, top ? id : 0xffffffffu);
+    m = __ballot_sync(0xffffffffu, top && id == least);
+  }
+  return __ffs(static_cast<int>(m)) - 1;
+}
+
+template <int kRows>
+__global__ void __launch_bounds__(32) jacobi_kernel(const double* __restrict__ alpha, const double* __restrict__ beta,
+                                                    const int* __restrict__ nv, int ld, int max_rot_in, double tol,
+                                                    double* __restrict__ lam, double* __restrict__ w0,
+                                                    int* __restrict__ bad) {
   extern __shared__ double sm[];
-  __shared__ double red_v[kJacThreads / 32];
-  __shared__ int red_i[kJacThreads / 32];
-  __shared__ double s_c, s_s, s_app, s_aqq, s_apq;
-  __shared__ int s_p, s_q, s_stop;
   const int ch = blockIdx.x;
   int n = nv[ch];
-  const int tid = threadIdx.x;
-  // A chain length outside [0, ld] would overrun the ld x ld shared matrix and the chain's rows of
+  const int lane = threadIdx.x;
+  // A chain length outside [0, ld] would overrun the shared triangle and the chain's rows of
   // alpha/beta/lam/w0: such a chain is skipped and reported through *bad (when given).
   if (n < 0 || n > ld) {
-    if (tid == 0 && bad) atomicOr(bad, 1);
+    if (lane == 0 && bad) atomicOr(bad, 1);
     n = 0;
   }
   const double* a = alpha + static_cast<int64_t>(ch) * ld;
@@ -49,110 +80,166 @@ __global__ void __launch_bounds__(kJacThreads) jacobi_kernel(const double* __res
   double* wo = w0 + static_cast<int64_t>(ch) * ld;
   if (n <= 0) return;
   if (n == 1) {
-    if (tid == 0) {
+    if (lane == 0) {
       lo[0] = a[0];
       wo[0] = 1.0;
     }
     return;
   }
-  double* A = sm;
-  double* v0 = sm + n * n;
-  for (int i = tid; i < n * n; i += kJacThreads) {
-    const int r = i / n, c = i - r * n;
-    double v = 0.0;
-    if (r == c) v = a[r];
-    else if (c == r + 1) v = b[r];
-    else if (r == c + 1) v = b[c];
-    A[i] = v;
-  }
-  for (int i = tid; i < n; i += kJacThreads) v0[i] = (i == 0) ? 1.0 : 0.0;
-  __syncthreads();
-  const int max_rot = max_rot_in > 0 ? max_rot_in : max(3000, 120 * n);
-  const int lane = tid & 31, warp = tid >> 5;
-  for (int rot = 0; rot < max_rot; ++rot) {
-    // Pivot: largest |A_ij| over i<j, first in row-major order (strict > as the reference).
-    double best = 0.0;
-    int bidx = 0x7fffffff;
-    for (int L = tid; L < n * n; L += kJacThreads) {
-      const int r = L / n, c = L - r * n;
-      if (c <= r) continue;
-      const double v = fabs(A[L]);
-      if (v > best) {
-        best = v;
-        bidx = L;
-      }
-    }
+  double* D = sm;
+  double* v0 = sm + n;
+  double* A = sm + 2 * n;
+  for (int i = lane; i < n * (n - 1) / 2; i += 32) A[i] = 0.0;
+  __syncwarp();
+  unsigned long long rk[kRows];  // per owned row k: key of its largest |A_kj|, j > k
+  unsigned rc[kRows];            // and the first such column
+  int ro[kRows];                 // tri_row of the row
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-      const double ov = __shfl_down_sync(0xffffffffu, best, off);
-      const int oi = __shfl_down_sync(0xffffffffu, bidx, off);
-      if (ov > best || (ov == best && oi < bidx)) {
-        best = ov;
-        bidx = oi;
-      }
+  for (int i = 0; i < kRows; ++i) {
+    const int k = lane + 32 * i;
+    rk[i] = 0ull;
+    rc[i] = static_cast<unsigned>(k + 1);
+    ro[i] = tri_row(k, n);
+    if (k < n) {
+      D[k] = a[k];
+      v0[k] = (k == 0) ? 1.0 : 0.0;
     }
-    if (lane == 0) {
-      red_v[warp] = best;
-      red_i[warp] = bidx;
+    if (k + 1 < n) {
+      A[ro[i] + k + 1] = b[k];
+      rk[i] = jac_key(b[k]);
     }
-    __syncthreads();
-    if (tid == 0) {
-      double bv = red_v[0];
-      int bi = red_i[0];
-      for (int w = 1; w < kJacThreads / 32; ++w)
-        if (red_v[w] > bv || (red_v[w] == bv && red_i[w] < bi)) {
-          bv = red_v[w];
-          bi = red_i[w];
+  }
+  __syncwarp();
+  const int max_rot = max_rot_in > 0 ? max_rot_in : max(3000, 120 * n);
+  for (int rot = 0; rot < max_rot; ++rot) {
+    // Pivot: largest |A_ij| over i < j, first in row-major order (strict > as the reference).
+    int p, q;
+    unsigned long long big;
+    for (;;) {
+      unsigned long long v = rk[0];
+      unsigned code = static_cast<unsigned>(lane) << 8 | rc[0];
+#pragma unroll
+      for (int i = 1; i < kRows; ++i)
+        if (rk[i] > v) {
+          v = rk[i];
+          code = static_cast<unsigned>(lane + 32 * i) << 8 | rc[i];
         }
-      int p = 0, q = 1;
-      if (bi != 0x7fffffff) {
-        p = bi / n;
-        q = bi - p * n;
+      const int src = warp_top(v, code, __reduce_max_sync(0xffffffffu, static_cast<unsigned>(v >> 32)));
+      big = __shfl_sync(0xffffffffu, v, src);
+      code = __shfl_sync(0xffffffffu, code, src);
+      p = static_cast<int>(code >> 8);
+      q = static_cast<int>(code & 255u);
+      if (big == 0ull) {  // nothing off the diagonal: the reference's (0, 1)
+        p = 0;
+        q = 1;
+        break;
       }
-      s_stop = !(bv >= tol);  // reference: break if max_abs < tol (max_abs starts at 0)
-      if (!s_stop) {
-        const double app = A[p * n + p], aqq = A[q * n + q], apq = A[p * n + q];
-        const double phi = mul(0.5, atan2(mul(2.0, apq), sub(aqq, app)));
-        s_c = cos(phi);
-        s_s = sin(phi);
-        s_app = app;
-        s_aqq = aqq;
-        s_apq = apq;
-        s_p = p;
-        s_q = q;
+      if (q != static_cast<int>(kNoCol)) break;
+      const double* row = A + tri_row(p, n);
+      v = 0ull;
+      code = 0u;
+#pragma unroll
+      for (int i = 0; i < kRows; ++i) {
+        const int j = lane + 32 * i;
+        const unsigned long long x = j > p && j < n ? jac_key(row[j]) : 0ull;
+        if (x > v) {
+          v = x;
+          code = static_cast<unsigned>(j);
+        }
+      }
+      const int at = warp_top(v, code, __reduce_max_sync(0xffffffffu, static_cast<unsigned>(v >> 32)));
+      v = __shfl_sync(0xffffffffu, v, at);
+      code = __shfl_sync(0xffffffffu, code, at);
+#pragma unroll
+      for (int i = 0; i < kRows; ++i)
+        if (lane + 32 * i == p) {
+          rk[i] = v;
+          rc[i] = v ? code : static_cast<unsigned>(p + 1);
+        }
+    }
+    if (!(__longlong_as_double(static_cast<long long>(big)) >= tol)) break;  // reference: break if max_abs < tol
+    const int op = tri_row(p, n), oq = tri_row(q, n);
+    const double app = D[p], aqq = D[q], apq = A[op + q];
+    const double vip = v0[p], viq = v0[q];
+    double apk[kRows], aqk[kRows];
+    int ip[kRows], iq[kRows];
+    bool in[kRows];
+#pragma unroll
+    for (int i = 0; i < kRows; ++i) {
+      const int k = lane + 32 * i;
+      in[i] = k < n && k != p && k != q;
+      ip[i] = k < p ? ro[i] + p : op + k;
+      iq[i] = k < q ? ro[i] + q : oq + k;
+      apk[i] = in[i] ? A[ip[i]] : 0.0;
+      aqk[i] = in[i] ? A[iq[i]] : 0.0;
+    }
+    const double phi = mul(0.5, atan2(mul(2.0, apq), sub(aqq, app)));
+    double c, s;
+    sincos(phi, &s, &c);
+    unsigned long long mp = 0ull, mq = 0ull;  // this lane's largest new entries of rows p and q
+    unsigned cp = 0u, cq = 0u;
+#pragma unroll
+    for (int i = 0; i < kRows; ++i) {
+      const int k = lane + 32 * i;
+      const double rpk = sub(mul(c, apk[i]), mul(s, aqk[i]));
+      const double rqk = add(mul(c, aqk[i]), mul(s, apk[i]));
+      if (in[i]) {
+        A[ip[i]] = rpk;
+        A[iq[i]] = rqk;
+      }
+      const unsigned long long kp = in[i] ? jac_key(rpk) : 0ull, kq = in[i] ? jac_key(rqk) : 0ull;
+      if (k > p && kp > mp) {
+        mp = kp;
+        cp = static_cast<unsigned>(k);
+      }
+      if (k > q && kq > mq) {
+        mq = kq;
+        cq = static_cast<unsigned>(k);
+      }
+      if (in[i] && k < q) {  // (k, q), and (k, p) where k < p, are entries of row k
+        const bool both = k < p && kp >= kq;
+        const unsigned long long x = both ? kp : kq;
+        const unsigned xc = static_cast<unsigned>(both ? p : q);
+        const bool was = rc[i] == static_cast<unsigned>(p) || rc[i] == static_cast<unsigned>(q);
+        const bool up = x > rk[i];
+        const bool tie = x == rk[i] && xc < rc[i] && rc[i] != kNoCol;
+        rc[i] = up ? xc : was ? kNoCol : tie ? xc : rc[i];
+        rk[i] = up ? x : rk[i];
       }
     }
-    __syncthreads();
-    if (s_stop) break;
-    const int p = s_p, q = s_q;
-    const double c = s_c, s = s_s;
-    for (int k = tid; k < n; k += kJacThreads) {
-      if (k == p || k == q) continue;
-      const double apk = A[p * n + k], aqk = A[q * n + k];
-      const double rpk = sub(mul(c, apk), mul(s, aqk));
-      const double rqk = add(mul(c, aqk), mul(s, apk));
-      A[p * n + k] = rpk;
-      A[k * n + p] = rpk;
-      A[q * n + k] = rqk;
-      A[k * n + q] = rqk;
+    const unsigned hp = __reduce_max_sync(0xffffffffu, static_cast<unsigned>(mp >> 32));
+    const unsigned hq = __reduce_max_sync(0xffffffffu, static_cast<unsigned>(mq >> 32));
+    const int lp = warp_top(mp, cp, hp), lq = warp_top(mq, cq, hq);
+    mp = __shfl_sync(0xffffffffu, mp, lp);
+    cp = __shfl_sync(0xffffffffu, cp, lp);
+    mq = __shfl_sync(0xffffffffu, mq, lq);
+    cq = __shfl_sync(0xffffffffu, cq, lq);
+#pragma unroll
+    for (int i = 0; i < kRows; ++i) {
+      const int k = lane + 32 * i;
+      if (k == p) {
+        rk[i] = mp;
+        rc[i] = mp ? cp : static_cast<unsigned>(k + 1);
+      }
+      if (k == q) {
+        rk[i] = mq;
+        rc[i] = mq ? cq : static_cast<unsigned>(k + 1);
+      }
     }
-    if (tid == 0) {
-      const double app = s_app, aqq = s_aqq, apq = s_apq;
-      const double cc = mul(c, c), ss = mul(s, s), tsc = mul(mul(2.0, s), c);
-      const double npp = add(sub(mul(cc, app), mul(tsc, apq)), mul(ss, aqq));
-      const double nqq = add(add(mul(ss, app), mul(tsc, apq)), mul(cc, aqq));
-      A[p * n + q] = 0.0;
-      A[q * n + p] = 0.0;
-      A[p * n + p] = npp;
-      A[q * n + q] = nqq;
-      const double vip = v0[p], viq = v0[q];
+    const double cc = mul(c, c), ss = mul(s, s), tsc = mul(mul(2.0, s), c);
+    const double npp = add(sub(mul(cc, app), mul(tsc, apq)), mul(ss, aqq));
+    const double nqq = add(add(mul(ss, app), mul(tsc, apq)), mul(cc, aqq));
+    if (lane == 0) {
+      D[p] = npp;
+      D[q] = nqq;
+      A[op + q] = 0.0;
       v0[p] = sub(mul(c, vip), mul(s, viq));
       v0[q] = add(mul(s, vip), mul(c, viq));
     }
-    __syncthreads();
+    __syncwarp();
   }
-  for (int k = tid; k < n; k += kJacThreads) {
-    lo[k] = A[k * n + k];
+  for (int k = lane; k < n; k += 32) {
+    lo[k] = D[k];
     wo[k] = mul(v0[k], v0[k]);
   }
 }
@@ -308,10 +395,15 @@ __global__ void ritz_kernel(const double* __restrict__ a, const double* __restri
 cudaError_t quad_jacobi(const double* alpha, const double* beta, const int* n, int nc, int ld, int max_rot,
                         double tol, double* lam, double* w0, cudaStream_t st, int* bad) {
   if (nc <= 0) return cudaSuccess;
-  const size_t sm = (static_cast<size_t>(ld) * ld + ld) * sizeof(double);
-  cudaError_t e = cudaFuncSetAttribute(jacobi_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sm));
+  if (ld <= 0 || ld > 32 * kJacMaxRows) return cudaErrorInvalidValue;
+  using K = void (*)(const double*, const double*, const int*, int, int, double, double*, double*, int*);
+  static const K kernels[kJacMaxRows] = {jacobi_kernel<1>, jacobi_kernel<2>, jacobi_kernel<3>, jacobi_kernel<4>,
+                                         jacobi_kernel<5>};
+  const K k = kernels[(ld - 1) / 32];
+  const size_t sm = (static_cast<size_t>(ld) * (ld - 1) / 2 + 2 * static_cast<size_t>(ld)) * sizeof(double);
+  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sm));
   if (e != cudaSuccess) return e;
-  jacobi_kernel<<<nc, kJacThreads, sm, st>>>(alpha, beta, n, ld, max_rot, tol, lam, w0, bad);
+  k<<<nc, 32, sm, st>>>(alpha, beta, n, ld, max_rot, tol, lam, w0, bad);
   return cudaGetLastError();
 }
 

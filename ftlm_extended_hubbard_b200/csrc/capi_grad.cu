@@ -19,7 +19,7 @@ struct ChainGrad {
   double lmin = 0.0, g = 0.0, m[3] = {0.0, 0.0, 0.0};
 };
 
-// Weight matrices of up to nc chains on the GPU (symeig.cu: Jacobi eigen-decomposition of each
+// Weight matrices of up to nc chains on the GPU (symeig.cu: QL eigen-decomposition of each
 // chain's tridiagonal, then K = Z P Z^T), written to g_grad.Kp in the layout [i][ld][nc] (chain
 // fastest) with the scales 1/(sc_i sc_l); g and the lowest Ritz value per chain to `out`.
 int fill_weights(ftlm_sector* s, int nc, int ld, double bT, const std::vector<int>& n, const std::vector<double>& A,
@@ -63,7 +63,7 @@ int fill_weights(ftlm_sector* s, int nc, int ld, double bT, const std::vector<in
     ChainGrad& cg = (*out)[static_cast<size_t>(c)];
     cg = ChainGrad{};
     if (n[static_cast<size_t>(c)] <= 0) continue;
-    if (info[static_cast<size_t>(c)] != 0) return fail(FTLM_ERR_NUMERIC, "GPU Jacobi eigen-solver did not converge");
+    if (info[static_cast<size_t>(c)] != 0) return fail(FTLM_ERR_NUMERIC, "GPU eigen-solver did not converge");
     cg.ok = true;
     cg.g = g[static_cast<size_t>(c)];
     cg.lmin = lm[static_cast<size_t>(c)];
@@ -445,8 +445,8 @@ int ftlm_gpu_gc_logz_grad(const ftlm_params* p, double mu, double bT, int R, int
   return FTLM_OK;
 }
 
-// Per-chain log quadrature and energy ratio with a converged eigen-decomposition (parallel cyclic
-// Jacobi on the GPU, symeig.cu), the quadrature the gradient differentiates; same layout as
+// Per-chain log quadrature and energy ratio with a converged eigen-decomposition (implicit QL
+// on the GPU, symeig.cu), the quadrature the gradient differentiates; same layout as
 // ftlm_gpu_tridiag_quadrature.
 int ftlm_gpu_tridiag_quadrature_exact(const double* alpha, const double* beta, const int* n, int nc, int ld,
                                       const double* bts, int n_bt, double* logq, double* energy) {
@@ -480,7 +480,7 @@ int ftlm_gpu_tridiag_quadrature_exact(const double* alpha, const double* beta, c
   std::vector<int> info(static_cast<size_t>(nc));
   CU_TRY(cudaMemcpy(info.data(), di.p, nc * sizeof(int), cudaMemcpyDeviceToHost));
   for (int c = 0; c < nc; ++c)
-    if (n[c] > 0 && info[static_cast<size_t>(c)] != 0) return fail(FTLM_ERR_NUMERIC, "GPU Jacobi eigen-solver did not converge");
+    if (n[c] > 0 && info[static_cast<size_t>(c)] != 0) return fail(FTLM_ERR_NUMERIC, "GPU eigen-solver did not converge");
   CU_TRY(cudaMemcpy(logq, dq.p, outb, cudaMemcpyDeviceToHost));
   CU_TRY(cudaMemcpy(energy, de.p, outb, cudaMemcpyDeviceToHost));
   return FTLM_OK;

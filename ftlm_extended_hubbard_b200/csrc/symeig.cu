@@ -3,10 +3,13 @@
 //   symeig_kernel   parallel cyclic Jacobi (Brent-Luk round-robin ordering: m/2 disjoint rotations
 //                   per round, m-1 rounds per sweep, sweeps until the off-diagonal Frobenius norm is
 //                   below 1e-15 of the matrix norm), the matrix in shared memory (m <= 160, row
-//                   stride m+1 so that column accesses of a warp fall in distinct bank pairs).  Input
-//                   dense or tridiagonal; output eigenvalues in ascending order, optionally the squared
-//                   first row of the eigenvector matrix (the quadrature weights) or all eigenvectors
-//                   (row j of Vt = eigenvector j).
+//                   stride m+1 so that column accesses of a warp fall in distinct bank pairs):
+//                   eigenvalues of a dense matrix in ascending order.
+//   tql_weights_kernel, tql_vectors_kernel
+//                   implicit QL iteration of a tridiagonal matrix (Bowdler, Martin, Reinsch and
+//                   Wilkinson, Numer. Math. 11, 293 (1968)): eigenvalues in ascending order with the
+//                   squared first row of the eigenvector matrix (the quadrature weights), or with all
+//                   eigenvectors (row j of Vt = eigenvector j).
 //   duhamel_kernel  the Duhamel weight matrix of one Lanczos chain from its eigen-decomposition:
 //                   K = Z P Z^T, P_jk = Z_0j Z_0k (e^{-b l_j} - e^{-b l_k}) / (l_k - l_j) (the limit
 //                   b e^{-b l_j} on the diagonal), with the same shift l_0 and the same expm1 form
@@ -39,13 +42,9 @@ __device__ __forceinline__ void rr_pair(int r, int k, int m, int* p, int* q) {
   *q = max(a, b);
 }
 
-template <int kV>  // 0: eigenvalues only, 1: + first row of V, 2: + all eigenvectors (Vt rows)
 __global__ void __launch_bounds__(kEigThreads) symeig_kernel(const double* __restrict__ dense,
-                                                             const double* __restrict__ alpha,
-                                                             const double* __restrict__ beta,
                                                              const int* __restrict__ nv, int ld,
-                                                             double* __restrict__ lam, double* __restrict__ v0,
-                                                             double* __restrict__ vt, int* __restrict__ info) {
+                                                             double* __restrict__ lam, int* __restrict__ info) {
   extern __shared__ double sm[];
   __shared__ double rc[kMaxEig / 2], rs[kMaxEig / 2];
   __shared__ int rp[kMaxEig / 2], rq[kMaxEig / 2];
@@ -66,31 +65,12 @@ __global__ void __launch_bounds__(kEigThreads) symeig_kernel(const double* __res
   const int m = n + (n & 1);  // even order; a padding index stays decoupled (zero row and column)
   const int S = m + 1;        // row stride in shared memory
   double* A = sm;
-  double* V0 = sm + static_cast<size_t>(m) * S;  // first row of V (kV == 1)
-  double* Vt = vt ? vt + static_cast<int64_t>(ch) * ld * ld : nullptr;  // kV == 2, rows = eigenvectors
   for (int i = tid; i < m * S; i += kEigThreads) {
     const int r = i / S, c = i - r * S;
     double v = 0.0;
-    if (r < n && c < n) {
-      if (dense) {
-        v = dense[static_cast<int64_t>(ch) * ld * ld + static_cast<int64_t>(r) * ld + c];
-      } else {
-        const double* a = alpha + static_cast<int64_t>(ch) * ld;
-        const double* b = beta + static_cast<int64_t>(ch) * ld;
-        if (r == c) v = a[r];
-        else if (c == r + 1) v = b[r];
-        else if (r == c + 1) v = b[c];
-      }
-    }
+    if (r < n && c < n) v = dense[static_cast<int64_t>(ch) * ld * ld + static_cast<int64_t>(r) * ld + c];
     A[i] = v;
   }
-  if (kV == 1)
-    for (int i = tid; i < m; i += kEigThreads) V0[i] = (i == 0) ? 1.0 : 0.0;
-  if (kV == 2)
-    for (int i = tid; i < m * m; i += kEigThreads) {
-      const int r = i / m, c = i - r * m;
-      if (r < n && c < n) Vt[static_cast<int64_t>(r) * ld + c] = (r == c) ? 1.0 : 0.0;
-    }
   __syncthreads();
   // Frobenius norm for the stopping rule
   double fro = 0.0;
@@ -153,7 +133,7 @@ __global__ void __launch_bounds__(kEigThreads) symeig_kernel(const double* __res
         A[q * S + j] = s * x + c * y;
       }
       __syncthreads();
-      // columns: A <- A J (and V <- V J)
+      // columns: A <- A J
       for (int i = tid; i < half * m; i += kEigThreads) {
         const int k = i / m, j = i - k * m;
         const int p = rp[k], q = rq[k];
@@ -162,26 +142,6 @@ __global__ void __launch_bounds__(kEigThreads) symeig_kernel(const double* __res
         A[j * S + p] = c * x - s * y;
         A[j * S + q] = s * x + c * y;
       }
-      if (kV == 1)
-        for (int k = tid; k < half; k += kEigThreads) {
-          const int p = rp[k], q = rq[k];
-          const double c = rc[k], s = rs[k];
-          const double x = V0[p], y = V0[q];
-          V0[p] = c * x - s * y;
-          V0[q] = s * x + c * y;
-        }
-      if (kV == 2)
-        for (int i = tid; i < half * m; i += kEigThreads) {
-          const int k = i / m, j = i - k * m;
-          const int p = rp[k], q = rq[k];
-          if (p >= n || q >= n || j >= n) continue;  // the padding index never mixes (its column is zero)
-          const double c = rc[k], s = rs[k];
-          double* vp = Vt + static_cast<int64_t>(p) * ld;
-          double* vq = Vt + static_cast<int64_t>(q) * ld;
-          const double x = vp[j], y = vq[j];
-          vp[j] = c * x - s * y;
-          vq[j] = s * x + c * y;
-        }
       __syncthreads();
       for (int k = tid; k < half; k += kEigThreads) {  // the rotation annihilates a_pq
         const int p = rp[k], q = rq[k];
@@ -205,36 +165,216 @@ __global__ void __launch_bounds__(kEigThreads) symeig_kernel(const double* __res
       rank += (lk < lj || (lk == lj && k < j)) ? 1 : 0;
     }
     lo[rank] = lj;
-    if (kV == 1) v0[static_cast<int64_t>(ch) * ld + rank] = V0[j] * V0[j];  // weight Z_0j^2
-    if (kV == 2) reinterpret_cast<int*>(V0)[j] = rank;  // permutation for the row move below
   }
-  if (kV == 2) {
-    // Vt rows to ascending order: eigenvector j belongs at row rank(j); move through the row-0
-    // scratch of shared memory one destination row at a time (rows are n <= 160 doubles).
-    __syncthreads();
-    const int* rk = reinterpret_cast<const int*>(V0);
-    double* tmp = A;  // A's diagonal was consumed above; reuse its storage
-    for (int i = tid; i < n * n; i += kEigThreads) {
-      const int j = i / n, c = i - j * n;
-      tmp[rk[j] * n + c] = Vt[static_cast<int64_t>(j) * ld + c];
+}
+
+// Implicit QL iteration of one symmetric tridiagonal of order n: d[i * st] the diagonal and e[i * st] the entry
+// below it (e[n - 1] = 0), overwritten by the eigenvalues and zeros; every rotation is applied to columns i and
+// i + 1 of one row of the eigenvector matrix, z[i * zst].  The rotations of a sweep are a serial chain (one rsqrt and
+// about eight multiply-adds each), which bounds both kernels below; the loads of the next rotation are issued before
+// the chain of this one.  Returns whether every eigenvalue converged within 60 sweeps.
+__device__ __forceinline__ bool tql(double* d, double* e, int st, double* z, int zst, int n) {
+  constexpr double kEps = 2.220446049250313e-16;
+  for (int l = 0; l < n; ++l) {
+    for (int it = 0;; ++it) {
+      int m = l;
+      double dm = d[l * st];
+      for (; m < n - 1; ++m) {
+        const double dn = d[(m + 1) * st];
+        if (fabs(e[m * st]) <= kEps * (fabs(dm) + fabs(dn))) break;
+        dm = dn;
+      }
+      if (m == l) break;
+      if (it == 60) return false;
+      const double el = e[l * st], dl = d[l * st];
+      double g = (d[(l + 1) * st] - dl) / (2.0 * el);
+      const double r0 = sqrt(fma(g, g, 1.0));
+      g = dm - dl + el / (g + copysign(r0, g));
+      double s = 1.0, c = 1.0, p = 0.0;
+      double dnext = dm, ei = e[(m - 1) * st], di = d[(m - 1) * st], zi = z[(m - 1) * zst], zn = z[m * zst];
+      int i = m - 1;
+      for (; i >= l; --i) {
+        const double f = s * ei, b = c * ei, dcur = di, zcur = zi;
+        if (i > l) {
+          ei = e[(i - 1) * st];
+          di = d[(i - 1) * st];
+          zi = z[(i - 1) * zst];
+        }
+        const double h = fma(f, f, g * g);
+        if (h == 0.0) {  // the matrix splits at i + 1
+          d[(i + 1) * st] = dnext - p;
+          e[(i + 1) * st] = 0.0;
+          e[m * st] = 0.0;
+          z[(i + 1) * zst] = zn;
+          break;
+        }
+        const double inv = rsqrt(h);
+        e[(i + 1) * st] = h * inv;
+        s = f * inv;
+        c = g * inv;
+        g = dnext - p;
+        const double t = fma(dcur - g, s, 2.0 * c * b);
+        p = s * t;
+        d[(i + 1) * st] = g + p;
+        g = fma(c, t, -b);
+        dnext = dcur;
+        z[(i + 1) * zst] = fma(s, zcur, c * zn);
+        zn = fma(c, zcur, -s * zn);
+      }
+      if (i >= l) continue;
+      d[l * st] = dnext - p;
+      e[l * st] = g;
+      e[m * st] = 0.0;
+      z[l * zst] = zn;
     }
-    __syncthreads();
-    for (int i = tid; i < n * n; i += kEigThreads) {
-      const int j = i / n, c = i - j * n;
-      Vt[static_cast<int64_t>(j) * ld + c] = tmp[i];
+  }
+  return true;
+}
+
+// Power of two that brings the largest |a_i|, |b_i| (n of the former, n - 1 of the latter) into [1, 2), so that the
+// squares in tql neither overflow nor underflow; 0 for a zero matrix or entries that are not finite.
+__device__ __forceinline__ double tql_scale(double big) {
+  if (!(big > 0.0) || !(big <= DBL_MAX)) return 0.0;
+  return scalbn(1.0, -ilogb(big));
+}
+
+// Chains per block: one lane each.  A chain is one lane's serial work, so few share a warp (the others wait for the
+// longest); 32 chains of n = 80 are 8 blocks.
+constexpr int kTqlChains = 4;
+
+// Eigenvalues (ascending) and first-row weights.  Bound by the serial chain of about 0.85 n^2 rotations: 32 chains of
+// n = 80 take 1.1 ms, against 2.3 ms for the parallel cyclic Jacobi on the dense matrix.
+__global__ void __launch_bounds__(32) tql_weights_kernel(const double* __restrict__ alpha,
+                                                         const double* __restrict__ beta, const int* __restrict__ nv,
+                                                         int nm, int ld, double* __restrict__ lam,
+                                                         double* __restrict__ w0, int* __restrict__ info) {
+  extern __shared__ double sm[];
+  const int lane = threadIdx.x;
+  const int ch0 = blockIdx.x * kTqlChains;
+  double* d = sm;
+  double* e = d + ld * kTqlChains;
+  double* z = e + ld * kTqlChains;
+  for (int i = lane; i < ld * kTqlChains; i += 32) {
+    const int ch = ch0 + i / ld, k = i % ld, at = k * kTqlChains + i / ld;
+    const int n = ch < nm ? nv[ch] : 0;
+    const bool in = k < n && n <= ld;
+    d[at] = in ? alpha[static_cast<int64_t>(ch) * ld + k] : 0.0;
+    e[at] = in && k + 1 < n ? beta[static_cast<int64_t>(ch) * ld + k] : 0.0;
+    z[at] = k == 0 ? 1.0 : 0.0;
+  }
+  __syncwarp();
+  double unscale = 1.0;
+  if (lane < kTqlChains && ch0 + lane < nm) {
+    const int n = nv[ch0 + lane];
+    if (n < 0 || n > ld) {  // out of range: report, write nothing
+      if (info) info[ch0 + lane] = 2;
+    } else {
+      double big = 0.0;
+      bool finite = true;
+      for (int k = 0; k < n; ++k) {
+        const double a = fabs(d[k * kTqlChains + lane]), b = fabs(e[k * kTqlChains + lane]);
+        finite = finite && a <= DBL_MAX && b <= DBL_MAX;
+        big = fmax(big, fmax(a, b));
+      }
+      const double sc = finite ? tql_scale(big) : 0.0;
+      bool ok = true;
+      if (sc != 0.0) {
+        for (int k = 0; k < n; ++k) {
+          d[k * kTqlChains + lane] *= sc;
+          e[k * kTqlChains + lane] *= sc;
+        }
+        ok = tql(d + lane, e + lane, kTqlChains, z + lane, kTqlChains, n);
+        unscale = 1.0 / sc;
+      }
+      if (info) info[ch0 + lane] = ok ? 0 : 1;
     }
+  }
+  __syncwarp();
+  for (int c = 0; c < kTqlChains && ch0 + c < nm; ++c) {
+    const int n = nv[ch0 + c];
+    if (n < 0 || n > ld) continue;
+    const double us = __shfl_sync(0xffffffffu, unscale, c);
+    for (int j = lane; j < n; j += 32) {
+      const double lj = d[j * kTqlChains + c];
+      int rank = 0;
+      for (int k = 0; k < n; ++k) {
+        const double lk = d[k * kTqlChains + c];
+        rank += (lk < lj || (lk == lj && k < j)) ? 1 : 0;
+      }
+      const double zj = z[j * kTqlChains + c];
+      lam[static_cast<int64_t>(ch0 + c) * ld + rank] = lj * us;
+      w0[static_cast<int64_t>(ch0 + c) * ld + rank] = zj * zj;
+    }
+  }
+}
+
+// Eigenvalues (ascending) and all eigenvectors, one block per matrix: thread k owns row k of the eigenvector matrix
+// (Z[i][k] in shared memory, conflict-free), and every warp runs the scalar recurrence on its own copy of the
+// tridiagonal, identically, so no barrier is needed until the end.
+__global__ void __launch_bounds__(kMaxEig) tql_vectors_kernel(const double* __restrict__ alpha,
+                                                              const double* __restrict__ beta,
+                                                              const int* __restrict__ nv, int ld,
+                                                              double* __restrict__ lam, double* __restrict__ vt,
+                                                              int* __restrict__ info) {
+  extern __shared__ double sm[];
+  const int ch = blockIdx.x;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int n = nv[ch];
+  if (n < 0 || n > ld) {
+    if (tid == 0 && info) info[ch] = 2;
+    return;
+  }
+  double* d = sm + 2 * ld * warp;
+  double* e = d + ld;
+  double* z = sm + 2 * ld * (blockDim.x >> 5) + tid;
+  const int zst = blockDim.x;
+  double big = 0.0;
+  bool finite = true;
+  for (int i = lane; i < n; i += 32) {
+    d[i] = alpha[static_cast<int64_t>(ch) * ld + i];
+    e[i] = i + 1 < n ? beta[static_cast<int64_t>(ch) * ld + i] : 0.0;
+    finite = finite && fabs(d[i]) <= DBL_MAX && fabs(e[i]) <= DBL_MAX;
+    big = fmax(big, fmax(fabs(d[i]), fabs(e[i])));
+  }
+  for (int o = 16; o > 0; o >>= 1) big = fmax(big, __shfl_xor_sync(0xffffffffu, big, o));
+  finite = __all_sync(0xffffffffu, finite);
+  for (int i = 0; i < n; ++i) z[i * zst] = i == tid ? 1.0 : 0.0;
+  const double sc = finite ? tql_scale(big) : 0.0;
+  bool ok = true;
+  if (sc != 0.0) {
+    for (int i = lane; i < n; i += 32) {
+      d[i] *= sc;
+      e[i] *= sc;
+    }
+    __syncwarp();
+    ok = tql(d, e, 1, z, zst, n);
+  }
+  __syncwarp();
+  if (tid == 0 && info) info[ch] = ok ? 0 : 1;
+  const double us = sc != 0.0 ? 1.0 / sc : 1.0;
+  for (int j = 0; j < n; ++j) {
+    const double lj = d[j];
+    int rank = 0;
+    for (int k = lane; k < n; k += 32) rank += (d[k] < lj || (d[k] == lj && k < j)) ? 1 : 0;
+    rank = __reduce_add_sync(0xffffffffu, rank);
+    if (tid == 0) lam[static_cast<int64_t>(ch) * ld + rank] = lj * us;
+    if (tid < n) vt[(static_cast<int64_t>(ch) * ld + rank) * ld + tid] = z[j * zst];
   }
 }
 
 // K = Z P Z^T in the moment kernel's layout Kp[(i*ld + l)*nc + c] / (sc_i sc_l), with
 // Z[i][j] = Vt[j][i] (ascending l_j); g = sum_j Z_0j^2 e^{-b (l_j - l_0)}, lmin = l_0.
-__global__ void __launch_bounds__(kEigThreads) duhamel_kernel(const double* __restrict__ lam,
+// P is formed once in shared memory (one expm1 and one division an entry); both products then read it and V.
+constexpr int kDuhThreads = 512;
+
+__global__ void __launch_bounds__(kDuhThreads) duhamel_kernel(const double* __restrict__ lam,
                                                               const double* __restrict__ vt,
                                                               const int* __restrict__ nv, int ld, int nc, double bT,
                                                               const double* __restrict__ scale,
                                                               double* __restrict__ Y, double* __restrict__ Kp,
                                                               double* __restrict__ g_out,
                                                               double* __restrict__ lmin_out) {
+  extern __shared__ double P[];  // [n][n]
   const int ch = blockIdx.x;
   const int tid = threadIdx.x;
   const int n = nv[ch];
@@ -244,36 +384,40 @@ __global__ void __launch_bounds__(kEigThreads) duhamel_kernel(const double* __re
   double* y = Y + static_cast<int64_t>(ch) * ld * ld;
   const double* sc = scale + static_cast<int64_t>(ch) * ld;
   const double shift = l[0];
-  __shared__ double ew[kMaxEig];
-  for (int j = tid; j < n; j += kEigThreads) ew[j] = exp(-bT * (l[j] - shift));
-  __syncthreads();
-  // Y[i][k] = sum_j Z_ij Z_0j D_jk, then K_il = sum_k Y_ik Z_0k Z_lk
-  for (int e = tid; e < n * n; e += kEigThreads) {
-    const int i = e / n, k = e - i * n;
-    double acc = 0.0;
-    for (int j = 0; j < n; ++j) {
-      const int a = min(j, k), b = max(j, k);
-      const double ea = ew[a];
-      const double delta = l[b] - l[a];
-      const double D = (a == b || delta == 0.0) ? bT * ea : ea * (-expm1(-bT * delta)) / delta;
-      acc += V[static_cast<int64_t>(j) * ld + i] * V[static_cast<int64_t>(j) * ld] * D;
-    }
-    y[static_cast<int64_t>(i) * ld + k] = acc;
+  __shared__ double ew[kMaxEig], z0[kMaxEig];
+  for (int j = tid; j < n; j += kDuhThreads) {
+    ew[j] = exp(-bT * (l[j] - shift));
+    z0[j] = V[static_cast<int64_t>(j) * ld];
   }
   __syncthreads();
-  for (int e = tid; e < n * n; e += kEigThreads) {
+  for (int e = tid; e < n * n; e += kDuhThreads) {
+    const int j = e / n, k = e - j * n;
+    const int a = min(j, k), b = max(j, k);
+    const double ea = ew[a];
+    const double delta = l[b] - l[a];
+    P[e] = z0[j] * ((a == b || delta == 0.0) ? bT * ea : ea * (-expm1(-bT * delta)) / delta);
+  }
+  __syncthreads();
+  // Y[i][k] = sum_j Z_ij Z_0j D_jk, then K_il = sum_k Y_ik Z_0k Z_lk
+  for (int e = tid; e < n * n; e += kDuhThreads) {
+    const int k = e / n, i = e - k * n;
+    double acc = 0.0;
+#pragma unroll 4
+    for (int j = 0; j < n; ++j) acc = fma(V[static_cast<int64_t>(j) * ld + i], P[j * n + k], acc);
+    y[static_cast<int64_t>(k) * ld + i] = acc * z0[k];
+  }
+  __syncthreads();
+  for (int e = tid; e < n * n; e += kDuhThreads) {
     const int i = e / n, lq = e - i * n;
     double acc = 0.0;
+#pragma unroll 4
     for (int k = 0; k < n; ++k)
-      acc += y[static_cast<int64_t>(i) * ld + k] * V[static_cast<int64_t>(k) * ld] * V[static_cast<int64_t>(k) * ld + lq];
+      acc = fma(y[static_cast<int64_t>(k) * ld + i], V[static_cast<int64_t>(k) * ld + lq], acc);
     Kp[(static_cast<int64_t>(i) * ld + lq) * nc + ch] = acc / (sc[i] * sc[lq]);
   }
   if (tid == 0) {
     double gs = 0.0;
-    for (int j = 0; j < n; ++j) {
-      const double z0 = V[static_cast<int64_t>(j) * ld];
-      gs += z0 * z0 * ew[j];
-    }
+    for (int j = 0; j < n; ++j) gs += z0[j] * z0[j] * ew[j];
     g_out[ch] = gs;
     lmin_out[ch] = shift;
   }
@@ -305,21 +449,18 @@ cudaError_t embed_hermitian(const double2* cols, int dk, double* R, cudaStream_t
 cudaError_t symeig_tridiag(const double* alpha, const double* beta, const int* n, int nm, int ld, double* lam,
                            double* v0, double* vt, int* info, cudaStream_t st) {
   if (nm <= 0) return cudaSuccess;
-  if (ld > kMaxEig || ld <= 0) return cudaErrorInvalidValue;
-  const int m = ld + (ld & 1);
-  const size_t sm = (static_cast<size_t>(m) * (m + 1) + m) * sizeof(double);
-  cudaError_t e;
+  if (ld > kMaxEig || ld <= 0 || (!v0 && !vt)) return cudaErrorInvalidValue;
   if (vt) {
-    e = cudaFuncSetAttribute(symeig_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sm));
-    if (e == cudaSuccess) symeig_kernel<2><<<nm, kEigThreads, sm, st>>>(nullptr, alpha, beta, n, ld, lam, v0, vt, info);
-  } else if (v0) {
-    e = cudaFuncSetAttribute(symeig_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sm));
-    if (e == cudaSuccess) symeig_kernel<1><<<nm, kEigThreads, sm, st>>>(nullptr, alpha, beta, n, ld, lam, v0, vt, info);
+    const int threads = (ld + 31) / 32 * 32;
+    const size_t sm = (static_cast<size_t>(2) * ld * (threads / 32) + static_cast<size_t>(ld) * threads) * sizeof(double);
+    const cudaError_t e = cudaFuncSetAttribute(tql_vectors_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               static_cast<int>(sm));
+    if (e != cudaSuccess) return e;
+    tql_vectors_kernel<<<nm, threads, sm, st>>>(alpha, beta, n, ld, lam, vt, info);
   } else {
-    e = cudaFuncSetAttribute(symeig_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sm));
-    if (e == cudaSuccess) symeig_kernel<0><<<nm, kEigThreads, sm, st>>>(nullptr, alpha, beta, n, ld, lam, v0, vt, info);
+    const size_t sm = static_cast<size_t>(3) * ld * kTqlChains * sizeof(double);
+    tql_weights_kernel<<<(nm + kTqlChains - 1) / kTqlChains, 32, sm, st>>>(alpha, beta, n, nm, ld, lam, v0, info);
   }
-  if (e != cudaSuccess) return e;
   return cudaGetLastError();
 }
 
@@ -328,16 +469,19 @@ cudaError_t symeig_dense(const double* A, const int* n, int nm, int ld, double* 
   if (ld > kMaxEig || ld <= 0) return cudaErrorInvalidValue;
   const int m = ld + (ld & 1);
   const size_t sm = (static_cast<size_t>(m) * (m + 1) + m) * sizeof(double);
-  cudaError_t e = cudaFuncSetAttribute(symeig_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sm));
+  cudaError_t e = cudaFuncSetAttribute(symeig_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sm));
   if (e != cudaSuccess) return e;
-  symeig_kernel<0><<<nm, kEigThreads, sm, st>>>(A, nullptr, nullptr, n, ld, lam, nullptr, nullptr, info);
+  symeig_kernel<<<nm, kEigThreads, sm, st>>>(A, n, ld, lam, info);
   return cudaGetLastError();
 }
 
 cudaError_t duhamel_weights_dev(const double* lam, const double* vt, const int* n, int nc, int ld, double bT,
                                 const double* scale, double* Y, double* Kp, double* g, double* lmin, cudaStream_t st) {
   if (nc <= 0) return cudaSuccess;
-  duhamel_kernel<<<nc, kEigThreads, 0, st>>>(lam, vt, n, ld, nc, bT, scale, Y, Kp, g, lmin);
+  const size_t sm = static_cast<size_t>(ld) * ld * sizeof(double);
+  const cudaError_t e = cudaFuncSetAttribute(duhamel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sm));
+  if (e != cudaSuccess) return e;
+  duhamel_kernel<<<nc, kDuhThreads, sm, st>>>(lam, vt, n, ld, nc, bT, scale, Y, Kp, g, lmin);
   return cudaGetLastError();
 }
 

@@ -1,5 +1,5 @@
-// Small dense symmetric eigen-problems on the GPU (symeig.cu): parallel cyclic Jacobi, one CTA per
-// matrix, and the Duhamel weights of the parameter gradient.
+// Small symmetric eigen-problems on the GPU (symeig.cu): implicit QL for tridiagonals, parallel cyclic
+// Jacobi for dense matrices, and the Duhamel weights of the parameter gradient.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -9,8 +9,8 @@ namespace ftlm_b200 {
 constexpr int kMaxEig = 160;  // largest order (the matrix sits in shared memory)
 
 // Tridiagonals alpha/beta [nm][ld] of orders n[nm] (0 <= n <= ld <= 160): eigenvalues ascending
-// into lam [nm][ld]; v0 (may be null): squared first components [nm][ld] (quadrature weights);
-// vt (may be null): eigenvectors as rows, [nm][ld][ld].  info [nm] (may be null): 0 converged,
+// into lam [nm][ld], and either vt (eigenvectors as rows, [nm][ld][ld]) or, when vt is null, v0 (squared
+// first components [nm][ld], the quadrature weights).  info [nm] (may be null): 0 converged,
 // 1 not converged after 60 sweeps, 2 order out of range (nothing written).
 cudaError_t symeig_tridiag(const double* alpha, const double* beta, const int* n, int nm, int ld, double* lam,
                            double* v0, double* vt, int* info, cudaStream_t st);

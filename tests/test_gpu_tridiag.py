@@ -54,3 +54,42 @@ def test_jacobi_with_equal_and_zero_entries(gpu):
             T = np.diag(a[i]) + np.diag(b[i, :n - 1], 1) + np.diag(b[i, :n - 1], -1)
             assert np.abs(np.sort(lam[i]) - np.linalg.eigvalsh(T)).max() <= 1e-11
             assert abs(w[i].sum() - 1.0) <= 1e-11
+
+
+@pytest.mark.parametrize("n", [1, *SIZES])
+def test_converged_quadrature_against_eigh(gpu, n):
+    """log sum_k w_k exp(-b lam_k) and its energy from the converged solver: five chains (one past a block of four),
+    one of them shorter, one scaled far from 1, one of a split matrix.  lam is good to a few n eps ||T|| (1e-12 of the
+    norm), so the logarithm to b times that."""
+    rng = np.random.default_rng(n)
+    a, b = 20 + 6 * rng.random((5, n)), 8 + rng.random((5, n))
+    b[3, ::3] = 0.0
+    scale = np.array([1.0, 1.0, 1e-160, 1.0, 1.0])
+    a, b = a * scale[:, None], b * scale[:, None]
+    size = np.array([n, max(1, n - 1), n, n, n])
+    for beta in (0.01, 1.0, 10.0):
+        lq, e = quadrature_exact(a, b, size, beta)
+        for c in range(5):
+            m = size[c]
+            T = np.diag(a[c, :m]) + np.diag(b[c, :m - 1], 1) + np.diag(b[c, :m - 1], -1)
+            lam, z = np.linalg.eigh(T / scale[c])
+            lam *= scale[c]
+            w = z[0] ** 2
+            x = np.log(np.maximum(w, 1e-300)) - beta * lam
+            ref = x.max() + np.log(np.exp(x - x.max()).sum())
+            tol = 1e-12 * (1.0 + beta * np.abs(lam).max())
+            assert abs(lq[c] - ref) <= tol
+            p = np.exp(x - ref)
+            assert abs(e[c] - (p * lam).sum()) <= 1e-11 * np.abs(lam).max()
+
+
+def quadrature_exact(a, b, n, beta):
+    import ctypes as C
+
+    from ftlm_extended_hubbard_b200._lib import call
+    n = np.ascontiguousarray(n, np.int32)
+    bt = np.array([beta])
+    lq, e = np.zeros(len(n)), np.zeros(len(n))
+    call("ftlm_gpu_tridiag_quadrature_exact", *[x.ctypes.data_as(C.c_void_p) for x in (a, b, n)], a.shape[0],
+         a.shape[1], bt.ctypes.data_as(C.c_void_p), 1, lq.ctypes.data_as(C.c_void_p), e.ctypes.data_as(C.c_void_p))
+    return lq, e

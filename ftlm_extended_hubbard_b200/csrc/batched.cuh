@@ -20,27 +20,34 @@ constexpr int kBtActive = 4;  // 1 while the chain has not broken down
 constexpr int kBtFields = 8;
 constexpr int kBtPartialDoubles = kBtBlocks * kBtChains * 2;
 
-// W <- complex64 Philox start vectors (chain r: key seed + r*100003), norms -> scalar state.
-// flags: 2 ints (tiny-entry flags of the current and next vector, cleared here).  gauge: the sector
-// whose spin-ordered basis the block vectors of bt_step live in (the start vector G r, G the
-// diagonal sign matrix of gauge_sign); null for orbit blocks (their own basis).
-cudaError_t bt_start(float2* W, int64_t dim, unsigned seed, double* st, double* partial, int* used, int* flags,
-                     cudaStream_t s, const DevSector* gauge);
-// One Lanczos step k for all chains on block vectors in the sector's gauge basis (bt_start with
-// gauge = &S): Y <- H W_k, z, W_{k+1} (into Y), beta_k; alpha/beta [M][32].  G H G has the same
-// spectrum and the start vectors are G r, so alpha/beta are those of the original basis.
-cudaError_t bt_step(const DevSector& S, const float2* Wk, const float2* Wkm1, float2* Y, int k, double* st,
-                    double* partial, double* alpha, double* beta, int* used, int* flags, cudaStream_t s);
+struct Neu {  // Neumaier-compensated FP64 sum
+  double s = 0.0, c = 0.0;
+  __device__ __forceinline__ void add(double v) {
+    const double t = s + v;
+    c += (fabs(s) >= fabs(v)) ? ((s - t) + v) : ((v - t) + s);
+    s = t;
+  }
+  __device__ __forceinline__ double value() const { return s + c; }
+};
 
-// One Lanczos step for 32 chains of an orbit momentum block (block vectors over its dk
-// representatives); same contract as bt_step.  Needs the sector's max up-degree <= 120 and at most
-// 256 sources per representative.
+// |v|^2 < 1e-28 in FP32 (squares below FLT_MIN flush towards zero, which is still below the bound).
+__device__ __forceinline__ bool tinyf(float2 v) { return fmaf(v.x, v.x, v.y * v.y) < 1e-28f; }
+
+// Totals of nblocks partial sums per chain (partial[(block * 32 + chain) * values]) and the recurrence's scalars for
+// the first `lanes` chains.  mode 0: start norms; 1: dot products, alpha_k; 2: norms, beta_k and breakdown.  scaled:
+// the dot products are of H q_k (complex128 chains) instead of H W_k.  clear (mode 1): set to 0.
+void bt_scalars(const double* partial, int nblocks, int mode, int k, int lanes, bool scaled, double* st, double* alpha,
+                double* beta, int* used, int* clear, cudaStream_t s);
+
+// W <- complex64 Philox start vectors of the block's representatives (chain r: key seed + r*100003), norms -> scalar
+// state.  flags: 2 ints (tiny-entry flags of the current and next vector, cleared here).
+cudaError_t bt_start(float2* W, int64_t dim, unsigned seed, double* st, double* partial, int* used, int* flags,
+                     cudaStream_t s);
+
+// One Lanczos step k of 32 chains of an orbit momentum block (block vectors over its dk representatives, 256 bytes
+// each): Y <- H_K W_k, z, W_{k+1} (into Y), beta_k; alpha/beta [M][32].  Needs the sector's max up-degree <= 120 and at
+// most 256 sources per representative.
 cudaError_t bt_orbit_step(const OrbitApplyDev& A, const float2* Wk, const float2* Wkm1, float2* Y, int k, double* st,
                           double* partial, double* alpha, double* beta, int* used, int* flags, cudaStream_t s);
-
-// Y = (G H G) X for one block vector in the gauge basis, without Lanczos bookkeeping (st_unit is
-// unused), zero_flag points to an int 0 (no small-entry filter), partial receives unused dot sums.
-cudaError_t bt_apply(const DevSector& S, const float2* X, float2* Y, const double* st_unit, double* partial,
-                     const int* zero_flag, cudaStream_t s);
 
 }  // namespace ftlm_b200

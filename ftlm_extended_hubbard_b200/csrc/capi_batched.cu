@@ -1,5 +1,5 @@
-// C ABI of the batched complex64 FTLM (batched.cu): 32 chains per block vector, the M Lanczos steps
-// of a block captured once into a CUDA graph and launched without host synchronisation.
+// C ABI of the batched complex64 FTLM of a sector (planes.cu): blocks of 32 chains in groups of planes, the M Lanczos
+// steps of a block launched without host synchronisation.
 #include <map>
 
 #include "capi_internal.hpp"
@@ -16,13 +16,49 @@ GradWs g_grad;
 
 int bt_run_chains(ftlm_sector* s, int R, int M, unsigned seed, std::vector<double>* A, std::vector<double>* B,
                   std::vector<int>* used) {
-  cudaStream_t st = s->stream;
+  A->assign(static_cast<size_t>(R) * M, 0.0);
+  B->assign(static_cast<size_t>(R) * M, 0.0);
+  used->assign(static_cast<size_t>(R), 0);
+  const int64_t dim = s->plan.dim;
   const DevSector& S = s->dev;
-  return bt_run_chains_impl(
-      s->plan.dim, st,
-      [&S, st](const float2* wk, const float2* wkm1, float2* y, int k, double* sd, double* part, double* al, double* be,
-               int* us, int* fl) { return bt_step(S, wk, wkm1, y, k, sd, part, al, be, us, fl, st); },
-      R, M, seed, A, B, used, &S);
+  cudaStream_t st = s->stream;
+  const int group = pl_group(dim, (std::min(R, kBtChains) + 1) / 2);
+  std::lock_guard<std::mutex> lock(g_bt_mu);
+  CU_TRY(g_bt.ensure(static_cast<size_t>(group) * dim * sizeof(float4), M));
+  const size_t tab = static_cast<size_t>(M) * kBtChains * sizeof(double);
+  std::vector<double> ha(static_cast<size_t>(M) * kBtChains), hb(static_cast<size_t>(M) * kBtChains);
+  std::vector<int> hu(kBtChains);
+  for (int blk = 0; blk * kBtChains < R; ++blk) {
+    const int nc = std::min(kBtChains, R - blk * kBtChains), planes = (nc + 1) / 2;
+    CU_TRY(cudaMemsetAsync(g_bt.alpha.p, 0, tab, st));
+    CU_TRY(cudaMemsetAsync(g_bt.beta.p, 0, tab, st));
+    for (int p0 = 0; p0 < planes; p0 += group) {
+      const int np = std::min(group, planes - p0);
+      const PlaneState z = g_bt.state(2 * p0);
+      float4 *wk = g_bt.buf[0].as<float4>(), *y = g_bt.buf[1].as<float4>(), *wkm1 = g_bt.buf[2].as<float4>();
+      CU_TRY(pl_start(S, wk, np, seed + static_cast<unsigned>(blk * kBtChains + 2 * p0) * 100003u, z, st));
+      for (int k = 0; k < M; ++k) {
+        CU_TRY(pl_step(S, wk, wkm1, y, np, k, z, st));
+        float4* t = wkm1;
+        wkm1 = wk;
+        wk = y;
+        y = t;
+      }
+    }
+    CU_TRY(cudaMemcpyAsync(ha.data(), g_bt.alpha.p, tab, cudaMemcpyDeviceToHost, st));
+    CU_TRY(cudaMemcpyAsync(hb.data(), g_bt.beta.p, tab, cudaMemcpyDeviceToHost, st));
+    CU_TRY(cudaMemcpyAsync(hu.data(), g_bt.used.p, hu.size() * sizeof(int), cudaMemcpyDeviceToHost, st));
+    CU_TRY(cudaStreamSynchronize(st));
+    for (int r = 0; r < nc; ++r) {
+      const size_t ch = static_cast<size_t>(blk * kBtChains + r);
+      (*used)[ch] = hu[static_cast<size_t>(r)];
+      for (int k = 0; k < M; ++k) {
+        (*A)[ch * M + k] = ha[static_cast<size_t>(k) * kBtChains + r];
+        (*B)[ch * M + k] = hb[static_cast<size_t>(k) * kBtChains + r];
+      }
+    }
+  }
+  return FTLM_OK;
 }
 
 }  // namespace capi
@@ -63,12 +99,12 @@ int ftlm_gpu_batched_autotune(ftlm_sector* s, int reps, int* variant, float* ms)
   float best = 3.4e38f;
   {
     std::lock_guard<std::mutex> lock(g_bt_mu);
-    CU_TRY(g_bt.ensure(P.dim, 1));
-    float2* W = g_bt.buf[0].as<float2>();
-    float2* Y = g_bt.buf[1].as<float2>();
+    const int planes = pl_group(P.dim, kBtChains / 2);
+    CU_TRY(g_bt.ensure(static_cast<size_t>(planes) * P.dim * sizeof(float4), 1));
+    float4* W = g_bt.buf[0].as<float4>();
+    float4* Y = g_bt.buf[1].as<float4>();
     int* fl = g_bt.flags.as<int>();
-    CU_TRY(bt_start(W, P.dim, 7u, g_bt.st.as<double>(), g_bt.partial.as<double>(), g_bt.used.as<int>(), fl, st,
-                    &s->dev));
+    CU_TRY(pl_start(s->dev, W, planes, 7u, g_bt.state(0), st));
     CU_TRY(cudaMemsetAsync(fl, 0, sizeof(int), st));
     cudaEvent_t e0, e1;
     CU_TRY(cudaEventCreate(&e0));
@@ -77,9 +113,9 @@ int ftlm_gpu_batched_autotune(ftlm_sector* s, int reps, int* variant, float* ms)
     for (int v = 0; v < 3 && ce == cudaSuccess; ++v) {
       DevSector d = s->dev;
       d.bt_cols = v;
-      ce = bt_apply(d, W, Y, nullptr, g_bt.partial.as<double>(), fl, st);  // warm-up
+      ce = pl_apply(d, W, Y, planes, fl, st);  // warm-up
       if (ce == cudaSuccess) ce = cudaEventRecord(e0, st);
-      for (int r = 0; r < reps && ce == cudaSuccess; ++r) ce = bt_apply(d, W, Y, nullptr, g_bt.partial.as<double>(), fl, st);
+      for (int r = 0; r < reps && ce == cudaSuccess; ++r) ce = pl_apply(d, W, Y, planes, fl, st);
       if (ce == cudaSuccess) ce = cudaEventRecord(e1, st);
       if (ce == cudaSuccess) ce = cudaEventSynchronize(e1);
       float t = 0.0f;

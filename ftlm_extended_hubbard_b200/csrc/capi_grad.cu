@@ -71,20 +71,16 @@ int fill_weights(ftlm_sector* s, int nc, int ld, double bT, const std::vector<in
   return FTLM_OK;
 }
 
-// Moments of one batch of chains: Q [n][vstride], AQ likewise (or null), weights already in
-// g_grad.Kp [n][ld][nc] (fill_weights).
+// Moments of one batch of nc chains: Q [n][planes][dim] with strides vstride and pstride, AQ likewise (or null),
+// weights already in g_grad.Kp [n][ld][nc] (fill_weights).
 template <class T>
-int run_moments(ftlm_sector* s, const T* Q, const T* AQ, int64_t vstride, int n, int ld, int nc,
-                std::vector<ChainGrad>* out) {
+int run_moments(ftlm_sector* s, const T* Q, const T* AQ, int64_t vstride, int64_t pstride, int planes, int n, int ld,
+                int nc, std::vector<ChainGrad>* out) {
   cudaStream_t st = s->stream;
-  CU_TRY(g_grad.grow(g_grad.part, g_grad.pcap, static_cast<size_t>(2048) * 32 * 3 * sizeof(double)));
+  CU_TRY(g_grad.grow(g_grad.part, g_grad.pcap, static_cast<size_t>(kGradMaxBlocks) * nc * 3 * sizeof(double)));
   int grid = 0;
-  cudaError_t e;
-  if constexpr (sizeof(T) == sizeof(float2))
-    e = grad_moments_c64(s->dev, Q, AQ ? AQ : Q, vstride, g_grad.Kp.as<double>(), n, ld, g_grad.part.as<double>(), &grid, st);
-  else
-    e = grad_moments_c128(s->dev, Q, AQ ? AQ : Q, vstride, g_grad.Kp.as<double>(), n, ld, g_grad.part.as<double>(), &grid,
-                          st);
+  const cudaError_t e = grad_moments(s->dev, Q, AQ ? AQ : Q, vstride, pstride, planes, g_grad.Kp.as<double>(), n, ld, nc,
+                                     g_grad.part.as<double>(), &grid, st);
   if (e == cudaErrorInvalidValue)
     return fail(FTLM_ERR_UNSUPPORTED, "gradient: Lanczos vectors of one block do not fit in shared memory");
   CU_TRY(e);
@@ -131,7 +127,7 @@ int grad_plain(ftlm_sector* s, ftlm_sector* op, double bT, int R, int M, unsigne
     std::vector<std::vector<double>> scale(1, std::vector<double>(static_cast<size_t>(n), 1.0));
     rc = fill_weights(s, 1, M, bT, std::vector<int>{n}, A, B, scale, &one);
     if (rc) return rc;
-    rc = run_moments<double2>(s, Q, AQ, dim, n, M, 1, &one);
+    rc = run_moments<double2>(s, Q, AQ, dim, dim, 1, n, M, 1, &one);
     if (rc) return rc;
     (*out)[static_cast<size_t>(r)] = one[0];
   }
@@ -141,52 +137,53 @@ int grad_plain(ftlm_sector* s, ftlm_sector* op, double bT, int R, int M, unsigne
 // Batched path: complex64 32-chain blocks of ftlm_gpu_batched_ftlm_sector, replayed step by step.
 int grad_batched(ftlm_sector* s, ftlm_sector* op, double bT, int R, int M, unsigned seed, std::vector<ChainGrad>* out) {
   const int64_t dim = s->plan.dim;
-  const int64_t vs = dim * kBtChains;
+  const int max_planes = (std::min(R, kBtChains) + 1) / 2, group = pl_group(dim, max_planes);
+  const int64_t vs = dim * max_planes;  // elements of two chains per stored vector
   std::lock_guard<std::mutex> lock(g_bt_mu);
-  CU_TRY(g_bt.ensure(dim, M));
-  CU_TRY(g_grad.grow(g_grad.Q, g_grad.qcap, static_cast<size_t>(M + 1) * vs * sizeof(float2)));
-  if (op) CU_TRY(g_grad.grow(g_grad.AQ, g_grad.acap, static_cast<size_t>(M) * vs * sizeof(float2)));
-  if (!g_grad.stunit.p) {
-    std::vector<double> unit(static_cast<size_t>(kBtFields) * kBtChains, 0.0);
-    for (int c = 0; c < kBtChains; ++c) unit[static_cast<size_t>(kBtSin) * kBtChains + c] = 1.0;
-    CU_TRY(g_grad.stunit.alloc(unit.size() * sizeof(double)));
-    CU_TRY(cudaMemcpy(g_grad.stunit.p, unit.data(), unit.size() * sizeof(double), cudaMemcpyHostToDevice));
+  CU_TRY(g_bt.ensure(0, M));
+  CU_TRY(g_grad.grow(g_grad.Q, g_grad.qcap, static_cast<size_t>(M + 1) * vs * sizeof(float4)));
+  if (op) CU_TRY(g_grad.grow(g_grad.AQ, g_grad.acap, static_cast<size_t>(M) * vs * sizeof(float4)));
+  if (!g_grad.zflag.p) {
     CU_TRY(g_grad.zflag.alloc(sizeof(int)));
     CU_TRY(cudaMemset(g_grad.zflag.p, 0, sizeof(int)));
   }
   cudaStream_t st = s->stream;
-  float2* Q = g_grad.Q.as<float2>();
-  float2* AQ = op ? g_grad.AQ.as<float2>() : nullptr;
+  float4* Q = g_grad.Q.as<float4>();
+  float4* AQ = op ? g_grad.AQ.as<float4>() : nullptr;
   double* sd = g_bt.st.as<double>();
-  double* part = g_bt.partial.as<double>();
   double* al = g_bt.alpha.as<double>();
   double* be = g_bt.beta.as<double>();
   int* us = g_bt.used.as<int>();
-  int* fl = g_bt.flags.as<int>();
   out->assign(static_cast<size_t>(R), ChainGrad{});
   std::vector<double> ha(static_cast<size_t>(M) * kBtChains), hb(static_cast<size_t>(M) * kBtChains),
-      hs(static_cast<size_t>(kBtFields) * kBtChains);
+      hs(kBtChains);  // 1 / ||raw start||
   std::vector<int> hu(kBtChains);
   for (int blk = 0; blk * kBtChains < R; ++blk) {
     const unsigned seed_b = seed + static_cast<unsigned>(blk * kBtChains) * 100003u;
     CU_TRY(cudaMemsetAsync(al, 0, static_cast<size_t>(M) * kBtChains * sizeof(double), st));
     CU_TRY(cudaMemsetAsync(be, 0, static_cast<size_t>(M) * kBtChains * sizeof(double), st));
-    CU_TRY(bt_start(Q, dim, seed_b, sd, part, us, fl, st, &s->dev));
-    CU_TRY(cudaMemcpyAsync(hs.data(), sd, hs.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
-    for (int k = 0; k < M; ++k)
-      CU_TRY(bt_step(s->dev, Q + static_cast<int64_t>(k) * vs, Q + static_cast<int64_t>(k > 0 ? k - 1 : 0) * vs,
-                     Q + static_cast<int64_t>(k + 1) * vs, k, sd, part, al, be, us, fl, st));
+    const int nc = std::min(kBtChains, R - blk * kBtChains), planes = (nc + 1) / 2;
+    // the forward's groups and kernels; W_0's scale (st) is read before the steps overwrite it
+    for (int p0 = 0; p0 < planes; p0 += group) {
+      const int np = std::min(group, planes - p0);
+      const PlaneState z = g_bt.state(2 * p0);
+      float4* Qp = Q + p0 * dim;
+      CU_TRY(pl_start(s->dev, Qp, np, seed_b + static_cast<unsigned>(2 * p0) * 100003u, z, st));
+      CU_TRY(cudaMemcpyAsync(hs.data() + 2 * p0, sd + kBtSin * kBtChains + 2 * p0, 2 * np * sizeof(double),
+                             cudaMemcpyDeviceToHost, st));
+      for (int k = 0; k < M; ++k)
+        CU_TRY(pl_step(s->dev, Qp + k * vs, Qp + (k > 0 ? k - 1 : 0) * vs, Qp + (k + 1) * vs, np, k, z, st));
+    }
     CU_TRY(cudaMemcpyAsync(ha.data(), al, ha.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
     CU_TRY(cudaMemcpyAsync(hb.data(), be, hb.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
     CU_TRY(cudaMemcpyAsync(hu.data(), us, hu.size() * sizeof(int), cudaMemcpyDeviceToHost, st));
     CU_TRY(cudaStreamSynchronize(st));
-    const int nc = std::min(kBtChains, R - blk * kBtChains);
     std::vector<int> n(static_cast<size_t>(kBtChains), 0);
     std::vector<double> A(static_cast<size_t>(kBtChains) * M, 0.0), B(static_cast<size_t>(kBtChains) * M, 0.0);
     std::vector<std::vector<double>> scale(static_cast<size_t>(kBtChains));
     int nmax = 0;
     for (int c = 0; c < nc; ++c) {
-      const double sin0 = hs[static_cast<size_t>(kBtSin) * kBtChains + c];
+      const double sin0 = hs[static_cast<size_t>(c)];
       const int nn = (sin0 > 0.0) ? hu[static_cast<size_t>(c)] : 0;
       n[static_cast<size_t>(c)] = nn;
       nmax = std::max(nmax, nn);
@@ -202,14 +199,18 @@ int grad_batched(ftlm_sector* s, ftlm_sector* op, double bT, int R, int M, unsig
       }
     }
     if (nmax == 0) continue;
-    if (op)
-      for (int i = 0; i < nmax; ++i)
-        CU_TRY(bt_apply(op->dev, Q + static_cast<int64_t>(i) * vs, AQ + static_cast<int64_t>(i) * vs,
-                        g_grad.stunit.as<double>(), part, g_grad.zflag.as<int>(), st));
+    if (op) {  // the operator on every stored vector: planes are contiguous over the vectors of a full store
+      if (planes == max_planes) {
+        CU_TRY(pl_apply(op->dev, Q, AQ, nmax * planes, g_grad.zflag.as<int>(), st));
+      } else {
+        for (int i = 0; i < nmax; ++i)
+          CU_TRY(pl_apply(op->dev, Q + i * vs, AQ + i * vs, planes, g_grad.zflag.as<int>(), st));
+      }
+    }
     std::vector<ChainGrad> cg(static_cast<size_t>(kBtChains));
     int rc = fill_weights(s, kBtChains, M, bT, n, A, B, scale, &cg);
     if (rc) return rc;
-    rc = run_moments<float2>(s, Q, AQ, vs, nmax, M, kBtChains, &cg);
+    rc = run_moments<float4>(s, Q, AQ, vs, dim, planes, nmax, M, kBtChains, &cg);
     if (rc) return rc;
     for (int c = 0; c < nc; ++c) (*out)[static_cast<size_t>(blk * kBtChains + c)] = cg[static_cast<size_t>(c)];
   }

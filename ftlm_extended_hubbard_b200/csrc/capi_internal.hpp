@@ -20,6 +20,7 @@
 #include "grad.cuh"
 #include "hv.cuh"
 #include "orbit.cuh"
+#include "planes.cuh"
 #include "plan.hpp"
 #include "symeig.cuh"
 #include "tridiag.hpp"
@@ -209,20 +210,21 @@ int need_device(const ftlm_sector* s);
 
 // ---- batched complex64 path (capi_batched.cu) ------------------------------------------------
 struct BtWs {
-  int64_t cap = 0;
+  size_t cap = 0;
   int mcap = 0;
   DevBuf buf[3], st, partial, alpha, beta, used, flags;
-  cudaError_t ensure(int64_t dim, int M) {
+  // three vectors of `bytes` each and the scalars of 32 chains of M steps
+  cudaError_t ensure(size_t bytes, int M) {
     cudaError_t e = cudaSuccess;
-    if (dim > cap) {
-      for (auto& b : buf) b.alloc(0);  // release before growing
+    if (bytes > cap) {
+      release();
       for (auto& b : buf)
-        if ((e = b.alloc(static_cast<size_t>(dim) * kBtChains * sizeof(float2))) != cudaSuccess) return e;
-      cap = dim;
+        if ((e = b.alloc(bytes)) != cudaSuccess) return e;
+      cap = bytes;
     }
     if (!st.p) {
       if ((e = st.alloc(kBtFields * kBtChains * sizeof(double))) != cudaSuccess) return e;
-      if ((e = partial.alloc(kBtPartialDoubles * sizeof(double))) != cudaSuccess) return e;
+      if ((e = partial.alloc(std::max<int64_t>(kBtPartialDoubles, kPlPartialDoubles) * sizeof(double))) != cudaSuccess) return e;
       if ((e = used.alloc(kBtChains * sizeof(int))) != cudaSuccess) return e;
       if ((e = flags.alloc(2 * sizeof(int))) != cudaSuccess) return e;
     }
@@ -233,8 +235,13 @@ struct BtWs {
     }
     return e;
   }
+  // the scalar state of a group whose first chain is c0 of the block
+  PlaneState state(int c0) const {
+    return PlaneState{st.as<double>() + c0,    partial.as<double>(), alpha.as<double>() + c0,
+                      beta.as<double>() + c0,  used.as<int>() + c0,  flags.as<int>()};
+  }
   void release() {
-    for (auto& b : buf) b.alloc(0);
+    for (auto& b : buf) b.alloc(0);  // release before growing
     cap = 0;
   }
 };
@@ -244,7 +251,7 @@ extern std::mutex g_bt_mu;
 
 // Krylov vector store of the gradient replay (grows to the largest sector seen).
 struct GradWs {
-  DevBuf Q, AQ, Kp, part, stunit, zflag;
+  DevBuf Q, AQ, Kp, part, zflag;
   size_t qcap = 0, acap = 0, kcap = 0, pcap = 0;
   cudaError_t grow(DevBuf& b, size_t& cap, size_t bytes) {
     if (bytes <= cap && b.p) return cudaSuccess;
@@ -260,15 +267,16 @@ struct GradWs {
 extern GradWs g_grad;
 
 
-// Runs ceil(R/32) blocks of 32 chains on sector s; A/B [R][M] (beta zero-padded), used [R].
+// Runs ceil(R/32) blocks of 32 chains of a momentum block of dim states, the M steps of a block as one graph; A/B
+// [R][M] (beta zero-padded), used [R].
 template <class Step>
 int bt_run_chains_impl(int64_t dim, cudaStream_t st, Step&& step, int R, int M, unsigned seed, std::vector<double>* A,
-                       std::vector<double>* B, std::vector<int>* used, const DevSector* gauge) {
+                       std::vector<double>* B, std::vector<int>* used) {
   A->assign(static_cast<size_t>(R) * M, 0.0);
   B->assign(static_cast<size_t>(R) * M, 0.0);
   used->assign(static_cast<size_t>(R), 0);
   std::lock_guard<std::mutex> lock(g_bt_mu);
-  CU_TRY(g_bt.ensure(dim, M));
+  CU_TRY(g_bt.ensure(static_cast<size_t>(dim) * kBtChains * sizeof(float2), M));
   float2* bufs[3] = {g_bt.buf[0].as<float2>(), g_bt.buf[1].as<float2>(), g_bt.buf[2].as<float2>()};
   double* sd = g_bt.st.as<double>();
   double* part = g_bt.partial.as<double>();
@@ -282,7 +290,7 @@ int bt_run_chains_impl(int64_t dim, cudaStream_t st, Step&& step, int R, int M, 
     const unsigned seed_b = seed + static_cast<unsigned>(blk * kBtChains) * 100003u;
     CU_TRY(cudaMemsetAsync(al, 0, static_cast<size_t>(M) * kBtChains * sizeof(double), st));
     CU_TRY(cudaMemsetAsync(be, 0, static_cast<size_t>(M) * kBtChains * sizeof(double), st));
-    CU_TRY(bt_start(bufs[0], dim, seed_b, sd, part, us, fl, st, gauge));
+    CU_TRY(bt_start(bufs[0], dim, seed_b, sd, part, us, fl, st));
     cudaGraph_t graph = nullptr;
     CU_TRY(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
     float2 *wk = bufs[0], *y = bufs[1], *wkm1 = bufs[2];
@@ -341,7 +349,7 @@ int fused_sectors_ftlm(const std::vector<ftlm_sector*>& secs, const std::vector<
                        unsigned seed, int start_mode, const double* bts, int n_bt, double* lnz_s, double* e_s,
                        bool converged);
 
-// 32-chain blocks of one sector (bt_step), alpha/beta [R][M], steps used [R].
+// The complex64 chains of one sector in groups of planes (planes.cu), alpha/beta [R][M] (beta zero-padded), used [R].
 int bt_run_chains(ftlm_sector* s, int R, int M, unsigned seed, std::vector<double>* A, std::vector<double>* B,
                   std::vector<int>* used);
 

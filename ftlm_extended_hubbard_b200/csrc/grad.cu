@@ -1,11 +1,12 @@
 // Krylov moments for the FTLM parameter gradient; contract in grad.cuh.
 //
-// Block = E consecutive elements (state, chain) of the flattened [state][NC] vectors.  The block
-// stages its slice of every W_l in shared memory (each thread only reads its own element's
-// column, conflict-free), then for rows i in pairs stages K'[i][*][*] and forms
+// Block = kE consecutive states of one plane (of the planes' one or two chains).  A thread keeps its own state's
+// entry of every W_l in shared memory (only it reads them: conflict-free, no barrier), then for rows i, kIB at a time,
+// the block stages K'[i][*] of the plane's chains and forms
 //   X_i = sum_l K'_il W_l   (FP64),
-// accumulating Re(conj W_i X_i) (times the diagonal operators) and Re(conj(A W_i) X_i).  Fixed
-// grid and fixed per-block order: the sums are bitwise repeatable.
+// accumulating Re(conj W_i X_i) (times the diagonal operators) and Re(conj(A W_i) X_i).  Bound by the FP64 rate for
+// long chains (4 n^2 operations per chain and state); kIB rows share each conversion of W_l to FP64 and each load.
+// Fixed grid and fixed per-block order: the sums are bitwise repeatable.
 #include <algorithm>
 
 #include "grad.cuh"
@@ -14,133 +15,161 @@ namespace ftlm_b200 {
 
 namespace {
 
-constexpr int kIB = 2;  // rows of K' staged per pass
+constexpr int kIB = 4;  // rows of K' staged per pass
 
-__device__ __forceinline__ double2 ld_c(const float2* p, int64_t i) {
-  const float2 v = p[i];
-  return make_double2(v.x, v.y);
-}
-__device__ __forceinline__ double2 ld_c(const double2* p, int64_t i) { return p[i]; }
+template <typename T>
+struct Elem;
+template <>
+struct Elem<float4> {  // two complex64 chains
+  static constexpr int kC = 2;
+  static __device__ __forceinline__ void get(const float4& v, double (&re)[2], double (&im)[2]) {
+    re[0] = v.x;
+    im[0] = v.y;
+    re[1] = v.z;
+    im[1] = v.w;
+  }
+};
+template <>
+struct Elem<double2> {  // one complex128 chain
+  static constexpr int kC = 1;
+  static __device__ __forceinline__ void get(const double2& v, double (&re)[1], double (&im)[1]) {
+    re[0] = v.x;
+    im[0] = v.y;
+  }
+};
 
-template <typename T, int NC>
+template <typename T>
 __global__ void __launch_bounds__(256) moments_kernel(DevSector S, const T* __restrict__ W, const T* __restrict__ AW,
-                                                      int64_t vstride, const double* __restrict__ Kp, int n, int ld,
-                                                      double* __restrict__ partial) {
+                                                      int64_t vstride, int64_t pstride, const double* __restrict__ Kp,
+                                                      int n, int ld, int nc, int nb, double* __restrict__ partial) {
+  constexpr int kC = Elem<T>::kC;
   extern __shared__ __align__(16) unsigned char smraw[];
   const int E = blockDim.x;
   T* Ws = reinterpret_cast<T*>(smraw);                                                    // [n][E]
-  double* Ks = reinterpret_cast<double*>(smraw + static_cast<size_t>(n) * E * sizeof(T));  // [kIB][n][NC]
+  double* Ks = reinterpret_cast<double*>(smraw + static_cast<size_t>(n) * E * sizeof(T));  // [n][kIB][kC]
   const int t = threadIdx.x;
-  const int c = t % NC;  // E and every block start are multiples of NC
-  const int64_t nch = (vstride + E - 1) / E;
-  double accD = 0.0, accP = 0.0, accA = 0.0;
-  for (int64_t ch = blockIdx.x; ch < nch; ch += gridDim.x) {
+  const int plane = blockIdx.x / nb, b = blockIdx.x - plane * nb;
+  const T* Wp = W + plane * pstride;
+  const T* Ap = AW + plane * pstride;
+  const double* Kc = Kp + plane * kC;
+  double accD[kC] = {}, accP[kC] = {}, accA[kC] = {};
+  const int64_t nch = (S.dim + E - 1) / E;
+  for (int64_t ch = b; ch < nch; ch += nb) {
     const int64_t e = ch * E + t;
-    const bool valid = e < vstride;
-    __syncthreads();
-    for (int l = 0; l < n; ++l) {
-      T v{};
-      if (valid) v = W[static_cast<int64_t>(l) * vstride + e];
-      Ws[l * E + t] = v;
-    }
+    const bool valid = e < S.dim;
     double aD = 0.0, aP = 0.0;
     if (valid) {
-      const int64_t s = e / NC;
-      const int64_t ru = s / S.Dd, rd = s - ru * S.Dd;
+      for (int l = 0; l < n; ++l) Ws[l * E + t] = Wp[static_cast<int64_t>(l) * vstride + e];
+      const int64_t ru = e / S.Dd, rd = e - ru * S.Dd;
       const uint32_t u = S.umask[ru], d = S.dmask[rd];
       const uint4 w = S.wpl[ru];
       aD = static_cast<double>(__popc(u & d));
       aP = static_cast<double>(S.cnt_uu[ru] + S.cnt_dd[rd] + __popc(d & w.x) + 2 * __popc(d & w.y) +
                                4 * __popc(d & w.z) + 8 * __popc(d & w.w));
     }
-    double sW = 0.0, sA = 0.0;
+    double sW[kC] = {}, sA[kC] = {};
     for (int i0 = 0; i0 < n; i0 += kIB) {
       __syncthreads();
-      for (int idx = t; idx < kIB * n * NC; idx += E) {
-        const int ib = idx / (n * NC), rem = idx - ib * (n * NC);
-        const int i = i0 + ib;
-        Ks[idx] = (i < n) ? Kp[(static_cast<int64_t>(i) * ld) * NC + rem] : 0.0;
+      for (int idx = t; idx < kIB * n * kC; idx += E) {
+        const int q = idx % kC, ib = idx / kC % kIB, l = idx / (kC * kIB);
+        Ks[idx] = (i0 + ib < n) ? Kc[(static_cast<int64_t>(i0 + ib) * ld + l) * nc + q] : 0.0;
       }
       __syncthreads();
       if (!valid) continue;
-      double xr[kIB], xi[kIB];
-#pragma unroll
-      for (int ib = 0; ib < kIB; ++ib) xr[ib] = xi[ib] = 0.0;
+      double xr[kIB][kC] = {}, xi[kIB][kC] = {};
       for (int l = 0; l < n; ++l) {
-        const double2 wl = ld_c(Ws, l * E + t);
+        double re[kC], im[kC];
+        Elem<T>::get(Ws[l * E + t], re, im);
 #pragma unroll
         for (int ib = 0; ib < kIB; ++ib) {
-          const double k = Ks[(ib * n + l) * NC + c];
-          xr[ib] = fma(k, wl.x, xr[ib]);
-          xi[ib] = fma(k, wl.y, xi[ib]);
+#pragma unroll
+          for (int q = 0; q < kC; ++q) {
+            const double k = Ks[(l * kIB + ib) * kC + q];
+            xr[ib][q] = fma(k, re[q], xr[ib][q]);
+            xi[ib][q] = fma(k, im[q], xi[ib][q]);
+          }
         }
       }
 #pragma unroll
       for (int ib = 0; ib < kIB; ++ib) {
         const int i = i0 + ib;
         if (i >= n) break;
-        const double2 wi = ld_c(Ws, i * E + t);
-        sW = fma(wi.x, xr[ib], fma(wi.y, xi[ib], sW));
-        const double2 ai = ld_c(AW, static_cast<int64_t>(i) * vstride + e);
-        sA = fma(ai.x, xr[ib], fma(ai.y, xi[ib], sA));
+        double re[kC], im[kC];
+        Elem<T>::get(Ws[i * E + t], re, im);
+#pragma unroll
+        for (int q = 0; q < kC; ++q) sW[q] = fma(re[q], xr[ib][q], fma(im[q], xi[ib][q], sW[q]));
+        Elem<T>::get(Ap[static_cast<int64_t>(i) * vstride + e], re, im);
+#pragma unroll
+        for (int q = 0; q < kC; ++q) sA[q] = fma(re[q], xr[ib][q], fma(im[q], xi[ib][q], sA[q]));
       }
     }
-    accD = fma(aD, sW, accD);
-    accP = fma(aP, sW, accP);
-    accA += sA;
-  }
-  // per-chain block sums (threads t, t + NC, ... hold chain c)
-  __syncthreads();
-  double* red = reinterpret_cast<double*>(smraw);
-  red[t] = accD;
-  red[E + t] = accP;
-  red[2 * E + t] = accA;
-  __syncthreads();
-  if (t < NC) {
-    for (int q = 0; q < 3; ++q) {
-      double sum = 0.0;
-      for (int j = t; j < E; j += NC) sum += red[q * E + j];
-      partial[(static_cast<int64_t>(blockIdx.x) * NC + t) * 3 + q] = sum;
+#pragma unroll
+    for (int q = 0; q < kC; ++q) {
+      accD[q] = fma(aD, sW[q], accD[q]);
+      accP[q] = fma(aP, sW[q], accP[q]);
+      accA[q] += sA[q];
     }
+  }
+  // block sums per chain
+  __syncthreads();
+  double* red = reinterpret_cast<double*>(smraw);  // [3 * kC][E]
+#pragma unroll
+  for (int q = 0; q < kC; ++q) {
+    red[(3 * q) * E + t] = accD[q];
+    red[(3 * q + 1) * E + t] = accP[q];
+    red[(3 * q + 2) * E + t] = accA[q];
+  }
+  __syncthreads();
+  const int warp = t >> 5, lane = t & 31;
+  for (int v = warp; v < 3 * kC; v += E >> 5) {
+    double sum = 0.0;
+    for (int j = lane; j < E; j += 32) sum += red[v * E + j];
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_down_sync(0xffffffffu, sum, o);
+    if (lane == 0) partial[(static_cast<int64_t>(b) * nc + plane * kC + v / 3) * 3 + v % 3] = sum;
   }
 }
 
-template <typename T, int NC, int kE>
-cudaError_t launch(const DevSector& S, const T* W, const T* AW, int64_t vstride, const double* Kp, int n, int ld,
-                   double* partial, int* grid, cudaStream_t st) {
+template <typename T>
+cudaError_t launch(const DevSector& S, const T* W, const T* AW, int64_t vstride, int64_t pstride, int planes,
+                   const double* Kp, int n, int ld, int nc, double* partial, int* blocks, cudaStream_t st) {
+  constexpr int kC = Elem<T>::kC;
   int dev = 0, sms = 0, optin = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-  const size_t smem = std::max(static_cast<size_t>(n) * kE * sizeof(T) + static_cast<size_t>(kIB) * n * NC * sizeof(double),
-                               static_cast<size_t>(3) * kE * sizeof(double));
+  // widest block whose slice of the n vectors fits in shared memory, not wider than the sector
+  int E = 256;
+  auto bytes = [&](int e) {
+    return std::max(static_cast<size_t>(n) * e * sizeof(T) + static_cast<size_t>(kIB) * n * kC * sizeof(double),
+                    static_cast<size_t>(3 * kC) * e * sizeof(double));
+  };
+  while (E > 32 && (bytes(E) > static_cast<size_t>(optin) || E / 2 >= S.dim)) E /= 2;
+  const size_t smem = bytes(E);
   if (n <= 0 || smem > static_cast<size_t>(optin)) return cudaErrorInvalidValue;
-  cudaError_t e = cudaFuncSetAttribute(moments_kernel<T, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  cudaError_t e = cudaFuncSetAttribute(moments_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        static_cast<int>(smem));
   if (e != cudaSuccess) return e;
-  const int64_t nch = (vstride + kE - 1) / kE;
-  const int per_sm = std::max(1, static_cast<int>(static_cast<size_t>(optin) / smem));
-  const int64_t cap = static_cast<int64_t>(sms) * std::min(per_sm, 2);
-  *grid = static_cast<int>(nch < cap ? (nch > 0 ? nch : 1) : cap);
-  moments_kernel<T, NC><<<*grid, kE, smem, st>>>(S, W, AW, vstride, Kp, n, ld, partial);
+  const int64_t nch = (S.dim + E - 1) / E;
+  const int per_sm = std::max(1, std::min(static_cast<int>(static_cast<size_t>(optin) / smem), 2048 / E));
+  const int64_t cap = std::max<int64_t>(1, (static_cast<int64_t>(sms) * per_sm + planes - 1) / planes);
+  const int nb = static_cast<int>(std::min<int64_t>({nch, cap, kGradMaxBlocks}));
+  *blocks = nb;
+  moments_kernel<T><<<nb * planes, E, smem, st>>>(S, W, AW, vstride, pstride, Kp, n, ld, nc, nb, partial);
   return cudaGetLastError();
 }
 
 }  // namespace
 
-// Widest block whose slice of the n vectors fits in shared memory.
-cudaError_t grad_moments_c64(const DevSector& S, const float2* W, const float2* AW, int64_t vstride, const double* Kp,
-                             int n, int ld, double* partial, int* grid, cudaStream_t st) {
-  cudaError_t e = launch<float2, 32, 256>(S, W, AW, vstride, Kp, n, ld, partial, grid, st);
-  if (e == cudaErrorInvalidValue) e = launch<float2, 32, 128>(S, W, AW, vstride, Kp, n, ld, partial, grid, st);
-  return e;
+cudaError_t grad_moments(const DevSector& S, const float4* W, const float4* AW, int64_t vstride, int64_t pstride,
+                         int planes, const double* Kp, int n, int ld, int nc, double* partial, int* blocks,
+                         cudaStream_t st) {
+  return launch(S, W, AW, vstride, pstride, planes, Kp, n, ld, nc, partial, blocks, st);
 }
 
-cudaError_t grad_moments_c128(const DevSector& S, const double2* W, const double2* AW, int64_t vstride,
-                              const double* Kp, int n, int ld, double* partial, int* grid, cudaStream_t st) {
-  cudaError_t e = launch<double2, 1, 128>(S, W, AW, vstride, Kp, n, ld, partial, grid, st);
-  if (e == cudaErrorInvalidValue) e = launch<double2, 1, 64>(S, W, AW, vstride, Kp, n, ld, partial, grid, st);
-  return e;
+cudaError_t grad_moments(const DevSector& S, const double2* W, const double2* AW, int64_t vstride, int64_t pstride,
+                         int planes, const double* Kp, int n, int ld, int nc, double* partial, int* blocks,
+                         cudaStream_t st) {
+  return launch(S, W, AW, vstride, pstride, planes, Kp, n, ld, nc, partial, blocks, st);
 }
 
 }  // namespace ftlm_b200

@@ -5,8 +5,9 @@
 //   m0 = sum_il K'_il <W_i| D |W_l>,  m1 = sum_il K'_il <W_i| P |W_l>,  m2 = sum_il K'_il <A W_i|W_l>
 // with D = number of doubly occupied sites, P = sum over neighbour pairs of n_i n_j (both
 // diagonal, evaluated from the sector tables) and A W_i supplied by the caller (the t' hopping
-// operator applied to each W_i).  Vectors are [state][NC chains]: NC = 32 complex64 (block
-// vectors of the batched path) or NC = 1 complex128 (one chain of the plain path).
+// operator applied to each W_i).  Vectors are planes over the sector's states: two complex64 chains
+// (the batched path) or one complex128 chain (the plain path) per element; plane p of vector i starts
+// at W + i * vstride + p * pstride.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -15,13 +16,16 @@
 
 namespace ftlm_b200 {
 
-// Kp: [n][ld][NC] (row i, column l, chain fastest).  partial: [grid][NC][3] doubles, grid returned
-// in *grid (at most 2 * SM count blocks).  smem needs n * E * sizeof(element) + 2 * n * NC * 8
-// bytes with E = 256 (NC = 32) or 128 (NC = 1) elements per block; fails with
-// cudaErrorInvalidValue when that exceeds the device's limit.
-cudaError_t grad_moments_c64(const DevSector& S, const float2* W, const float2* AW, int64_t vstride, const double* Kp,
-                             int n, int ld, double* partial, int* grid, cudaStream_t st);
-cudaError_t grad_moments_c128(const DevSector& S, const double2* W, const double2* AW, int64_t vstride,
-                              const double* Kp, int n, int ld, double* partial, int* grid, cudaStream_t st);
+constexpr int64_t kGradMaxBlocks = 2048;
+
+// Kp: [n][ld][nc] (row i, column l, chain fastest), nc = the planes' chains.  partial: [blocks][nc][3] doubles, blocks
+// (<= kGradMaxBlocks) returned in *blocks.  Shared memory: the n vectors' entries of a block of 32 to 256 states;
+// cudaErrorInvalidValue when that does not fit.
+cudaError_t grad_moments(const DevSector& S, const float4* W, const float4* AW, int64_t vstride, int64_t pstride,
+                         int planes, const double* Kp, int n, int ld, int nc, double* partial, int* blocks,
+                         cudaStream_t st);
+cudaError_t grad_moments(const DevSector& S, const double2* W, const double2* AW, int64_t vstride, int64_t pstride,
+                         int planes, const double* Kp, int n, int ld, int nc, double* partial, int* blocks,
+                         cudaStream_t st);
 
 }  // namespace ftlm_b200

@@ -4,12 +4,9 @@
 // the parameter gradient and the momentum blocks are in capi_batched.cu, capi_grad.cu and
 // capi_orbit.cu.
 #include <map>
-#include <thread>
-
 #include <atomic>
 
 #include "capi_internal.hpp"
-#include "chains.cuh"
 
 using namespace ftlm_b200;
 using namespace ftlm_b200::capi;
@@ -841,129 +838,18 @@ namespace capi {
 
 int64_t g_fused_max_dim = int64_t(1) << 17;
 
-// ftlm_gpu_ftlm_sector for many small sectors at once: every chain of every sector in one
-// chains_lanczos launch (one CTA per chain), then one batched quadrature; per-sector results in
-// lnz_s/e_s rows out_idx[i].  Same start vectors and seeds as the per-sector path.
-int fused_sectors_lanczos(const std::vector<ftlm_sector*>& secs, int R, int M, unsigned seed, int start_mode,
-                          std::vector<double>* Aout, std::vector<double>* Bout, std::vector<int>* Uout) {
-  if (secs.empty()) return FTLM_OK;
-  if (start_mode != FTLM_START_REFERENCE && start_mode != FTLM_START_PHILOX)
-    return fail(FTLM_ERR_INVALID, "unknown start_mode");
-  const int ns = static_cast<int>(secs.size());
-  const int nc = ns * R;
-  std::vector<DevSector> devs(static_cast<size_t>(ns));
-  std::vector<ChainDesc> cds(static_cast<size_t>(nc));
-  int64_t total = 0;
-  for (int i = 0; i < ns; ++i) {
-    devs[static_cast<size_t>(i)] = secs[static_cast<size_t>(i)]->dev;
-    for (int r = 0; r < R; ++r) {
-      cds[static_cast<size_t>(i) * R + r] = ChainDesc{i, i * R + r, total};
-      total += 3 * secs[static_cast<size_t>(i)]->plan.dim;
-    }
-  }
-  cudaStream_t st = secs[0]->stream;
-  DevBuf d_sec, d_cd, d_scr, d_a, d_b, d_u, d_red;
-  CU_TRY(d_sec.alloc(devs.size() * sizeof(DevSector)));
-  CU_TRY(d_cd.alloc(cds.size() * sizeof(ChainDesc)));
-  CU_TRY(d_scr.alloc(static_cast<size_t>(total) * sizeof(double2)));
-  CU_TRY(d_a.alloc(static_cast<size_t>(nc) * M * sizeof(double)));
-  CU_TRY(d_b.alloc(static_cast<size_t>(nc) * M * sizeof(double)));
-  CU_TRY(d_u.alloc(static_cast<size_t>(nc) * sizeof(int)));
-  CU_TRY(cudaMemcpyAsync(d_sec.p, devs.data(), devs.size() * sizeof(DevSector), cudaMemcpyHostToDevice, st));
-  // chains of larger sectors first, 1024 threads each; the rest 256 threads each
-  std::vector<ChainDesc> ordered;
-  ordered.reserve(cds.size());
-  for (const auto& c : cds)
-    if (secs[static_cast<size_t>(c.sector)]->plan.dim > 8192) ordered.push_back(c);
-  const int n_wide = static_cast<int>(ordered.size());
-  for (const auto& c : cds)
-    if (secs[static_cast<size_t>(c.sector)]->plan.dim <= 8192) ordered.push_back(c);
-  CU_TRY(cudaMemcpyAsync(d_cd.p, ordered.data(), ordered.size() * sizeof(ChainDesc), cudaMemcpyHostToDevice, st));
-  CU_TRY(cudaMemsetAsync(d_a.p, 0, static_cast<size_t>(nc) * M * sizeof(double), st));
-  CU_TRY(cudaMemsetAsync(d_b.p, 0, static_cast<size_t>(nc) * M * sizeof(double), st));
-  double2* scr = d_scr.as<double2>();
-  if (start_mode == FTLM_START_REFERENCE) {
-    // host RNG (libstdc++ mt19937 + normal_distribution, as the reference), chains in parallel
-    std::vector<std::complex<double>> host(static_cast<size_t>(total));
-    const unsigned hw = std::max(1u, std::min(32u, std::thread::hardware_concurrency()));
-    std::vector<std::thread> pool;
-    for (unsigned w = 0; w < hw; ++w)
-      pool.emplace_back([&, w]() {
-        std::vector<std::complex<double>> q;
-        for (int c = static_cast<int>(w); c < nc; c += static_cast<int>(hw)) {
-          const int i = c / R, r = c % R;
-          reference_start(secs[static_cast<size_t>(i)]->plan.dim, seed + static_cast<unsigned>(r) * 100003u, &q);
-          std::copy(q.begin(), q.end(), host.begin() + cds[static_cast<size_t>(c)].off);
-        }
-      });
-    for (auto& th : pool) th.join();
-    CU_TRY(cudaMemcpyAsync(scr, host.data(), host.size() * sizeof(double2), cudaMemcpyHostToDevice, st));
-    CU_TRY(cudaStreamSynchronize(st));
-  } else {
-    CU_TRY(d_red.alloc(kScratchDoubles * sizeof(double)));
-    for (int c = 0; c < nc; ++c) {
-      const int i = c / R, r = c % R;
-      const int64_t dim = secs[static_cast<size_t>(i)]->plan.dim;
-      double2* q = scr + cds[static_cast<size_t>(c)].off;
-      CU_TRY(lz_philox_start(q, dim, seed + static_cast<unsigned>(r) * 100003u, d_red.as<double>(), st));
-      CU_TRY(lz_normalise_start(q, dim, d_red.as<double>(), st));
-    }
-  }
-  // the two launches run concurrently: the small chains on a second stream ordered after the copies
-  cudaStream_t st2 = nullptr;
-  cudaEvent_t ready = nullptr, done = nullptr;
-  CU_TRY(cudaStreamCreateWithFlags(&st2, cudaStreamNonBlocking));
-  cudaError_t ce = cudaEventCreateWithFlags(&ready, cudaEventDisableTiming);
-  if (ce == cudaSuccess) ce = cudaEventCreateWithFlags(&done, cudaEventDisableTiming);
-  if (ce == cudaSuccess) ce = cudaEventRecord(ready, st);
-  if (ce == cudaSuccess) ce = cudaStreamWaitEvent(st2, ready, 0);
-  if (ce == cudaSuccess)
-    ce = chains_lanczos(d_sec.as<DevSector>(), d_cd.as<ChainDesc>(), n_wide, M, scr, d_a.as<double>(),
-                        d_b.as<double>(), d_u.as<int>(), true, st);
-  if (ce == cudaSuccess)
-    ce = chains_lanczos(d_sec.as<DevSector>(), d_cd.as<ChainDesc>() + n_wide, nc - n_wide, M, scr, d_a.as<double>(),
-                        d_b.as<double>(), d_u.as<int>(), false, st2);
-  if (ce == cudaSuccess) ce = cudaEventRecord(done, st2);
-  if (ce == cudaSuccess) ce = cudaStreamWaitEvent(st, done, 0);
-  const cudaError_t se = cudaStreamSynchronize(st);
-  if (ready) cudaEventDestroy(ready);
-  if (done) cudaEventDestroy(done);
-  cudaStreamDestroy(st2);
-  CU_TRY(ce);
-  CU_TRY(se);
-  std::vector<double>& A = *Aout;
-  std::vector<double>& B = *Bout;
-  std::vector<int>& used = *Uout;
-  A.assign(static_cast<size_t>(nc) * M, 0.0);
-  B.assign(static_cast<size_t>(nc) * M, 0.0);
-  used.assign(static_cast<size_t>(nc), 0);
-  CU_TRY(cudaMemcpyAsync(A.data(), d_a.p, A.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
-  CU_TRY(cudaMemcpyAsync(B.data(), d_b.p, B.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
-  CU_TRY(cudaMemcpyAsync(used.data(), d_u.p, used.size() * sizeof(int), cudaMemcpyDeviceToHost, st));
-  CU_TRY(cudaStreamSynchronize(st));
-  return FTLM_OK;
-}
-
 int fused_sectors_ftlm(const std::vector<ftlm_sector*>& secs, const std::vector<int>& out_idx, int R, int M,
-                       unsigned seed, int start_mode, const double* bts, int n_bt, double* lnz_s, double* e_s,
+                       unsigned seed, int start_mode, bool c64, const double* bts, int n_bt, double* lnz_s, double* e_s,
                        bool converged) {
   if (secs.empty()) return FTLM_OK;
-  const int ns = static_cast<int>(secs.size());
-  const int nc = ns * R;
-  std::vector<double> A, B;
-  std::vector<int> used;
-  int rc0 = fused_sectors_lanczos(secs, R, M, seed, start_mode, &A, &B, &used);
-  if (rc0) return rc0;
-  std::vector<double> lq(static_cast<size_t>(nc) * n_bt), eq(static_cast<size_t>(nc) * n_bt);
-  int rc = chain_quadrature(A.data(), B.data(), used.data(), nc, M, bts, n_bt, lq.data(), eq.data(), converged);
+  const size_t n = static_cast<size_t>(n_bt);
+  std::vector<double> lz(secs.size() * n), en(secs.size() * n);
+  const int rc = chains_ftlm(secs, R, M, seed, start_mode, c64, bts, n_bt, converged, lz.data(), en.data());
   if (rc) return rc;
-  for (int i = 0; i < ns; ++i) {
-    const size_t o = static_cast<size_t>(i) * R;
-    const size_t dst = static_cast<size_t>(out_idx[static_cast<size_t>(i)]) * n_bt;
-    rc = ftlm_gpu_ftlm_combine(lq.data() + o * n_bt, eq.data() + o * n_bt, used.data() + o, R, n_bt,
-                               std::log(static_cast<double>(secs[static_cast<size_t>(i)]->plan.dim)), lnz_s + dst,
-                               e_s + dst);
-    if (rc) return rc;
+  for (size_t i = 0; i < secs.size(); ++i) {
+    const size_t dst = static_cast<size_t>(out_idx[i]) * n;
+    std::copy(lz.begin() + i * n, lz.begin() + (i + 1) * n, lnz_s + dst);
+    std::copy(en.begin() + i * n, en.begin() + (i + 1) * n, e_s + dst);
   }
   return FTLM_OK;
 }
@@ -976,18 +862,39 @@ extern "C" {
 int ftlm_gpu_lanczos_sectors(ftlm_sector* const* secs, int n_sectors, int R, int M, unsigned seed, int start_mode,
                              double* alpha, double* beta, int* used) {
   if (!secs || n_sectors < 0 || R <= 0 || M <= 0 || !alpha || !beta || !used) return fail(FTLM_ERR_INVALID, "bad arguments");
-  std::vector<ftlm_sector*> v(secs, secs + n_sectors);
-  for (ftlm_sector* s : v) {
-    const int rc = need_device(s);
+  // Sectors far beyond the fused path's range run their chains one at a time.
+  constexpr int64_t kFusedMost = int64_t(1) << 22;
+  std::vector<ftlm_sector*> v;
+  std::vector<int> at;
+  for (int i = 0; i < n_sectors; ++i) {
+    int rc = need_device(secs[i]);
     if (rc) return rc;
+    if (secs[i]->plan.dim <= kFusedMost) {
+      v.push_back(secs[i]);
+      at.push_back(i);
+      continue;
+    }
+    for (int r = 0; r < R; ++r) {
+      const size_t row = static_cast<size_t>(i) * R + r;
+      std::fill(alpha + row * M, alpha + (row + 1) * M, 0.0);
+      std::fill(beta + row * M, beta + (row + 1) * M, 0.0);
+      int nb = 0;
+      rc = ftlm_gpu_lanczos(secs[i], M, seed + static_cast<unsigned>(r) * 100003u, start_mode, alpha + row * M,
+                            beta + row * M, &nb, used + row);
+      if (rc) return rc;
+    }
   }
-  std::vector<double> A, B;
-  std::vector<int> u;
-  const int rc = fused_sectors_lanczos(v, R, M, seed, start_mode, &A, &B, &u);
+  if (v.empty()) return FTLM_OK;
+  ChainRun run;
+  const int rc = chains_run(v, R, M, seed, start_mode, false, &run);
   if (rc) return rc;
-  std::copy(A.begin(), A.end(), alpha);
-  std::copy(B.begin(), B.end(), beta);
-  std::copy(u.begin(), u.end(), used);
+  const size_t rows = static_cast<size_t>(R), tab = rows * M;
+  for (size_t i = 0; i < v.size(); ++i) {
+    const size_t o = static_cast<size_t>(at[i]) * rows;
+    CU_TRY(cudaMemcpy(alpha + o * M, run.alpha.as<double>() + i * tab, tab * sizeof(double), cudaMemcpyDeviceToHost));
+    CU_TRY(cudaMemcpy(beta + o * M, run.beta.as<double>() + i * tab, tab * sizeof(double), cudaMemcpyDeviceToHost));
+    CU_TRY(cudaMemcpy(used + o, run.used.as<int>() + i * rows, rows * sizeof(int), cudaMemcpyDeviceToHost));
+  }
   return FTLM_OK;
 }
 
@@ -1109,7 +1016,7 @@ int ftlm_gpu_gc_sweep(const ftlm_params* p, int R, int M, unsigned seed, int sta
       ftlm_gpu_sector_destroy(s);
       if (rc) return clear_and(small, rc);
     }
-  const int rcf = fused_sectors_ftlm(small, small_idx, std::max(1, R), std::max(1, M), seed, start_mode, bts, n_bt,
+  const int rcf = fused_sectors_ftlm(small, small_idx, std::max(1, R), std::max(1, M), seed, start_mode, false, bts, n_bt,
                                      lnz_s, e_s, plain_quadrature_converged());
   clear_and(small, FTLM_OK);
   if (rcf) return rcf;

@@ -275,12 +275,15 @@ int batched_sweep(const ftlm_params* p, int R, int M, unsigned seed, const doubl
   if (n <= 0 || n > 32) return fail(FTLM_ERR_INVALID, "FockBasis: require 1 <= n_sites <= 32 (bit packing)");
   const int nsec = (n + 1) * (n + 1);
   std::vector<int> N(static_cast<size_t>(nsec));
-  // sectors the batched path runs in complex128 (dim <= 2M, Philox starts) go to one fused launch
-  std::vector<ftlm_sector*> small;
-  std::vector<int> small_idx;
-  auto clear_and = [&small](int rc) {
+  // small sectors go to fused launches: those the batched path runs in complex128 (dim <= 2M, Philox starts), and
+  // those whose complex64 chains need no check against complex128
+  std::vector<ftlm_sector*> small, mid;
+  std::vector<int> small_idx, mid_idx;
+  auto clear_and = [&small, &mid](int rc) {
     for (ftlm_sector* x : small) ftlm_gpu_sector_destroy(x);
+    for (ftlm_sector* x : mid) ftlm_gpu_sector_destroy(x);
     small.clear();
+    mid.clear();
     return rc;
   };
   for (int nu = 0; nu <= n; ++nu)
@@ -295,14 +298,22 @@ int batched_sweep(const ftlm_params* p, int R, int M, unsigned seed, const doubl
         small_idx.push_back(idx);
         continue;
       }
+      if (n_check <= 0 && M <= 160 && s->plan.dim >= 2 && s->plan.dim <= kFusedSweepMax && s->plan.max_up_deg <= 120) {
+        mid.push_back(s);
+        mid_idx.push_back(idx);
+        continue;
+      }
       rc = batched_sector(s, bts, n_bt, R, M, seed, n_check, lnz_s + static_cast<size_t>(idx) * n_bt,
                           e_s + static_cast<size_t>(idx) * n_bt,
                           lnz_s_err ? lnz_s_err + static_cast<size_t>(idx) * n_bt : nullptr);
       ftlm_gpu_sector_destroy(s);
       if (rc) return clear_and(rc);
     }
-  const int rcf = fused_sectors_ftlm(small, small_idx, std::max(1, R), std::max(1, M), seed, FTLM_START_PHILOX, bts,
-                                     n_bt, lnz_s, e_s, true);
+  int rcf = fused_sectors_ftlm(small, small_idx, std::max(1, R), std::max(1, M), seed, FTLM_START_PHILOX, false, bts, n_bt,
+                               lnz_s, e_s, true);
+  if (!rcf)
+    rcf = fused_sectors_ftlm(mid, mid_idx, std::max(1, R), std::max(1, M), seed, FTLM_START_PHILOX, true, bts, n_bt, lnz_s,
+                             e_s, true);
   clear_and(FTLM_OK);
   if (rcf) return rcf;
   if (lnz_s_err)  // the fused small sectors ran in complex128

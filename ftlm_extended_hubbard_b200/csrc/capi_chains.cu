@@ -1,0 +1,229 @@
+// Host side of the fused Lanczos chains of many sectors (chains.cu): launches by size class, and the sectors' ln Z and
+// energy with the chains' tridiagonals never leaving the device.
+#include <thread>
+
+#include "capi_internal.hpp"
+#include "chains.cuh"
+
+using namespace ftlm_b200;
+using namespace ftlm_b200::capi;
+
+namespace ftlm_b200 {
+namespace capi {
+
+namespace {
+
+// The reference's start vectors (src/lanczos.cpp:140-175) before normalisation.  The entries of a shorter vector are
+// the first ones of a longer vector of the same seed, so the longest of each seed serves every sector.
+void reference_normals(int64_t dim, int R, unsigned seed, std::vector<std::complex<double>>* out) {
+  out->resize(static_cast<size_t>(R) * dim);
+  const int hw = static_cast<int>(std::max(1u, std::min(32u, std::thread::hardware_concurrency())));
+  auto work = [&](int w, int n) {
+    for (int r = w; r < R; r += n) {
+      std::mt19937 rng(seed + static_cast<unsigned>(r) * 100003u);
+      std::normal_distribution<double> gauss(0.0, 1.0);
+      std::complex<double>* v = out->data() + static_cast<size_t>(r) * dim;
+      for (int64_t i = 0; i < dim; ++i) {
+        const double re = gauss(rng);
+        const double im = gauss(rng);
+        v[i] = {re, im};
+      }
+    }
+  };
+  const int n = std::min(hw, R);
+  if (n <= 1 || static_cast<int64_t>(R) * dim < 4096) {
+    work(0, 1);
+    return;
+  }
+  std::vector<std::thread> pool;
+  for (int w = 1; w < n; ++w) pool.emplace_back(work, w, n);
+  work(0, n);
+  for (auto& th : pool) th.join();
+}
+
+}  // namespace
+
+int chains_run(const std::vector<ftlm_sector*>& secs, int R, int M, unsigned seed, int start_mode, bool c64,
+               ChainRun* run, void* store, const std::vector<int64_t>* store_base, bool keep_scale) {
+  if (start_mode != FTLM_START_REFERENCE && start_mode != FTLM_START_PHILOX)
+    return fail(FTLM_ERR_INVALID, "unknown start_mode");
+  const int ns = static_cast<int>(secs.size());
+  const int per = c64 ? 2 : 1, planes = (R + per - 1) / per;
+  struct Item {
+    ChainDesc d;
+    int size;
+    bool smem;
+    int64_t dim;
+    size_t bytes;
+  };
+  std::vector<DevSector> devs;
+  std::vector<Item> items;
+  int64_t max_dim = 0;
+  bool phase = true;  // one kernel for all: the register form of the table entries where every table has it
+  for (const ftlm_sector* s : secs)
+    if (s->dev.dn_g.ent && s->dev.dn_g.nt > 0 && !s->dev.dn_g.phase) phase = false;
+  for (int i = 0; i < ns; ++i) {
+    const DevSector& S = secs[static_cast<size_t>(i)]->dev;
+    devs.push_back(S);
+    max_dim = std::max(max_dim, S.dim);
+    const bool smem = chain_in_smem(S, c64, phase);
+    for (int p = 0; p < planes; ++p) {
+      ChainDesc d{};
+      d.sector = i;
+      d.out = i * R + per * p;
+      d.chains = std::min(per, R - per * p);
+      d.seed = seed + static_cast<unsigned>(per * p) * 100003u;
+      if (store_base) {
+        d.store = (*store_base)[static_cast<size_t>(i)] + static_cast<int64_t>(p) * S.dim;
+        d.store_step = static_cast<int64_t>(planes) * S.dim;
+      }
+      items.push_back(Item{d, chain_class(S.dim), smem, S.dim, chain_elements(S) * 16 * (smem ? 3 : 4)});
+    }
+  }
+  std::stable_sort(items.begin(), items.end(), [](const Item& a, const Item& b) {
+    if (a.size != b.size) return a.size < b.size;
+    if (a.smem != b.smem) return b.smem;
+    return a.dim > b.dim;
+  });
+  cudaStream_t st = secs[0]->stream;
+  const size_t nc = static_cast<size_t>(ns) * R;
+  CU_TRY(run->alpha.alloc(nc * M * sizeof(double)));
+  CU_TRY(run->beta.alloc(nc * M * sizeof(double)));
+  CU_TRY(run->used.alloc(nc * sizeof(int)));
+  CU_TRY(cudaMemsetAsync(run->alpha.p, 0, nc * M * sizeof(double), st));
+  CU_TRY(cudaMemsetAsync(run->beta.p, 0, nc * M * sizeof(double), st));
+  if (keep_scale) {
+    std::vector<double> one(nc * M, 1.0);
+    CU_TRY(run->scale.alloc(nc * M * sizeof(double)));
+    CU_TRY(cudaMemcpyAsync(run->scale.p, one.data(), nc * M * sizeof(double), cudaMemcpyHostToDevice, st));
+    CU_TRY(cudaStreamSynchronize(st));
+  }
+  DevBuf d_sec, d_desc, d_scr, d_init;
+  CU_TRY(d_sec.alloc(devs.size() * sizeof(DevSector)));
+  CU_TRY(cudaMemcpyAsync(d_sec.p, devs.data(), devs.size() * sizeof(DevSector), cudaMemcpyHostToDevice, st));
+  if (start_mode == FTLM_START_REFERENCE) {
+    std::vector<std::complex<double>> host;
+    reference_normals(max_dim, R, seed, &host);
+    CU_TRY(d_init.alloc(host.size() * sizeof(double2)));
+    CU_TRY(cudaMemcpyAsync(d_init.p, host.data(), host.size() * sizeof(double2), cudaMemcpyHostToDevice, st));
+    CU_TRY(cudaStreamSynchronize(st));
+    for (auto& it : items) it.d.init = static_cast<int64_t>(it.d.out % R) * max_dim;
+  }
+  // The planes in pieces whose vectors fit a bounded scratch; the classes of a piece run side by side.
+  constexpr size_t kScratch = size_t(16) << 30;
+  size_t largest = 0, total = 0;
+  for (const auto& it : items) {
+    largest = std::max(largest, it.bytes);
+    total += it.bytes;
+  }
+  CU_TRY(d_scr.alloc(std::min(total, std::max(kScratch, largest))));
+  CU_TRY(d_desc.alloc(items.size() * sizeof(ChainDesc)));
+  std::vector<ChainDesc> descs(items.size());
+  const size_t room = std::max(kScratch, largest);
+  std::vector<size_t> piece{0};  // first items of the pieces
+  {
+    size_t at = 0;
+    for (size_t i = 0; i < items.size(); ++i) {
+      if (at + items[i].bytes > room) {
+        piece.push_back(i);
+        at = 0;
+      }
+      items[i].d.off = static_cast<int64_t>(at / 16);
+      at += items[i].bytes;
+      descs[i] = items[i].d;
+    }
+  }
+  piece.push_back(items.size());
+  CU_TRY(cudaMemcpyAsync(d_desc.p, descs.data(), descs.size() * sizeof(ChainDesc), cudaMemcpyHostToDevice, st));
+  cudaEvent_t ev[2] = {nullptr, nullptr};
+  cudaError_t ce = cudaEventCreateWithFlags(&ev[0], cudaEventDisableTiming);
+  if (ce == cudaSuccess) ce = cudaEventCreateWithFlags(&ev[1], cudaEventDisableTiming);
+  for (size_t pc = 0; pc + 1 < piece.size() && ce == cudaSuccess; ++pc) {
+    ce = cudaEventRecord(ev[0], st);
+    int stream = 0;
+    for (size_t i = piece[pc]; i < piece[pc + 1] && ce == cudaSuccess;) {
+      size_t j = i;
+      size_t smem_bytes = 0;
+      for (; j < piece[pc + 1] && items[j].size == items[i].size && items[j].smem == items[i].smem; ++j)
+        smem_bytes = std::max(smem_bytes, chain_smem_bytes(devs[static_cast<size_t>(items[j].d.sector)], c64, phase, items[j].smem));
+      cudaStream_t s2 = secs[static_cast<size_t>(std::min(stream, ns - 1))]->stream;
+      ++stream;
+      if (s2 != st) ce = cudaStreamWaitEvent(s2, ev[0], 0);
+      ChainLaunch L{};
+      L.sectors = d_sec.as<DevSector>();
+      L.descs = d_desc.as<ChainDesc>() + i;
+      L.blocks = static_cast<int>(j - i);
+      L.size = items[i].size;
+      L.smem = items[i].smem;
+      L.phase = phase;
+      L.smem_bytes = smem_bytes;
+      L.M = M;
+      L.scratch = d_scr.p;
+      L.init = d_init.as<double2>();
+      L.alpha = run->alpha.as<double>();
+      L.beta = run->beta.as<double>();
+      L.used = run->used.as<int>();
+      L.scale = keep_scale ? run->scale.as<double>() : nullptr;
+      L.store = store;
+      if (ce == cudaSuccess) ce = chains_lanczos(L, c64, s2);
+      if (s2 != st && ce == cudaSuccess) {
+        ce = cudaEventRecord(ev[1], s2);
+        if (ce == cudaSuccess) ce = cudaStreamWaitEvent(st, ev[1], 0);
+      }
+      i = j;
+    }
+  }
+  const cudaError_t se = cudaStreamSynchronize(st);  // the scratch goes back to the device here
+  if (ce != cudaSuccess) cudaDeviceSynchronize();
+  for (auto& e : ev)
+    if (e) cudaEventDestroy(e);
+  CU_TRY(ce);
+  CU_TRY(se);
+  return FTLM_OK;
+}
+
+int chains_ftlm(const std::vector<ftlm_sector*>& secs, int R, int M, unsigned seed, int start_mode, bool c64,
+                const double* bts, int n_bt, bool converged, double* lnz, double* energy) {
+  if (secs.empty() || n_bt == 0) return FTLM_OK;
+  if (M > 160) return fail(FTLM_ERR_UNSUPPORTED, "tridiagonal size > 160 is not supported by the on-chip eigen-solver");
+  const int ns = static_cast<int>(secs.size()), nc = ns * R;
+  if (static_cast<long long>(nc) * n_bt > 0x7fffffffLL) return fail(FTLM_ERR_INVALID, "n_chains * n_bt exceeds 2^31 - 1");
+  ChainRun run;
+  int rc = chains_run(secs, R, M, seed, start_mode, c64, &run);
+  if (rc) return rc;
+  cudaStream_t st = secs[0]->stream;
+  const size_t outb = static_cast<size_t>(nc) * n_bt * sizeof(double), secb = static_cast<size_t>(ns) * n_bt * sizeof(double);
+  std::vector<double> logd;
+  for (const ftlm_sector* s : secs) logd.push_back(std::log(static_cast<double>(s->plan.dim)));
+  DevBuf lam, w, bt, lq, eq, info, ld, z, e;
+  CU_TRY(lam.alloc(static_cast<size_t>(nc) * M * sizeof(double)));
+  CU_TRY(w.alloc(static_cast<size_t>(nc) * M * sizeof(double)));
+  CU_TRY(bt.alloc(n_bt * sizeof(double)));
+  CU_TRY(lq.alloc(outb));
+  CU_TRY(eq.alloc(outb));
+  CU_TRY(info.alloc(nc * sizeof(int)));
+  CU_TRY(ld.alloc(logd.size() * sizeof(double)));
+  CU_TRY(z.alloc(secb));
+  CU_TRY(e.alloc(secb));
+  CU_TRY(cudaMemcpyAsync(bt.p, bts, n_bt * sizeof(double), cudaMemcpyHostToDevice, st));
+  CU_TRY(cudaMemcpyAsync(ld.p, logd.data(), logd.size() * sizeof(double), cudaMemcpyHostToDevice, st));
+  const double *al = run.alpha.as<double>(), *be = run.beta.as<double>();
+  const int* us = run.used.as<int>();
+  if (converged)
+    CU_TRY(symeig_tridiag(al, be, us, nc, M, lam.as<double>(), w.as<double>(), nullptr, info.as<int>(), st));
+  else
+    CU_TRY(quad_jacobi(al, be, us, nc, M, 0, 1e-14, lam.as<double>(), w.as<double>(), st));
+  CU_TRY(quad_eval(lam.as<double>(), w.as<double>(), us, nc, M, bt.as<double>(), n_bt, lq.as<double>(), eq.as<double>(), st));
+  CU_TRY(quad_sectors(lq.as<double>(), eq.as<double>(), us, ns, R, n_bt, ld.as<double>(), z.as<double>(), e.as<double>(), st));
+  CU_TRY(cudaMemcpyAsync(lnz, z.p, secb, cudaMemcpyDeviceToHost, st));
+  CU_TRY(cudaMemcpyAsync(energy, e.p, secb, cudaMemcpyDeviceToHost, st));
+  std::vector<int> bad(static_cast<size_t>(nc), 0);
+  if (converged) CU_TRY(cudaMemcpyAsync(bad.data(), info.p, nc * sizeof(int), cudaMemcpyDeviceToHost, st));
+  CU_TRY(cudaStreamSynchronize(st));
+  for (int b : bad)
+    if (b == 1) return fail(FTLM_ERR_NUMERIC, "GPU eigen-solver did not converge");
+  return FTLM_OK;
+}
+
+}  // namespace capi
+}  // namespace ftlm_b200

@@ -329,8 +329,8 @@ int ftlm_gpu_gc_logz(const ftlm_params* p, double mu, double bT, int R, int M, u
   const int nsec = (n + 1) * (n + 1);
   const int st_mode = method == 1 ? FTLM_START_PHILOX : start_mode;
   const long long limit = method == 1 ? 2LL * M : kGcFusedPlainMax;
-  std::vector<SectorPtr> small;
-  std::vector<int> small_idx;
+  std::vector<SectorPtr> small, mid;  // chains in fused launches below: complex128 and complex64
+  std::vector<int> small_idx, mid_idx;
   std::vector<double> A, B;
   std::vector<int> used;
   for (int nu = 0; nu <= n; ++nu)
@@ -341,9 +341,14 @@ int ftlm_gpu_gc_logz(const ftlm_params* p, double mu, double bT, int R, int M, u
       if (rc) return rc;
       SectorPtr s(raw);
       const int64_t dim = s->plan.dim;
-      if (dim <= limit) {  // chains of all small sectors in one launch below
+      if (dim <= limit) {
         small.push_back(std::move(s));
         small_idx.push_back(idx);
+        continue;
+      }
+      if (method == 1 && dim <= kFusedSweepMax && s->plan.max_up_deg <= 120) {
+        mid.push_back(std::move(s));
+        mid_idx.push_back(idx);
         continue;
       }
       if (method == 1) {
@@ -368,21 +373,14 @@ int ftlm_gpu_gc_logz(const ftlm_params* p, double mu, double bT, int R, int M, u
       rc = gc_quadrature(A.data(), B.data(), used.data(), R, M, bT, dim, lnz_s + idx, e_s + idx);
       if (rc) return rc;
     }
-  if (!small.empty()) {
+  auto fused = [&](const std::vector<SectorPtr>& v, const std::vector<int>& at, bool c64) {
     std::vector<ftlm_sector*> hs;
-    for (auto& s : small) hs.push_back(s.get());
-    const size_t ns = hs.size();
-    A.assign(ns * R * M, 0.0);
-    B.assign(ns * R * M, 0.0);
-    used.assign(ns * R, 0);
-    rc = ftlm_gpu_lanczos_sectors(hs.data(), static_cast<int>(ns), R, M, seed, st_mode, A.data(), B.data(), used.data());
-    if (rc) return rc;
-    for (size_t i = 0; i < ns; ++i) {
-      rc = gc_quadrature(A.data() + i * R * M, B.data() + i * R * M, used.data() + i * R, R, M, bT, hs[i]->plan.dim,
-                         lnz_s + small_idx[i], e_s + small_idx[i]);
-      if (rc) return rc;
-    }
-  }
+    for (const auto& s : v) hs.push_back(s.get());
+    return fused_sectors_ftlm(hs, at, R, M, seed, st_mode, c64, &bT, 1, lnz_s, e_s, true);
+  };
+  rc = fused(small, small_idx, false);
+  if (!rc) rc = fused(mid, mid_idx, true);
+  if (rc) return rc;
   std::vector<double> x(static_cast<size_t>(nsec));
   for (int nu = 0; nu <= n; ++nu)
     for (int nd = 0; nd <= n; ++nd) {

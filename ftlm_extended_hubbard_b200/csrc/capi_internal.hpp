@@ -343,11 +343,26 @@ bool plain_quadrature_converged();
 int plain_sector_ftlm(ftlm_sector* s, const double* bts, int n_bt, int R, int M, unsigned seed, int start_mode,
                       bool converged, double* lnz, double* energy);
 
-// ftlm_gpu_ftlm_sector for many small sectors in one chains_lanczos launch (capi.cu); results in
-// rows out_idx[i] of lnz_s / e_s.
+// The fused chains of many sectors (capi_chains.cu), results on the device: rows [sector][chain] of alpha/beta [M]
+// (zero-padded), steps used and, with keep_scale, the norms of the stored vectors.
+struct ChainRun {
+  DevBuf alpha, beta, used, scale;
+};
+// c64: complex64 chains (Philox starts), else complex128.  store: the chains' vectors W_k go to store + store_base[i] +
+// (k * planes + p) * dim for plane p (two chains of complex64, one of complex128) of sector i.
+int chains_run(const std::vector<ftlm_sector*>& secs, int R, int M, unsigned seed, int start_mode, bool c64,
+               ChainRun* run, void* store = nullptr, const std::vector<int64_t>* store_base = nullptr,
+               bool keep_scale = false);
+// ln Z and energy of each sector on the temperature grid, [sector][n_bt].
+int chains_ftlm(const std::vector<ftlm_sector*>& secs, int R, int M, unsigned seed, int start_mode, bool c64,
+                const double* bts, int n_bt, bool converged, double* lnz, double* energy);
+// The same into rows out_idx[i] of lnz_s / e_s.
 int fused_sectors_ftlm(const std::vector<ftlm_sector*>& secs, const std::vector<int>& out_idx, int R, int M,
-                       unsigned seed, int start_mode, const double* bts, int n_bt, double* lnz_s, double* e_s,
+                       unsigned seed, int start_mode, bool c64, const double* bts, int n_bt, double* lnz_s, double* e_s,
                        bool converged);
+
+// Largest sector of a batched sweep that joins the fused launch (beyond it a sector fills the GPU by itself).
+constexpr int64_t kFusedSweepMax = 1 << 15;
 
 // The complex64 chains of one sector in groups of planes (planes.cu), alpha/beta [R][M] (beta zero-padded), used [R].
 int bt_run_chains(ftlm_sector* s, int R, int M, unsigned seed, std::vector<double>* A, std::vector<double>* B,

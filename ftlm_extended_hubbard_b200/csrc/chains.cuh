@@ -1,6 +1,6 @@
-// Fused Lanczos for many small sectors (chains.cu): one CTA per chain runs all M steps of the
-// src/lanczos.cpp:180-205 recurrence on vectors of its own sector, so a whole sweep of small
-// sectors is one launch instead of M host-synchronised steps per chain.
+// Fused Lanczos of many small sectors (chains.cu): one block per plane of one sector runs all M steps of the
+// src/lanczos.cpp:180-205 recurrence on its own vectors, so a whole sweep of small sectors is a few launches instead of
+// M times five kernels per sector.  A plane is two complex64 chains or one complex128 chain of a sector.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -10,15 +10,41 @@
 namespace ftlm_b200 {
 
 struct ChainDesc {
-  int sector;   // index into the DevSector array
-  int out;      // row of alpha/beta/used written by this chain
-  int64_t off;  // first element of the chain's three vectors (q, q_prev, w) in the scratch
+  int sector;          // index into the DevSector array
+  int out;             // first row of alpha/beta/used/scale written by this plane
+  int chains;          // chains of the plane that are wanted (a plane's second complex64 chain may not be)
+  unsigned seed;       // Philox key of its first chain
+  int64_t off;         // first element of its vectors in the scratch (3 of chain_elements(); 4 outside shared memory)
+  int64_t init;        // first element of its start vector in ChainLaunch::init
+  int64_t store;       // first element of its stored vectors, and their distance
+  int64_t store_step;
 };
 
-// q_0 of every chain (normalised) at scratch[off]; outputs alpha/beta [out][M] (beta of a chain
-// that broke down at step k: k entries), used [out].  Deterministic (fixed per-CTA order).
-// wide: 1024 threads per chain (for larger sectors) instead of 256.
-cudaError_t chains_lanczos(const DevSector* sectors, const ChainDesc* chains, int nc, int M, double2* scratch,
-                           double* alpha, double* beta, int* used, bool wide, cudaStream_t st);
+// Planes of one size class whose gathered vector is (or is not) in shared memory.
+struct ChainLaunch {
+  const DevSector* sectors;
+  const ChainDesc* descs;
+  int blocks;
+  int size;             // chain_class of the sectors
+  bool smem;            // the gathered vector is in shared memory
+  bool phase;           // every gauge table with table entries has the phase form
+  size_t smem_bytes;    // largest chain_smem_bytes of the sectors
+  int M;
+  void* scratch;
+  const double2* init;  // complex128 start vectors, not normalised, in the sector's order; null: Philox
+  double* alpha;        // [rows][M], zero-filled by the caller; entries of a chain that broke down at step k: k + 1
+  double* beta;         // (beta: k)
+  int* used;            // [rows]
+  double* scale;        // [rows][M] or null: norm of the stored vector k (1 where the chain has ended)
+  void* store;          // or null: the unnormalised vectors W_k in the spin-ordered basis, for a gradient's replay
+};
+
+int chain_class(int64_t dim);
+// Elements of one vector: rows have a pitch of Dd + 8.
+inline size_t chain_elements(const DevSector& S) { return static_cast<size_t>(S.Du) * static_cast<size_t>(S.Dd + 8); }
+// Shared memory of a plane of the sector, and whether its gathered vector fits there too.
+size_t chain_smem_bytes(const DevSector& S, bool c64, bool phase, bool with_vector);
+bool chain_in_smem(const DevSector& S, bool c64, bool phase);
+cudaError_t chains_lanczos(const ChainLaunch& L, bool c64, cudaStream_t st);
 
 }  // namespace ftlm_b200

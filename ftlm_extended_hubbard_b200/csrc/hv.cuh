@@ -59,6 +59,9 @@ cudaError_t quad_eval(const double* lam, const double* w0, const int* n, int nc,
 // Sector ln Z from R chain values: lnz[b] = ln(dim) + log mean_r exp(logq[r][b]); energy weighted.
 cudaError_t quad_sector(const double* logq, const double* eq, const int* n, int R, int nbt, double log_dim,
                         double* lnz, double* energy, cudaStream_t st);
+// The same for ns sectors of R chains each (log_dims [ns] on the device; lnz, energy [ns][nbt]).
+cudaError_t quad_sectors(const double* logq, const double* eq, const int* n, int ns, int R, int nbt,
+                         const double* log_dims, double* lnz, double* energy, cudaStream_t st);
 cudaError_t gc_reduce_dev(const double* lnz_s, const double* e_s, const int* N_s, int n_sec, const double* bts,
                           int n_bt, const double* mus, int n_mu, int n_sites, double* lnz_gc, double* n_avg,
                           double* e_avg, cudaStream_t st);

@@ -63,6 +63,42 @@ struct C64 {
   }
 };
 
+struct C128 {
+  using T = double2;
+  using Cf = double2;
+  static constexpr int kC = 1;
+  static constexpr bool kScaled = true;
+  static __device__ __forceinline__ T zero() { return make_double2(0.0, 0.0); }
+  static __device__ __forceinline__ bool small(T v) { return tiny(v) && (v.x != 0.0 || v.y != 0.0); }
+  static __device__ __forceinline__ T filtered(T v, double s) { return tiny(make_double2(s * v.x, s * v.y)) ? zero() : v; }
+  static __device__ __forceinline__ T times(double g, T v) { return make_double2(g * v.x, g * v.y); }
+  static __device__ __forceinline__ T add_scaled(T y, T a, double s) { return make_double2(fma(s, a.x, y.x), fma(s, a.y, y.y)); }
+  static __device__ __forceinline__ Cf coef(double2 c) { return c; }
+  static __device__ __forceinline__ Cf signed_coef(Cf c, uint32_t e) {
+    const int f = static_cast<int>(e & 0x80000000u);
+    return make_double2(__hiloint2double(__double2hiint(c.x) ^ f, __double2loint(c.x)),
+                        __hiloint2double(__double2hiint(c.y) ^ f, __double2loint(c.y)));
+  }
+  static __device__ __forceinline__ void cmac(T& acc, Cf c, T v) {
+    acc.x = fma(c.x, v.x, acc.x);
+    acc.x = fma(-c.y, v.y, acc.x);
+    acc.y = fma(c.x, v.y, acc.y);
+    acc.y = fma(c.y, v.x, acc.y);
+  }
+  static __device__ __forceinline__ void dot(double (&d)[2], T w, T y, double s) {  // conj(s w) y
+    const double x = s * w.x, z = s * w.y;
+    d[0] += x * y.x + z * y.y;
+    d[1] += x * y.y - z * y.x;
+  }
+  static __device__ __forceinline__ Cf up_coef(const DevSector& S, int j) { return S.up_coef[j]; }
+  static __device__ __forceinline__ Cf dn_coef(const DevSector& S, uint32_t e) {
+    return signed_coef(S.dn_coef[(e >> 1) & 255u], e << 31);
+  }
+  static __device__ __forceinline__ double2 get(T v, int) { return v; }
+  static __device__ __forceinline__ T make(const double2 (&z)[1]) { return z[0]; }
+  static __device__ __forceinline__ double2 narrow(double re, double im) { return make_double2(re, im); }
+};
+
 // The two real coefficients of the gauge table as registers: an entry picks the second one where (entry & cls) is not
 // zero and flips the sign by its bit 31.  In the XOR form the entry carries the bits by which the high words differ,
 // so the second value is the first with the differing bits other than the sign flipped.
@@ -99,6 +135,30 @@ struct RowCoefs<C64> {
     acc.y = fmaf(c, v.y, acc.y);
     acc.z = fmaf(c, v.z, acc.z);
     acc.w = fmaf(c, v.w, acc.w);
+  }
+};
+
+template <>
+struct RowCoefs<C128> {
+  double a0, a1, pc, ps;
+  bool xor_real;
+  __device__ __forceinline__ explicit RowCoefs(const DevGauge& G)
+      : a0(G.real2[0]), a1(G.real2[1]), pc(G.pc), ps(G.ps), xor_real(G.xor_real != 0) {}
+  static __device__ __forceinline__ double flip(double v, uint32_t bits) {
+    return __hiloint2double(__double2hiint(v) ^ static_cast<int>(bits), __double2loint(v));
+  }
+  __device__ __forceinline__ double pick(uint32_t e) const {
+    if (xor_real) return flip(a0, e & 0xFFFC0000u);
+    return flip((e & 0x40000000u) ? a1 : a0, e & 0x80000000u);
+  }
+  // Table-section entry in the phase form: real2[cls] (pc, +-ps), bit for bit the table's value.
+  __device__ __forceinline__ double2 phase(uint32_t e) const {
+    const double c = flip((e & 0x40000000u) ? a1 : a0, e & 0x80000000u);
+    return make_double2(c * pc, flip(c * ps, (e << 4) & 0x80000000u));
+  }
+  static __device__ __forceinline__ void mac(double2& acc, double c, double2 v) {
+    acc.x = fma(c, v.x, acc.x);
+    acc.y = fma(c, v.y, acc.y);
   }
 };
 

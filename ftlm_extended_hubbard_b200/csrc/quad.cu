@@ -287,11 +287,20 @@ __global__ void eval_kernel(const double* __restrict__ lam, const double* __rest
 
 // src/ftlm_thermo.cpp:246-256: ln(dim) + max_l + log(sum_r e^{L_r - max_l} / count), chains
 // with n <= 0 skipped.  Energy: e^{L_r}-weighted mean of the chain energies.
-__global__ void sector_kernel(const double* __restrict__ logq, const double* __restrict__ eq,
-                              const int* __restrict__ nv, int R, int nbt, double log_dim, double* __restrict__ lnz,
-                              double* __restrict__ energy) {
-  const int bi = blockIdx.x * blockDim.x + threadIdx.x;
-  if (bi >= nbt) return;
+// One thread per sector and temperature; log_dims null: log_dim for all.
+__global__ void sector_kernel(const double* __restrict__ logq_all, const double* __restrict__ eq_all,
+                              const int* __restrict__ nv_all, int ns, int R, int nbt, double log_dim,
+                              const double* __restrict__ log_dims, double* __restrict__ lnz_all,
+                              double* __restrict__ energy_all) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= ns * nbt) return;
+  const int sec = i / nbt, bi = i - sec * nbt;
+  const double* logq = logq_all + static_cast<int64_t>(sec) * R * nbt;
+  const double* eq = eq_all + static_cast<int64_t>(sec) * R * nbt;
+  const int* nv = nv_all + static_cast<int64_t>(sec) * R;
+  double* lnz = lnz_all + static_cast<int64_t>(sec) * nbt;
+  double* energy = energy_all + static_cast<int64_t>(sec) * nbt;
+  if (log_dims) log_dim = log_dims[sec];
   double mx = -CUDART_INF;
   int cnt = 0;
   bool first = true;
@@ -420,7 +429,14 @@ cudaError_t quad_eval(const double* lam, const double* w0, const int* n, int nc,
 cudaError_t quad_sector(const double* logq, const double* eq, const int* n, int R, int nbt, double log_dim,
                         double* lnz, double* energy, cudaStream_t st) {
   if (nbt <= 0) return cudaSuccess;
-  sector_kernel<<<(nbt + 127) / 128, 128, 0, st>>>(logq, eq, n, R, nbt, log_dim, lnz, energy);
+  sector_kernel<<<(nbt + 127) / 128, 128, 0, st>>>(logq, eq, n, 1, R, nbt, log_dim, nullptr, lnz, energy);
+  return cudaGetLastError();
+}
+
+cudaError_t quad_sectors(const double* logq, const double* eq, const int* n, int ns, int R, int nbt,
+                         const double* log_dims, double* lnz, double* energy, cudaStream_t st) {
+  if (nbt <= 0 || ns <= 0) return cudaSuccess;
+  sector_kernel<<<(ns * nbt + 63) / 64, 64, 0, st>>>(logq, eq, n, ns, R, nbt, 0.0, log_dims, lnz, energy);
   return cudaGetLastError();
 }
 

@@ -7,6 +7,7 @@
 #include <complex>
 #include <cstring>
 #include <map>
+#include <thread>
 #include <utility>
 
 namespace ftlm_b200 {
@@ -236,12 +237,19 @@ void build_gauge_table(const SpinSpace& sp, const std::vector<MergedHop>& hops, 
     const uint32_t extra = G.phase ? tab_bits[static_cast<size_t>(k - 2)] : 0u;
     return (src << 4) | (static_cast<uint32_t>(k - 2) << 18) | extra | (sg << 31);
   };
+  // Groups are independent: built by several threads for the large tables, then put together in order.
+  struct Group {
+    bool ok = false;
+    uint8_t perm[32];
+    size_t KR0 = 0, KT0 = 0;
+    std::vector<uint32_t> ent;
+  };
   const int64_t ngroups = (D + 31) / 32;
-  std::vector<std::vector<uint32_t>> lr(32), lt(32), sr(32), st(32);
-  for (int64_t g = 0; g < ngroups; ++g) {
+  std::vector<Group> groups(static_cast<size_t>(ngroups));
+  auto build_group = [&](int64_t g) {
+    Group& R = groups[static_cast<size_t>(g)];
+    std::vector<uint32_t> lr[32], lt[32], sr[32], st[32];
     for (int l = 0; l < 32; ++l) {
-      lr[l].clear();
-      lt[l].clear();
       const int64_t r = g * 32 + l;
       if (r >= D) continue;
       const uint32_t m2 = sp.masks[static_cast<size_t>(r)];
@@ -260,7 +268,7 @@ void build_gauge_table(const SpinSpace& sp, const std::vector<MergedHop>& hops, 
     // max(its longest lane, its busiest bank group), so move strings between quarters to balance the
     // bank-group loads (local search over swaps, deterministic per group); lane L serves string
     // g*32 + perm[L].  The last, partial group keeps the identity.
-    uint8_t perm[32];
+    uint8_t* perm = R.perm;
     for (int l = 0; l < 32; ++l) perm[l] = static_cast<uint8_t>(l);
     if (g * 32 + 32 <= D) {
       int dl[2][32], dgp[2][32][8];
@@ -271,23 +279,25 @@ void build_gauge_table(const SpinSpace& sp, const std::vector<MergedHop>& hops, 
           for (int b = 0; b < 8; ++b) dgp[sct][l][b] = 0;
           for (uint32_t e : lst) ++dgp[sct][l][(e >> 10) & 7u];
         }
-      auto cost = [&](const uint8_t* pm) {
-        int tot = 0;
-        for (int sct = 0; sct < 2; ++sct) {
-          int dm = 0;
-          for (int q = 0; q < 4; ++q) {
-            int m = 0, gs[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-            for (int k = 0; k < 8; ++k) {
-              const int l = pm[q * 8 + k];
-              m = std::max(m, dl[sct][l]);
-              for (int b = 0; b < 8; ++b) gs[b] += dgp[sct][l][b];
-            }
-            for (int b = 0; b < 8; ++b) m = std::max(m, gs[b]);
-            dm = std::max(dm, m);
+      // rounds of a quarter, and of the group: the sum over sections of the worst quarter's
+      int load[2][4][8], rounds[2][4];
+      auto quarter = [&](int sct, int q, const int* gs) {
+        int m = 0;
+        for (int k = 0; k < 8; ++k) m = std::max(m, std::max(dl[sct][perm[q * 8 + k]], gs[k]));
+        return m;
+      };
+      for (int sct = 0; sct < 2; ++sct)
+        for (int q = 0; q < 4; ++q) {
+          for (int b = 0; b < 8; ++b) {
+            load[sct][q][b] = 0;
+            for (int k = 0; k < 8; ++k) load[sct][q][b] += dgp[sct][perm[q * 8 + k]][b];
           }
-          tot += dm;
+          rounds[sct][q] = quarter(sct, q, load[sct][q]);
         }
-        return tot;
+      auto total = [](const int (&r)[2][4]) {
+        int t = 0;
+        for (int sct = 0; sct < 2; ++sct) t += std::max(std::max(r[sct][0], r[sct][1]), std::max(r[sct][2], r[sct][3]));
+        return t;
       };
       uint64_t st64 = 0x9E3779B97F4A7C15ull ^ static_cast<uint64_t>(g);
       auto rnd = [&st64]() {  // splitmix64
@@ -296,18 +306,37 @@ void build_gauge_table(const SpinSpace& sp, const std::vector<MergedHop>& hops, 
         z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
         return z ^ (z >> 31);
       };
-      int best = cost(perm);
+      int best = total(rounds);
       for (int it = 0; it < 1500; ++it) {
         const int a = static_cast<int>(rnd() % 32), b = static_cast<int>(rnd() % 32);
-        if (a / 8 == b / 8) continue;
+        const int qa = a / 8, qb = b / 8;
+        if (qa == qb) continue;
+        const int pa = perm[a], pb = perm[b];
         std::swap(perm[a], perm[b]);
-        const int c = cost(perm);
-        if (c <= best)
+        int la[2][8], lb[2][8], r2[2][4];
+        std::memcpy(r2, rounds, sizeof(r2));
+        for (int sct = 0; sct < 2; ++sct) {
+          for (int k = 0; k < 8; ++k) {
+            const int diff = dgp[sct][pb][k] - dgp[sct][pa][k];
+            la[sct][k] = load[sct][qa][k] + diff;
+            lb[sct][k] = load[sct][qb][k] - diff;
+          }
+          r2[sct][qa] = quarter(sct, qa, la[sct]);
+          r2[sct][qb] = quarter(sct, qb, lb[sct]);
+        }
+        const int c = total(r2);
+        if (c <= best) {
           best = c;
-        else
+          std::memcpy(rounds, r2, sizeof(r2));
+          for (int sct = 0; sct < 2; ++sct) {
+            std::memcpy(load[sct][qa], la[sct], sizeof(la[sct]));
+            std::memcpy(load[sct][qb], lb[sct], sizeof(lb[sct]));
+          }
+        } else {
           std::swap(perm[a], perm[b]);
+        }
       }
-      std::vector<std::vector<uint32_t>> tr(32), tt(32);
+      std::vector<uint32_t> tr[32], tt[32];
       for (int l = 0; l < 32; ++l) {
         tr[l].swap(lr[perm[l]]);
         tt[l].swap(lt[perm[l]]);
@@ -317,7 +346,6 @@ void build_gauge_table(const SpinSpace& sp, const std::vector<MergedHop>& hops, 
         lt[l].swap(tt[l]);
       }
     }
-    for (int l = 0; l < 32; ++l) G.perm.push_back(perm[l]);
     size_t KR = 0, KT = 0;
     for (int qw = 0; qw < 4; ++qw) {
       schedule_quarter(&lr[8 * qw], &sr[8 * qw], pad_hop, D);
@@ -327,30 +355,51 @@ void build_gauge_table(const SpinSpace& sp, const std::vector<MergedHop>& hops, 
     }
     // each section padded to whole 4-entry loads: the row pass runs one loop per section with no
     // per-entry section test, and skips the padding rounds of each section's last load
-    const size_t KR0 = KR, KT0 = KT;
+    R.KR0 = KR;
+    R.KT0 = KT;
     KR = (KR + 3) / 4 * 4;
     KT = (KT + 3) / 4 * 4;
     const size_t K4 = KR + KT;
-    const size_t off = G.ent.size();
-    if (off + K4 * 32 > static_cast<size_t>(INT32_MAX) || KR0 > 0xFFFF || KT0 > 0x7FFF) return;
-    G.grp.push_back(static_cast<int32_t>(off));
-    G.grp.push_back(static_cast<int32_t>(KR));
-    G.grp.push_back(static_cast<int32_t>(KT));
-    G.grp.push_back(static_cast<int32_t>(KR0 | (KT0 << 16)));
-    // round k of lane l at off + ((k / 4) * 32 + l) * 4 + k % 4: a lane loads 4 rounds with one
+    // round k of lane l at ((k / 4) * 32 + l) * 4 + k % 4: a lane loads 4 rounds with one
     // 16-byte load.  Rounds a quarter does not need, and the rounds that pad the group to a
     // multiple of 4: lane l reads the sentinel of bank group l % 8.
-    G.ent.resize(off + K4 * 32);
+    R.ent.resize(K4 * 32);
     for (size_t k = 0; k < K4; ++k)
       for (int l = 0; l < 32; ++l) {
         uint32_t e = sentinel(static_cast<uint32_t>(l) & 7u);
         if (k < KR) {
           if (k < sr[l].size()) e = encode(sr[l][k]);
-        } else if (k < KR + KT) {
-          if (k - KR < st[l].size()) e = encode(st[l][k - KR]);
+        } else if (k - KR < st[l].size()) {
+          e = encode(st[l][k - KR]);
         }
-        G.ent[off + ((k / 4) * 32 + static_cast<size_t>(l)) * 4 + k % 4] = e;
+        R.ent[((k / 4) * 32 + static_cast<size_t>(l)) * 4 + k % 4] = e;
       }
+    R.ok = true;
+  };
+  const int nthreads = static_cast<int>(
+      std::max<int64_t>(1, std::min<int64_t>({static_cast<int64_t>(std::thread::hardware_concurrency()), 16, ngroups / 16})));
+  if (nthreads == 1) {
+    for (int64_t g = 0; g < ngroups; ++g) build_group(g);
+  } else {
+    std::vector<std::thread> pool;
+    for (int w = 0; w < nthreads; ++w)
+      pool.emplace_back([&, w]() {
+        for (int64_t g = w; g < ngroups; g += nthreads) build_group(g);
+      });
+    for (auto& t : pool) t.join();
+  }
+  for (const Group& R : groups) {
+    const size_t off = G.ent.size();
+    if (!R.ok || off + R.ent.size() > static_cast<size_t>(INT32_MAX) || R.KR0 > 0xFFFF || R.KT0 > 0x7FFF) {
+      G.grp.clear();
+      return;
+    }
+    G.perm.insert(G.perm.end(), R.perm, R.perm + 32);
+    G.grp.push_back(static_cast<int32_t>(off));
+    G.grp.push_back(static_cast<int32_t>((R.KR0 + 3) / 4 * 4));
+    G.grp.push_back(static_cast<int32_t>((R.KT0 + 3) / 4 * 4));
+    G.grp.push_back(static_cast<int32_t>(R.KR0 | (R.KT0 << 16)));
+    G.ent.insert(G.ent.end(), R.ent.begin(), R.ent.end());
   }
   // two all-sentinel loads after the last group: the row pass loads two ahead of use unconditionally
   G.ent.resize(G.ent.size() + 2 * 32 * 4, sentinel(0u));
@@ -535,65 +584,32 @@ void build_up_packed(SectorPlan* Pp) {
 
 }  // namespace
 
-std::string build_plan(int n_sites, int n_up, int n_dn, double U, double V, const std::vector<HopIn>& hops,
-                       const std::vector<PairIn>& pairs, SectorPlan* out) {
-  init_binom();
-  if (n_sites <= 0 || n_sites > 32) return "FockBasis: require 1 <= n_sites <= 32 (bit packing)";
-  if (n_up < 0 || n_dn < 0 || n_up > n_sites || n_dn > n_sites) return "FockBasis: particle numbers out of range";
-  for (const auto& h : hops) {
-    if (h.from < 0 || h.to < 0 || h.from >= n_sites || h.to >= n_sites || (h.spin != 0 && h.spin != 1))
-      return "hopping out of range";
-    if (h.from == h.to) return "on-site hopping entries are not supported";
-  }
-  for (const auto& pr : pairs)
-    if (pr.i < 0 || pr.j < 0 || pr.i >= n_sites || pr.j >= n_sites) return "nn pair out of range";
-  const uint64_t Du = binom(n_sites, n_up), Dd = binom(n_sites, n_dn);
-  if (Du > (1u << 22) || Dd > (1u << 22)) return "spin space larger than 2^22 strings is not supported";
-  if (Du * Dd >= (1ull << 31)) return "sector dimension must fit the reference's int index (< 2^31)";
+namespace {
 
+// The tables that depend on one species' strings alone (with the lattice): sectors that share N_up or N_down share them.
+std::string build_up(SectorPlan* out) {
   SectorPlan& P = *out;
-  P = SectorPlan{};
-  P.n = n_sites;
-  P.nu = n_up;
-  P.nd = n_dn;
-  P.U = U;
-  P.V = V;
-  P.pairs = pairs;
-  P.up.build(n_sites, n_up);
-  P.dn.build(n_sites, n_dn);
-  P.dim = P.up.D * P.dn.D;
-  P.hu = merge_hops(hops, 0);
-  P.hd = merge_hops(hops, 1);
-  if (P.hd.size() + 1 > 256) return "more than 255 distinct down hoppings are not supported";
-
+  P.up.build(P.n, P.nu);
   // Diagonal tables.  sum_pairs (u_i+d_i)(u_j+d_j) = uu + dd + sum_s d_s * c_u(s).
   P.cnt_uu.resize(static_cast<size_t>(P.up.D));
-  P.cnt_dd.resize(static_cast<size_t>(P.dn.D));
   P.wpl.assign(static_cast<size_t>(P.up.D) * 4, 0u);
   for (int64_t r = 0; r < P.up.D; ++r) {
     const uint32_t u = P.up.masks[static_cast<size_t>(r)];
     int uu = 0;
     int cu[32] = {0};
-    for (const auto& pr : pairs) {
+    for (const auto& pr : P.pairs) {
       const int ui = (u >> pr.i) & 1u, uj = (u >> pr.j) & 1u;
       uu += ui * uj;
       cu[pr.i] += uj;
       cu[pr.j] += ui;
     }
     P.cnt_uu[static_cast<size_t>(r)] = uu;
-    for (int s = 0; s < n_sites; ++s) {
+    for (int s = 0; s < P.n; ++s) {
       if (cu[s] > 15) return "more than 15 nn pairs on one site are not supported";
       for (int b = 0; b < 4; ++b)
         if ((cu[s] >> b) & 1) P.wpl[static_cast<size_t>(r) * 4 + b] |= (1u << s);
     }
   }
-  for (int64_t r = 0; r < P.dn.D; ++r) {
-    const uint32_t d = P.dn.masks[static_cast<size_t>(r)];
-    int dd = 0;
-    for (const auto& pr : pairs) dd += static_cast<int>(((d >> pr.i) & 1u) * ((d >> pr.j) & 1u));
-    P.cnt_dd[static_cast<size_t>(r)] = dd;
-  }
-
   // Up part: for output up string u', hop f->t contributes from source u = u' ^ f ^ t when
   // u' has t and not f; the up-string factor (-1)^#up(lo,hi) is the same on u and u'.
   P.up_ptr.assign(static_cast<size_t>(P.up.D) + 1, 0);
@@ -617,6 +633,19 @@ std::string build_plan(int n_sites, int n_up, int n_dn, double U, double V, cons
   }
   P.mean_up_sources = P.up.D ? static_cast<double>(P.up_src.size()) / static_cast<double>(P.up.D) : 0.0;
   build_up_packed(&P);
+  return "";
+}
+
+std::string build_dn(SectorPlan* out) {
+  SectorPlan& P = *out;
+  P.dn.build(P.n, P.nd);
+  P.cnt_dd.resize(static_cast<size_t>(P.dn.D));
+  for (int64_t r = 0; r < P.dn.D; ++r) {
+    const uint32_t d = P.dn.masks[static_cast<size_t>(r)];
+    int dd = 0;
+    for (const auto& pr : P.pairs) dd += static_cast<int>(((d >> pr.i) & 1u) * ((d >> pr.j) & 1u));
+    P.cnt_dd[static_cast<size_t>(r)] = dd;
+  }
 
   // Down part: per output down string d', hop f->t contributes from d = d' ^ f ^ t; the
   // down-string factor (-1)^#dn(lo,hi) goes into the entry, the up-string factor per row.
@@ -678,6 +707,83 @@ std::string build_plan(int n_sites, int n_up, int n_dn, double U, double V, cons
   P.mean_dn_sources = P.dn.D ? static_cast<double>(total_src) / static_cast<double>(P.dn.D) : 0.0;
   build_gauge_table(P.dn, P.hd, P.n, &P.dn_g);
   return "";
+}
+
+void copy_up(const SectorPlan& A, SectorPlan* P) {
+  P->up = A.up;
+  P->cnt_uu = A.cnt_uu;
+  P->wpl = A.wpl;
+  P->up_ptr = A.up_ptr;
+  P->up_src = A.up_src;
+  P->up_coef = A.up_coef;
+  P->up_lohi = A.up_lohi;
+  P->up_pk_ok = A.up_pk_ok;
+  P->up_real2[0] = A.up_real2[0];
+  P->up_real2[1] = A.up_real2[1];
+  P->up_pc = A.up_pc;
+  P->up_ps = A.up_ps;
+  P->up_pk = A.up_pk;
+  P->mean_up_sources = A.mean_up_sources;
+  P->max_up_deg = A.max_up_deg;
+}
+
+void copy_dn(const SectorPlan& A, SectorPlan* P) {
+  P->dn = A.dn;
+  P->cnt_dd = A.cnt_dd;
+  P->dn_gptr = A.dn_gptr;
+  P->dn_ent = A.dn_ent;
+  P->dn_pad_hop = A.dn_pad_hop;
+  P->dn_csr_ptr = A.dn_csr_ptr;
+  P->dn_csr_ent = A.dn_csr_ent;
+  P->dn_coef = A.dn_coef;
+  P->dn_nmask = A.dn_nmask;
+  P->dn_g = A.dn_g;
+  P->mean_dn_sources = A.mean_dn_sources;
+  P->max_dn_deg = A.max_dn_deg;
+}
+
+}  // namespace
+
+std::string build_plan(int n_sites, int n_up, int n_dn, double U, double V, const std::vector<HopIn>& hops,
+                       const std::vector<PairIn>& pairs, SectorPlan* out, const SectorPlan* up_like,
+                       const SectorPlan* dn_like) {
+  init_binom();
+  if (n_sites <= 0 || n_sites > 32) return "FockBasis: require 1 <= n_sites <= 32 (bit packing)";
+  if (n_up < 0 || n_dn < 0 || n_up > n_sites || n_dn > n_sites) return "FockBasis: particle numbers out of range";
+  for (const auto& h : hops) {
+    if (h.from < 0 || h.to < 0 || h.from >= n_sites || h.to >= n_sites || (h.spin != 0 && h.spin != 1))
+      return "hopping out of range";
+    if (h.from == h.to) return "on-site hopping entries are not supported";
+  }
+  for (const auto& pr : pairs)
+    if (pr.i < 0 || pr.j < 0 || pr.i >= n_sites || pr.j >= n_sites) return "nn pair out of range";
+  const uint64_t Du = binom(n_sites, n_up), Dd = binom(n_sites, n_dn);
+  if (Du > (1u << 22) || Dd > (1u << 22)) return "spin space larger than 2^22 strings is not supported";
+  if (Du * Dd >= (1ull << 31)) return "sector dimension must fit the reference's int index (< 2^31)";
+
+  SectorPlan& P = *out;
+  P = SectorPlan{};
+  P.n = n_sites;
+  P.nu = n_up;
+  P.nd = n_dn;
+  P.U = U;
+  P.V = V;
+  P.pairs = pairs;
+  P.hu = merge_hops(hops, 0);
+  P.hd = merge_hops(hops, 1);
+  if (P.hd.size() + 1 > 256) return "more than 255 distinct down hoppings are not supported";
+  std::string err;
+  if (up_like)
+    copy_up(*up_like, &P);
+  else
+    err = build_up(&P);
+  if (!err.empty()) return err;
+  if (dn_like)
+    copy_dn(*dn_like, &P);
+  else
+    err = build_dn(&P);
+  P.dim = P.up.D * P.dn.D;
+  return err;
 }
 
 }  // namespace ftlm_b200

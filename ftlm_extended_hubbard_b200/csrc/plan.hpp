@@ -139,8 +139,11 @@ struct SectorPlan {
 
 // Builds the plan; returns "" on success or an error message (reference argument errors:
 // src/fock_basis.cpp:19-24).
+// up_like / dn_like (may be null): a plan of the same lattice, hops and pairs with the same N_up / N_down, whose tables
+// of that species are copied instead of built (a sweep's (n+1)^2 sectors have n+1 tables of each species).
 std::string build_plan(int n_sites, int n_up, int n_dn, double U, double V, const std::vector<HopIn>& hops,
-                       const std::vector<PairIn>& pairs, SectorPlan* out);
+                       const std::vector<PairIn>& pairs, SectorPlan* out, const SectorPlan* up_like = nullptr,
+                       const SectorPlan* dn_like = nullptr);
 
 // Diagonal entry from the plan tables (host).
 double plan_diag(const SectorPlan& p, int64_t ru, int64_t rd);

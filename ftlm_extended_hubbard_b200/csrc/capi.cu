@@ -25,6 +25,97 @@ int ftlm_b200::capi::fail(int code, const std::string& msg) {
 
 int ftlm_b200::set_error(int code, const char* msg) { return fail(code, msg); }
 
+namespace {
+
+struct PoolBlock {
+  void* p;
+  size_t bytes;
+};
+struct Pool {
+  std::mutex mu;
+  std::map<int, std::vector<PoolBlock>> free;  // by device
+  std::map<void*, int> device;                 // of every block taken or kept
+  size_t kept = 0;
+};
+Pool& pool() {
+  static Pool* p = new Pool;  // not destroyed: its blocks end with the context
+  return *p;
+}
+
+}  // namespace
+
+cudaError_t ftlm_b200::capi::pool_take(size_t bytes, void** p, size_t* got) {
+  *p = nullptr;
+  *got = 0;
+  bytes = std::max<size_t>(bytes, 256);
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  Pool& P = pool();
+  {
+    std::lock_guard<std::mutex> lock(P.mu);
+    auto& v = P.free[dev];
+    size_t best = v.size();
+    for (size_t i = 0; i < v.size(); ++i)  // the smallest that fits, unless most of it would lie idle
+      if (v[i].bytes >= bytes && v[i].bytes <= 8 * bytes + (size_t(1) << 20) && (best == v.size() || v[i].bytes < v[best].bytes))
+        best = i;
+    if (best < v.size()) {
+      *p = v[best].p;
+      *got = v[best].bytes;
+      P.kept -= v[best].bytes;
+      v[best] = v.back();
+      v.pop_back();
+      return cudaSuccess;
+    }
+  }
+  size_t want = bytes;  // rounded up to an eighth of its power of two, so that blocks fit each other's uses
+  size_t unit = 256;
+  while (unit * 16 < bytes) unit *= 2;
+  want = (bytes + unit - 1) / unit * unit;
+  e = cudaMalloc(p, want);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    pool_trim();
+    e = cudaMalloc(p, want);
+  }
+  if (e != cudaSuccess) return e;
+  *got = want;
+  std::lock_guard<std::mutex> lock(P.mu);
+  P.device[*p] = dev;
+  return cudaSuccess;
+}
+
+void ftlm_b200::capi::pool_give(void* p, size_t got) {
+  if (!p) return;
+  Pool& P = pool();
+  {
+    std::lock_guard<std::mutex> lock(P.mu);
+    auto it = P.device.find(p);
+    if (it != P.device.end() && P.kept + got <= kPoolKeep) {
+      P.free[it->second].push_back(PoolBlock{p, got});
+      P.kept += got;
+      return;
+    }
+    if (it != P.device.end()) P.device.erase(it);
+  }
+  cudaFree(p);
+}
+
+void ftlm_b200::capi::pool_trim() {
+  Pool& P = pool();
+  std::vector<PoolBlock> all;
+  {
+    std::lock_guard<std::mutex> lock(P.mu);
+    for (auto& d : P.free) {
+      all.insert(all.end(), d.second.begin(), d.second.end());
+      d.second.clear();
+    }
+    for (const PoolBlock& b : all) P.device.erase(b.p);
+    P.kept = 0;
+  }
+  for (const PoolBlock& b : all) cudaFree(b.p);
+}
+
 namespace ftlm_b200 {
 namespace capi {
 
@@ -56,6 +147,33 @@ void reference_start(int64_t dim, unsigned seed, std::vector<std::complex<double
 
 namespace {
 
+// A sector's tables in one block: laid out in a host image, copied at once.
+class TableArena {
+ public:
+  template <class T>
+  size_t add(const std::vector<T>& v) {
+    const size_t at = (image_.size() + 255) / 256 * 256, bytes = std::max<size_t>(v.size(), 1) * sizeof(T);
+    image_.resize(at + bytes);
+    if (!v.empty()) std::memcpy(image_.data() + at, v.data(), v.size() * sizeof(T));
+    return at;
+  }
+  cudaError_t upload(void** block, size_t* got) {
+    const cudaError_t e = pool_take(image_.size(), block, got);
+    if (e != cudaSuccess) return e;
+    base_ = static_cast<char*>(*block);
+    const cudaError_t c = cudaMemcpy(base_, image_.data(), image_.size(), cudaMemcpyHostToDevice);
+    return c == cudaSuccess ? cudaStreamSynchronize(cudaStreamLegacy) : c;  // other streams may read it now
+  }
+  template <class T>
+  const T* at(size_t off) const {
+    return reinterpret_cast<const T*>(base_ + off);
+  }
+
+ private:
+  std::vector<char> image_;
+  char* base_ = nullptr;
+};
+
 int upload_plan(ftlm_sector* s) {
   const SectorPlan& P = s->plan;
   DevSector& D = s->dev;
@@ -66,118 +184,69 @@ int upload_plan(ftlm_sector* s) {
   D.dim = P.dim;
   D.U = P.U;
   D.V = P.V;
-  std::vector<uint4> w4(static_cast<size_t>(P.up.D));
-  for (size_t i = 0; i < w4.size(); ++i) w4[i] = make_uint4(P.wpl[4 * i], P.wpl[4 * i + 1], P.wpl[4 * i + 2], P.wpl[4 * i + 3]);
-  std::vector<double2> upc(P.up_src.size()), dnc(P.dn_coef.size() / 2);
-  std::vector<float2> upc32(upc.size()), dnc32(dnc.size());
-  for (size_t i = 0; i < upc.size(); ++i) {
-    upc[i] = make_double2(P.up_coef[2 * i], P.up_coef[2 * i + 1]);
-    upc32[i] = make_float2(static_cast<float>(upc[i].x), static_cast<float>(upc[i].y));
+  std::vector<float2> upc32(P.up_src.size()), dnc32s(P.dn_coef.size());
+  for (size_t i = 0; i < upc32.size(); ++i)
+    upc32[i] = make_float2(static_cast<float>(P.up_coef[2 * i]), static_cast<float>(P.up_coef[2 * i + 1]));
+  for (size_t i = 0; i < dnc32s.size() / 2; ++i) {
+    const float x = static_cast<float>(P.dn_coef[2 * i]), y = static_cast<float>(P.dn_coef[2 * i + 1]);
+    dnc32s[2 * i] = make_float2(x, y);
+    dnc32s[2 * i + 1] = make_float2(-x, -y);
   }
-  for (size_t i = 0; i < dnc.size(); ++i) {
-    dnc[i] = make_double2(P.dn_coef[2 * i], P.dn_coef[2 * i + 1]);
-    dnc32[i] = make_float2(static_cast<float>(dnc[i].x), static_cast<float>(dnc[i].y));
+  TableArena A;
+  const size_t um = A.add(P.up.masks), dm = A.add(P.dn.masks), cuu = A.add(P.cnt_uu), cdd = A.add(P.cnt_dd);
+  const size_t wp = A.add(P.wpl), uptr = A.add(P.up_ptr), usrc = A.add(P.up_src), ucf = A.add(P.up_coef);
+  const size_t ulh = A.add(P.up_lohi), ucf32 = A.add(upc32), gptr = A.add(P.dn_gptr), dent = A.add(P.dn_ent);
+  const size_t cptr = A.add(P.dn_csr_ptr), cent = A.add(P.dn_csr_ent), dcf = A.add(P.dn_coef), dcf32s = A.add(dnc32s);
+  const size_t dnm = A.add(P.dn_nmask), fl = A.add(std::vector<int>(4, 0));
+  const GaugeTable& G = P.dn_g;
+  const size_t gent = G.ok ? A.add(G.ent) : 0, ggrp = G.ok ? A.add(G.grp) : 0, gperm = G.ok ? A.add(G.perm) : 0;
+  const size_t gtab = G.ok && !G.tab.empty() ? A.add(G.tab) : 0, upk = P.up_pk_ok ? A.add(P.up_pk) : 0;
+  CU_TRY(A.upload(&s->tables, &s->tables_bytes));
+  D.bt_cols = 1;  // 128-column slabs of the batched column pass (ftlm_gpu_batched_autotune times the others)
+  D.dn_g = DevGauge{};
+  D.dn_g.real2[0] = G.real2[0];
+  D.dn_g.real2[1] = G.real2[1];
+  if (G.ok) {
+    D.dn_g.ent = A.at<uint32_t>(gent);
+    D.dn_g.grp = A.at<int4>(ggrp);
+    D.dn_g.perm = A.at<uint8_t>(gperm);
+    D.dn_g.nt = static_cast<int>(G.tab.size() / 2);
+    D.dn_g.phase = G.phase ? 1 : 0;
+    D.dn_g.xor_real = G.xor_real ? 1 : 0;
+    D.dn_g.pc = G.pc;
+    D.dn_g.ps = G.ps;
+    if (D.dn_g.nt > 0) D.dn_g.tab = A.at<double2>(gtab);
   }
-  std::vector<float2> dnc32s(2 * dnc32.size());
-  for (size_t i = 0; i < dnc32.size(); ++i) {
-    dnc32s[2 * i] = dnc32[i];
-    dnc32s[2 * i + 1] = make_float2(-dnc32[i].x, -dnc32[i].y);
-  }
-  float2 *ucf32, *dcf32, *dcf32s;
-  CU_TRY(upload(upc32, &ucf32, &s->owned));
-  CU_TRY(upload(dnc32, &dcf32, &s->owned));
-  CU_TRY(upload(dnc32s, &dcf32s, &s->owned));
-  uint32_t *um, *dm, *ulh, *dent, *dnm;
-  int32_t *cuu, *cdd, *uptr, *usrc;
-  uint4* wp;
-  double2 *ucf, *dcf;
-  int64_t* gptr;
-  int64_t* cptr;
-  uint32_t* cent;
-  CU_TRY(upload(P.dn_csr_ptr, &cptr, &s->owned));
-  CU_TRY(upload(P.dn_csr_ent, &cent, &s->owned));
-  CU_TRY(upload(P.up.masks, &um, &s->owned));
-  CU_TRY(upload(P.dn.masks, &dm, &s->owned));
-  CU_TRY(upload(P.cnt_uu, &cuu, &s->owned));
-  CU_TRY(upload(P.cnt_dd, &cdd, &s->owned));
-  CU_TRY(upload(w4, &wp, &s->owned));
-  CU_TRY(upload(P.up_ptr, &uptr, &s->owned));
-  CU_TRY(upload(P.up_src, &usrc, &s->owned));
-  CU_TRY(upload(upc, &ucf, &s->owned));
-  CU_TRY(upload(P.up_lohi, &ulh, &s->owned));
-  CU_TRY(upload(P.dn_gptr, &gptr, &s->owned));
-  CU_TRY(upload(P.dn_ent, &dent, &s->owned));
-  CU_TRY(upload(dnc, &dcf, &s->owned));
-  CU_TRY(upload(P.dn_nmask, &dnm, &s->owned));
-  std::vector<int> flags(4, 0);
-  int* fl;
-  CU_TRY(upload(flags, &fl, &s->owned));
-  D.bt_cols = 1;  // 8-column chunks: the fastest at 4x4 (4,4), (6,6), (8,8) (ftlm_gpu_batched_autotune)
-  auto upload_gauge = [&](const GaugeTable& G, DevGauge* out) -> cudaError_t {
-    *out = DevGauge{};
-    out->real2[0] = G.real2[0];
-    out->real2[1] = G.real2[1];
-    if (!G.ok) return cudaSuccess;
-    uint32_t* ge;
-    int32_t* gg;
-    cudaError_t e = upload(G.ent, &ge, &s->owned);
-    if (e == cudaSuccess) e = upload(G.grp, &gg, &s->owned);
-    if (e != cudaSuccess) return e;
-    out->ent = ge;
-    out->grp = reinterpret_cast<const int4*>(gg);
-    uint8_t* gp;
-    if ((e = upload(G.perm, &gp, &s->owned)) != cudaSuccess) return e;
-    out->perm = gp;
-    out->nt = static_cast<int>(G.tab.size() / 2);
-    out->phase = G.phase ? 1 : 0;
-    out->xor_real = G.xor_real ? 1 : 0;
-    out->pc = G.pc;
-    out->ps = G.ps;
-    if (out->nt > 0) {
-      double* gt;
-      if ((e = upload(G.tab, &gt, &s->owned)) != cudaSuccess) return e;
-      out->tab = reinterpret_cast<const double2*>(gt);
-    }
-    return cudaSuccess;
-  };
-  CU_TRY(upload_gauge(P.dn_g, &D.dn_g));
-  D.up_pk = nullptr;
+  D.up_pk = P.up_pk_ok ? A.at<uint32_t>(upk) : nullptr;
   D.up_real2[0] = P.up_real2[0];
   D.up_real2[1] = P.up_real2[1];
   D.up_pc = P.up_pc;
   D.up_ps = P.up_ps;
-  if (P.up_pk_ok) {
-    uint32_t* upk;
-    CU_TRY(upload(P.up_pk, &upk, &s->owned));
-    D.up_pk = upk;
-  }
-  D.umask = um;
-  D.dmask = dm;
-  D.cnt_uu = cuu;
-  D.cnt_dd = cdd;
-  D.wpl = wp;
-  D.up_ptr = uptr;
-  D.up_src = usrc;
-  D.up_coef = ucf;
-  D.up_lohi = ulh;
-  D.dn_gptr = gptr;
-  D.dn_ent = dent;
-  D.dn_csr_ptr = cptr;
-  D.up_coef32 = ucf32;
-  D.dn_coef32 = dcf32;
-  D.dn_coef32s = dcf32s;
-  D.dn_csr_ent = cent;
-  D.dn_coef = dcf;
-  D.dn_nmask = dnm;
+  D.umask = A.at<uint32_t>(um);
+  D.dmask = A.at<uint32_t>(dm);
+  D.cnt_uu = A.at<int32_t>(cuu);
+  D.cnt_dd = A.at<int32_t>(cdd);
+  D.wpl = A.at<uint4>(wp);
+  D.up_ptr = A.at<int32_t>(uptr);
+  D.up_src = A.at<int32_t>(usrc);
+  D.up_coef = A.at<double2>(ucf);
+  D.up_lohi = A.at<uint32_t>(ulh);
+  D.dn_gptr = A.at<int64_t>(gptr);
+  D.dn_ent = A.at<uint32_t>(dent);
+  D.dn_csr_ptr = A.at<int64_t>(cptr);
+  D.up_coef32 = A.at<float2>(ucf32);
+  D.dn_coef32s = A.at<float2>(dcf32s);
+  D.dn_csr_ent = A.at<uint32_t>(cent);
+  D.dn_coef = A.at<double2>(dcf);
+  D.dn_nmask = A.at<uint32_t>(dnm);
   D.n_dn_hops = P.dn_pad_hop;
-  D.flags = fl;
-  CU_TRY(cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking));
+  D.flags = const_cast<int*>(A.at<int>(fl));
   s->on_device = true;
   return FTLM_OK;
 }
 
 int create_common(int n_sites, int n_up, int n_dn, double U, double V, const ftlm_hop* hops, int n_hops,
-                  const ftlm_pair* pairs, int n_pairs, bool device, ftlm_sector** out) {
+                  const ftlm_pair* pairs, int n_pairs, bool device, ftlm_sector** out, PlanParts* parts = nullptr) {
   if (!out) return fail(FTLM_ERR_INVALID, "null output handle");
   *out = nullptr;
   if (n_hops < 0 || n_pairs < 0 || (n_hops > 0 && !hops) || (n_pairs > 0 && !pairs))
@@ -190,7 +259,9 @@ int create_common(int n_sites, int n_up, int n_dn, double U, double V, const ftl
   if (!s) return fail(FTLM_ERR_NOMEM, "host allocation failed");
   std::string err;
   try {
-    err = build_plan(n_sites, n_up, n_dn, U, V, hv, pv, &s->plan);
+    err = build_plan(n_sites, n_up, n_dn, U, V, hv, pv, &s->plan, parts ? parts->find(parts->up, n_up) : nullptr,
+                     parts ? parts->find(parts->dn, n_dn) : nullptr);
+    if (parts && err.empty()) parts->keep(s->plan);
   } catch (const std::bad_alloc&) {
     delete s;
     return fail(FTLM_ERR_NOMEM, "host allocation failed while building the sector plan");
@@ -218,6 +289,25 @@ int ftlm_b200::capi::need_device(const ftlm_sector* s) {
   if (!s) return fail(FTLM_ERR_INVALID, "null sector");
   if (!s->on_device) return fail(FTLM_ERR_INVALID, "sector was created host-only");
   return FTLM_OK;
+}
+
+int ftlm_b200::capi::sector_create(const ftlm_params* p, int n_up, int n_dn, PlanParts* parts, ftlm_sector** out) {
+  if (!p) return fail(FTLM_ERR_INVALID, "null params");
+  if (p->Lx <= 0 || p->Ly <= 0) return fail(FTLM_ERR_INVALID, "Lx, Ly must be positive");
+  std::vector<HopIn> hv;
+  std::vector<PairIn> pv;
+  build_geometry(p->Lx, p->Ly, p->t, p->tp, p->phi_x, p->phi_y, &hv, &pv);
+  std::vector<ftlm_hop> h(hv.size());
+  for (size_t i = 0; i < hv.size(); ++i) h[i] = ftlm_hop{hv[i].from, hv[i].to, hv[i].spin, hv[i].cre, hv[i].cim};
+  std::vector<ftlm_pair> q(pv.size());
+  for (size_t i = 0; i < pv.size(); ++i) q[i] = ftlm_pair{pv[i].i, pv[i].j};
+  const int rc = create_common(p->Lx * p->Ly, n_up, n_dn, p->U, p->V, h.data(), static_cast<int>(h.size()), q.data(),
+                               static_cast<int>(q.size()), true, out, parts);
+  if (rc == FTLM_OK) {
+    (*out)->Lx = p->Lx;
+    (*out)->Ly = p->Ly;
+  }
+  return rc;
 }
 
 extern "C" {
@@ -263,22 +353,7 @@ int ftlm_gpu_sector_create_host(int n_sites, int n_up, int n_dn, double U, doubl
 }
 
 int ftlm_gpu_sector_create(const ftlm_params* p, int n_up, int n_dn, ftlm_sector** out) {
-  if (!p) return fail(FTLM_ERR_INVALID, "null params");
-  if (p->Lx <= 0 || p->Ly <= 0) return fail(FTLM_ERR_INVALID, "Lx, Ly must be positive");
-  std::vector<HopIn> hv;
-  std::vector<PairIn> pv;
-  build_geometry(p->Lx, p->Ly, p->t, p->tp, p->phi_x, p->phi_y, &hv, &pv);
-  std::vector<ftlm_hop> h(hv.size());
-  for (size_t i = 0; i < hv.size(); ++i) h[i] = ftlm_hop{hv[i].from, hv[i].to, hv[i].spin, hv[i].cre, hv[i].cim};
-  std::vector<ftlm_pair> q(pv.size());
-  for (size_t i = 0; i < pv.size(); ++i) q[i] = ftlm_pair{pv[i].i, pv[i].j};
-  const int rc = create_common(p->Lx * p->Ly, n_up, n_dn, p->U, p->V, h.data(), static_cast<int>(h.size()), q.data(),
-                               static_cast<int>(q.size()), true, out);
-  if (rc == FTLM_OK) {
-    (*out)->Lx = p->Lx;
-    (*out)->Ly = p->Ly;
-  }
-  return rc;
+  return sector_create(p, n_up, n_dn, nullptr, out);
 }
 
 int ftlm_gpu_sector_destroy(ftlm_sector* s) {
@@ -534,7 +609,20 @@ int ftlm_gpu_lanczos(ftlm_sector* s, int max_steps, unsigned seed, int start_mod
   int rc = need_device(s);
   if (rc) return rc;
   std::vector<double> a, b;
-  if (s->effective_path() >= 2)
+  if (s->apply_path == 0 && fused_alone(s->dev) && max_steps > 0) {
+    // few states: all steps in one kernel
+    ChainRun run;
+    rc = chains_run({s}, 1, max_steps, seed, start_mode, false, &run);
+    if (rc) return rc;
+    int n = 0;
+    CU_TRY(cudaMemcpy(&n, run.used, sizeof(int), cudaMemcpyDeviceToHost));
+    a.resize(static_cast<size_t>(max_steps));
+    b.resize(static_cast<size_t>(max_steps));
+    CU_TRY(cudaMemcpy(a.data(), run.alpha, a.size() * sizeof(double), cudaMemcpyDeviceToHost));
+    CU_TRY(cudaMemcpy(b.data(), run.beta, b.size() * sizeof(double), cudaMemcpyDeviceToHost));
+    a.resize(static_cast<size_t>(n));
+    b.resize(static_cast<size_t>(n > 0 && b[static_cast<size_t>(n) - 1] > 0.0 ? n : std::max(0, n - 1)));  // a chain that ended has no last beta
+  } else if (s->effective_path() >= 2)
     rc = run_lanczos_fused(s, max_steps, seed, start_mode, &a, &b);
   else
     rc = run_lanczos(
@@ -605,19 +693,18 @@ int ftlm_gpu_ftlm_combine(const double* logq, const double* energy_r, const int*
   if (R <= 0 || n_bt < 0 || !logq || !energy_r || !used || !lnz || !energy) return fail(FTLM_ERR_INVALID, "bad arguments");
   if (n_bt == 0) return FTLM_OK;
   const size_t qb = static_cast<size_t>(R) * n_bt * sizeof(double);
-  DevBuf dq, de, dn, dz, den;
-  CU_TRY(dq.alloc(qb));
-  CU_TRY(de.alloc(qb));
-  CU_TRY(dn.alloc(R * sizeof(int)));
-  CU_TRY(dz.alloc(n_bt * sizeof(double)));
-  CU_TRY(den.alloc(n_bt * sizeof(double)));
-  CU_TRY(cudaMemcpy(dq.p, logq, qb, cudaMemcpyHostToDevice));
-  CU_TRY(cudaMemcpy(de.p, energy_r, qb, cudaMemcpyHostToDevice));
-  CU_TRY(cudaMemcpy(dn.p, used, R * sizeof(int), cudaMemcpyHostToDevice));
-  CU_TRY(quad_sector(dq.as<double>(), de.as<double>(), dn.as<int>(), R, n_bt, log_dim, dz.as<double>(),
-                     den.as<double>(), nullptr));
-  CU_TRY(cudaMemcpy(lnz, dz.p, n_bt * sizeof(double), cudaMemcpyDeviceToHost));
-  CU_TRY(cudaMemcpy(energy, den.p, n_bt * sizeof(double), cudaMemcpyDeviceToHost));
+  Scratch mem;
+  const size_t o_dq = mem.add(qb), o_de = mem.add(qb), o_dn = mem.add(R * sizeof(int));
+  const size_t o_dz = mem.add(n_bt * sizeof(double)), o_den = mem.add(n_bt * sizeof(double));
+  CU_TRY(mem.commit());
+  CU_TRY(cudaMemcpy(mem.at<void>(o_dq), logq, qb, cudaMemcpyHostToDevice));
+  CU_TRY(cudaMemcpy(mem.at<void>(o_de), energy_r, qb, cudaMemcpyHostToDevice));
+  CU_TRY(cudaMemcpy(mem.at<void>(o_dn), used, R * sizeof(int), cudaMemcpyHostToDevice));
+  CU_TRY(quad_sector(mem.at<double>(o_dq), mem.at<double>(o_de), mem.at<int>(o_dn), R, n_bt, log_dim, mem.at<double>(o_dz),
+                     mem.at<double>(o_den), nullptr));
+  CU_TRY(cudaMemcpy(lnz, mem.at<void>(o_dz), n_bt * sizeof(double), cudaMemcpyDeviceToHost));
+  CU_TRY(cudaMemcpy(energy, mem.at<void>(o_den), n_bt * sizeof(double), cudaMemcpyDeviceToHost));
+  mem.idle();
   return FTLM_OK;
 }
 
@@ -629,19 +716,18 @@ int ftlm_gpu_tridiag_eig(const double* alpha, const double* beta, const int* n, 
     if (n[c] < 0 || n[c] > ld) return fail(FTLM_ERR_INVALID, "chain length outside [0, ld]");
   if (nc == 0) return FTLM_OK;
   const size_t mat = static_cast<size_t>(nc) * ld * sizeof(double);
-  DevBuf da, db, dn, dl, dw;
-  CU_TRY(da.alloc(mat));
-  CU_TRY(db.alloc(mat));
-  CU_TRY(dn.alloc(nc * sizeof(int)));
-  CU_TRY(dl.alloc(mat));
-  CU_TRY(dw.alloc(mat));
-  CU_TRY(cudaMemcpy(da.p, alpha, mat, cudaMemcpyHostToDevice));
-  CU_TRY(cudaMemcpy(db.p, beta, mat, cudaMemcpyHostToDevice));
-  CU_TRY(cudaMemcpy(dn.p, n, nc * sizeof(int), cudaMemcpyHostToDevice));
-  CU_TRY(quad_jacobi(da.as<double>(), db.as<double>(), dn.as<int>(), nc, ld, max_rot, tol, dl.as<double>(),
-                     dw.as<double>(), nullptr));
-  CU_TRY(cudaMemcpy(lam, dl.p, mat, cudaMemcpyDeviceToHost));
-  CU_TRY(cudaMemcpy(w0, dw.p, mat, cudaMemcpyDeviceToHost));
+  Scratch mem;
+  const size_t o_da = mem.add(mat), o_db = mem.add(mat), o_dn = mem.add(nc * sizeof(int)), o_dl = mem.add(mat);
+  const size_t o_dw = mem.add(mat);
+  CU_TRY(mem.commit());
+  CU_TRY(cudaMemcpy(mem.at<void>(o_da), alpha, mat, cudaMemcpyHostToDevice));
+  CU_TRY(cudaMemcpy(mem.at<void>(o_db), beta, mat, cudaMemcpyHostToDevice));
+  CU_TRY(cudaMemcpy(mem.at<void>(o_dn), n, nc * sizeof(int), cudaMemcpyHostToDevice));
+  CU_TRY(quad_jacobi(mem.at<double>(o_da), mem.at<double>(o_db), mem.at<int>(o_dn), nc, ld, max_rot, tol, mem.at<double>(o_dl),
+                     mem.at<double>(o_dw), nullptr));
+  CU_TRY(cudaMemcpy(lam, mem.at<void>(o_dl), mat, cudaMemcpyDeviceToHost));
+  CU_TRY(cudaMemcpy(w0, mem.at<void>(o_dw), mat, cudaMemcpyDeviceToHost));
+  mem.idle();
   return FTLM_OK;
 }
 
@@ -656,39 +742,37 @@ int ftlm_gpu_tridiag_quadrature(const double* alpha, const double* beta, const i
   if (nc == 0 || n_bt == 0) return FTLM_OK;
   const size_t mat = static_cast<size_t>(nc) * ld * sizeof(double);
   const size_t outb = static_cast<size_t>(nc) * n_bt * sizeof(double);
-  DevBuf da, db, dn, dl, dw, dbt, dq, de;
-  CU_TRY(da.alloc(mat));
-  CU_TRY(db.alloc(mat));
-  CU_TRY(dn.alloc(nc * sizeof(int)));
-  CU_TRY(dl.alloc(mat));
-  CU_TRY(dw.alloc(mat));
-  CU_TRY(dbt.alloc(n_bt * sizeof(double)));
-  CU_TRY(dq.alloc(outb));
-  CU_TRY(de.alloc(outb));
-  CU_TRY(cudaMemcpy(da.p, alpha, mat, cudaMemcpyHostToDevice));
-  CU_TRY(cudaMemcpy(db.p, beta, mat, cudaMemcpyHostToDevice));
-  CU_TRY(cudaMemcpy(dn.p, n, nc * sizeof(int), cudaMemcpyHostToDevice));
-  CU_TRY(cudaMemcpy(dbt.p, bts, n_bt * sizeof(double), cudaMemcpyHostToDevice));
-  CU_TRY(quad_jacobi(da.as<double>(), db.as<double>(), dn.as<int>(), nc, ld, 0, 1e-14, dl.as<double>(), dw.as<double>(),
+  Scratch mem;
+  const size_t o_da = mem.add(mat), o_db = mem.add(mat), o_dn = mem.add(nc * sizeof(int)), o_dl = mem.add(mat);
+  const size_t o_dw = mem.add(mat), o_dbt = mem.add(n_bt * sizeof(double)), o_dq = mem.add(outb);
+  const size_t o_de = mem.add(outb);
+  CU_TRY(mem.commit());
+  CU_TRY(cudaMemcpy(mem.at<void>(o_da), alpha, mat, cudaMemcpyHostToDevice));
+  CU_TRY(cudaMemcpy(mem.at<void>(o_db), beta, mat, cudaMemcpyHostToDevice));
+  CU_TRY(cudaMemcpy(mem.at<void>(o_dn), n, nc * sizeof(int), cudaMemcpyHostToDevice));
+  CU_TRY(cudaMemcpy(mem.at<void>(o_dbt), bts, n_bt * sizeof(double), cudaMemcpyHostToDevice));
+  CU_TRY(quad_jacobi(mem.at<double>(o_da), mem.at<double>(o_db), mem.at<int>(o_dn), nc, ld, 0, 1e-14, mem.at<double>(o_dl), mem.at<double>(o_dw),
                      nullptr));
-  CU_TRY(quad_eval(dl.as<double>(), dw.as<double>(), dn.as<int>(), nc, ld, dbt.as<double>(), n_bt, dq.as<double>(),
-                   de.as<double>(), nullptr));
-  CU_TRY(cudaMemcpy(logq, dq.p, outb, cudaMemcpyDeviceToHost));
-  CU_TRY(cudaMemcpy(energy, de.p, outb, cudaMemcpyDeviceToHost));
+  CU_TRY(quad_eval(mem.at<double>(o_dl), mem.at<double>(o_dw), mem.at<int>(o_dn), nc, ld, mem.at<double>(o_dbt), n_bt, mem.at<double>(o_dq),
+                   mem.at<double>(o_de), nullptr));
+  CU_TRY(cudaMemcpy(logq, mem.at<void>(o_dq), outb, cudaMemcpyDeviceToHost));
+  CU_TRY(cudaMemcpy(energy, mem.at<void>(o_de), outb, cudaMemcpyDeviceToHost));
+  mem.idle();
   return FTLM_OK;
 }
 
 int ftlm_gpu_ritz_values(const double* alpha, const double* beta, int n, int k, double* ritz) {
   if (n <= 0 || k <= 0 || !alpha || !ritz || (n > 1 && !beta)) return fail(FTLM_ERR_INVALID, "bad arguments");
   k = std::min(k, n);
-  DevBuf da, db, dr;
-  CU_TRY(da.alloc(n * sizeof(double)));
-  CU_TRY(db.alloc(n * sizeof(double)));
-  CU_TRY(dr.alloc(k * sizeof(double)));
-  CU_TRY(cudaMemcpy(da.p, alpha, n * sizeof(double), cudaMemcpyHostToDevice));
-  if (n > 1) CU_TRY(cudaMemcpy(db.p, beta, (n - 1) * sizeof(double), cudaMemcpyHostToDevice));
-  CU_TRY(ritz_bisect(da.as<double>(), db.as<double>(), n, k, dr.as<double>(), nullptr));
-  CU_TRY(cudaMemcpy(ritz, dr.p, k * sizeof(double), cudaMemcpyDeviceToHost));
+  Scratch mem;
+  const size_t o_da = mem.add(n * sizeof(double)), o_db = mem.add(n * sizeof(double));
+  const size_t o_dr = mem.add(k * sizeof(double));
+  CU_TRY(mem.commit());
+  CU_TRY(cudaMemcpy(mem.at<void>(o_da), alpha, n * sizeof(double), cudaMemcpyHostToDevice));
+  if (n > 1) CU_TRY(cudaMemcpy(mem.at<void>(o_db), beta, (n - 1) * sizeof(double), cudaMemcpyHostToDevice));
+  CU_TRY(ritz_bisect(mem.at<double>(o_da), mem.at<double>(o_db), n, k, mem.at<double>(o_dr), nullptr));
+  CU_TRY(cudaMemcpy(ritz, mem.at<void>(o_dr), k * sizeof(double), cudaMemcpyDeviceToHost));
+  mem.idle();
   return FTLM_OK;
 }
 
@@ -758,6 +842,8 @@ int plain_sector_ftlm(ftlm_sector* s, const double* bts, int n_bt, int R, int M,
     }
     return FTLM_OK;
   }
+  if (s->apply_path == 0 && fused_alone(s->dev))
+    return chains_ftlm({s}, R, M, seed, start_mode, false, bts, n_bt, converged, lnz, energy);
   std::vector<double> A(static_cast<size_t>(R) * M, 0.0), B(static_cast<size_t>(R) * M, 0.0);
   std::vector<int> nv(static_cast<size_t>(R), 0);
   for (int r = 0; r < R; ++r) {
@@ -771,19 +857,19 @@ int plain_sector_ftlm(ftlm_sector* s, const double* bts, int n_bt, int R, int M,
   std::vector<double> lq(static_cast<size_t>(R) * n_bt), eq(static_cast<size_t>(R) * n_bt);
   rc = chain_quadrature(A.data(), B.data(), nv.data(), R, M, bts, n_bt, lq.data(), eq.data(), converged);
   if (rc) return rc;
-  DevBuf dq, de, dn, dz, den;
-  CU_TRY(dq.alloc(lq.size() * sizeof(double)));
-  CU_TRY(de.alloc(eq.size() * sizeof(double)));
-  CU_TRY(dn.alloc(nv.size() * sizeof(int)));
-  CU_TRY(dz.alloc(n_bt * sizeof(double)));
-  CU_TRY(den.alloc(n_bt * sizeof(double)));
-  CU_TRY(cudaMemcpy(dq.p, lq.data(), lq.size() * sizeof(double), cudaMemcpyHostToDevice));
-  CU_TRY(cudaMemcpy(de.p, eq.data(), eq.size() * sizeof(double), cudaMemcpyHostToDevice));
-  CU_TRY(cudaMemcpy(dn.p, nv.data(), nv.size() * sizeof(int), cudaMemcpyHostToDevice));
-  CU_TRY(quad_sector(dq.as<double>(), de.as<double>(), dn.as<int>(), R, n_bt, std::log(static_cast<double>(dim)),
-                     dz.as<double>(), den.as<double>(), nullptr));
-  CU_TRY(cudaMemcpy(lnz, dz.p, n_bt * sizeof(double), cudaMemcpyDeviceToHost));
-  CU_TRY(cudaMemcpy(energy, den.p, n_bt * sizeof(double), cudaMemcpyDeviceToHost));
+  Scratch mem;
+  const size_t o_dq = mem.add(lq.size() * sizeof(double)), o_de = mem.add(eq.size() * sizeof(double));
+  const size_t o_dn = mem.add(nv.size() * sizeof(int)), o_dz = mem.add(n_bt * sizeof(double));
+  const size_t o_den = mem.add(n_bt * sizeof(double));
+  CU_TRY(mem.commit());
+  CU_TRY(cudaMemcpy(mem.at<void>(o_dq), lq.data(), lq.size() * sizeof(double), cudaMemcpyHostToDevice));
+  CU_TRY(cudaMemcpy(mem.at<void>(o_de), eq.data(), eq.size() * sizeof(double), cudaMemcpyHostToDevice));
+  CU_TRY(cudaMemcpy(mem.at<void>(o_dn), nv.data(), nv.size() * sizeof(int), cudaMemcpyHostToDevice));
+  CU_TRY(quad_sector(mem.at<double>(o_dq), mem.at<double>(o_de), mem.at<int>(o_dn), R, n_bt, std::log(static_cast<double>(dim)),
+                     mem.at<double>(o_dz), mem.at<double>(o_den), nullptr));
+  CU_TRY(cudaMemcpy(lnz, mem.at<void>(o_dz), n_bt * sizeof(double), cudaMemcpyDeviceToHost));
+  CU_TRY(cudaMemcpy(energy, mem.at<void>(o_den), n_bt * sizeof(double), cudaMemcpyDeviceToHost));
+  mem.idle();
   return FTLM_OK;
 }
 
@@ -807,27 +893,24 @@ int ftlm_gpu_gc_reduce(const double* lnz_s, const double* e_s, const int* N_s, i
   if (n_bt == 0 || n_mu == 0) return FTLM_OK;
   const size_t sb = static_cast<size_t>(std::max(n_sec, 1)) * n_bt * sizeof(double);
   const size_t gb = static_cast<size_t>(n_bt) * n_mu * sizeof(double);
-  DevBuf dl, de, dN, db, dm, o1, o2, o3;
-  CU_TRY(dl.alloc(sb));
-  CU_TRY(de.alloc(sb));
-  CU_TRY(dN.alloc(std::max(n_sec, 1) * sizeof(int)));
-  CU_TRY(db.alloc(n_bt * sizeof(double)));
-  CU_TRY(dm.alloc(n_mu * sizeof(double)));
-  CU_TRY(o1.alloc(gb));
-  CU_TRY(o2.alloc(gb));
-  CU_TRY(o3.alloc(gb));
+  Scratch mem;
+  const size_t o_dl = mem.add(sb), o_de = mem.add(sb), o_dN = mem.add(std::max(n_sec, 1) * sizeof(int));
+  const size_t o_db = mem.add(n_bt * sizeof(double)), o_dm = mem.add(n_mu * sizeof(double)), o_o1 = mem.add(gb);
+  const size_t o_o2 = mem.add(gb), o_o3 = mem.add(gb);
+  CU_TRY(mem.commit());
   if (n_sec > 0) {
-    CU_TRY(cudaMemcpy(dl.p, lnz_s, static_cast<size_t>(n_sec) * n_bt * sizeof(double), cudaMemcpyHostToDevice));
-    CU_TRY(cudaMemcpy(de.p, e_s, static_cast<size_t>(n_sec) * n_bt * sizeof(double), cudaMemcpyHostToDevice));
-    CU_TRY(cudaMemcpy(dN.p, N_s, n_sec * sizeof(int), cudaMemcpyHostToDevice));
+    CU_TRY(cudaMemcpy(mem.at<void>(o_dl), lnz_s, static_cast<size_t>(n_sec) * n_bt * sizeof(double), cudaMemcpyHostToDevice));
+    CU_TRY(cudaMemcpy(mem.at<void>(o_de), e_s, static_cast<size_t>(n_sec) * n_bt * sizeof(double), cudaMemcpyHostToDevice));
+    CU_TRY(cudaMemcpy(mem.at<void>(o_dN), N_s, n_sec * sizeof(int), cudaMemcpyHostToDevice));
   }
-  CU_TRY(cudaMemcpy(db.p, bts, n_bt * sizeof(double), cudaMemcpyHostToDevice));
-  CU_TRY(cudaMemcpy(dm.p, mus, n_mu * sizeof(double), cudaMemcpyHostToDevice));
-  CU_TRY(gc_reduce_dev(dl.as<double>(), de.as<double>(), dN.as<int>(), n_sec, db.as<double>(), n_bt, dm.as<double>(),
-                       n_mu, n_sites, o1.as<double>(), o2.as<double>(), o3.as<double>(), nullptr));
-  CU_TRY(cudaMemcpy(lnz_gc, o1.p, gb, cudaMemcpyDeviceToHost));
-  CU_TRY(cudaMemcpy(n_avg, o2.p, gb, cudaMemcpyDeviceToHost));
-  CU_TRY(cudaMemcpy(e_avg, o3.p, gb, cudaMemcpyDeviceToHost));
+  CU_TRY(cudaMemcpy(mem.at<void>(o_db), bts, n_bt * sizeof(double), cudaMemcpyHostToDevice));
+  CU_TRY(cudaMemcpy(mem.at<void>(o_dm), mus, n_mu * sizeof(double), cudaMemcpyHostToDevice));
+  CU_TRY(gc_reduce_dev(mem.at<double>(o_dl), mem.at<double>(o_de), mem.at<int>(o_dN), n_sec, mem.at<double>(o_db), n_bt, mem.at<double>(o_dm),
+                       n_mu, n_sites, mem.at<double>(o_o1), mem.at<double>(o_o2), mem.at<double>(o_o3), nullptr));
+  CU_TRY(cudaMemcpy(lnz_gc, mem.at<void>(o_o1), gb, cudaMemcpyDeviceToHost));
+  CU_TRY(cudaMemcpy(n_avg, mem.at<void>(o_o2), gb, cudaMemcpyDeviceToHost));
+  CU_TRY(cudaMemcpy(e_avg, mem.at<void>(o_o3), gb, cudaMemcpyDeviceToHost));
+  mem.idle();
   return FTLM_OK;
 }
 
@@ -836,7 +919,7 @@ int ftlm_gpu_gc_reduce(const double* lnz_s, const double* e_s, const int* N_s, i
 namespace ftlm_b200 {
 namespace capi {
 
-int64_t g_fused_max_dim = int64_t(1) << 17;
+int64_t g_fused_max_dim = kFusedSweepMax;
 
 int fused_sectors_ftlm(const std::vector<ftlm_sector*>& secs, const std::vector<int>& out_idx, int R, int M,
                        unsigned seed, int start_mode, bool c64, const double* bts, int n_bt, double* lnz_s, double* e_s,
@@ -862,14 +945,14 @@ extern "C" {
 int ftlm_gpu_lanczos_sectors(ftlm_sector* const* secs, int n_sectors, int R, int M, unsigned seed, int start_mode,
                              double* alpha, double* beta, int* used) {
   if (!secs || n_sectors < 0 || R <= 0 || M <= 0 || !alpha || !beta || !used) return fail(FTLM_ERR_INVALID, "bad arguments");
-  // Sectors far beyond the fused path's range run their chains one at a time.
+  // Sectors far beyond the fused path's range, or with rows too long for it, run their chains one at a time.
   constexpr int64_t kFusedMost = int64_t(1) << 22;
   std::vector<ftlm_sector*> v;
   std::vector<int> at;
   for (int i = 0; i < n_sectors; ++i) {
     int rc = need_device(secs[i]);
     if (rc) return rc;
-    if (secs[i]->plan.dim <= kFusedMost) {
+    if (secs[i]->plan.dim <= kFusedMost && chain_rows(secs[i]->dev, false, false) > 0) {
       v.push_back(secs[i]);
       at.push_back(i);
       continue;
@@ -891,9 +974,9 @@ int ftlm_gpu_lanczos_sectors(ftlm_sector* const* secs, int n_sectors, int R, int
   const size_t rows = static_cast<size_t>(R), tab = rows * M;
   for (size_t i = 0; i < v.size(); ++i) {
     const size_t o = static_cast<size_t>(at[i]) * rows;
-    CU_TRY(cudaMemcpy(alpha + o * M, run.alpha.as<double>() + i * tab, tab * sizeof(double), cudaMemcpyDeviceToHost));
-    CU_TRY(cudaMemcpy(beta + o * M, run.beta.as<double>() + i * tab, tab * sizeof(double), cudaMemcpyDeviceToHost));
-    CU_TRY(cudaMemcpy(used + o, run.used.as<int>() + i * rows, rows * sizeof(int), cudaMemcpyDeviceToHost));
+    CU_TRY(cudaMemcpy(alpha + o * M, run.alpha + i * tab, tab * sizeof(double), cudaMemcpyDeviceToHost));
+    CU_TRY(cudaMemcpy(beta + o * M, run.beta + i * tab, tab * sizeof(double), cudaMemcpyDeviceToHost));
+    CU_TRY(cudaMemcpy(used + o, run.used + i * rows, rows * sizeof(int), cudaMemcpyDeviceToHost));
   }
   return FTLM_OK;
 }
@@ -992,6 +1075,7 @@ int ftlm_gpu_gc_sweep(const ftlm_params* p, int R, int M, unsigned seed, int sta
   if (n <= 0 || n > 32) return fail(FTLM_ERR_INVALID, "FockBasis: require 1 <= n_sites <= 32 (bit packing)");
   const int nsec = (n + 1) * (n + 1);
   std::vector<int> N(static_cast<size_t>(nsec));
+  PlanParts parts(n);
   std::vector<ftlm_sector*> small;  // sectors for the fused small-sector launch
   std::vector<int> small_idx;
   auto clear_and = [](std::vector<ftlm_sector*>& v, int rc) {
@@ -1004,9 +1088,9 @@ int ftlm_gpu_gc_sweep(const ftlm_params* p, int R, int M, unsigned seed, int sta
       const int idx = nu * (n + 1) + nd;  // benchmarks/bench_ftlm_nmu_rect.cpp:62
       N[static_cast<size_t>(idx)] = nu + nd;
       ftlm_sector* s = nullptr;
-      int rc = ftlm_gpu_sector_create(p, nu, nd, &s);
+      int rc = sector_create(p, nu, nd, &parts, &s);
       if (rc) return clear_and(small, rc);
-      if (s->plan.dim >= 2 && s->plan.dim <= g_fused_max_dim && M <= 160) {  // fused below
+      if (s->plan.dim >= 2 && s->plan.dim <= g_fused_max_dim && M <= 160 && chain_rows(s->dev, false, false) > 0) {  // fused below
         small.push_back(s);
         small_idx.push_back(idx);
         continue;

@@ -178,6 +178,8 @@ int batched_sector(ftlm_sector* s, const double* bts, int n_bt, int R, int M, un
     return plain_sector_ftlm(s, bts, n_bt, R, M, seed, FTLM_START_PHILOX, true, lnz, energy);
   if (s->plan.max_up_deg > 120)
     return fail(FTLM_ERR_UNSUPPORTED, "batched path: more than 120 up-hop sources per string");
+  if (n_check <= 0 && fused_alone(s->dev))
+    return chains_ftlm({s}, R, M, seed, FTLM_START_PHILOX, true, bts, n_bt, true, lnz, energy);
   std::vector<double> A, B;
   std::vector<int> used;
   rc = bt_run_chains(s, R, M, seed, &A, &B, &used);
@@ -277,6 +279,7 @@ int batched_sweep(const ftlm_params* p, int R, int M, unsigned seed, const doubl
   std::vector<int> N(static_cast<size_t>(nsec));
   // small sectors go to fused launches: those the batched path runs in complex128 (dim <= 2M, Philox starts), and
   // those whose complex64 chains need no check against complex128
+  PlanParts parts(n);
   std::vector<ftlm_sector*> small, mid;
   std::vector<int> small_idx, mid_idx;
   auto clear_and = [&small, &mid](int rc) {
@@ -291,14 +294,15 @@ int batched_sweep(const ftlm_params* p, int R, int M, unsigned seed, const doubl
       const int idx = nu * (n + 1) + nd;
       N[static_cast<size_t>(idx)] = nu + nd;
       ftlm_sector* s = nullptr;
-      int rc = ftlm_gpu_sector_create(p, nu, nd, &s);
+      int rc = sector_create(p, nu, nd, &parts, &s);
       if (rc) return clear_and(rc);
-      if (s->plan.dim >= 2 && s->plan.dim <= 2 * static_cast<int64_t>(std::max(1, M)) && M <= 160) {
+      if (s->plan.dim >= 2 && s->plan.dim <= 2 * static_cast<int64_t>(std::max(1, M)) && M <= 160) {  // a row fits: <= 320
         small.push_back(s);
         small_idx.push_back(idx);
         continue;
       }
-      if (n_check <= 0 && M <= 160 && s->plan.dim >= 2 && s->plan.dim <= kFusedSweepMax && s->plan.max_up_deg <= 120) {
+      if (n_check <= 0 && M <= 160 && s->plan.dim >= 2 && s->plan.dim <= kFusedSweepMax && s->plan.max_up_deg <= 120 &&
+          chain_rows(s->dev, true, false) > 0) {
         mid.push_back(s);
         mid_idx.push_back(idx);
         continue;
@@ -329,6 +333,7 @@ int ftlm_gpu_batched_release(void) {
   std::lock_guard<std::mutex> lock(g_bt_mu);
   g_bt.release();
   g_grad.release();
+  pool_trim();
   return FTLM_OK;
 }
 

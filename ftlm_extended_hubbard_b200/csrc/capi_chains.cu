@@ -3,7 +3,6 @@
 #include <thread>
 
 #include "capi_internal.hpp"
-#include "chains.cuh"
 
 using namespace ftlm_b200;
 using namespace ftlm_b200::capi;
@@ -66,18 +65,21 @@ int chains_run(const std::vector<ftlm_sector*>& secs, int R, int M, unsigned see
     const DevSector& S = secs[static_cast<size_t>(i)]->dev;
     devs.push_back(S);
     max_dim = std::max(max_dim, S.dim);
-    const bool smem = chain_in_smem(S, c64, phase);
+    const int rows = chain_rows(S, c64, phase);
+    const bool smem = rows == static_cast<int>(S.Du);
+    if (rows == 0) return fail(FTLM_ERR_UNSUPPORTED, "fused chains: a row of the sector does not fit shared memory");
     for (int p = 0; p < planes; ++p) {
       ChainDesc d{};
       d.sector = i;
       d.out = i * R + per * p;
       d.chains = std::min(per, R - per * p);
       d.seed = seed + static_cast<unsigned>(per * p) * 100003u;
+      d.rows = rows;
       if (store_base) {
         d.store = (*store_base)[static_cast<size_t>(i)] + static_cast<int64_t>(p) * S.dim;
         d.store_step = static_cast<int64_t>(planes) * S.dim;
       }
-      items.push_back(Item{d, chain_class(S.dim), smem, S.dim, chain_elements(S) * 16 * (smem ? 3 : 4)});
+      items.push_back(Item{d, chain_class(S.dim), smem, S.dim, chain_elements(S) * 16 * 3});
     }
   }
   std::stable_sort(items.begin(), items.end(), [](const Item& a, const Item& b) {
@@ -87,26 +89,24 @@ int chains_run(const std::vector<ftlm_sector*>& secs, int R, int M, unsigned see
   });
   cudaStream_t st = secs[0]->stream;
   const size_t nc = static_cast<size_t>(ns) * R;
-  CU_TRY(run->alpha.alloc(nc * M * sizeof(double)));
-  CU_TRY(run->beta.alloc(nc * M * sizeof(double)));
-  CU_TRY(run->used.alloc(nc * sizeof(int)));
-  CU_TRY(cudaMemsetAsync(run->alpha.p, 0, nc * M * sizeof(double), st));
-  CU_TRY(cudaMemsetAsync(run->beta.p, 0, nc * M * sizeof(double), st));
+  const size_t o_a = run->mem.array<double>(nc * M), o_b = run->mem.array<double>(nc * M);
+  const size_t o_u = run->mem.array<int>(nc);
+  const size_t o_s = keep_scale ? run->mem.array<double>(nc * M) : 0;
+  CU_TRY(run->mem.commit());
+  run->alpha = run->mem.at<double>(o_a);
+  run->beta = run->mem.at<double>(o_b);
+  run->used = run->mem.at<int>(o_u);
+  CU_TRY(cudaMemsetAsync(run->alpha, 0, nc * M * sizeof(double), st));
+  CU_TRY(cudaMemsetAsync(run->beta, 0, nc * M * sizeof(double), st));
+  std::vector<double> ones;
   if (keep_scale) {
-    std::vector<double> one(nc * M, 1.0);
-    CU_TRY(run->scale.alloc(nc * M * sizeof(double)));
-    CU_TRY(cudaMemcpyAsync(run->scale.p, one.data(), nc * M * sizeof(double), cudaMemcpyHostToDevice, st));
-    CU_TRY(cudaStreamSynchronize(st));
+    ones.assign(nc * M, 1.0);
+    run->scale = run->mem.at<double>(o_s);
+    CU_TRY(cudaMemcpyAsync(run->scale, ones.data(), nc * M * sizeof(double), cudaMemcpyHostToDevice, st));
   }
-  DevBuf d_sec, d_desc, d_scr, d_init;
-  CU_TRY(d_sec.alloc(devs.size() * sizeof(DevSector)));
-  CU_TRY(cudaMemcpyAsync(d_sec.p, devs.data(), devs.size() * sizeof(DevSector), cudaMemcpyHostToDevice, st));
+  std::vector<std::complex<double>> host;
   if (start_mode == FTLM_START_REFERENCE) {
-    std::vector<std::complex<double>> host;
     reference_normals(max_dim, R, seed, &host);
-    CU_TRY(d_init.alloc(host.size() * sizeof(double2)));
-    CU_TRY(cudaMemcpyAsync(d_init.p, host.data(), host.size() * sizeof(double2), cudaMemcpyHostToDevice, st));
-    CU_TRY(cudaStreamSynchronize(st));
     for (auto& it : items) it.d.init = static_cast<int64_t>(it.d.out % R) * max_dim;
   }
   // The planes in pieces whose vectors fit a bounded scratch; the classes of a piece run side by side.
@@ -116,8 +116,14 @@ int chains_run(const std::vector<ftlm_sector*>& secs, int R, int M, unsigned see
     largest = std::max(largest, it.bytes);
     total += it.bytes;
   }
-  CU_TRY(d_scr.alloc(std::min(total, std::max(kScratch, largest))));
-  CU_TRY(d_desc.alloc(items.size() * sizeof(ChainDesc)));
+  Scratch mem;
+  const size_t o_sec = mem.array<DevSector>(devs.size()), o_desc = mem.array<ChainDesc>(items.size());
+  const size_t o_init = mem.array<double2>(host.size());
+  const size_t o_scr = mem.add(std::min(total, std::max(kScratch, largest)));
+  CU_TRY(mem.commit());
+  CU_TRY(cudaMemcpyAsync(mem.at<void>(o_sec), devs.data(), devs.size() * sizeof(DevSector), cudaMemcpyHostToDevice, st));
+  if (!host.empty())
+    CU_TRY(cudaMemcpyAsync(mem.at<void>(o_init), host.data(), host.size() * sizeof(double2), cudaMemcpyHostToDevice, st));
   std::vector<ChainDesc> descs(items.size());
   const size_t room = std::max(kScratch, largest);
   std::vector<size_t> piece{0};  // first items of the pieces
@@ -134,7 +140,7 @@ int chains_run(const std::vector<ftlm_sector*>& secs, int R, int M, unsigned see
     }
   }
   piece.push_back(items.size());
-  CU_TRY(cudaMemcpyAsync(d_desc.p, descs.data(), descs.size() * sizeof(ChainDesc), cudaMemcpyHostToDevice, st));
+  CU_TRY(cudaMemcpyAsync(mem.at<void>(o_desc), descs.data(), descs.size() * sizeof(ChainDesc), cudaMemcpyHostToDevice, st));
   cudaEvent_t ev[2] = {nullptr, nullptr};
   cudaError_t ce = cudaEventCreateWithFlags(&ev[0], cudaEventDisableTiming);
   if (ce == cudaSuccess) ce = cudaEventCreateWithFlags(&ev[1], cudaEventDisableTiming);
@@ -145,25 +151,25 @@ int chains_run(const std::vector<ftlm_sector*>& secs, int R, int M, unsigned see
       size_t j = i;
       size_t smem_bytes = 0;
       for (; j < piece[pc + 1] && items[j].size == items[i].size && items[j].smem == items[i].smem; ++j)
-        smem_bytes = std::max(smem_bytes, chain_smem_bytes(devs[static_cast<size_t>(items[j].d.sector)], c64, phase, items[j].smem));
+        smem_bytes = std::max(smem_bytes, chain_smem_bytes(devs[static_cast<size_t>(items[j].d.sector)], c64, phase, items[j].d.rows));
       cudaStream_t s2 = secs[static_cast<size_t>(std::min(stream, ns - 1))]->stream;
       ++stream;
       if (s2 != st) ce = cudaStreamWaitEvent(s2, ev[0], 0);
       ChainLaunch L{};
-      L.sectors = d_sec.as<DevSector>();
-      L.descs = d_desc.as<ChainDesc>() + i;
+      L.sectors = mem.at<DevSector>(o_sec);
+      L.descs = mem.at<ChainDesc>(o_desc) + i;
       L.blocks = static_cast<int>(j - i);
       L.size = items[i].size;
       L.smem = items[i].smem;
       L.phase = phase;
       L.smem_bytes = smem_bytes;
       L.M = M;
-      L.scratch = d_scr.p;
-      L.init = d_init.as<double2>();
-      L.alpha = run->alpha.as<double>();
-      L.beta = run->beta.as<double>();
-      L.used = run->used.as<int>();
-      L.scale = keep_scale ? run->scale.as<double>() : nullptr;
+      L.scratch = mem.at<void>(o_scr);
+      L.init = host.empty() ? nullptr : mem.at<double2>(o_init);
+      L.alpha = run->alpha;
+      L.beta = run->beta;
+      L.used = run->used;
+      L.scale = run->scale;
       L.store = store;
       if (ce == cudaSuccess) ce = chains_lanczos(L, c64, s2);
       if (s2 != st && ce == cudaSuccess) {
@@ -173,12 +179,13 @@ int chains_run(const std::vector<ftlm_sector*>& secs, int R, int M, unsigned see
       i = j;
     }
   }
-  const cudaError_t se = cudaStreamSynchronize(st);  // the scratch goes back to the device here
-  if (ce != cudaSuccess) cudaDeviceSynchronize();
+  const cudaError_t se = cudaStreamSynchronize(st);
   for (auto& e : ev)
     if (e) cudaEventDestroy(e);
   CU_TRY(ce);
   CU_TRY(se);
+  mem.idle();
+  run->mem.idle();
   return FTLM_OK;
 }
 
@@ -192,34 +199,36 @@ int chains_ftlm(const std::vector<ftlm_sector*>& secs, int R, int M, unsigned se
   int rc = chains_run(secs, R, M, seed, start_mode, c64, &run);
   if (rc) return rc;
   cudaStream_t st = secs[0]->stream;
-  const size_t outb = static_cast<size_t>(nc) * n_bt * sizeof(double), secb = static_cast<size_t>(ns) * n_bt * sizeof(double);
+  const size_t outb = static_cast<size_t>(nc) * n_bt * sizeof(double);
   std::vector<double> logd;
   for (const ftlm_sector* s : secs) logd.push_back(std::log(static_cast<double>(s->plan.dim)));
-  DevBuf lam, w, bt, lq, eq, info, ld, z, e;
-  CU_TRY(lam.alloc(static_cast<size_t>(nc) * M * sizeof(double)));
-  CU_TRY(w.alloc(static_cast<size_t>(nc) * M * sizeof(double)));
-  CU_TRY(bt.alloc(n_bt * sizeof(double)));
-  CU_TRY(lq.alloc(outb));
-  CU_TRY(eq.alloc(outb));
-  CU_TRY(info.alloc(nc * sizeof(int)));
-  CU_TRY(ld.alloc(logd.size() * sizeof(double)));
-  CU_TRY(z.alloc(secb));
-  CU_TRY(e.alloc(secb));
-  CU_TRY(cudaMemcpyAsync(bt.p, bts, n_bt * sizeof(double), cudaMemcpyHostToDevice, st));
-  CU_TRY(cudaMemcpyAsync(ld.p, logd.data(), logd.size() * sizeof(double), cudaMemcpyHostToDevice, st));
-  const double *al = run.alpha.as<double>(), *be = run.beta.as<double>();
-  const int* us = run.used.as<int>();
+  Scratch mem;
+  const size_t mat = static_cast<size_t>(nc) * M;
+  const size_t o_l = mem.array<double>(mat), o_w = mem.array<double>(mat), o_q = mem.add(outb), o_e = mem.add(outb);
+  const size_t o_i = mem.array<int>(nc), o_in = mem.array<double>(n_bt + logd.size());
+  const size_t o_out = mem.array<double>(2 * ns * n_bt);
+  CU_TRY(mem.commit());
+  std::vector<double> in(bts, bts + n_bt), out(2 * static_cast<size_t>(ns) * n_bt);
+  in.insert(in.end(), logd.begin(), logd.end());
+  CU_TRY(cudaMemcpyAsync(mem.at<void>(o_in), in.data(), in.size() * sizeof(double), cudaMemcpyHostToDevice, st));
+  const double *bt = mem.at<double>(o_in), *ld = bt + n_bt;
+  double *lam = mem.at<double>(o_l), *w = mem.at<double>(o_w), *lq = mem.at<double>(o_q), *eq = mem.at<double>(o_e);
+  double *z = mem.at<double>(o_out), *e = z + static_cast<size_t>(ns) * n_bt;
   if (converged)
-    CU_TRY(symeig_tridiag(al, be, us, nc, M, lam.as<double>(), w.as<double>(), nullptr, info.as<int>(), st));
+    CU_TRY(symeig_tridiag(run.alpha, run.beta, run.used, nc, M, lam, w, nullptr, mem.at<int>(o_i), st));
   else
-    CU_TRY(quad_jacobi(al, be, us, nc, M, 0, 1e-14, lam.as<double>(), w.as<double>(), st));
-  CU_TRY(quad_eval(lam.as<double>(), w.as<double>(), us, nc, M, bt.as<double>(), n_bt, lq.as<double>(), eq.as<double>(), st));
-  CU_TRY(quad_sectors(lq.as<double>(), eq.as<double>(), us, ns, R, n_bt, ld.as<double>(), z.as<double>(), e.as<double>(), st));
-  CU_TRY(cudaMemcpyAsync(lnz, z.p, secb, cudaMemcpyDeviceToHost, st));
-  CU_TRY(cudaMemcpyAsync(energy, e.p, secb, cudaMemcpyDeviceToHost, st));
+    CU_TRY(quad_jacobi(run.alpha, run.beta, run.used, nc, M, 0, 1e-14, lam, w, st));
+  run.mem.busy();
+  CU_TRY(quad_eval(lam, w, run.used, nc, M, bt, n_bt, lq, eq, st));
+  CU_TRY(quad_sectors(lq, eq, run.used, ns, R, n_bt, ld, z, e, st));
+  CU_TRY(cudaMemcpyAsync(out.data(), z, out.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
   std::vector<int> bad(static_cast<size_t>(nc), 0);
-  if (converged) CU_TRY(cudaMemcpyAsync(bad.data(), info.p, nc * sizeof(int), cudaMemcpyDeviceToHost, st));
+  if (converged) CU_TRY(cudaMemcpyAsync(bad.data(), mem.at<void>(o_i), nc * sizeof(int), cudaMemcpyDeviceToHost, st));
   CU_TRY(cudaStreamSynchronize(st));
+  mem.idle();
+  run.mem.idle();
+  std::copy(out.begin(), out.begin() + ns * n_bt, lnz);
+  std::copy(out.begin() + ns * n_bt, out.end(), energy);
   for (int b : bad)
     if (b == 1) return fail(FTLM_ERR_NUMERIC, "GPU eigen-solver did not converge");
   return FTLM_OK;

@@ -31,33 +31,28 @@ int fill_weights(ftlm_sector* s, int nc, int ld, double bT, const std::vector<in
     for (size_t i = 0; i < scale[static_cast<size_t>(c)].size() && i < static_cast<size_t>(ld); ++i)
       sc[static_cast<size_t>(c) * ld + i] = scale[static_cast<size_t>(c)][i];
   const size_t mat = static_cast<size_t>(nc) * ld * sizeof(double);
-  DevBuf da, db, dn, dsc, dl, dvt, dy, dg, dlm, di;
-  CU_TRY(da.alloc(mat));
-  CU_TRY(db.alloc(mat));
-  CU_TRY(dn.alloc(nc * sizeof(int)));
-  CU_TRY(dsc.alloc(mat));
-  CU_TRY(dl.alloc(mat));
-  CU_TRY(dvt.alloc(mat * ld));
-  CU_TRY(dy.alloc(mat * ld));
-  CU_TRY(dg.alloc(nc * sizeof(double)));
-  CU_TRY(dlm.alloc(nc * sizeof(double)));
-  CU_TRY(di.alloc(nc * sizeof(int)));
-  CU_TRY(cudaMemcpyAsync(da.p, A.data(), mat, cudaMemcpyHostToDevice, st));
-  CU_TRY(cudaMemcpyAsync(db.p, B.data(), mat, cudaMemcpyHostToDevice, st));
-  CU_TRY(cudaMemcpyAsync(dn.p, n.data(), nc * sizeof(int), cudaMemcpyHostToDevice, st));
-  CU_TRY(cudaMemcpyAsync(dsc.p, sc.data(), mat, cudaMemcpyHostToDevice, st));
-  CU_TRY(cudaMemsetAsync(dg.p, 0, nc * sizeof(double), st));
+  Scratch mem;
+  const size_t o_da = mem.add(mat), o_db = mem.add(mat), o_dn = mem.add(nc * sizeof(int)), o_dsc = mem.add(mat);
+  const size_t o_dl = mem.add(mat), o_dvt = mem.add(mat * ld), o_dy = mem.add(mat * ld);
+  const size_t o_dg = mem.add(nc * sizeof(double)), o_dlm = mem.add(nc * sizeof(double));
+  const size_t o_di = mem.add(nc * sizeof(int));
+  CU_TRY(mem.commit());
+  CU_TRY(cudaMemcpyAsync(mem.at<void>(o_da), A.data(), mat, cudaMemcpyHostToDevice, st));
+  CU_TRY(cudaMemcpyAsync(mem.at<void>(o_db), B.data(), mat, cudaMemcpyHostToDevice, st));
+  CU_TRY(cudaMemcpyAsync(mem.at<void>(o_dn), n.data(), nc * sizeof(int), cudaMemcpyHostToDevice, st));
+  CU_TRY(cudaMemcpyAsync(mem.at<void>(o_dsc), sc.data(), mat, cudaMemcpyHostToDevice, st));
+  CU_TRY(cudaMemsetAsync(mem.at<void>(o_dg), 0, nc * sizeof(double), st));
   CU_TRY(g_grad.grow(g_grad.Kp, g_grad.kcap, static_cast<size_t>(ld) * ld * nc * sizeof(double)));
   CU_TRY(cudaMemsetAsync(g_grad.Kp.p, 0, static_cast<size_t>(ld) * ld * nc * sizeof(double), st));
-  CU_TRY(symeig_tridiag(da.as<double>(), db.as<double>(), dn.as<int>(), nc, ld, dl.as<double>(), nullptr,
-                        dvt.as<double>(), di.as<int>(), st));
-  CU_TRY(duhamel_weights_dev(dl.as<double>(), dvt.as<double>(), dn.as<int>(), nc, ld, bT, dsc.as<double>(),
-                             dy.as<double>(), g_grad.Kp.as<double>(), dg.as<double>(), dlm.as<double>(), st));
+  CU_TRY(symeig_tridiag(mem.at<double>(o_da), mem.at<double>(o_db), mem.at<int>(o_dn), nc, ld, mem.at<double>(o_dl), nullptr,
+                        mem.at<double>(o_dvt), mem.at<int>(o_di), st));
+  CU_TRY(duhamel_weights_dev(mem.at<double>(o_dl), mem.at<double>(o_dvt), mem.at<int>(o_dn), nc, ld, bT, mem.at<double>(o_dsc),
+                             mem.at<double>(o_dy), g_grad.Kp.as<double>(), mem.at<double>(o_dg), mem.at<double>(o_dlm), st));
   std::vector<double> g(static_cast<size_t>(nc)), lm(static_cast<size_t>(nc));
   std::vector<int> info(static_cast<size_t>(nc));
-  CU_TRY(cudaMemcpyAsync(g.data(), dg.p, nc * sizeof(double), cudaMemcpyDeviceToHost, st));
-  CU_TRY(cudaMemcpyAsync(lm.data(), dlm.p, nc * sizeof(double), cudaMemcpyDeviceToHost, st));
-  CU_TRY(cudaMemcpyAsync(info.data(), di.p, nc * sizeof(int), cudaMemcpyDeviceToHost, st));
+  CU_TRY(cudaMemcpyAsync(g.data(), mem.at<void>(o_dg), nc * sizeof(double), cudaMemcpyDeviceToHost, st));
+  CU_TRY(cudaMemcpyAsync(lm.data(), mem.at<void>(o_dlm), nc * sizeof(double), cudaMemcpyDeviceToHost, st));
+  CU_TRY(cudaMemcpyAsync(info.data(), mem.at<void>(o_di), nc * sizeof(int), cudaMemcpyDeviceToHost, st));
   CU_TRY(cudaStreamSynchronize(st));
   for (int c = 0; c < nc; ++c) {
     ChainGrad& cg = (*out)[static_cast<size_t>(c)];
@@ -68,6 +63,7 @@ int fill_weights(ftlm_sector* s, int nc, int ld, double bT, const std::vector<in
     cg.g = g[static_cast<size_t>(c)];
     cg.lmin = lm[static_cast<size_t>(c)];
   }
+  mem.idle();
   return FTLM_OK;
 }
 
@@ -281,7 +277,7 @@ int ftlm_gpu_grad_sector(ftlm_sector* s, ftlm_sector* op_tp, double bT, int R, i
 namespace {
 
 constexpr double kGcWeightCutoff = 1e-13;
-constexpr long long kGcFusedPlainMax = 1LL << 17;
+constexpr long long kGcFusedPlainMax = kFusedSweepMax;
 
 struct SectorDeleter {
   void operator()(ftlm_sector* s) const { ftlm_gpu_sector_destroy(s); }
@@ -329,6 +325,7 @@ int ftlm_gpu_gc_logz(const ftlm_params* p, double mu, double bT, int R, int M, u
   const int nsec = (n + 1) * (n + 1);
   const int st_mode = method == 1 ? FTLM_START_PHILOX : start_mode;
   const long long limit = method == 1 ? 2LL * M : kGcFusedPlainMax;
+  PlanParts parts(n);
   std::vector<SectorPtr> small, mid;  // chains in fused launches below: complex128 and complex64
   std::vector<int> small_idx, mid_idx;
   std::vector<double> A, B;
@@ -337,16 +334,16 @@ int ftlm_gpu_gc_logz(const ftlm_params* p, double mu, double bT, int R, int M, u
     for (int nd = 0; nd <= n; ++nd) {
       const int idx = nu * (n + 1) + nd;
       ftlm_sector* raw = nullptr;
-      rc = ftlm_gpu_sector_create(p, nu, nd, &raw);
+      rc = sector_create(p, nu, nd, &parts, &raw);
       if (rc) return rc;
       SectorPtr s(raw);
       const int64_t dim = s->plan.dim;
-      if (dim <= limit) {
+      if (dim <= limit && chain_rows(s->dev, false, false) > 0) {
         small.push_back(std::move(s));
         small_idx.push_back(idx);
         continue;
       }
-      if (method == 1 && dim <= kFusedSweepMax && s->plan.max_up_deg <= 120) {
+      if (method == 1 && dim <= kFusedSweepMax && s->plan.max_up_deg <= 120 && chain_rows(s->dev, true, false) > 0) {
         mid.push_back(std::move(s));
         mid_idx.push_back(idx);
         continue;
@@ -413,6 +410,7 @@ int ftlm_gpu_gc_logz_grad(const ftlm_params* p, double mu, double bT, int R, int
   pop.tp = 1.0;
   pop.U = 0.0;
   pop.V = 0.0;
+  PlanParts parts(n), op_parts(n);
   for (int nu = 0; nu <= n; ++nu)
     for (int nd = 0; nd <= n; ++nd) {
       const size_t idx = static_cast<size_t>(nu * (n + 1) + nd);
@@ -422,10 +420,10 @@ int ftlm_gpu_gc_logz_grad(const ftlm_params* p, double mu, double bT, int R, int
       dbeta += w * (mu * N[idx] - e_s[idx]);
       if (!(w >= kGcWeightCutoff)) continue;
       ftlm_sector *rs = nullptr, *ro = nullptr;
-      rc = ftlm_gpu_sector_create(p, nu, nd, &rs);
+      rc = sector_create(p, nu, nd, &parts, &rs);
       if (rc) return rc;
       SectorPtr s(rs);
-      rc = ftlm_gpu_sector_create(&pop, nu, nd, &ro);
+      rc = sector_create(&pop, nu, nd, &op_parts, &ro);
       if (rc) return rc;
       SectorPtr op(ro);
       double lz = 0.0, g[3] = {0.0, 0.0, 0.0};
@@ -458,30 +456,26 @@ int ftlm_gpu_tridiag_quadrature_exact(const double* alpha, const double* beta, c
   if (nc == 0 || n_bt == 0) return FTLM_OK;
   const size_t mat = static_cast<size_t>(nc) * ld * sizeof(double);
   const size_t outb = static_cast<size_t>(nc) * n_bt * sizeof(double);
-  DevBuf da, db, dn, dl, dw, dbt, dq, de, di;
-  CU_TRY(da.alloc(mat));
-  CU_TRY(db.alloc(mat));
-  CU_TRY(dn.alloc(nc * sizeof(int)));
-  CU_TRY(dl.alloc(mat));
-  CU_TRY(dw.alloc(mat));
-  CU_TRY(dbt.alloc(n_bt * sizeof(double)));
-  CU_TRY(dq.alloc(outb));
-  CU_TRY(de.alloc(outb));
-  CU_TRY(di.alloc(nc * sizeof(int)));
-  CU_TRY(cudaMemcpy(da.p, alpha, mat, cudaMemcpyHostToDevice));
-  CU_TRY(cudaMemcpy(db.p, beta, mat, cudaMemcpyHostToDevice));
-  CU_TRY(cudaMemcpy(dn.p, n, nc * sizeof(int), cudaMemcpyHostToDevice));
-  CU_TRY(cudaMemcpy(dbt.p, bts, n_bt * sizeof(double), cudaMemcpyHostToDevice));
-  CU_TRY(symeig_tridiag(da.as<double>(), db.as<double>(), dn.as<int>(), nc, ld, dl.as<double>(), dw.as<double>(),
-                        nullptr, di.as<int>(), nullptr));
-  CU_TRY(quad_eval(dl.as<double>(), dw.as<double>(), dn.as<int>(), nc, ld, dbt.as<double>(), n_bt, dq.as<double>(),
-                   de.as<double>(), nullptr));
+  Scratch mem;
+  const size_t o_da = mem.add(mat), o_db = mem.add(mat), o_dn = mem.add(nc * sizeof(int)), o_dl = mem.add(mat);
+  const size_t o_dw = mem.add(mat), o_dbt = mem.add(n_bt * sizeof(double)), o_dq = mem.add(outb);
+  const size_t o_de = mem.add(outb), o_di = mem.add(nc * sizeof(int));
+  CU_TRY(mem.commit());
+  CU_TRY(cudaMemcpy(mem.at<void>(o_da), alpha, mat, cudaMemcpyHostToDevice));
+  CU_TRY(cudaMemcpy(mem.at<void>(o_db), beta, mat, cudaMemcpyHostToDevice));
+  CU_TRY(cudaMemcpy(mem.at<void>(o_dn), n, nc * sizeof(int), cudaMemcpyHostToDevice));
+  CU_TRY(cudaMemcpy(mem.at<void>(o_dbt), bts, n_bt * sizeof(double), cudaMemcpyHostToDevice));
+  CU_TRY(symeig_tridiag(mem.at<double>(o_da), mem.at<double>(o_db), mem.at<int>(o_dn), nc, ld, mem.at<double>(o_dl), mem.at<double>(o_dw),
+                        nullptr, mem.at<int>(o_di), nullptr));
+  CU_TRY(quad_eval(mem.at<double>(o_dl), mem.at<double>(o_dw), mem.at<int>(o_dn), nc, ld, mem.at<double>(o_dbt), n_bt, mem.at<double>(o_dq),
+                   mem.at<double>(o_de), nullptr));
   std::vector<int> info(static_cast<size_t>(nc));
-  CU_TRY(cudaMemcpy(info.data(), di.p, nc * sizeof(int), cudaMemcpyDeviceToHost));
+  CU_TRY(cudaMemcpy(info.data(), mem.at<void>(o_di), nc * sizeof(int), cudaMemcpyDeviceToHost));
   for (int c = 0; c < nc; ++c)
     if (n[c] > 0 && info[static_cast<size_t>(c)] != 0) return fail(FTLM_ERR_NUMERIC, "GPU eigen-solver did not converge");
-  CU_TRY(cudaMemcpy(logq, dq.p, outb, cudaMemcpyDeviceToHost));
-  CU_TRY(cudaMemcpy(energy, de.p, outb, cudaMemcpyDeviceToHost));
+  CU_TRY(cudaMemcpy(logq, mem.at<void>(o_dq), outb, cudaMemcpyDeviceToHost));
+  CU_TRY(cudaMemcpy(energy, mem.at<void>(o_de), outb, cudaMemcpyDeviceToHost));
+  mem.idle();
   return FTLM_OK;
 }
 

@@ -17,6 +17,7 @@
 
 #include "../../include/ftlm_gpu.h"
 #include "batched.cuh"
+#include "chains.cuh"
 #include "grad.cuh"
 #include "hv.cuh"
 #include "orbit.cuh"
@@ -39,18 +40,49 @@ int fail(int code, const std::string& msg);
                   std::string(#expr) + ": " + cudaGetErrorString(e_));                                   \
   } while (0)
 
-template <class T>
-cudaError_t upload(const std::vector<T>& v, T** out, std::vector<void*>* owned) {
-  *out = nullptr;
-  const size_t bytes = std::max<size_t>(v.size(), 1) * sizeof(T);
-  void* p = nullptr;
-  cudaError_t e = cudaMalloc(&p, bytes);
-  if (e != cudaSuccess) return e;
-  owned->push_back(p);
-  if (!v.empty()) e = cudaMemcpy(p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice);
-  *out = static_cast<T*>(p);
-  return e;
-}
+// Device blocks kept between calls, for workspaces and tables that live for one call or one small sector: cudaMalloc and
+// cudaFree cost tens of microseconds to milliseconds each, more than many of the calls.  Per device, at most kPoolKeep
+// bytes stay here (given back by ftlm_gpu_batched_release, or when device memory runs out); thread-safe.  A block is
+// given only when no work on it is in flight.
+constexpr size_t kPoolKeep = size_t(1) << 30;
+cudaError_t pool_take(size_t bytes, void** p, size_t* got);
+void pool_give(void* p, size_t got);
+void pool_trim();
+
+// One block of the pool, laid out by add() and obtained by commit().  idle() says that the work on it has ended; without
+// it (an error on the way) the block is given back after the device has.
+class Scratch {
+ public:
+  Scratch() = default;
+  Scratch(const Scratch&) = delete;
+  Scratch& operator=(const Scratch&) = delete;
+  ~Scratch() {
+    if (!p_) return;
+    if (busy_) cudaDeviceSynchronize();
+    pool_give(p_, got_);
+  }
+  size_t add(size_t bytes) {
+    const size_t at = size_;
+    size_ += (std::max<size_t>(bytes, 1) + 255) / 256 * 256;
+    return at;
+  }
+  template <class T>
+  size_t array(size_t n) {
+    return add(n * sizeof(T));
+  }
+  cudaError_t commit() { return pool_take(size_, &p_, &got_); }
+  template <class T>
+  T* at(size_t off) const {
+    return reinterpret_cast<T*>(static_cast<char*>(p_) + off);
+  }
+  void idle() { busy_ = false; }
+  void busy() { busy_ = true; }
+
+ private:
+  void* p_ = nullptr;
+  size_t size_ = 0, got_ = 0;
+  bool busy_ = true;
+};
 
 // Device buffer that frees itself.
 struct DevBuf {
@@ -64,11 +96,52 @@ struct DevBuf {
   cudaError_t alloc(size_t bytes) {
     if (p) cudaFree(p);
     p = nullptr;
-    return cudaMalloc(&p, std::max<size_t>(bytes, 16));
+    cudaError_t e = cudaMalloc(&p, std::max<size_t>(bytes, 16));
+    if (e == cudaErrorMemoryAllocation) {
+      cudaGetLastError();
+      pool_trim();
+      e = cudaMalloc(&p, std::max<size_t>(bytes, 16));
+    }
+    return e;
   }
   template <class T>
   T* as() const {
     return static_cast<T*>(p);
+  }
+};
+
+// A non-blocking stream, created when it is first asked for: a sweep's sectors mostly share one launch and need none.
+class LazyStream {
+ public:
+  LazyStream() = default;
+  LazyStream(const LazyStream&) = delete;
+  LazyStream& operator=(const LazyStream&) = delete;
+  ~LazyStream() {
+    if (s_) cudaStreamDestroy(s_);
+  }
+  operator cudaStream_t() {  // the legacy default stream where none can be created
+    if (!s_ && cudaStreamCreateWithFlags(&s_, cudaStreamNonBlocking) != cudaSuccess) s_ = nullptr;
+    return s_;
+  }
+
+ private:
+  cudaStream_t s_ = nullptr;
+};
+
+// Plans of a sweep's sectors by N_up and by N_down, whose tables of that species the other sectors copy (build_plan).
+struct PlanParts {
+  explicit PlanParts(int n) : up(static_cast<size_t>(n) + 1), dn(static_cast<size_t>(n) + 1) {}
+  std::vector<std::shared_ptr<const SectorPlan>> up, dn;
+  static const SectorPlan* find(const std::vector<std::shared_ptr<const SectorPlan>>& v, int k) {
+    return k >= 0 && k < static_cast<int>(v.size()) ? v[static_cast<size_t>(k)].get() : nullptr;
+  }
+  void keep(const SectorPlan& P) {
+    auto& u = up[static_cast<size_t>(P.nu)];
+    auto& d = dn[static_cast<size_t>(P.nd)];
+    if (u && d) return;
+    auto copy = std::make_shared<const SectorPlan>(P);
+    if (!u) u = copy;
+    if (!d) d = copy;
   }
 };
 
@@ -160,15 +233,17 @@ struct ftlm_sector {
   bool on_device = false;
   int device = -1;
   ftlm_b200::DevSector dev{};
-  std::vector<void*> owned;
+  void* tables = nullptr;  // one block of the pool
+  size_t tables_bytes = 0;
   int apply_path = 0;    // 0 auto, 1 generic, 2 rows+cols, 3 rows (register coefficient classes)+cols
   int cols_variant = 0;  // column slab 256/128/512 (0/1/2); 3/4/5: the same over the packed up list (path 3)
   ftlm_b200::capi::LanczosWs ws;
   ftlm_b200::capi::DevBuf hx, hy;  // staging for the host-buffer apply
-  cudaStream_t stream = nullptr;
+  ftlm_b200::capi::LazyStream stream;
   ~ftlm_sector() {
-    for (void* p : owned) cudaFree(p);
-    if (stream) cudaStreamDestroy(stream);
+    if (!tables) return;
+    cudaDeviceSynchronize();  // as a free would: a caller's H v may still read the tables
+    ftlm_b200::capi::pool_give(tables, tables_bytes);
   }
   // Kernel choice for H·v: 1 = generic gather; 2 = row pass with the per-row coefficient table +
   // column-slab pass over the CSR up list; 3 = row pass in the gauge basis (register-held real
@@ -207,6 +282,8 @@ namespace ftlm_b200 {
 namespace capi {
 
 int need_device(const ftlm_sector* s);
+// ftlm_gpu_sector_create, with the tables that a sweep's sectors share (parts may be null).
+int sector_create(const ftlm_params* p, int n_up, int n_dn, PlanParts* parts, ftlm_sector** out);
 
 // ---- batched complex64 path (capi_batched.cu) ------------------------------------------------
 struct BtWs {
@@ -346,7 +423,9 @@ int plain_sector_ftlm(ftlm_sector* s, const double* bts, int n_bt, int R, int M,
 // The fused chains of many sectors (capi_chains.cu), results on the device: rows [sector][chain] of alpha/beta [M]
 // (zero-padded), steps used and, with keep_scale, the norms of the stored vectors.
 struct ChainRun {
-  DevBuf alpha, beta, used, scale;
+  Scratch mem;
+  double *alpha = nullptr, *beta = nullptr, *scale = nullptr;
+  int* used = nullptr;
 };
 // c64: complex64 chains (Philox starts), else complex128.  store: the chains' vectors W_k go to store + store_base[i] +
 // (k * planes + p) * dim for plane p (two chains of complex64, one of complex128) of sector i.
@@ -361,8 +440,15 @@ int fused_sectors_ftlm(const std::vector<ftlm_sector*>& secs, const std::vector<
                        unsigned seed, int start_mode, bool c64, const double* bts, int n_bt, double* lnz_s, double* e_s,
                        bool converged);
 
-// Largest sector of a batched sweep that joins the fused launch (beyond it a sector fills the GPU by itself).
-constexpr int64_t kFusedSweepMax = 1 << 15;
+// Whether a single sector's own chains run fused, by the lanes that a step of its block has to go through: a step takes
+// about 20 us at 8192 lanes, what the kernels of a step on the whole GPU take for their launches alone (3x3 (5,4), 15,876
+// states, one chain: 180 us a step fused).
+inline bool fused_alone(const DevSector& S) {  // and a row of it fits (chain_rows)
+  const int64_t lanes = S.Dd <= 16 ? S.Du / (32 / S.Dd) * 32 : S.Du * ((S.Dd + 31) / 32 * 32);
+  return lanes <= 8192 && chain_rows(S, false, false) > 0;
+}
+// Largest sector that joins the fused launch of a sweep; a larger one fills the GPU by itself.
+constexpr int64_t kFusedSweepMax = 1 << 14;
 
 // The complex64 chains of one sector in groups of planes (planes.cu), alpha/beta [R][M] (beta zero-padded), used [R].
 int bt_run_chains(ftlm_sector* s, int R, int M, unsigned seed, std::vector<double>* A, std::vector<double>* B,

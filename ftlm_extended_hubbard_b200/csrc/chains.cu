@@ -3,7 +3,9 @@
 // One block per plane (chains.cuh) runs all M steps: a warp takes 32 output strings of one row, a lane one state, with
 // the row pass's gauge-table walk for the down hops and the row's source list (the same for the whole warp) for the up
 // hops; then the dot products, the update and the norm over the block's own vectors.  The vector that the hops gather
-// from is staged in shared memory where it fits (14,336 states with their padding), else in the block's scratch.
+// from is staged in shared memory where it fits (14,336 states with their padding); else the rows are, a block of rows at
+// a time, and the up hops read the block's scratch (32 lanes that gather at random within a row from global memory touch
+// a line each: 3x3 (4,4), 15,876 states, took 142 us a step that way).
 // Rows have a pitch of Dd + 8 elements whose last 8 stay zero: the target of the table's padding entries, and harmless
 // to the flat elementwise passes.  Bound by the latency of the gathers and of four block reductions a step; it exists
 // because a step of a small sector otherwise costs five kernel launches, whatever its size: 3x3
@@ -79,7 +81,7 @@ __global__ void __launch_bounds__(1024, 1) chains_kernel(const DevSector* __rest
   typename P::Cf* tab = reinterpret_cast<typename P::Cf*>(smem_raw);
   const DevGauge G = S.dn_g;
   const size_t tab_bytes = kPhase ? 0 : (G.ent ? static_cast<size_t>(G.nt) * 8 * sizeof(typename P::Cf) : 0);
-  T* xs = kSmem ? reinterpret_cast<T*>(smem_raw + ((tab_bytes + 15) & ~size_t(15))) : wkm1 + V;
+  T* xs = reinterpret_cast<T*>(smem_raw + ((tab_bytes + 15) & ~size_t(15)));
   const RowCoefs<P> rc(G);
   if (!kPhase && G.ent)
     for (int i = tid; i < G.nt * 8; i += nt) tab[i] = P::coef(G.tab[i >> 3]);
@@ -88,7 +90,6 @@ __global__ void __launch_bounds__(1024, 1) chains_kernel(const DevSector* __rest
   for (int i = tid; i < Du * 8; i += nt) {
     const int o = (i >> 3) * pitch + Dd + (i & 7);
     wk[o] = y[o] = wkm1[o] = P::zero();
-    xs[o] = P::zero();
   }
   // start vector: Philox (chain q: key seed + q * 100003) or the caller's, in the gauge basis
   double n0[P::kC] = {};
@@ -117,13 +118,10 @@ __global__ void __launch_bounds__(1024, 1) chains_kernel(const DevSector* __rest
     steps[q] = 0;
     if (scale && tid == 0 && q < cd.chains) scale[static_cast<int64_t>(cd.out + q) * M] = active[q] ? n : 1.0;
   }
-  const int ng = (Dd + 31) >> 5, items = Du * ng;
+  // A warp's item is 32 strings of one row, or 32 / Dd whole rows where they are short.
+  const int rpw = Dd <= 16 ? 32 / Dd : 1, ng = (Dd + 31) >> 5;
+  const int sub = rpw > 1 ? lane / Dd : 0, pos0 = rpw > 1 ? lane - sub * Dd : lane;
   for (int k = 0; k < M; ++k) {
-    for (int i = tid; i < V; i += nt) {
-      T v = wk[i];
-      if (P::kScaled) v = P::times(s_in[0], v);
-      xs[i] = P::filtered(v, 1.0);
-    }
     if (store) {
       T* out = store + cd.store + static_cast<int64_t>(k) * cd.store_step;
       for (int i = tid; i < dim; i += nt) {
@@ -131,50 +129,64 @@ __global__ void __launch_bounds__(1024, 1) chains_kernel(const DevSector* __rest
         out[i] = wk[i + 8 * r];
       }
     }
-    __syncthreads();
     double d[2 * P::kC] = {};
-    for (int it = warp; it < items; it += nw) {
-      const int r = it / ng, pos = (it - r * ng) * 32 + lane;
-      const T* row = xs + r * pitch;
-      const bool in = pos < Dd;
-      const int c = !in ? 0 : G.ent ? gauge_string(G, pos) : pos;
-      const uint32_t u = S.umask[r];
-      T acc = P::times(diag_value(S, u, S.dmask[c], S.cnt_uu[r], S.cnt_dd[c], S.wpl[r]), row[c]);
-      if (G.ent) {
-        if (phase) {
-          RowSum<P, 1, kPhase> s;
-          s.base = reinterpret_cast<const unsigned char*>(row);
-          s.line = 0;
-          s.acc[0] = acc;
-          s.walk(G, pos, tab, rc);
-          acc = s.acc[0];
+    for (int rb = 0; rb < Du; rb += cd.rows) {  // all rows at once where the whole vector is staged
+      const int nr = min(cd.rows, Du - rb);
+      if (rb > 0) __syncthreads();
+      for (int i = tid; i < nr * pitch; i += nt) {
+        T v = wk[rb * pitch + i];
+        if (P::kScaled) v = P::times(s_in[0], v);
+        xs[i] = P::filtered(v, 1.0);
+      }
+      __syncthreads();
+      const int items = (nr + rpw - 1) / rpw * ng;
+      for (int it = warp; it < items; it += nw) {
+        const int rl = it / ng * rpw + sub, pos = (it - it / ng * ng) * 32 + pos0;
+        const bool in = rl < nr && sub < rpw && pos < Dd;
+        const int r = rb + (in ? rl : 0);
+        const T* row = xs + (in ? rl : 0) * pitch;
+        const int tp = in ? pos : 0, c = !G.ent ? tp : gauge_string(G, tp);
+        T acc = P::times(diag_value(S, S.umask[r], S.dmask[c], S.cnt_uu[r], S.cnt_dd[c], S.wpl[r]), row[c]);
+        if (G.ent) {
+          if (phase) {
+            RowSum<P, 1, kPhase> s;
+            s.base = reinterpret_cast<const unsigned char*>(row);
+            s.line = 0;
+            s.acc[0] = acc;
+            s.walk(G, rpw > 1 ? tp : pos, tab, rc);
+            acc = s.acc[0];
+          } else {
+            RowSum<P, 1, false> s;
+            s.base = reinterpret_cast<const unsigned char*>(row);
+            s.line = 0;
+            s.acc[0] = acc;
+            s.walk(G, rpw > 1 ? tp : pos, tab, rc);
+            acc = s.acc[0];
+          }
         } else {
-          RowSum<P, 1, false> s;
-          s.base = reinterpret_cast<const unsigned char*>(row);
-          s.line = 0;
-          s.acc[0] = acc;
-          s.walk(G, pos, tab, rc);
-          acc = s.acc[0];
+          acc = list_hops<P>(S, row, c, acc);
         }
-      } else if (in) {
-        acc = list_hops<P>(S, row, c, acc);
-      }
-      T up = P::zero();
-      const T* col = xs + c;
-      const int j1 = S.up_ptr[r + 1];
-      int j = S.up_ptr[r];
-      for (; j + 4 <= j1; j += 4) {
-        T v[4];
+        T up = P::zero();
+        const T* col = (kSmem ? xs : wk) + c;
+        auto source = [&](int j) {
+          const T v = col[S.up_src[j] * pitch];
+          return kSmem ? v : P::filtered(v, s_in[0]);
+        };
+        const int j1 = S.up_ptr[r + 1];
+        int j = S.up_ptr[r];
+        for (; j + 4 <= j1; j += 4) {
+          T v[4];
 #pragma unroll
-        for (int t = 0; t < 4; ++t) v[t] = col[S.up_src[j + t] * pitch];
+          for (int t = 0; t < 4; ++t) v[t] = source(j + t);
 #pragma unroll
-        for (int t = 0; t < 4; ++t) P::cmac(up, P::up_coef(S, j + t), v[t]);
-      }
-      for (; j < j1; ++j) P::cmac(up, P::up_coef(S, j), col[S.up_src[j] * pitch]);
-      if (in) {
-        const T v = P::add_scaled(acc, up, 1.0);
-        y[r * pitch + c] = v;
-        P::dot(d, wk[r * pitch + c], v, s_in[0]);
+          for (int t = 0; t < 4; ++t) P::cmac(up, P::up_coef(S, j + t), v[t]);
+        }
+        for (; j < j1; ++j) P::cmac(up, P::up_coef(S, j), source(j));
+        if (in) {
+          const T v = P::add_scaled(acc, up, kSmem ? 1.0 : s_in[0]);
+          y[r * pitch + c] = v;
+          P::dot(d, row[c], v, 1.0);
+        }
       }
     }
     all_totals<2 * P::kC>(d, sh);
@@ -188,21 +200,33 @@ __global__ void __launch_bounds__(1024, 1) chains_kernel(const DevSector* __rest
       if (active[q] && tid == 0 && q < cd.chains) alpha[static_cast<int64_t>(cd.out + q) * M + k] = zr;
     }
     double n2[P::kC] = {};
-    for (int i = tid; i < V; i += nt) {
-      const T yv = y[i], av = wk[i], pv = k > 0 ? wkm1[i] : P::zero();
-      decltype(P::narrow(0.0, 0.0)) w[P::kC];
+    constexpr int kBatch = P::kC == 1 ? 2 : 1;  // two complex64 chains need the registers
+    for (int i0 = tid; i0 < V; i0 += kBatch * nt) {
+      T yv[kBatch], av[kBatch], pv[kBatch];
 #pragma unroll
-      for (int q = 0; q < P::kC; ++q) {
-        const auto yy = P::get(yv, q), aa = P::get(av, q), pp = P::get(pv, q);
-        const double sy = P::kScaled ? 1.0 : s_in[q];
-        double wr = sy * static_cast<double>(yy.x) - (c1r[q] * aa.x - c1i[q] * aa.y);
-        double wi = sy * static_cast<double>(yy.y) - (c1r[q] * aa.y + c1i[q] * aa.x);
-        wr -= c2[q] * pp.x;
-        wi -= c2[q] * pp.y;
-        w[q] = P::narrow(wr, wi);
-        n2[q] += static_cast<double>(w[q].x) * w[q].x + static_cast<double>(w[q].y) * w[q].y;
+      for (int t = 0; t < kBatch; ++t) {
+        const int i = i0 + t * nt < V ? i0 + t * nt : i0;
+        yv[t] = y[i];
+        av[t] = wk[i];
+        pv[t] = k > 0 ? wkm1[i] : P::zero();
       }
-      y[i] = P::make(w);
+#pragma unroll
+      for (int t = 0; t < kBatch; ++t) {
+        if (i0 + t * nt >= V) continue;
+        decltype(P::narrow(0.0, 0.0)) w[P::kC];
+#pragma unroll
+        for (int q = 0; q < P::kC; ++q) {
+          const auto yy = P::get(yv[t], q), aa = P::get(av[t], q), pp = P::get(pv[t], q);
+          const double sy = P::kScaled ? 1.0 : s_in[q];
+          double wr = sy * static_cast<double>(yy.x) - (c1r[q] * aa.x - c1i[q] * aa.y);
+          double wi = sy * static_cast<double>(yy.y) - (c1r[q] * aa.y + c1i[q] * aa.x);
+          wr -= c2[q] * pp.x;
+          wi -= c2[q] * pp.y;
+          w[q] = P::narrow(wr, wi);
+          n2[q] += static_cast<double>(w[q].x) * w[q].x + static_cast<double>(w[q].y) * w[q].y;
+        }
+        y[i0 + t * nt] = P::make(w);
+      }
     }
     all_totals<P::kC>(n2, sh);
     bool any = false;
@@ -243,13 +267,17 @@ constexpr int kClassThreads[4] = {1024, 512, 256, 64};
 
 int chain_class(int64_t dim) { return dim > 4096 ? 0 : dim > 1024 ? 1 : dim > 256 ? 2 : 3; }
 
-size_t chain_smem_bytes(const DevSector& S, bool c64, bool phase, bool with_vector) {
+size_t chain_smem_bytes(const DevSector& S, bool c64, bool phase, int rows) {
   const size_t tab = !S.dn_g.ent || phase ? 0 : static_cast<size_t>(S.dn_g.nt) * 8 * (c64 ? 8 : 16);
-  return (tab + 15) / 16 * 16 + (with_vector ? chain_elements(S) * 16 : 0);
+  return (tab + 15) / 16 * 16 + static_cast<size_t>(rows) * static_cast<size_t>(S.Dd + 8) * 16;
 }
 
-bool chain_in_smem(const DevSector& S, bool c64, bool phase) {
-  return chain_smem_bytes(S, c64, phase, true) + 2048 <= kMaxSmem;  // 2048: the reduction's own
+int chain_rows(const DevSector& S, bool c64, bool phase) {
+  const size_t most = kMaxSmem - 2048;  // 2048: the reductions' own
+  if (chain_smem_bytes(S, c64, phase, static_cast<int>(S.Du)) <= most) return static_cast<int>(S.Du);
+  const size_t base = chain_smem_bytes(S, c64, phase, 0), line = static_cast<size_t>(S.Dd + 8) * 16;
+  if (base + line > most) return 0;
+  return static_cast<int>(std::max<size_t>(1, base < most / 2 ? (most / 2 - base) / line : 1));
 }
 
 namespace {

@@ -14,7 +14,8 @@ struct ChainDesc {
   int out;             // first row of alpha/beta/used/scale written by this plane
   int chains;          // chains of the plane that are wanted (a plane's second complex64 chain may not be)
   unsigned seed;       // Philox key of its first chain
-  int64_t off;         // first element of its vectors in the scratch (3 of chain_elements(); 4 outside shared memory)
+  int rows;            // rows staged at once: all of them where the vector fits shared memory
+  int64_t off;         // first element of its three vectors of chain_elements() in the scratch
   int64_t init;        // first element of its start vector in ChainLaunch::init
   int64_t store;       // first element of its stored vectors, and their distance
   int64_t store_step;
@@ -42,9 +43,10 @@ struct ChainLaunch {
 int chain_class(int64_t dim);
 // Elements of one vector: rows have a pitch of Dd + 8.
 inline size_t chain_elements(const DevSector& S) { return static_cast<size_t>(S.Du) * static_cast<size_t>(S.Dd + 8); }
-// Shared memory of a plane of the sector, and whether its gathered vector fits there too.
-size_t chain_smem_bytes(const DevSector& S, bool c64, bool phase, bool with_vector);
-bool chain_in_smem(const DevSector& S, bool c64, bool phase);
+// Shared memory of a plane of the sector with `rows` rows staged, and the rows that are: all of them where they fit, else
+// as many as fit half of it (0: not even one).
+size_t chain_smem_bytes(const DevSector& S, bool c64, bool phase, int rows);
+int chain_rows(const DevSector& S, bool c64, bool phase);
 cudaError_t chains_lanczos(const ChainLaunch& L, bool c64, cudaStream_t st);
 
 }  // namespace ftlm_b200

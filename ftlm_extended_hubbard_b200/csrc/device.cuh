@@ -44,7 +44,6 @@ struct DevSector {
   const int64_t* dn_csr_ptr;   // [Dd+1] unpadded down-hop lists (batched path)
   const uint32_t* dn_csr_ent;
   const float2* up_coef32;     // [nnz_up] complex64 copies for the batched path
-  const float2* dn_coef32;     // [n_dn_hops+1]
   const float2* dn_coef32s;    // [2*(n_dn_hops+1)]: [2*hop + s] = (-1)^s coef (the gauge-basis row pass)
   const double2* dn_coef;  // [n_dn_hops+1]
   const uint32_t* dn_nmask;// [n_dn_hops+1]

@@ -265,7 +265,7 @@ int ftlm_gpu_batched_sweep_checked(const ftlm_params* p, int R, int M, unsigned 
 int ftlm_gpu_batched_release(void);
 
 /* Sectors with 2 <= dim <= max_dim in ftlm_gpu_gc_sweep run as one fused launch (one CTA per chain,
- * all M steps on the device; same start vectors and recurrence); default 131072, 0 disables.
+ * all M steps on the device; same start vectors and recurrence); default 16384, 0 disables.
  * No reference counterpart (scheduling only). */
 int ftlm_gpu_set_fused_max_dim(long long max_dim);
 /* Autotuner (no reference counterpart): times the sector's H·v variants — the generic gather kernel

@@ -536,68 +536,65 @@ int ftlm_gpu_apply_host(ftlm_sector* s, const double* x, double* y) {
 
 }  // extern "C"
 
-namespace {
-
-// The recurrence of src/lanczos.cpp:180-205 on a sector that runs the row + column-slab passes,
-// with the BLAS-1 work folded into them: vectors are kept unnormalised (q_k = s_k W_k, s_k =
-// 1/beta_{k-1}), the row pass stages s_k W_k, the column pass adds s_k times the up-hop sum and
-// emits the partials of z = <q_k, H q_k>, and one pass forms w = H q_k - z q_k - beta_{k-1} q_{k-1}
-// with ||w||^2.  Per step: 8 streaming vector passes instead of 12 and no normalisation pass.
-// alpha and ||w||^2 are read back once per step for the reference's breakdown test.
-int run_lanczos_fused(ftlm_sector* s, int max_steps, unsigned seed, int start_mode, std::vector<double>* alpha,
-                      std::vector<double>* beta) {
-  alpha->clear();
-  beta->clear();
-  const int64_t dim = s->plan.dim;
-  if (dim <= 0 || max_steps <= 0) return FTLM_OK;
-  LanczosWs& ws = s->ws;
-  cudaStream_t st = s->stream;
-  const int path = s->effective_path();
-  const DevSector d = s->dev_for(path);
-  if (hv_rows_smem_bytes(d) > 227 * 1024)
-    return fail(FTLM_ERR_UNSUPPORTED, "row pass does not fit in shared memory for this sector");
-  CU_TRY(ws.ensure(dim));
-  const int64_t nblk = hv_cols_blocks(d, s->cols_variant);
-  CU_TRY(ws.ensure_dotp(nblk));
-  double* scr = ws.scratch.as<double>();
-  if (start_mode == FTLM_START_PHILOX) {
-    CU_TRY(lz_philox_start(ws.q.as<double2>(), dim, seed, scr, st));
-    CU_TRY(lz_normalise_start(ws.q.as<double2>(), dim, scr, st));
-  } else if (start_mode == FTLM_START_REFERENCE) {
-    std::vector<std::complex<double>> h;
-    reference_start(dim, seed, &h);
-    CU_TRY(cudaMemcpyAsync(ws.q.p, h.data(), dim * sizeof(double2), cudaMemcpyHostToDevice, st));
-    CU_TRY(cudaStreamSynchronize(st));
-  } else {
+int ftlm_b200::capi::planes_lanczos(ftlm_sector* s, int R, int M, unsigned seed, int start_mode, std::vector<double>* A,
+                                    std::vector<double>* B, std::vector<int>* used) {
+  if (start_mode != FTLM_START_REFERENCE && start_mode != FTLM_START_PHILOX)
     return fail(FTLM_ERR_INVALID, "unknown start_mode");
-  }
-  double2* Wk = ws.q.as<double2>();
-  double2* Wkm1 = ws.qp.as<double2>();
-  double2* Y = ws.w.as<double2>();
-  double sk = 1.0, skm1 = 0.0, bprev = 0.0;
-  double res[4];
-  for (int k = 0; k < max_steps; ++k) {
-    CU_TRY(hv_launch_pass(d, Wk, Y, 0, st, s->cols_variant, sk, nullptr));
-    CU_TRY(hv_launch_pass(d, Wk, Y, 1, st, s->cols_variant, sk, ws.dotp.as<double>()));
-    CU_TRY(lz_reduce_pairs(ws.dotp.as<double>(), nblk, scr, st));
-    CU_TRY(lz_update_scaled(Y, Wk, sk, Wkm1, skm1, bprev, k > 0, dim, scr, st));
-    CU_TRY(cudaMemcpyAsync(res, scr + kResZ, 3 * sizeof(double), cudaMemcpyDeviceToHost, st));
+  A->assign(static_cast<size_t>(R) * M, 0.0);
+  B->assign(static_cast<size_t>(R) * M, 0.0);
+  used->assign(static_cast<size_t>(R), 0);
+  const int64_t dim = s->plan.dim;
+  const DevSector& S = s->dev;
+  cudaStream_t st = s->stream;
+  BtWs& ws = s->planes;
+  const int group = pl_group(S, false, std::min(R, kBtChains));
+  CU_TRY(ws.ensure(static_cast<size_t>(group) * dim * sizeof(double2), M, pl_items_doubles(S, false, group)));
+  const size_t tab = static_cast<size_t>(M) * kBtChains * sizeof(double);
+  std::vector<double> ha(static_cast<size_t>(M) * kBtChains), hb(static_cast<size_t>(M) * kBtChains);
+  std::vector<int> hu(kBtChains);
+  std::vector<std::complex<double>> start;
+  const bool given = start_mode == FTLM_START_REFERENCE;
+  for (int r0 = 0; r0 < R; r0 += group) {  // the scalars of a group are read before the next one starts
+    const int np = std::min(group, R - r0);
+    const unsigned seed_g = seed + static_cast<unsigned>(r0) * 100003u;
+    const PlaneState z = ws.state(0);
+    double2 *wk = ws.buf[0].as<double2>(), *y = ws.buf[1].as<double2>(), *wkm1 = ws.buf[2].as<double2>();
+    CU_TRY(cudaMemsetAsync(ws.alpha.p, 0, tab, st));
+    CU_TRY(cudaMemsetAsync(ws.beta.p, 0, tab, st));
+    if (given) {
+      reference_normals(dim, np, seed_g, &start);
+      CU_TRY(cudaMemcpyAsync(wk, start.data(), start.size() * sizeof(double2), cudaMemcpyHostToDevice, st));
+    }
+    CU_TRY(pl_start(S, wk, np, seed_g, given, z, st));
+    for (int k = 0; k < M; ++k) {
+      CU_TRY(pl_step(S, wk, wkm1, y, np, k, z, st));
+      double2* t = wkm1;
+      wkm1 = wk;
+      wk = y;
+      y = t;
+    }
+    CU_TRY(cudaMemcpyAsync(ha.data(), ws.alpha.p, tab, cudaMemcpyDeviceToHost, st));
+    CU_TRY(cudaMemcpyAsync(hb.data(), ws.beta.p, tab, cudaMemcpyDeviceToHost, st));
+    CU_TRY(cudaMemcpyAsync(hu.data(), ws.used.p, hu.size() * sizeof(int), cudaMemcpyDeviceToHost, st));
     CU_TRY(cudaStreamSynchronize(st));
-    alpha->push_back(res[0]);
-    const double nw2 = res[2];
-    if (nw2 < 1e-24) break;
-    const double b_k = std::sqrt(nw2);
-    beta->push_back(b_k);
-    // rotate: W_{k-1} <- W_k, W_k <- w (unnormalised, scale 1/b_k), the old W_{k-1} buffer is next Y
-    double2* t = Wkm1;
-    Wkm1 = Wk;
-    Wk = Y;
-    Y = t;
-    skm1 = sk;
-    sk = 1.0 / b_k;
-    bprev = b_k;
+    for (int r = 0; r < np; ++r) {
+      const size_t ch = static_cast<size_t>(r0 + r);
+      (*used)[ch] = hu[static_cast<size_t>(r)];
+      for (int k = 0; k < M; ++k) {
+        (*A)[ch * M + k] = ha[static_cast<size_t>(k) * kBtChains + r];
+        (*B)[ch * M + k] = hb[static_cast<size_t>(k) * kBtChains + r];
+      }
+    }
   }
   return FTLM_OK;
+}
+
+namespace {
+
+// A chain's alpha and beta without their padding: one that ended has no last beta.
+void trim_chain(int n, std::vector<double>* a, std::vector<double>* b) {
+  a->resize(static_cast<size_t>(n));
+  b->resize(static_cast<size_t>(n > 0 && (*b)[static_cast<size_t>(n) - 1] > 0.0 ? n : std::max(0, n - 1)));
 }
 
 }  // namespace
@@ -620,14 +617,17 @@ int ftlm_gpu_lanczos(ftlm_sector* s, int max_steps, unsigned seed, int start_mod
     b.resize(static_cast<size_t>(max_steps));
     CU_TRY(cudaMemcpy(a.data(), run.alpha, a.size() * sizeof(double), cudaMemcpyDeviceToHost));
     CU_TRY(cudaMemcpy(b.data(), run.beta, b.size() * sizeof(double), cudaMemcpyDeviceToHost));
-    a.resize(static_cast<size_t>(n));
-    b.resize(static_cast<size_t>(n > 0 && b[static_cast<size_t>(n) - 1] > 0.0 ? n : std::max(0, n - 1)));  // a chain that ended has no last beta
-  } else if (s->effective_path() >= 2)
-    rc = run_lanczos_fused(s, max_steps, seed, start_mode, &a, &b);
-  else
+    trim_chain(n, &a, &b);
+  } else if (s->apply_path != 1 && max_steps > 0 && pl_fits(s->dev, s->plan.max_up_deg)) {
+    std::vector<int> u;
+    rc = planes_lanczos(s, 1, max_steps, seed, start_mode, &a, &b, &u);
+    if (rc) return rc;
+    trim_chain(u[0], &a, &b);
+  } else {
     rc = run_lanczos(
         s->plan.dim, [s](const double2* x, double2* y, cudaStream_t st) { return s->apply(x, y, st); }, s->ws,
         max_steps, seed, start_mode, s->stream, &a, &b);
+  }
   if (rc) return rc;
   if (alpha) std::copy(a.begin(), a.end(), alpha);
   if (beta) std::copy(b.begin(), b.end(), beta);
@@ -846,13 +846,18 @@ int plain_sector_ftlm(ftlm_sector* s, const double* bts, int n_bt, int R, int M,
     return chains_ftlm({s}, R, M, seed, start_mode, false, bts, n_bt, converged, lnz, energy);
   std::vector<double> A(static_cast<size_t>(R) * M, 0.0), B(static_cast<size_t>(R) * M, 0.0);
   std::vector<int> nv(static_cast<size_t>(R), 0);
-  for (int r = 0; r < R; ++r) {
-    const unsigned seed_r = seed + static_cast<unsigned>(r) * 100003u;
-    int nb = 0, used = 0;
-    rc = ftlm_gpu_lanczos(s, M, seed_r, start_mode, &A[static_cast<size_t>(r) * M], &B[static_cast<size_t>(r) * M], &nb,
-                          &used);
+  if (s->apply_path != 1 && pl_fits(s->dev, s->plan.max_up_deg)) {
+    rc = planes_lanczos(s, R, M, seed, start_mode, &A, &B, &nv);
     if (rc) return rc;
-    nv[static_cast<size_t>(r)] = used;
+  } else {
+    for (int r = 0; r < R; ++r) {
+      const unsigned seed_r = seed + static_cast<unsigned>(r) * 100003u;
+      int nb = 0, used = 0;
+      rc = ftlm_gpu_lanczos(s, M, seed_r, start_mode, &A[static_cast<size_t>(r) * M], &B[static_cast<size_t>(r) * M], &nb,
+                            &used);
+      if (rc) return rc;
+      nv[static_cast<size_t>(r)] = used;
+    }
   }
   std::vector<double> lq(static_cast<size_t>(R) * n_bt), eq(static_cast<size_t>(R) * n_bt);
   rc = chain_quadrature(A.data(), B.data(), nv.data(), R, M, bts, n_bt, lq.data(), eq.data(), converged);

@@ -22,9 +22,9 @@ int bt_run_chains(ftlm_sector* s, int R, int M, unsigned seed, std::vector<doubl
   const int64_t dim = s->plan.dim;
   const DevSector& S = s->dev;
   cudaStream_t st = s->stream;
-  const int group = pl_group(dim, (std::min(R, kBtChains) + 1) / 2);
+  const int group = pl_group(S, true, (std::min(R, kBtChains) + 1) / 2);
   std::lock_guard<std::mutex> lock(g_bt_mu);
-  CU_TRY(g_bt.ensure(static_cast<size_t>(group) * dim * sizeof(float4), M));
+  CU_TRY(g_bt.ensure(static_cast<size_t>(group) * dim * sizeof(float4), M, pl_items_doubles(S, true, group)));
   const size_t tab = static_cast<size_t>(M) * kBtChains * sizeof(double);
   std::vector<double> ha(static_cast<size_t>(M) * kBtChains), hb(static_cast<size_t>(M) * kBtChains);
   std::vector<int> hu(kBtChains);
@@ -99,7 +99,7 @@ int ftlm_gpu_batched_autotune(ftlm_sector* s, int reps, int* variant, float* ms)
   float best = 3.4e38f;
   {
     std::lock_guard<std::mutex> lock(g_bt_mu);
-    const int planes = pl_group(P.dim, kBtChains / 2);
+    const int planes = pl_group(s->dev, true, kBtChains / 2);
     CU_TRY(g_bt.ensure(static_cast<size_t>(planes) * P.dim * sizeof(float4), 1));
     float4* W = g_bt.buf[0].as<float4>();
     float4* Y = g_bt.buf[1].as<float4>();

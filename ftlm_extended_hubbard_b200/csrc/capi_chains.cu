@@ -10,8 +10,6 @@ using namespace ftlm_b200::capi;
 namespace ftlm_b200 {
 namespace capi {
 
-namespace {
-
 // The reference's start vectors (src/lanczos.cpp:140-175) before normalisation.  The entries of a shorter vector are
 // the first ones of a longer vector of the same seed, so the longest of each seed serves every sector.
 void reference_normals(int64_t dim, int R, unsigned seed, std::vector<std::complex<double>>* out) {
@@ -40,8 +38,6 @@ void reference_normals(int64_t dim, int R, unsigned seed, std::vector<std::compl
   for (auto& th : pool) th.join();
 }
 
-}  // namespace
-
 int chains_run(const std::vector<ftlm_sector*>& secs, int R, int M, unsigned seed, int start_mode, bool c64,
                ChainRun* run, void* store, const std::vector<int64_t>* store_base, bool keep_scale) {
   if (start_mode != FTLM_START_REFERENCE && start_mode != FTLM_START_PHILOX)
@@ -51,20 +47,19 @@ int chains_run(const std::vector<ftlm_sector*>& secs, int R, int M, unsigned see
   struct Item {
     ChainDesc d;
     int size;
-    bool smem;
+    bool smem, phase, xor_real;
     int64_t dim;
     size_t bytes;
+    int group() const { return size * 8 + (smem ? 4 : 0) + (phase ? 2 : 0) + (xor_real ? 1 : 0); }
   };
   std::vector<DevSector> devs;
   std::vector<Item> items;
   int64_t max_dim = 0;
-  bool phase = true;  // one kernel for all: the register form of the table entries where every table has it
-  for (const ftlm_sector* s : secs)
-    if (s->dev.dn_g.ent && s->dev.dn_g.nt > 0 && !s->dev.dn_g.phase) phase = false;
   for (int i = 0; i < ns; ++i) {
     const DevSector& S = secs[static_cast<size_t>(i)]->dev;
     devs.push_back(S);
     max_dim = std::max(max_dim, S.dim);
+    const bool phase = S.dn_g.ent && S.dn_g.phase, xor_real = S.dn_g.ent && S.dn_g.xor_real;  // forms of its table entries
     const int rows = chain_rows(S, c64, phase);
     const bool smem = rows == static_cast<int>(S.Du);
     if (rows == 0) return fail(FTLM_ERR_UNSUPPORTED, "fused chains: a row of the sector does not fit shared memory");
@@ -79,12 +74,11 @@ int chains_run(const std::vector<ftlm_sector*>& secs, int R, int M, unsigned see
         d.store = (*store_base)[static_cast<size_t>(i)] + static_cast<int64_t>(p) * S.dim;
         d.store_step = static_cast<int64_t>(planes) * S.dim;
       }
-      items.push_back(Item{d, chain_class(S.dim), smem, S.dim, chain_elements(S) * 16 * 3});
+      items.push_back(Item{d, chain_class(S.dim), smem, phase, xor_real, S.dim, chain_elements(S) * 16 * 3});
     }
   }
   std::stable_sort(items.begin(), items.end(), [](const Item& a, const Item& b) {
-    if (a.size != b.size) return a.size < b.size;
-    if (a.smem != b.smem) return b.smem;
+    if (a.group() != b.group()) return a.group() < b.group();
     return a.dim > b.dim;
   });
   cudaStream_t st = secs[0]->stream;
@@ -150,8 +144,8 @@ int chains_run(const std::vector<ftlm_sector*>& secs, int R, int M, unsigned see
     for (size_t i = piece[pc]; i < piece[pc + 1] && ce == cudaSuccess;) {
       size_t j = i;
       size_t smem_bytes = 0;
-      for (; j < piece[pc + 1] && items[j].size == items[i].size && items[j].smem == items[i].smem; ++j)
-        smem_bytes = std::max(smem_bytes, chain_smem_bytes(devs[static_cast<size_t>(items[j].d.sector)], c64, phase, items[j].d.rows));
+      for (; j < piece[pc + 1] && items[j].group() == items[i].group(); ++j)
+        smem_bytes = std::max(smem_bytes, chain_smem_bytes(devs[static_cast<size_t>(items[j].d.sector)], c64, items[j].phase, items[j].d.rows));
       cudaStream_t s2 = secs[static_cast<size_t>(std::min(stream, ns - 1))]->stream;
       ++stream;
       if (s2 != st) ce = cudaStreamWaitEvent(s2, ev[0], 0);
@@ -161,7 +155,8 @@ int chains_run(const std::vector<ftlm_sector*>& secs, int R, int M, unsigned see
       L.blocks = static_cast<int>(j - i);
       L.size = items[i].size;
       L.smem = items[i].smem;
-      L.phase = phase;
+      L.phase = items[i].phase;
+      L.xor_real = items[i].xor_real;
       L.smem_bytes = smem_bytes;
       L.M = M;
       L.scratch = mem.at<void>(o_scr);

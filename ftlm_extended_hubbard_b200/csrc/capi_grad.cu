@@ -133,10 +133,10 @@ int grad_plain(ftlm_sector* s, ftlm_sector* op, double bT, int R, int M, unsigne
 // Batched path: complex64 32-chain blocks of ftlm_gpu_batched_ftlm_sector, replayed step by step.
 int grad_batched(ftlm_sector* s, ftlm_sector* op, double bT, int R, int M, unsigned seed, std::vector<ChainGrad>* out) {
   const int64_t dim = s->plan.dim;
-  const int max_planes = (std::min(R, kBtChains) + 1) / 2, group = pl_group(dim, max_planes);
+  const int max_planes = (std::min(R, kBtChains) + 1) / 2, group = pl_group(s->dev, true, max_planes);
   const int64_t vs = dim * max_planes;  // elements of two chains per stored vector
   std::lock_guard<std::mutex> lock(g_bt_mu);
-  CU_TRY(g_bt.ensure(0, M));
+  CU_TRY(g_bt.ensure(0, M, pl_items_doubles(s->dev, true, group)));
   CU_TRY(g_grad.grow(g_grad.Q, g_grad.qcap, static_cast<size_t>(M + 1) * vs * sizeof(float4)));
   if (op) CU_TRY(g_grad.grow(g_grad.AQ, g_grad.acap, static_cast<size_t>(M) * vs * sizeof(float4)));
   if (!g_grad.zflag.p) {
@@ -356,15 +356,20 @@ int ftlm_gpu_gc_logz(const ftlm_params* p, double mu, double bT, int R, int M, u
         rc = bt_run_chains(s.get(), R, M, seed, &A, &B, &used);
         if (rc) return rc;
       } else {
-        A.assign(static_cast<size_t>(R) * M, 0.0);
-        B.assign(static_cast<size_t>(R) * M, 0.0);
-        used.assign(static_cast<size_t>(R), 0);
-        for (int r = 0; r < R; ++r) {
-          int nb = 0, u = 0;
-          rc = ftlm_gpu_lanczos(s.get(), M, seed + static_cast<unsigned>(r) * 100003u, st_mode,
-                                A.data() + static_cast<size_t>(r) * M, B.data() + static_cast<size_t>(r) * M, &nb, &u);
+        if (s->apply_path != 1 && pl_fits(s->dev, s->plan.max_up_deg)) {
+          rc = planes_lanczos(s.get(), R, M, seed, st_mode, &A, &B, &used);
           if (rc) return rc;
-          used[static_cast<size_t>(r)] = u;
+        } else {
+          A.assign(static_cast<size_t>(R) * M, 0.0);
+          B.assign(static_cast<size_t>(R) * M, 0.0);
+          used.assign(static_cast<size_t>(R), 0);
+          for (int r = 0; r < R; ++r) {
+            int nb = 0, u = 0;
+            rc = ftlm_gpu_lanczos(s.get(), M, seed + static_cast<unsigned>(r) * 100003u, st_mode,
+                                  A.data() + static_cast<size_t>(r) * M, B.data() + static_cast<size_t>(r) * M, &nb, &u);
+            if (rc) return rc;
+            used[static_cast<size_t>(r)] = u;
+          }
         }
       }
       rc = gc_quadrature(A.data(), B.data(), used.data(), R, M, bT, dim, lnz_s + idx, e_s + idx);

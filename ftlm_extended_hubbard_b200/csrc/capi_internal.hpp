@@ -49,6 +49,29 @@ cudaError_t pool_take(size_t bytes, void** p, size_t* got);
 void pool_give(void* p, size_t got);
 void pool_trim();
 
+// One array in a block of the pool; its owner gives it back when no work on it is in flight.
+struct PoolBuf {
+  void* p = nullptr;
+  size_t got = 0;
+  PoolBuf() = default;
+  PoolBuf(const PoolBuf&) = delete;
+  PoolBuf& operator=(const PoolBuf&) = delete;
+  ~PoolBuf() { free(); }
+  void free() {
+    if (p) pool_give(p, got);
+    p = nullptr;
+    got = 0;
+  }
+  cudaError_t alloc(size_t bytes) {
+    free();
+    return pool_take(bytes, &p, &got);
+  }
+  template <class T>
+  T* as() const {
+    return static_cast<T*>(p);
+  }
+};
+
 // One block of the pool, laid out by add() and obtained by commit().  idle() says that the work on it has ended; without
 // it (an error on the way) the block is given back after the device has.
 class Scratch {
@@ -148,17 +171,12 @@ struct PlanParts {
 // Reference start vector (src/lanczos.cpp:140-175): re, im from std::normal_distribution<double>
 // over std::mt19937(seed), normalised with a serial sum; falls back to e_0 when ||q|| < 1e-18.
 void reference_start(int64_t dim, unsigned seed, std::vector<std::complex<double>>* q);
+// R such vectors before normalisation (seed + r*100003), drawn by several threads.
+void reference_normals(int64_t dim, int R, unsigned seed, std::vector<std::complex<double>>* out);
 
 struct LanczosWs {
   int64_t n = 0;
   DevBuf q, qp, w, scratch;
-  DevBuf dotp;  // column-pass partials of the fused sector recurrence
-  int64_t dotp_n = 0;
-  cudaError_t ensure_dotp(int64_t nblocks) {
-    if (nblocks <= dotp_n && dotp.p) return cudaSuccess;
-    dotp_n = nblocks;
-    return dotp.alloc(static_cast<size_t>(nblocks) * 2 * sizeof(double));
-  }
   cudaError_t ensure(int64_t dim) {
     if (n == dim && q.p) return cudaSuccess;
     n = dim;
@@ -223,6 +241,57 @@ int run_lanczos(int64_t dim, Apply&& apply, LanczosWs& ws, int max_steps, unsign
 }  // namespace capi
 }  // namespace ftlm_b200
 
+namespace ftlm_b200 {
+namespace capi {
+
+// Vectors and scalars of Lanczos chains on planes (or of a momentum block's 32 chains), kept between calls.
+struct BtWs {
+  size_t cap = 0;
+  int mcap = 0;
+  int64_t icap = 0;
+  PoolBuf buf[3], st, partial, items, alpha, beta, used, flags;
+  // three vectors of `bytes` each, the scalars of 32 chains of M steps, n_items partial sums of the column pass's items
+  cudaError_t ensure(size_t bytes, int M, int64_t n_items = 0) {
+    cudaError_t e = cudaSuccess;
+    if (bytes > cap) {
+      release();
+      for (auto& b : buf)
+        if ((e = b.alloc(bytes)) != cudaSuccess) return e;
+      cap = bytes;
+    }
+    if (n_items > icap) {
+      icap = 0;
+      if ((e = items.alloc(static_cast<size_t>(n_items) * sizeof(double))) != cudaSuccess) return e;
+      icap = n_items;
+    }
+    if (!st.p) {
+      if ((e = partial.alloc(std::max<int64_t>(kBtPartialDoubles, kPlPartialDoubles) * sizeof(double))) != cudaSuccess) return e;
+      if ((e = used.alloc(kBtChains * sizeof(int))) != cudaSuccess) return e;
+      if ((e = flags.alloc(2 * sizeof(int))) != cudaSuccess) return e;
+      if ((e = st.alloc(kBtFields * kBtChains * sizeof(double))) != cudaSuccess) return e;
+    }
+    if (M > mcap) {
+      mcap = 0;
+      if ((e = alpha.alloc(static_cast<size_t>(M) * kBtChains * sizeof(double))) != cudaSuccess) return e;
+      if ((e = beta.alloc(static_cast<size_t>(M) * kBtChains * sizeof(double))) != cudaSuccess) return e;
+      mcap = M;
+    }
+    return e;
+  }
+  // the scalar state of a group whose first chain is c0 of the block
+  PlaneState state(int c0) const {
+    return PlaneState{st.as<double>() + c0,   partial.as<double>(),  items.as<double>(),   alpha.as<double>() + c0,
+                      beta.as<double>() + c0, used.as<int>() + c0, flags.as<int>()};
+  }
+  void release() {  // before growing, too
+    for (auto& b : buf) b.free();
+    cap = 0;
+  }
+};
+
+}  // namespace capi
+}  // namespace ftlm_b200
+
 struct OrbitSectorData;
 
 // The opaque C handle: a sector plan, its device tables and per-sector workspaces.
@@ -235,6 +304,7 @@ struct ftlm_sector {
   ftlm_b200::DevSector dev{};
   void* tables = nullptr;  // one block of the pool
   size_t tables_bytes = 0;
+  ftlm_b200::capi::BtWs planes;  // vectors and scalars of its complex128 Lanczos chains
   int apply_path = 0;    // 0 auto, 1 generic, 2 rows+cols, 3 rows (register coefficient classes)+cols
   int cols_variant = 0;  // column slab 256/128/512 (0/1/2); 3/4/5: the same over the packed up list (path 3)
   ftlm_b200::capi::LanczosWs ws;
@@ -242,7 +312,7 @@ struct ftlm_sector {
   ftlm_b200::capi::LazyStream stream;
   ~ftlm_sector() {
     if (!tables) return;
-    cudaDeviceSynchronize();  // as a free would: a caller's H v may still read the tables
+    cudaDeviceSynchronize();  // as a free would: a caller's H v may still read the tables (and before `planes` goes back)
     ftlm_b200::capi::pool_give(tables, tables_bytes);
   }
   // Kernel choice for H·v: 1 = generic gather; 2 = row pass with the per-row coefficient table +
@@ -286,43 +356,6 @@ int need_device(const ftlm_sector* s);
 int sector_create(const ftlm_params* p, int n_up, int n_dn, PlanParts* parts, ftlm_sector** out);
 
 // ---- batched complex64 path (capi_batched.cu) ------------------------------------------------
-struct BtWs {
-  size_t cap = 0;
-  int mcap = 0;
-  DevBuf buf[3], st, partial, alpha, beta, used, flags;
-  // three vectors of `bytes` each and the scalars of 32 chains of M steps
-  cudaError_t ensure(size_t bytes, int M) {
-    cudaError_t e = cudaSuccess;
-    if (bytes > cap) {
-      release();
-      for (auto& b : buf)
-        if ((e = b.alloc(bytes)) != cudaSuccess) return e;
-      cap = bytes;
-    }
-    if (!st.p) {
-      if ((e = st.alloc(kBtFields * kBtChains * sizeof(double))) != cudaSuccess) return e;
-      if ((e = partial.alloc(std::max<int64_t>(kBtPartialDoubles, kPlPartialDoubles) * sizeof(double))) != cudaSuccess) return e;
-      if ((e = used.alloc(kBtChains * sizeof(int))) != cudaSuccess) return e;
-      if ((e = flags.alloc(2 * sizeof(int))) != cudaSuccess) return e;
-    }
-    if (M > mcap) {
-      if ((e = alpha.alloc(static_cast<size_t>(M) * kBtChains * sizeof(double))) != cudaSuccess) return e;
-      if ((e = beta.alloc(static_cast<size_t>(M) * kBtChains * sizeof(double))) != cudaSuccess) return e;
-      mcap = M;
-    }
-    return e;
-  }
-  // the scalar state of a group whose first chain is c0 of the block
-  PlaneState state(int c0) const {
-    return PlaneState{st.as<double>() + c0,    partial.as<double>(), alpha.as<double>() + c0,
-                      beta.as<double>() + c0,  used.as<int>() + c0,  flags.as<int>()};
-  }
-  void release() {
-    for (auto& b : buf) b.alloc(0);  // release before growing
-    cap = 0;
-  }
-};
-
 extern BtWs g_bt;
 extern std::mutex g_bt_mu;
 
@@ -449,6 +482,10 @@ inline bool fused_alone(const DevSector& S) {  // and a row of it fits (chain_ro
 }
 // Largest sector that joins the fused launch of a sweep; a larger one fills the GPU by itself.
 constexpr int64_t kFusedSweepMax = 1 << 14;
+
+// R complex128 chains of one sector (seed + r*100003) in groups of planes (planes.cu; pl_fits), layout as below.
+int planes_lanczos(ftlm_sector* s, int R, int M, unsigned seed, int start_mode, std::vector<double>* A,
+                   std::vector<double>* B, std::vector<int>* used);
 
 // The complex64 chains of one sector in groups of planes (planes.cu), alpha/beta [R][M] (beta zero-padded), used [R].
 int bt_run_chains(ftlm_sector* s, int R, int M, unsigned seed, std::vector<double>* A, std::vector<double>* B,

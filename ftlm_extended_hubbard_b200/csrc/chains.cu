@@ -60,7 +60,7 @@ __device__ __forceinline__ typename P::T list_hops(const DevSector& S, const typ
   return acc;
 }
 
-template <class P, bool kSmem, bool kPhase>
+template <class P, bool kSmem, bool kPhase, bool kXor>
 __global__ void __launch_bounds__(1024, 1) chains_kernel(const DevSector* __restrict__ sectors,
                                                          const ChainDesc* __restrict__ descs, int M,
                                                          typename P::T* __restrict__ scratch,
@@ -82,10 +82,9 @@ __global__ void __launch_bounds__(1024, 1) chains_kernel(const DevSector* __rest
   const DevGauge G = S.dn_g;
   const size_t tab_bytes = kPhase ? 0 : (G.ent ? static_cast<size_t>(G.nt) * 8 * sizeof(typename P::Cf) : 0);
   T* xs = reinterpret_cast<T*>(smem_raw + ((tab_bytes + 15) & ~size_t(15)));
-  const RowCoefs<P> rc(G);
+  const RowCoefs<P, kXor> rc(G);
   if (!kPhase && G.ent)
     for (int i = tid; i < G.nt * 8; i += nt) tab[i] = P::coef(G.tab[i >> 3]);
-  const bool phase = kPhase && G.phase;
   // padding: zero in every vector
   for (int i = tid; i < Du * 8; i += nt) {
     const int o = (i >> 3) * pitch + Dd + (i & 7);
@@ -148,21 +147,12 @@ __global__ void __launch_bounds__(1024, 1) chains_kernel(const DevSector* __rest
         const int tp = in ? pos : 0, c = !G.ent ? tp : gauge_string(G, tp);
         T acc = P::times(diag_value(S, S.umask[r], S.dmask[c], S.cnt_uu[r], S.cnt_dd[c], S.wpl[r]), row[c]);
         if (G.ent) {
-          if (phase) {
-            RowSum<P, 1, kPhase> s;
-            s.base = reinterpret_cast<const unsigned char*>(row);
-            s.line = 0;
-            s.acc[0] = acc;
-            s.walk(G, rpw > 1 ? tp : pos, tab, rc);
-            acc = s.acc[0];
-          } else {
-            RowSum<P, 1, false> s;
-            s.base = reinterpret_cast<const unsigned char*>(row);
-            s.line = 0;
-            s.acc[0] = acc;
-            s.walk(G, rpw > 1 ? tp : pos, tab, rc);
-            acc = s.acc[0];
-          }
+          RowSum<P, 1, kPhase, kXor> s;
+          s.base = reinterpret_cast<const unsigned char*>(row);
+          s.line = 0;
+          s.acc[0] = acc;
+          s.walk(G, rpw > 1 ? tp : pos, tab, rc);
+          acc = s.acc[0];
         } else {
           acc = list_hops<P>(S, row, c, acc);
         }
@@ -286,8 +276,11 @@ template <class P>
 cudaError_t launch(const ChainLaunch& L, cudaStream_t st) {
   using T = typename P::T;
   using K = void (*)(const DevSector*, const ChainDesc*, int, T*, const double2*, double*, double*, int*, double*, T*);
-  const K k = L.smem ? (L.phase ? chains_kernel<P, true, true> : chains_kernel<P, true, false>)
-                     : (L.phase ? chains_kernel<P, false, true> : chains_kernel<P, false, false>);
+  static const K kernels[8] = {chains_kernel<P, false, false, false>, chains_kernel<P, false, false, true>,
+                               chains_kernel<P, false, true, false>,  chains_kernel<P, false, true, true>,
+                               chains_kernel<P, true, false, false>,  chains_kernel<P, true, false, true>,
+                               chains_kernel<P, true, true, false>,   chains_kernel<P, true, true, true>};
+  const K k = kernels[(L.smem ? 4 : 0) + (L.phase ? 2 : 0) + (L.xor_real ? 1 : 0)];
   const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(L.smem_bytes));
   if (e != cudaSuccess) return e;
   k<<<L.blocks, kClassThreads[L.size], L.smem_bytes, st>>>(L.sectors, L.descs, L.M, static_cast<T*>(L.scratch), L.init, L.alpha,

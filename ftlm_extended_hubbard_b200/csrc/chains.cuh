@@ -21,14 +21,15 @@ struct ChainDesc {
   int64_t store_step;
 };
 
-// Planes of one size class whose gathered vector is (or is not) in shared memory.
+// Planes of one size class, staging and form of the sectors' gauge tables.
 struct ChainLaunch {
   const DevSector* sectors;
   const ChainDesc* descs;
   int blocks;
   int size;             // chain_class of the sectors
   bool smem;            // the gathered vector is in shared memory
-  bool phase;           // every gauge table with table entries has the phase form
+  bool phase;           // the tables' coefficients have the phase form
+  bool xor_real;        // and the XOR form
   size_t smem_bytes;    // largest chain_smem_bytes of the sectors
   int M;
   void* scratch;

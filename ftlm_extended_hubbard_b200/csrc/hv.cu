@@ -49,7 +49,7 @@ __device__ __forceinline__ double flip_sign(double v, uint32_t neg) {
 }
 
 __global__ void __launch_bounds__(kRowThreads, 1) hv_rows_kernel(DevSector S, const double2* __restrict__ x,
-                                                                   double2* __restrict__ y, double sx) {
+                                                                   double2* __restrict__ y) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int Dd = static_cast<int>(S.Dd);
   double2* xs = reinterpret_cast<double2*>(smem_raw);
@@ -64,8 +64,6 @@ __global__ void __launch_bounds__(kRowThreads, 1) hv_rows_kernel(DevSector S, co
     int saw_tiny = 0;
     for (int c = tid; c < Dd; c += kRowThreads) {
       double2 v = xrow[c];
-      v.x *= sx;  // the input is sx * x (sx = 1: unchanged)
-      v.y *= sx;
       if (tiny(v)) {
         saw_tiny |= (v.x != 0.0 || v.y != 0.0);
         v = make_double2(0.0, 0.0);
@@ -103,7 +101,7 @@ __global__ void __launch_bounds__(kRowThreads, 1) hv_rows_kernel(DevSector S, co
   }
 }
 
-using RowsKernel = void (*)(DevSector, const double2*, double2*, double);
+using RowsKernel = void (*)(DevSector, const double2*, double2*);
 
 // Column pass: two columns per thread, chunk = 2 * threads columns (variants: 64 / 128 / 256
 // threads = 128 / 256 / 512-column slabs of Du * chunk * 16 bytes kept in L2; the autotuner picks).
@@ -213,7 +211,7 @@ __device__ __forceinline__ void gauge_hops(double2& acc, const DevGauge& G, int 
 // GaugeTable (plan.hpp).
 template <bool kPhase, bool kXor>
 __global__ void __launch_bounds__(kRowThreads, 1) hv_rows_gauge_kernel(DevSector S, const double2* __restrict__ x,
-                                                                         double2* __restrict__ y, double sx) {
+                                                                         double2* __restrict__ y) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int Dd = static_cast<int>(S.Dd);
   double2* xs = reinterpret_cast<double2*>(smem_raw);
@@ -233,8 +231,6 @@ __global__ void __launch_bounds__(kRowThreads, 1) hv_rows_gauge_kernel(DevSector
     int saw_tiny = 0;
     for (int c = tid; c < Dd; c += kRowThreads) {
       double2 v = xrow[c];
-      v.x *= sx;  // the input is sx * x (sx = 1: unchanged)
-      v.y *= sx;
       if (tiny(v)) {
         saw_tiny |= (v.x != 0.0 || v.y != 0.0);
         v = make_double2(0.0, 0.0);
@@ -259,24 +255,20 @@ __global__ void __launch_bounds__(kRowThreads, 1) hv_rows_gauge_kernel(DevSector
   }
 }
 
-// kFused: the input is sx * x; the up-hop sum is formed on its own and added as
-// y = y_rows + sx * sum, and the thread's share of <sx x, y> over its columns goes to dot
-// (the Lanczos step's alpha without a separate pass: x[r, c] is in the L2-resident slab).
-template <int kColThreads, bool kFilter, bool kFused>
+template <int kColThreads, bool kFilter>
 __device__ __forceinline__ void cols_body(const DevSector& S, const double2* __restrict__ x, double2* __restrict__ y,
                                           int64_t r, int64_t c0, int deg, const int64_t* s_off, const double2* s_coef,
-                                          const uint32_t* s_lh, double sx, double (&dot)[2]) {
+                                          const uint32_t* s_lh) {
   const int64_t c1 = c0 + kColThreads;
   const bool has1 = c1 < S.Dd;
   const int64_t c1s = has1 ? c1 : c0;  // in-bounds column for the second lane slot
   const uint32_t q0 = prefix_parity_shifted(S.dmask[c0]);
   const uint32_t q1 = prefix_parity_shifted(S.dmask[c1s]);
   double2* y0 = y + r * S.Dd + c0;
-  double2 acc0 = kFused ? make_double2(0.0, 0.0) : *y0;
-  double2 acc1 = (has1 && !kFused) ? y[r * S.Dd + c1] : make_double2(0.0, 0.0);
+  double2 acc0 = *y0;
+  double2 acc1 = has1 ? y[r * S.Dd + c1] : make_double2(0.0, 0.0);
   const double2* x0 = x + c0;
   const double2* x1 = x + c1s;
-  auto skip = [sx](double2 v) { return kFused ? tiny(make_double2(sx * v.x, sx * v.y)) : tiny(v); };
   int j = 0;
   for (; j + 4 <= deg; j += 4) {
     double2 v0[4], v1[4];
@@ -291,8 +283,8 @@ __device__ __forceinline__ void cols_body(const DevSector& S, const double2* __r
       const uint32_t lh = s_lh[j + t];
       const uint32_t lo = lh & 255u, hi = lh >> 8;
       const double2 cf = s_coef[j + t];
-      if (!kFilter || !skip(v0[t])) cmac_xor(acc0, cf, v0[t], ((q0 >> lo) ^ (q0 >> hi)) & 1u);
-      if (!kFilter || !skip(v1[t])) cmac_xor(acc1, cf, v1[t], ((q1 >> lo) ^ (q1 >> hi)) & 1u);
+      if (!kFilter || !tiny(v0[t])) cmac_xor(acc0, cf, v0[t], ((q0 >> lo) ^ (q0 >> hi)) & 1u);
+      if (!kFilter || !tiny(v1[t])) cmac_xor(acc1, cf, v1[t], ((q1 >> lo) ^ (q1 >> hi)) & 1u);
     }
   }
   for (; j < deg; ++j) {
@@ -301,24 +293,8 @@ __device__ __forceinline__ void cols_body(const DevSector& S, const double2* __r
     const uint32_t lh = s_lh[j];
     const uint32_t lo = lh & 255u, hi = lh >> 8;
     const double2 cf = s_coef[j];
-    if (!kFilter || !skip(v0)) cmac_xor(acc0, cf, v0, ((q0 >> lo) ^ (q0 >> hi)) & 1u);
-    if (!kFilter || !skip(v1)) cmac_xor(acc1, cf, v1, ((q1 >> lo) ^ (q1 >> hi)) & 1u);
-  }
-  if constexpr (kFused) {
-    const double2 r0 = *y0;
-    acc0 = make_double2(fma(sx, acc0.x, r0.x), fma(sx, acc0.y, r0.y));
-    const double2 xq0 = x[r * S.Dd + c0];
-    const double qx = sx * xq0.x, qy = sx * xq0.y;  // conj(q) * y
-    dot[0] += qx * acc0.x + qy * acc0.y;
-    dot[1] += qx * acc0.y - qy * acc0.x;
-    if (has1) {
-      const double2 r1 = y[r * S.Dd + c1];
-      acc1 = make_double2(fma(sx, acc1.x, r1.x), fma(sx, acc1.y, r1.y));
-      const double2 xq1 = x[r * S.Dd + c1];
-      const double px = sx * xq1.x, py = sx * xq1.y;
-      dot[0] += px * acc1.x + py * acc1.y;
-      dot[1] += px * acc1.y - py * acc1.x;
-    }
+    if (!kFilter || !tiny(v0)) cmac_xor(acc0, cf, v0, ((q0 >> lo) ^ (q0 >> hi)) & 1u);
+    if (!kFilter || !tiny(v1)) cmac_xor(acc1, cf, v1, ((q1 >> lo) ^ (q1 >> hi)) & 1u);
   }
   *y0 = acc0;
   if (has1) y[r * S.Dd + c1] = acc1;
@@ -330,23 +306,22 @@ __device__ __forceinline__ void cols_body(const DevSector& S, const double2* __r
 // two FMAs per column instead of a complex multiply, and the list costs a quarter of a shared load per
 // source instead of three.  The kind of each source is the same for every thread of the block, so
 // the phase test does not diverge.  Same products and sums as cols_body on the CSR list.
-template <int kColThreads, bool kFilter, bool kFused>
+template <int kColThreads, bool kFilter>
 __device__ __forceinline__ void cols_body_packed(const DevSector& S, const double2* __restrict__ x,
                                                  double2* __restrict__ y, int64_t r, int64_t c0, int deg,
-                                                 const uint32_t* s_pk, double sx, double (&dot)[2]) {
+                                                 const uint32_t* s_pk) {
   const int64_t c1 = c0 + kColThreads;
   const bool has1 = c1 < S.Dd;
   const int64_t c1s = has1 ? c1 : c0;
   const uint32_t q0 = prefix_parity_shifted(S.dmask[c0]);
   const uint32_t q1 = prefix_parity_shifted(S.dmask[c1s]);
   double2* y0 = y + r * S.Dd + c0;
-  double2 acc0 = kFused ? make_double2(0.0, 0.0) : *y0;
-  double2 acc1 = (has1 && !kFused) ? y[r * S.Dd + c1] : make_double2(0.0, 0.0);
+  double2 acc0 = *y0;
+  double2 acc1 = has1 ? y[r * S.Dd + c1] : make_double2(0.0, 0.0);
   const double2* x0 = x + c0;
   const double2* x1 = x + c1s;
   const int64_t Dd = S.Dd;
   const double a0 = S.up_real2[0], a1 = S.up_real2[1], pc = S.up_pc, ps = S.up_ps;
-  auto skip = [sx](double2 v) { return kFused ? tiny(make_double2(sx * v.x, sx * v.y)) : tiny(v); };
   auto term = [&](uint32_t pk, double2 v0, double2 v1) {
     const uint32_t lo = (pk >> 14) & 31u, hi = (pk >> 19) & 31u;
     const double cf = flip_sign((pk & 0x40000000u) ? a1 : a0, pk >> 31);
@@ -355,15 +330,15 @@ __device__ __forceinline__ void cols_body_packed(const DevSector& S, const doubl
       const double cr = cf * pc;
       const double ci = flip_sign(cf * ps, (pk >> 28) & 1u);
       const double2 c = make_double2(cr, ci);
-      if (!kFilter || !skip(v0)) cmac_xor(acc0, c, v0, f0);
-      if (!kFilter || !skip(v1)) cmac_xor(acc1, c, v1, f1);
+      if (!kFilter || !tiny(v0)) cmac_xor(acc0, c, v0, f0);
+      if (!kFilter || !tiny(v1)) cmac_xor(acc1, c, v1, f1);
     } else {
-      if (!kFilter || !skip(v0)) {
+      if (!kFilter || !tiny(v0)) {
         const double c = flip_sign(cf, f0);
         acc0.x = fma(c, v0.x, acc0.x);
         acc0.y = fma(c, v0.y, acc0.y);
       }
-      if (!kFilter || !skip(v1)) {
+      if (!kFilter || !tiny(v1)) {
         const double c = flip_sign(cf, f1);
         acc1.x = fma(c, v1.x, acc1.x);
         acc1.y = fma(c, v1.y, acc1.y);
@@ -389,32 +364,14 @@ __device__ __forceinline__ void cols_body_packed(const DevSector& S, const doubl
     const int64_t off = static_cast<int64_t>(pk & 0x3FFFu) * Dd;
     term(pk, x0[off], x1[off]);
   }
-  if constexpr (kFused) {
-    const double2 r0 = *y0;
-    acc0 = make_double2(fma(sx, acc0.x, r0.x), fma(sx, acc0.y, r0.y));
-    const double2 xq0 = x[r * S.Dd + c0];
-    const double qx = sx * xq0.x, qy = sx * xq0.y;  // conj(q) * y
-    dot[0] += qx * acc0.x + qy * acc0.y;
-    dot[1] += qx * acc0.y - qy * acc0.x;
-    if (has1) {
-      const double2 r1 = y[r * S.Dd + c1];
-      acc1 = make_double2(fma(sx, acc1.x, r1.x), fma(sx, acc1.y, r1.y));
-      const double2 xq1 = x[r * S.Dd + c1];
-      const double px = sx * xq1.x, py = sx * xq1.y;
-      dot[0] += px * acc1.x + py * acc1.y;
-      dot[1] += px * acc1.y - py * acc1.x;
-    }
-  }
   *y0 = acc0;
   if (has1) y[r * S.Dd + c1] = acc1;
 }
 
-// At least 896 resident threads per SM (28 warps): the L2 gathers need the bytes in flight, and the
-// fused form would otherwise take a few registers more and drop to 24 warps.
-template <int kColThreads, bool kFused, bool kPacked>
+// At least 896 resident threads per SM (28 warps): the L2 gathers need the bytes in flight.
+template <int kColThreads, bool kPacked>
 __global__ void __launch_bounds__(kColThreads, 896 / kColThreads) hv_cols_kernel(DevSector S, const double2* __restrict__ x,
-                                                              double2* __restrict__ y, double sx,
-                                                              double* __restrict__ dotp) {
+                                                              double2* __restrict__ y) {
   constexpr int kColChunk = 2 * kColThreads;
   constexpr int kListDeg = kPacked ? 4 : kMaxUpDeg;  // the list arrays of the form this launch does not use
   __shared__ int64_t s_off[kListDeg];
@@ -438,43 +395,17 @@ __global__ void __launch_bounds__(kColThreads, 896 / kColThreads) hv_cols_kernel
   const bool filt = (*S.flags) != 0;
   __syncthreads();
   const int64_t c0 = chunk * kColChunk + threadIdx.x;
-  double dot[2] = {0.0, 0.0};
   if (c0 < S.Dd) {
     if constexpr (kPacked) {
       if (filt)
-        cols_body_packed<kColThreads, true, kFused>(S, x, y, r, c0, deg, s_pk, sx, dot);
+        cols_body_packed<kColThreads, true>(S, x, y, r, c0, deg, s_pk);
       else
-        cols_body_packed<kColThreads, false, kFused>(S, x, y, r, c0, deg, s_pk, sx, dot);
+        cols_body_packed<kColThreads, false>(S, x, y, r, c0, deg, s_pk);
     } else {
       if (filt)
-        cols_body<kColThreads, true, kFused>(S, x, y, r, c0, deg, s_off, s_coef, s_lh, sx, dot);
+        cols_body<kColThreads, true>(S, x, y, r, c0, deg, s_off, s_coef, s_lh);
       else
-        cols_body<kColThreads, false, kFused>(S, x, y, r, c0, deg, s_off, s_coef, s_lh, sx, dot);
-    }
-  }
-  if constexpr (kFused) {  // fixed tree over the block (warp shuffles, then warps in order): one partial
-    constexpr int kWarps = kColThreads / 32;
-    __shared__ double red[2][kWarps];
-#pragma unroll
-    for (int h = 16; h > 0; h >>= 1) {
-      dot[0] += __shfl_down_sync(0xFFFFFFFFu, dot[0], h);
-      dot[1] += __shfl_down_sync(0xFFFFFFFFu, dot[1], h);
-    }
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (lane == 0) {
-      red[0][warp] = dot[0];
-      red[1][warp] = dot[1];
-    }
-    __syncthreads();
-    if (threadIdx.x == 0 && dotp) {
-      double s0 = red[0][0], s1 = red[1][0];
-#pragma unroll
-      for (int w = 1; w < kWarps; ++w) {
-        s0 += red[0][w];
-        s1 += red[1][w];
-      }
-      dotp[2 * b] = s0;
-      dotp[2 * b + 1] = s1;
+        cols_body<kColThreads, false>(S, x, y, r, c0, deg, s_off, s_coef, s_lh);
     }
   }
 }
@@ -502,32 +433,18 @@ void init_sm_count() {
 }
 
 template <int kThreads>
-cudaError_t launch_cols(const DevSector& S, const double2* x, double2* y, cudaStream_t st, double sx, double* dotp) {
+cudaError_t launch_cols(const DevSector& S, const double2* x, double2* y, cudaStream_t st) {
   const int64_t nchunks = (S.Dd + 2 * kThreads - 1) / (2 * kThreads);
   const unsigned grid = static_cast<unsigned>(nchunks * S.Du);
-  const bool fused = dotp || sx != 1.0;
-  if (S.up_pk) {
-    if (fused)
-      hv_cols_kernel<kThreads, true, true><<<grid, kThreads, 0, st>>>(S, x, y, sx, dotp);
-    else
-      hv_cols_kernel<kThreads, false, true><<<grid, kThreads, 0, st>>>(S, x, y, sx, dotp);
-  } else {
-    if (fused)
-      hv_cols_kernel<kThreads, true, false><<<grid, kThreads, 0, st>>>(S, x, y, sx, dotp);
-    else
-      hv_cols_kernel<kThreads, false, false><<<grid, kThreads, 0, st>>>(S, x, y, sx, dotp);
-  }
+  if (S.up_pk)
+    hv_cols_kernel<kThreads, true><<<grid, kThreads, 0, st>>>(S, x, y);
+  else
+    hv_cols_kernel<kThreads, false><<<grid, kThreads, 0, st>>>(S, x, y);
   return cudaGetLastError();
 }
 
-int64_t hv_cols_blocks(const DevSector& S, int cols_variant) {
-  cols_variant %= 3;  // 3..5: the same slabs over the packed list
-  const int threads = cols_variant == 1 ? 64 : (cols_variant == 2 ? 256 : 128);
-  return (S.Dd + 2 * threads - 1) / (2 * threads) * S.Du;
-}
-
 cudaError_t hv_launch_pass(const DevSector& S, const double2* x, double2* y, int pass, cudaStream_t st,
-                           int cols_variant, double sx, double* dotp) {
+                           int cols_variant) {
   if (S.dim <= 0) return cudaSuccess;
   init_sm_count();
   if (pass == 0) {
@@ -540,13 +457,13 @@ cudaError_t hv_launch_pass(const DevSector& S, const double2* x, double2* y, int
     e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sm));
     if (e != cudaSuccess) return e;
     const int grid_r = static_cast<int>(std::min<int64_t>(S.Du, g_num_sms));
-    k<<<grid_r, kRowThreads, sm, st>>>(S, x, y, sx);
+    k<<<grid_r, kRowThreads, sm, st>>>(S, x, y);
     return cudaGetLastError();
   }
   cols_variant %= 3;  // 3..5: the same slabs; the list form comes with S (S.up_pk)
-  if (cols_variant == 1) return launch_cols<64>(S, x, y, st, sx, dotp);
-  if (cols_variant == 2) return launch_cols<256>(S, x, y, st, sx, dotp);
-  return launch_cols<128>(S, x, y, st, sx, dotp);
+  if (cols_variant == 1) return launch_cols<64>(S, x, y, st);
+  if (cols_variant == 2) return launch_cols<256>(S, x, y, st);
+  return launch_cols<128>(S, x, y, st);
 }
 
 cudaError_t hv_launch(const DevSector& S, const double2* x, double2* y, int path, cudaStream_t st, int cols_variant) {

@@ -2,6 +2,7 @@
 // a fixed grid of kRedBlocks blocks, a fixed in-block tree, and a single-block final pass, so
 // repeated runs give bitwise identical alpha/beta.
 #include "hv.cuh"
+#include "philox.cuh"
 
 namespace ftlm_b200 {
 
@@ -86,53 +87,6 @@ __global__ void __launch_bounds__(kRedThreads) update_kernel(double2* __restrict
   if (threadIdx.x == 0) partial[blockIdx.x] = v[0];
 }
 
-// Lanczos update with the scales of the unnormalised vectors applied on the fly.
-__global__ void __launch_bounds__(kRedThreads) update_scaled_kernel(double2* __restrict__ w,
-                                                                    const double2* __restrict__ Wk, double sk,
-                                                                    const double2* __restrict__ Wkm1, double skm1,
-                                                                    const double* __restrict__ zp, double bprev,
-                                                                    int use_prev, int64_t n,
-                                                                    double* __restrict__ partial) {
-  __shared__ double sh[kRedThreads];
-  const double zr = zp[0], zi = zp[1];
-  double v[1] = {0.0};
-  const int64_t stride = static_cast<int64_t>(gridDim.x) * kRedThreads;
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * kRedThreads + threadIdx.x; i < n; i += stride) {
-    double2 a = w[i];
-    const double2 b0 = Wk[i];
-    const double bx = sk * b0.x, by = sk * b0.y;
-    a.x -= zr * bx - zi * by;
-    a.y -= zr * by + zi * bx;
-    if (use_prev) {
-      const double2 c = Wkm1[i];
-      a.x -= bprev * (skm1 * c.x);
-      a.y -= bprev * (skm1 * c.y);
-    }
-    w[i] = a;
-    v[0] += a.x * a.x + a.y * a.y;
-  }
-  block_sum<1>(v, sh);
-  if (threadIdx.x == 0) partial[blockIdx.x] = v[0];
-}
-
-// First level of a pair reduction: block b sums pairs [b*per, (b+1)*per) in order.
-__global__ void __launch_bounds__(kRedThreads) pairs_kernel(const double* __restrict__ in, int64_t nb, int64_t per,
-                                                            double* __restrict__ out) {
-  __shared__ double sh[2 * kRedThreads];
-  double v[2] = {0.0, 0.0};
-  const int64_t b0 = static_cast<int64_t>(blockIdx.x) * per;
-  const int64_t b1 = min(nb, b0 + per);
-  for (int64_t i = b0 + threadIdx.x; i < b1; i += kRedThreads) {
-    v[0] += in[2 * i];
-    v[1] += in[2 * i + 1];
-  }
-  block_sum<2>(v, sh);
-  if (threadIdx.x == 0) {
-    out[2 * blockIdx.x] = v[0];
-    out[2 * blockIdx.x + 1] = v[1];
-  }
-}
-
 __global__ void scale_kernel(double2* __restrict__ dst, const double2* __restrict__ src, int64_t n,
                              const double* __restrict__ nw2) {
   const double b = sqrt(*nw2);
@@ -143,37 +97,13 @@ __global__ void scale_kernel(double2* __restrict__ dst, const double2* __restric
   }
 }
 
-// Philox4x32-10 (Salmon, Moraes, Dror, Shaw, SC'11): 10 rounds of the 4x32 S-box with the
-// published multipliers and Weyl key increments.
-__device__ __forceinline__ uint4 philox4x32_10(uint4 c, uint2 k) {
-  constexpr uint32_t M0 = 0xD2511F53u, M1 = 0xCD9E8D57u, W0 = 0x9E3779B9u, W1 = 0xBB67AE85u;
-#pragma unroll
-  for (int r = 0; r < 10; ++r) {
-    const uint32_t hi0 = __umulhi(M0, c.x), lo0 = M0 * c.x;
-    const uint32_t hi1 = __umulhi(M1, c.z), lo1 = M1 * c.z;
-    c = make_uint4(hi1 ^ c.y ^ k.x, lo1, hi0 ^ c.w ^ k.y, lo0);
-    k.x += W0;
-    k.y += W1;
-  }
-  return c;
-}
-
 __global__ void __launch_bounds__(kRedThreads) philox_start_kernel(double2* __restrict__ q, int64_t n, unsigned seed,
                                                                    double* __restrict__ partial) {
   __shared__ double sh[kRedThreads];
   double v[1] = {0.0};
   const int64_t stride = static_cast<int64_t>(gridDim.x) * kRedThreads;
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * kRedThreads + threadIdx.x; i < n; i += stride) {
-    const uint4 r = philox4x32_10(make_uint4(static_cast<uint32_t>(i), static_cast<uint32_t>(i >> 32), 0u, 0u),
-                                  make_uint2(seed, 0x7F4A7C15u));
-    const uint64_t a = (static_cast<uint64_t>(r.x) << 21) ^ (r.y >> 11);
-    const uint64_t b = (static_cast<uint64_t>(r.z) << 21) ^ (r.w >> 11);
-    const double u1 = (static_cast<double>(a & ((1ull << 53) - 1)) + 0.5) * 0x1.0p-53;  // (0,1)
-    const double u2 = (static_cast<double>(b & ((1ull << 53) - 1)) + 0.5) * 0x1.0p-53;
-    const double rad = sqrt(-2.0 * log(u1));
-    double s, c;
-    sincospi(2.0 * u2, &s, &c);
-    const double2 z = make_double2(rad * c, rad * s);
+    const double2 z = philox_normal(i, seed);
     q[i] = z;
     v[0] += z.x * z.x + z.y * z.y;
   }
@@ -207,21 +137,6 @@ cudaError_t lz_dotc(const double2* q, const double2* w, int64_t n, double* scrat
 cudaError_t lz_update(double2* w, const double2* q, const double2* qp, double bprev, int use_prev, int64_t n,
                       double* scratch, cudaStream_t st) {
   update_kernel<<<kRedBlocks, kRedThreads, 0, st>>>(w, q, qp, scratch + kResZ, bprev, use_prev, n, scratch);
-  final_kernel<1><<<1, kRedThreads, 0, st>>>(scratch, kRedBlocks, scratch + kResNw2);
-  return cudaGetLastError();
-}
-
-cudaError_t lz_reduce_pairs(const double* partial, int64_t nb, double* scratch, cudaStream_t st) {
-  const int64_t per = (nb + kRedBlocks - 1) / kRedBlocks;
-  pairs_kernel<<<kRedBlocks, kRedThreads, 0, st>>>(partial, nb, per, scratch);
-  final_kernel<2><<<1, kRedThreads, 0, st>>>(scratch, kRedBlocks, scratch + kResZ);
-  return cudaGetLastError();
-}
-
-cudaError_t lz_update_scaled(double2* w, const double2* Wk, double sk, const double2* Wkm1, double skm1, double bprev,
-                             int use_prev, int64_t n, double* scratch, cudaStream_t st) {
-  update_scaled_kernel<<<kRedBlocks, kRedThreads, 0, st>>>(w, Wk, sk, Wkm1, skm1, scratch + kResZ, bprev, use_prev, n,
-                                                          scratch);
   final_kernel<1><<<1, kRedThreads, 0, st>>>(scratch, kRedBlocks, scratch + kResNw2);
   return cudaGetLastError();
 }

@@ -31,13 +31,13 @@ constexpr int kMaxDeg = 128;       // up sources of a string
 constexpr int kStreamBlocks = 592; // start / update: blocks over all planes (4 per SM of 148, a multiple of 16)
 constexpr size_t kMaxSmem = 227 * 1024;
 
-// Start vectors: chain c of the group uses Philox4x32-10 with key seed + c*100003 and counter = state index, the
+// Start vectors: given ones (in W already, in the sector's order), or chain c of the group uses Philox4x32-10 with key seed + c*100003 and counter = state index, the
 // stream of FTLM_START_PHILOX, rounded to the chains' type and expressed in the gauge basis (W = G r).
 template <class P>
 __global__ void __launch_bounds__(kThreads) start_kernel(typename P::T* __restrict__ W, int64_t dim, unsigned seed, int nb,
                                                          double* __restrict__ partial, int* __restrict__ flag,
                                                          const uint32_t* __restrict__ umask,
-                                                         const uint32_t* __restrict__ dmask, int64_t Dd) {
+                                                         const uint32_t* __restrict__ dmask, int64_t Dd, bool given) {
   __shared__ double sh[P::kC * kThreads / 32];
   const int plane = blockIdx.x / nb, b = blockIdx.x - plane * nb;
   const unsigned key = seed + static_cast<unsigned>(P::kC * plane) * 100003u;
@@ -49,7 +49,13 @@ __global__ void __launch_bounds__(kThreads) start_kernel(typename P::T* __restri
     decltype(P::narrow(0.0, 0.0)) z[P::kC];
 #pragma unroll
     for (int q = 0; q < P::kC; ++q) {
-      const double2 n = philox_normal(i, key + static_cast<unsigned>(q) * 100003u);
+      double2 n;
+      if (given) {
+        const auto v = P::get(out[i], q);
+        n = make_double2(v.x, v.y);
+      } else {
+        n = philox_normal(i, key + static_cast<unsigned>(q) * 100003u);
+      }
       z[q] = P::narrow(g * n.x, g * n.y);
       acc[q].add(static_cast<double>(z[q].x) * z[q].x + static_cast<double>(z[q].y) * z[q].y);
     }
@@ -78,7 +84,7 @@ __device__ __forceinline__ void prefetch_l2(const void* from, uint32_t bytes) {
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p + off), "r"(min(32768u, bytes - off)) : "memory");
 }
 
-template <class P, int kP, bool kPhase>
+template <class P, int kP, bool kPhase, bool kXor>
 __global__ void __launch_bounds__(1024, 1) rows_kernel(DevSector S, const typename P::T* __restrict__ W,
                                                        typename P::T* __restrict__ Y, int planes,
                                                        const double* __restrict__ st, int* __restrict__ flag) {
@@ -90,7 +96,7 @@ __global__ void __launch_bounds__(1024, 1) rows_kernel(DevSector S, const typena
   typename P::Cf* tab = reinterpret_cast<typename P::Cf*>(smem_raw + kP * line);
   const int tid = threadIdx.x;
   const DevGauge G = S.dn_g;
-  const RowCoefs<P> rc(G);
+  const RowCoefs<P, kXor> rc(G);
   const bool filter = !P::kScaled && *flag != 0;
   if (!kPhase)
     for (int i = tid; i < G.nt * 8; i += nt) tab[i] = P::coef(G.tab[i >> 3]);
@@ -134,7 +140,7 @@ __global__ void __launch_bounds__(1024, 1) rows_kernel(DevSector S, const typena
     for (int c = tid; c < Dd; c += nt) {
       const int d = gauge_string(G, c);  // table position c serves output string d
       const double dg = diag_value(S, u, S.dmask[d], cuu, S.cnt_dd[d], wp);
-      RowSum<P, kP, kPhase> s;
+      RowSum<P, kP, kPhase, kXor> s;
       s.line = line;
       s.base = smem_raw;
 #pragma unroll
@@ -214,7 +220,7 @@ __device__ __forceinline__ void cols_sum(const typename P::T* __restrict__ x0, c
 }
 
 template <class P, int kT, bool kDot>
-__global__ void __launch_bounds__(kT, 1024 / kT) cols_kernel(DevSector S, const typename P::T* __restrict__ W,
+__global__ void __launch_bounds__(kT, P::kColThreads / kT) cols_kernel(DevSector S, const typename P::T* __restrict__ W,
                                                              typename P::T* __restrict__ Y, int planes,
                                                              const double* __restrict__ st, double* __restrict__ partial,
                                                              const int* __restrict__ flag) {
@@ -299,6 +305,81 @@ __global__ void __launch_bounds__(kT, 1024 / kT) cols_kernel(DevSector S, const 
   }
 }
 
+// The same, one block per item and one partial per item (items [plane][item][2 kC]): the hardware hands the items out in
+// order, so that all blocks stay within a chunk or two of each other and the slab stays in L2, where blocks of the
+// persistent grid drift apart over the hundreds of items that a large plane gives each of them.
+template <class P, int kT, bool kDot>
+__global__ void __launch_bounds__(kT, P::kColThreads / kT) cols_items_kernel(DevSector S, const typename P::T* __restrict__ W,
+                                                                             typename P::T* __restrict__ Y, uint32_t per,
+                                                                             const double* __restrict__ st,
+                                                                             double* __restrict__ items,
+                                                                             const int* __restrict__ flag) {
+  using T = typename P::T;
+  __shared__ uint32_t s_off[kMaxDeg];
+  __shared__ __align__(16) typename P::Cf s_cf[kMaxDeg];
+  __shared__ double sh[2 * P::kC * kT / 32];
+  const int t = threadIdx.x;
+  const bool filter = *flag != 0;
+  const uint32_t Dd = static_cast<uint32_t>(S.Dd), Du = static_cast<uint32_t>(S.Du);
+  const uint32_t p = blockIdx.x / per, it = blockIdx.x - p * per, chunk = it / Du, r = it - chunk * Du;
+  const int j0 = S.up_ptr[r], deg = S.up_ptr[r + 1] - j0;
+  for (int j = t; j < deg; j += kT) {
+    s_off[j] = static_cast<uint32_t>(S.up_src[j0 + j]) * Dd;
+    s_cf[j] = P::up_coef(S, j0 + j);
+  }
+  const T* Wp = W + static_cast<int64_t>(p) * S.dim;
+  T* Yp = Y + static_cast<int64_t>(p) * S.dim;
+  const double sx = P::kScaled && st ? st[kBtSin * 32 + p] : 1.0;
+  const uint32_t c0 = chunk * (2 * kT) + t, c1 = c0 + kT;
+  double d[2 * P::kC] = {};
+  __syncthreads();
+  if (c0 < Dd) {
+    const bool has1 = c1 < Dd;
+    const uint32_t c1s = has1 ? c1 : c0;
+    T a0, a1;
+    if (filter)
+      cols_sum<P, true>(Wp + c0, Wp + c1s, s_off, s_cf, deg, sx, a0, a1);
+    else
+      cols_sum<P, false>(Wp + c0, Wp + c1s, s_off, s_cf, deg, sx, a0, a1);
+    const uint32_t o0 = r * Dd + c0, o1 = r * Dd + c1s;
+    const T y0 = P::add_scaled(Yp[o0], a0, sx);
+    if (kDot) P::dot(d, Wp[o0], y0, sx);
+    Yp[o0] = y0;
+    if (has1) {
+      const T y1 = P::add_scaled(Yp[o1], a1, sx);
+      if (kDot) P::dot(d, Wp[o1], y1, sx);
+      Yp[o1] = y1;
+    }
+  }
+  if (kDot) {
+    block_totals<2 * P::kC, kT>(d, sh);
+    if (t == 0) {
+#pragma unroll
+      for (int v = 0; v < 2 * P::kC; ++v) items[static_cast<int64_t>(blockIdx.x) * (2 * P::kC) + v] = d[v];
+    }
+  }
+}
+
+// First level of the items' sums: block (plane, b) of nb adds its share of the plane's items into partial slot b.
+template <int kC>
+__global__ void __launch_bounds__(kThreads) fold_kernel(const double* __restrict__ items, uint32_t per, int nb,
+                                                        double* __restrict__ partial) {
+  __shared__ double sh[2 * kC * kThreads / 32];
+  const int plane = blockIdx.x / nb, b = blockIdx.x - plane * nb;
+  const uint32_t share = (per + nb - 1) / nb, i0 = b * share, i1 = min(per, i0 + share);
+  const double* in = items + static_cast<int64_t>(plane) * per * (2 * kC);
+  double d[2 * kC] = {};
+  for (uint32_t i = i0 + threadIdx.x; i < i1; i += kThreads) {
+#pragma unroll
+    for (int v = 0; v < 2 * kC; ++v) d[v] += in[static_cast<int64_t>(i) * (2 * kC) + v];
+  }
+  block_totals<2 * kC, kThreads>(d, sh);
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int v = 0; v < 2 * kC; ++v) partial[(static_cast<int64_t>(b) * 32 + kC * plane) * 2 + v] = d[v];
+  }
+}
+
 // W_{k+1} = s_in Y - c1 W_k - c2 W_{k-1} (in Y's buffer, FP64 then rounded), ||W_{k+1}||^2 partials per chain.  Streams
 // three vectors in and one out.
 template <class P>
@@ -366,13 +447,21 @@ int sm_count() {
   return n;
 }
 
+// Lines that the row pass can stage: 2, 1, or 0 (no gauge table, or a row does not fit).
+template <class P>
+int row_planes(const DevSector& S) {
+  const size_t line = static_cast<size_t>(S.Dd + 8) * 16;
+  const size_t tab = S.dn_g.phase ? 0 : static_cast<size_t>(S.dn_g.nt) * 8 * sizeof(typename P::Cf);
+  return !S.dn_g.ent || line + tab > kMaxSmem ? 0 : 2 * line + tab <= kMaxSmem ? 2 : 1;
+}
+
 // Planes per item and threads of the row pass: two planes where two lines fit, so that the entries are read once for
 // both; blocks no wider than a row, several on an SM, so that one block's staging overlaps another's hops (a single
 // 1024-thread block leaves the SM idle while it stages, and most of its threads where a row is short).
-template <class P, int kP, bool kPhase>
+template <class P, int kP, bool kPhase, bool kXor>
 cudaError_t launch_rows_p(const DevSector& S, const typename P::T* W, typename P::T* Y, int planes, const double* st,
                           int* flag, cudaStream_t s) {
-  const auto k = rows_kernel<P, kP, kPhase>;
+  const auto k = rows_kernel<P, kP, kPhase, kXor>;
   const size_t sm = static_cast<size_t>(kP) * (S.Dd + 8) * 16 + (kPhase ? 0 : S.dn_g.nt * 8 * sizeof(typename P::Cf));
   const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sm));
   if (e != cudaSuccess) return e;
@@ -386,49 +475,72 @@ cudaError_t launch_rows_p(const DevSector& S, const typename P::T* W, typename P
   return cudaGetLastError();
 }
 
+template <class P, int kP>
+cudaError_t launch_rows_n(const DevSector& S, const typename P::T* W, typename P::T* Y, int planes, const double* st,
+                          int* flag, cudaStream_t s) {
+  if (S.dn_g.phase)
+    return S.dn_g.xor_real ? launch_rows_p<P, kP, true, true>(S, W, Y, planes, st, flag, s)
+                           : launch_rows_p<P, kP, true, false>(S, W, Y, planes, st, flag, s);
+  return S.dn_g.xor_real ? launch_rows_p<P, kP, false, true>(S, W, Y, planes, st, flag, s)
+                         : launch_rows_p<P, kP, false, false>(S, W, Y, planes, st, flag, s);
+}
+
 template <class P>
 cudaError_t launch_rows(const DevSector& S, const typename P::T* W, typename P::T* Y, int planes, const double* st,
                         int* flag, cudaStream_t s) {
-  const size_t line = static_cast<size_t>(S.Dd + 8) * 16;
-  const size_t tab = S.dn_g.phase ? 0 : static_cast<size_t>(S.dn_g.nt) * 8 * sizeof(typename P::Cf);
-  if (S.dn_g.ent && planes > 1 && 2 * line + tab <= kMaxSmem)
-    return S.dn_g.phase ? launch_rows_p<P, 2, true>(S, W, Y, planes, st, flag, s)
-                        : launch_rows_p<P, 2, false>(S, W, Y, planes, st, flag, s);
-  if (S.dn_g.ent && line + tab <= kMaxSmem)
-    return S.dn_g.phase ? launch_rows_p<P, 1, true>(S, W, Y, planes, st, flag, s)
-                        : launch_rows_p<P, 1, false>(S, W, Y, planes, st, flag, s);
-  const int64_t blocks = std::min<int64_t>((S.dim * planes + kThreads - 1) / kThreads, static_cast<int64_t>(sm_count()) * 16);
-  rows_gather_kernel<P><<<static_cast<unsigned>(blocks), kThreads, 0, s>>>(S, W, Y, planes, flag);
-  return cudaGetLastError();
+  const int rp = row_planes<P>(S);
+  if (rp == 2 && planes > 1) return launch_rows_n<P, 2>(S, W, Y, planes, st, flag, s);
+  if (rp > 0) return launch_rows_n<P, 1>(S, W, Y, planes, st, flag, s);
+  if constexpr (P::kScaled) {
+    return cudaErrorNotSupported;  // pl_fits
+  } else {
+    const int64_t blocks = std::min<int64_t>((S.dim * planes + kThreads - 1) / kThreads, static_cast<int64_t>(sm_count()) * 16);
+    rows_gather_kernel<P><<<static_cast<unsigned>(blocks), kThreads, 0, s>>>(S, W, Y, planes, flag);
+    return cudaGetLastError();
+  }
 }
 
 template <class P, int kT>
 int launch_cols_t(const DevSector& S, const typename P::T* W, typename P::T* Y, int planes, const double* st,
-                  double* partial, const int* flag, cudaStream_t s) {
-  const int64_t items = (S.Dd + 2 * kT - 1) / (2 * kT) * S.Du * planes;
-  const int grid = static_cast<int>(std::min<int64_t>({items, static_cast<int64_t>(sm_count()) * (1024 / kT), kPlMaxBlocks}));
+                  double* partial, double* items, const int* flag, cudaStream_t s) {
+  const int64_t per = (S.Dd + 2 * kT - 1) / (2 * kT) * S.Du;
+  const int64_t grid = std::min<int64_t>({per * planes, static_cast<int64_t>(sm_count()) * (P::kColThreads / kT), kPlMaxBlocks});
+  // From 8 items of a plane for each block of the persistent grid, one block per item: 4x4 (6,6) complex128 2.19 -> 1.86 ms,
+  // 4x4 (5,6) complex64 1.09 -> 0.97 ms a plane; below, the persistent grid's prefetched lists: 4x3 (4,5) 40 us, 44 by items.
+  if (per >= 8 * grid && per * planes <= INT32_MAX) {
+    const unsigned n = static_cast<unsigned>(per * planes);
+    if (!partial) {
+      cols_items_kernel<P, kT, false><<<n, kT, 0, s>>>(S, W, Y, static_cast<uint32_t>(per), st, nullptr, flag);
+      return 0;
+    }
+    cols_items_kernel<P, kT, true><<<n, kT, 0, s>>>(S, W, Y, static_cast<uint32_t>(per), st, items, flag);
+    const int nb = std::max(1, kStreamBlocks / planes);
+    fold_kernel<P::kC><<<nb * planes, kThreads, 0, s>>>(items, static_cast<uint32_t>(per), nb, partial);
+    return nb;
+  }
   if (partial)
-    cols_kernel<P, kT, true><<<grid, kT, 0, s>>>(S, W, Y, planes, st, partial, flag);
+    cols_kernel<P, kT, true><<<static_cast<unsigned>(grid), kT, 0, s>>>(S, W, Y, planes, st, partial, flag);
   else
-    cols_kernel<P, kT, false><<<grid, kT, 0, s>>>(S, W, Y, planes, st, partial, flag);
-  return grid;
+    cols_kernel<P, kT, false><<<static_cast<unsigned>(grid), kT, 0, s>>>(S, W, Y, planes, st, partial, flag);
+  return static_cast<int>(grid);
 }
 
 // Returns the grid: the number of partials per chain.
 template <class P>
 int launch_cols(const DevSector& S, const typename P::T* W, typename P::T* Y, int planes, const double* st,
-                double* partial, const int* flag, cudaStream_t s) {
-  if (S.bt_cols == 1) return launch_cols_t<P, 64>(S, W, Y, planes, st, partial, flag, s);
-  if (S.bt_cols == 2) return launch_cols_t<P, 256>(S, W, Y, planes, st, partial, flag, s);
-  return launch_cols_t<P, 128>(S, W, Y, planes, st, partial, flag, s);
+                double* partial, double* items, const int* flag, cudaStream_t s) {
+  if (S.bt_cols == 1) return launch_cols_t<P, 64>(S, W, Y, planes, st, partial, items, flag, s);
+  if (S.bt_cols == 2) return launch_cols_t<P, 256>(S, W, Y, planes, st, partial, items, flag, s);
+  return launch_cols_t<P, 128>(S, W, Y, planes, st, partial, items, flag, s);
 }
 
 template <class P>
-cudaError_t start(const DevSector& S, typename P::T* W, int planes, unsigned seed, const PlaneState& z, cudaStream_t s) {
+cudaError_t start(const DevSector& S, typename P::T* W, int planes, unsigned seed, bool given, const PlaneState& z,
+                  cudaStream_t s) {
   const cudaError_t e = cudaMemsetAsync(z.flags, 0, 2 * sizeof(int), s);
   if (e != cudaSuccess) return e;
   const int nb = std::max(1, kStreamBlocks / planes);
-  start_kernel<P><<<nb * planes, kThreads, 0, s>>>(W, S.dim, seed, nb, z.partial, z.flags, S.umask, S.dmask, S.Dd);
+  start_kernel<P><<<nb * planes, kThreads, 0, s>>>(W, S.dim, seed, nb, z.partial, z.flags, S.umask, S.dmask, S.Dd, given);
   bt_scalars(z.partial, nb, 0, 0, P::kC * planes, P::kScaled, z.st, nullptr, nullptr, z.used, nullptr, s);
   return cudaGetLastError();
 }
@@ -442,7 +554,7 @@ cudaError_t step(const DevSector& S, const typename P::T* Wk, const typename P::
   int* fout = z.flags + (P::kScaled ? 0 : ((k + 1) & 1));
   const cudaError_t e = launch_rows<P>(S, Wk, Y, planes, z.st, fin, s);
   if (e != cudaSuccess) return e;
-  const int nc = launch_cols<P>(S, Wk, Y, planes, z.st, z.partial, fin, s);
+  const int nc = launch_cols<P>(S, Wk, Y, planes, z.st, z.partial, z.items, fin, s);
   bt_scalars(z.partial, nc, 1, k, P::kC * planes, P::kScaled, z.st, z.alpha, z.beta, z.used, fout, s);
   const int nb = std::max(1, kStreamBlocks / planes);
   update_kernel<P><<<nb * planes, kThreads, 0, s>>>(Y, Wk, Wkm1, S.dim, nb, z.st, k > 0, z.partial, fout);
@@ -452,14 +564,28 @@ cudaError_t step(const DevSector& S, const typename P::T* Wk, const typename P::
 
 }  // namespace
 
-int pl_group(int64_t dim, int planes) {
+int pl_group(const DevSector& S, bool c64, int planes) {
   constexpr int64_t kEnough = int64_t(256) << 20;
-  const int64_t bytes = 16 * std::max<int64_t>(dim, 1);
-  return static_cast<int>(std::min<int64_t>(planes, std::max<int64_t>(2, (kEnough + bytes - 1) / bytes)));
+  const int64_t bytes = 16 * std::max<int64_t>(S.dim, 1);
+  const int64_t least = (c64 ? row_planes<C64>(S) : row_planes<C128>(S));
+  return static_cast<int>(std::min<int64_t>(planes, std::max<int64_t>(least, (kEnough + bytes - 1) / bytes)));
 }
 
+int64_t pl_items_doubles(const DevSector& S, bool c64, int planes) {
+  const int kT = S.bt_cols == 1 ? 64 : S.bt_cols == 2 ? 256 : 128;
+  const int64_t per = (S.Dd + 2 * kT - 1) / (2 * kT) * S.Du;
+  return per * planes * (c64 ? 4 : 2);
+}
+
+bool pl_fits(const DevSector& S, int max_up_deg) { return row_planes<C128>(S) > 0 && max_up_deg <= kMaxDeg; }
+
 cudaError_t pl_start(const DevSector& S, float4* W, int planes, unsigned seed, const PlaneState& z, cudaStream_t s) {
-  return start<C64>(S, W, planes, seed, z, s);
+  return start<C64>(S, W, planes, seed, false, z, s);
+}
+
+cudaError_t pl_start(const DevSector& S, double2* W, int planes, unsigned seed, bool given, const PlaneState& z,
+                     cudaStream_t s) {
+  return start<C128>(S, W, planes, seed, given, z, s);
 }
 
 cudaError_t pl_step(const DevSector& S, const float4* Wk, const float4* Wkm1, float4* Y, int planes, int k,
@@ -467,10 +593,15 @@ cudaError_t pl_step(const DevSector& S, const float4* Wk, const float4* Wkm1, fl
   return step<C64>(S, Wk, Wkm1, Y, planes, k, z, s);
 }
 
+cudaError_t pl_step(const DevSector& S, const double2* Wk, const double2* Wkm1, double2* Y, int planes, int k,
+                    const PlaneState& z, cudaStream_t s) {
+  return step<C128>(S, Wk, Wkm1, Y, planes, k, z, s);
+}
+
 cudaError_t pl_apply(const DevSector& S, const float4* X, float4* Y, int planes, int* zero_flag, cudaStream_t s) {
   const cudaError_t e = launch_rows<C64>(S, X, Y, planes, nullptr, zero_flag, s);
   if (e != cudaSuccess) return e;
-  launch_cols<C64>(S, X, Y, planes, nullptr, nullptr, zero_flag, s);
+  launch_cols<C64>(S, X, Y, planes, nullptr, nullptr, nullptr, zero_flag, s);
   return cudaGetLastError();
 }
 

@@ -14,6 +14,7 @@ struct C64 {
   using Cf = float2;
   static constexpr int kC = 2;
   static constexpr bool kScaled = false;
+  static constexpr int kColThreads = 1024;  // resident threads per SM of the column pass (registers)
   static __device__ __forceinline__ T zero() { return make_float4(0.f, 0.f, 0.f, 0.f); }
   static __device__ __forceinline__ bool small(T v) {  // a non-zero entry that is skipped as a source
     return (tinyf(make_float2(v.x, v.y)) && (v.x != 0.f || v.y != 0.f)) ||
@@ -68,6 +69,7 @@ struct C128 {
   using Cf = double2;
   static constexpr int kC = 1;
   static constexpr bool kScaled = true;
+  static constexpr int kColThreads = 896;  // 4x4 (6,6): 2.19 ms, 2.33 with 1024
   static __device__ __forceinline__ T zero() { return make_double2(0.0, 0.0); }
   static __device__ __forceinline__ bool small(T v) { return tiny(v) && (v.x != 0.0 || v.y != 0.0); }
   static __device__ __forceinline__ T filtered(T v, double s) { return tiny(make_double2(s * v.x, s * v.y)) ? zero() : v; }
@@ -102,10 +104,10 @@ struct C128 {
 // The two real coefficients of the gauge table as registers: an entry picks the second one where (entry & cls) is not
 // zero and flips the sign by its bit 31.  In the XOR form the entry carries the bits by which the high words differ,
 // so the second value is the first with the differing bits other than the sign flipped.
-template <class P>
+template <class P, bool kXor>
 struct RowCoefs;
-template <>
-struct RowCoefs<C64> {
+template <bool kXor>
+struct RowCoefs<C64, kXor> {
   float a0, a1;
   float2 p0, p1;  // phase form: the two real values times (pc, ps)
   uint32_t cls;
@@ -113,7 +115,7 @@ struct RowCoefs<C64> {
     a0 = __double2float_rn(G.real2[0]);
     p0 = make_float2(__double2float_rn(G.real2[0] * G.pc), __double2float_rn(G.real2[0] * G.ps));
     p1 = make_float2(__double2float_rn(G.real2[1] * G.pc), __double2float_rn(G.real2[1] * G.ps));
-    if (G.xor_real) {
+    if (kXor) {
       cls = 0x7FFC0000u;
       const int d = (__double2hiint(G.real2[0]) ^ __double2hiint(G.real2[1])) & 0x7FFC0000;
       a1 = __double2float_rn(__hiloint2double(__double2hiint(G.real2[0]) ^ d, __double2loint(G.real2[0])));
@@ -138,17 +140,16 @@ struct RowCoefs<C64> {
   }
 };
 
-template <>
-struct RowCoefs<C128> {
+template <bool kXor>
+struct RowCoefs<C128, kXor> {
   double a0, a1, pc, ps;
-  bool xor_real;
   __device__ __forceinline__ explicit RowCoefs(const DevGauge& G)
-      : a0(G.real2[0]), a1(G.real2[1]), pc(G.pc), ps(G.ps), xor_real(G.xor_real != 0) {}
+      : a0(G.real2[0]), a1(G.real2[1]), pc(G.pc), ps(G.ps) {}
   static __device__ __forceinline__ double flip(double v, uint32_t bits) {
     return __hiloint2double(__double2hiint(v) ^ static_cast<int>(bits), __double2loint(v));
   }
   __device__ __forceinline__ double pick(uint32_t e) const {
-    if (xor_real) return flip(a0, e & 0xFFFC0000u);
+    if (kXor) return flip(a0, e & 0xFFFC0000u);
     return flip((e & 0x40000000u) ? a1 : a0, e & 0x80000000u);
   }
   // Table-section entry in the phase form: real2[cls] (pc, +-ps), bit for bit the table's value.
@@ -187,8 +188,9 @@ __device__ __forceinline__ void block_totals(double (&v)[NV], double* sh /* NV *
 // One output string of the row pass: the diagonal term and the down hops of kP staged lines (line p starts at base + p *
 // line, Dd elements and 8 zeros for the table's padding entries), walked in the gauge table's order, so the sums do not
 // depend on kP.
-template <class P, int kP, bool kPhase>
+template <class P, int kP, bool kPhase, bool kXor>
 struct RowSum {
+  using Coefs = RowCoefs<P, kXor>;
   typename P::T acc[kP];
   uint32_t line;  // bytes per staged line
   const unsigned char* base;
@@ -196,14 +198,14 @@ struct RowSum {
   __device__ __forceinline__ const typename P::T& at(uint32_t e, int p) const {
     return *reinterpret_cast<const typename P::T*>(base + (e & 0x3FFF0u) + p * line);
   }
-  __device__ __forceinline__ void real(uint32_t e, const RowCoefs<P>& rc) {
+  __device__ __forceinline__ void real(uint32_t e, const Coefs& rc) {
     const auto c = rc.pick(e);
 #pragma unroll
-    for (int p = 0; p < kP; ++p) RowCoefs<P>::mac(acc[p], c, at(e, p));
+    for (int p = 0; p < kP; ++p) Coefs::mac(acc[p], c, at(e, p));
   }
   // Complex coefficient: from registers where the table has the phase form (kPhase), else from the block's copy of the
   // table (8 copies, copy i % 8: the 8 lanes of a quarter-warp read 8 different bank groups), with the entry's sign.
-  __device__ __forceinline__ void cplx(uint32_t e, int i, const typename P::Cf* tab, const RowCoefs<P>& rc) {
+  __device__ __forceinline__ void cplx(uint32_t e, int i, const typename P::Cf* tab, const Coefs& rc) {
     typename P::Cf c;
     if constexpr (kPhase)
       c = rc.phase(e);
@@ -214,7 +216,7 @@ struct RowSum {
   }
   // The gauge-table walk of hv.cu's row pass for table position i (sections as whole 4-entry loads, the padding rounds
   // of each section's last load skipped, entry loads two ahead of use).
-  __device__ __forceinline__ void walk(const DevGauge& G, int i, const typename P::Cf* tab, const RowCoefs<P>& rc) {
+  __device__ __forceinline__ void walk(const DevGauge& G, int i, const typename P::Cf* tab, const Coefs& rc) {
     const int4 gp = G.grp[i >> 5];
     const int kr = gp.w & 0xFFFF, kt = gp.w >> 16;
     const uint4* ep = reinterpret_cast<const uint4*>(G.ent + gp.x) + (i & 31);

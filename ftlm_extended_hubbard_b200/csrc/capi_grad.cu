@@ -1,3 +1,5 @@
+#include <type_traits>
+
 #include "capi_internal.hpp"
 
 using namespace ftlm_b200;
@@ -19,91 +21,211 @@ struct ChainGrad {
   double lmin = 0.0, g = 0.0, m[3] = {0.0, 0.0, 0.0};
 };
 
-// Weight matrices of up to nc chains on the GPU (symeig.cu: QL eigen-decomposition of each
-// chain's tridiagonal, then K = Z P Z^T), written to g_grad.Kp in the layout [i][ld][nc] (chain
-// fastest) with the scales 1/(sc_i sc_l); g and the lowest Ritz value per chain to `out`.
-int fill_weights(ftlm_sector* s, int nc, int ld, double bT, const std::vector<int>& n, const std::vector<double>& A,
-                 const std::vector<double>& B, const std::vector<std::vector<double>>& scale,
-                 std::vector<ChainGrad>* out) {
-  cudaStream_t st = s->stream;
-  std::vector<double> sc(static_cast<size_t>(nc) * ld, 1.0);
-  for (int c = 0; c < nc; ++c)
-    for (size_t i = 0; i < scale[static_cast<size_t>(c)].size() && i < static_cast<size_t>(ld); ++i)
-      sc[static_cast<size_t>(c) * ld + i] = scale[static_cast<size_t>(c)][i];
-  const size_t mat = static_cast<size_t>(nc) * ld * sizeof(double);
-  Scratch mem;
-  const size_t o_da = mem.add(mat), o_db = mem.add(mat), o_dn = mem.add(nc * sizeof(int)), o_dsc = mem.add(mat);
-  const size_t o_dl = mem.add(mat), o_dvt = mem.add(mat * ld), o_dy = mem.add(mat * ld);
-  const size_t o_dg = mem.add(nc * sizeof(double)), o_dlm = mem.add(nc * sizeof(double));
-  const size_t o_di = mem.add(nc * sizeof(int));
-  CU_TRY(mem.commit());
-  CU_TRY(cudaMemcpyAsync(mem.at<void>(o_da), A.data(), mat, cudaMemcpyHostToDevice, st));
-  CU_TRY(cudaMemcpyAsync(mem.at<void>(o_db), B.data(), mat, cudaMemcpyHostToDevice, st));
-  CU_TRY(cudaMemcpyAsync(mem.at<void>(o_dn), n.data(), nc * sizeof(int), cudaMemcpyHostToDevice, st));
-  CU_TRY(cudaMemcpyAsync(mem.at<void>(o_dsc), sc.data(), mat, cudaMemcpyHostToDevice, st));
-  CU_TRY(cudaMemsetAsync(mem.at<void>(o_dg), 0, nc * sizeof(double), st));
-  CU_TRY(g_grad.grow(g_grad.Kp, g_grad.kcap, static_cast<size_t>(ld) * ld * nc * sizeof(double)));
-  CU_TRY(cudaMemsetAsync(g_grad.Kp.p, 0, static_cast<size_t>(ld) * ld * nc * sizeof(double), st));
-  CU_TRY(symeig_tridiag(mem.at<double>(o_da), mem.at<double>(o_db), mem.at<int>(o_dn), nc, ld, mem.at<double>(o_dl), nullptr,
-                        mem.at<double>(o_dvt), mem.at<int>(o_di), st));
-  CU_TRY(duhamel_weights_dev(mem.at<double>(o_dl), mem.at<double>(o_dvt), mem.at<int>(o_dn), nc, ld, bT, mem.at<double>(o_dsc),
-                             mem.at<double>(o_dy), g_grad.Kp.as<double>(), mem.at<double>(o_dg), mem.at<double>(o_dlm), st));
-  std::vector<double> g(static_cast<size_t>(nc)), lm(static_cast<size_t>(nc));
-  std::vector<int> info(static_cast<size_t>(nc));
-  CU_TRY(cudaMemcpyAsync(g.data(), mem.at<void>(o_dg), nc * sizeof(double), cudaMemcpyDeviceToHost, st));
-  CU_TRY(cudaMemcpyAsync(lm.data(), mem.at<void>(o_dlm), nc * sizeof(double), cudaMemcpyDeviceToHost, st));
-  CU_TRY(cudaMemcpyAsync(info.data(), mem.at<void>(o_di), nc * sizeof(int), cudaMemcpyDeviceToHost, st));
-  CU_TRY(cudaStreamSynchronize(st));
-  for (int c = 0; c < nc; ++c) {
-    ChainGrad& cg = (*out)[static_cast<size_t>(c)];
-    cg = ChainGrad{};
-    if (n[static_cast<size_t>(c)] <= 0) continue;
-    if (info[static_cast<size_t>(c)] != 0) return fail(FTLM_ERR_NUMERIC, "GPU eigen-solver did not converge");
-    cg.ok = true;
-    cg.g = g[static_cast<size_t>(c)];
-    cg.lmin = lm[static_cast<size_t>(c)];
-  }
-  mem.idle();
-  return FTLM_OK;
-}
-
-// Moments of one batch of nc chains: Q [n][planes][dim] with strides vstride and pstride, AQ likewise (or null),
-// weights already in g_grad.Kp [n][ld][nc] (fill_weights).
+// The moments of nc chains of one sector: tridiagonals, lengths and stored vectors' norms on the device, the vectors at Q
+// (Q + i * vstride + p * pstride: plane p of vector i) and their images under the operator at AQ (or null).
 template <class T>
-int run_moments(ftlm_sector* s, const T* Q, const T* AQ, int64_t vstride, int64_t pstride, int planes, int n, int ld,
-                int nc, std::vector<ChainGrad>* out) {
-  cudaStream_t st = s->stream;
-  CU_TRY(g_grad.grow(g_grad.part, g_grad.pcap, static_cast<size_t>(kGradMaxBlocks) * nc * 3 * sizeof(double)));
-  int grid = 0;
-  const cudaError_t e = grad_moments(s->dev, Q, AQ ? AQ : Q, vstride, pstride, planes, g_grad.Kp.as<double>(), n, ld, nc,
-                                     g_grad.part.as<double>(), &grid, st);
-  if (e == cudaErrorInvalidValue)
-    return fail(FTLM_ERR_UNSUPPORTED, "gradient: Lanczos vectors of one block do not fit in shared memory");
-  CU_TRY(e);
-  std::vector<double> hp(static_cast<size_t>(grid) * nc * 3);
-  CU_TRY(cudaMemcpyAsync(hp.data(), g_grad.part.p, hp.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
+struct SectorChains {
+  ftlm_sector* s;
+  int nc;
+  const T* Q;
+  const T* AQ;
+  int64_t vstride, pstride;
+};
+
+// Weights K = Z P Z^T of all chains (eigen-decomposition of each chain's tridiagonal, Duhamel's formula), then the
+// moments sector by sector; everything stays on the device until the end.
+template <class T>
+int chain_moments(const std::vector<SectorChains<T>>& v, int ld, double bT, const double* alpha, const double* beta,
+                  const int* used, const double* scale, cudaStream_t st, std::vector<ChainGrad>* out) {
+  int nc = 0, most = 0;
+  for (const auto& x : v) {
+    nc += x.nc;
+    most = std::max(most, x.nc);
+  }
+  const size_t mat = static_cast<size_t>(nc) * ld;
+  Scratch mem;
+  const size_t o_l = mem.array<double>(mat), o_v = mem.array<double>(mat * ld), o_y = mem.array<double>(mat * ld);
+  const size_t o_k = mem.array<double>(mat * ld), o_g = mem.array<double>(5 * static_cast<size_t>(nc));
+  const size_t o_i = mem.array<int>(2 * static_cast<size_t>(nc));
+  const size_t o_p = mem.array<double>(static_cast<size_t>(kGradMaxBlocks) * most * 3);
+  CU_TRY(mem.commit());
+  double *g = mem.at<double>(o_g), *lmin = g + nc, *m = lmin + nc;
+  CU_TRY(symeig_tridiag(alpha, beta, used, nc, ld, mem.at<double>(o_l), nullptr, mem.at<double>(o_v), mem.at<int>(o_i), st));
+  CU_TRY(duhamel_weights_dev(mem.at<double>(o_l), mem.at<double>(o_v), used, nc, ld, bT, scale, mem.at<double>(o_y),
+                             mem.at<double>(o_k), g, lmin, st));
+  int c0 = 0;
+  for (const auto& x : v) {
+    const cudaError_t e = grad_moments(x.s->dev, x.Q, x.AQ ? x.AQ : x.Q, x.vstride, x.pstride, x.nc,
+                                       mem.at<double>(o_k) + static_cast<size_t>(c0) * ld * ld, used + c0, ld,
+                                       mem.at<double>(o_p), m + 3 * c0, st);
+    if (e == cudaErrorInvalidValue)
+      return fail(FTLM_ERR_UNSUPPORTED, "gradient: Lanczos vectors of one block do not fit in shared memory");
+    CU_TRY(e);
+    c0 += x.nc;
+  }
+  std::vector<double> h(5 * static_cast<size_t>(nc));
+  std::vector<int> info(static_cast<size_t>(nc)), n(static_cast<size_t>(nc));
+  CU_TRY(cudaMemcpyAsync(h.data(), g, h.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
+  CU_TRY(cudaMemcpyAsync(info.data(), mem.at<void>(o_i), info.size() * sizeof(int), cudaMemcpyDeviceToHost, st));
+  CU_TRY(cudaMemcpyAsync(n.data(), used, n.size() * sizeof(int), cudaMemcpyDeviceToHost, st));
   CU_TRY(cudaStreamSynchronize(st));
-  for (int c = 0; c < nc; ++c) {
-    ChainGrad& cg = (*out)[static_cast<size_t>(c)];
-    for (int q = 0; q < 3; ++q) {
-      double sum = 0.0;
-      for (int b = 0; b < grid; ++b) sum += hp[(static_cast<size_t>(b) * nc + c) * 3 + q];
-      cg.m[q] = sum;
-    }
+  mem.idle();
+  out->assign(static_cast<size_t>(nc), ChainGrad{});
+  for (size_t c = 0; c < out->size(); ++c) {
+    if (n[c] <= 0) continue;
+    if (info[c] != 0) return fail(FTLM_ERR_NUMERIC, "GPU eigen-solver did not converge");
+    ChainGrad& cg = (*out)[c];
+    cg.ok = true;
+    cg.g = h[c];
+    cg.lmin = h[static_cast<size_t>(nc) + c];
+    for (int q = 0; q < 3; ++q) cg.m[q] = h[2 * static_cast<size_t>(nc) + 3 * c + q];
   }
   return FTLM_OK;
 }
 
-// Plain path: complex128 chains of ftlm_gpu_ftlm_sector (seed_r = seed + r*100003).
-int grad_plain(ftlm_sector* s, ftlm_sector* op, double bT, int R, int M, unsigned seed, int start_mode,
-               std::vector<ChainGrad>* out) {
+// Chains of small sectors (chains_run), replayed with their vectors kept; op[i] (may be null) is the operator's sector.
+// Sectors go in pieces whose stored vectors fit a bounded store.  out: [sector][R].
+template <class T>
+int grad_fused(const std::vector<ftlm_sector*>& secs, const std::vector<ftlm_sector*>& op, double bT, int R, int M,
+               unsigned seed, int start_mode, std::vector<std::vector<ChainGrad>>* out) {
+  constexpr bool c64 = sizeof(T) == sizeof(float4) && std::is_same<T, float4>::value;
+  constexpr size_t kStore = size_t(6) << 30;
+  const int planes = c64 ? (R + 1) / 2 : R;
+  out->assign(secs.size(), {});
+  std::lock_guard<std::mutex> lock(g_bt_mu);
+  if (!g_grad.flag.p) CU_TRY(g_grad.flag.alloc(sizeof(int)));
+  for (size_t i0 = 0; i0 < secs.size();) {
+    std::vector<ftlm_sector*> piece;
+    std::vector<int64_t> base;
+    int64_t at = 0;
+    size_t i1 = i0;
+    for (; i1 < secs.size(); ++i1) {
+      const int64_t add = static_cast<int64_t>(M) * planes * secs[i1]->plan.dim;
+      const size_t weights = (piece.size() + 1) * R * static_cast<size_t>(M) * M * sizeof(double) * 3;
+      if (!piece.empty() && (static_cast<size_t>(at + add) * sizeof(T) > kStore || weights > kStore / 2)) break;
+      piece.push_back(secs[i1]);
+      base.push_back(at);
+      at += add;
+    }
+    CU_TRY(g_grad.grow(g_grad.Q, g_grad.qcap, static_cast<size_t>(at) * sizeof(T)));
+    CU_TRY(g_grad.grow(g_grad.AQ, g_grad.acap, static_cast<size_t>(at) * sizeof(T)));
+    ChainRun run;
+    int rc = chains_run(piece, R, M, seed, start_mode, c64, &run, g_grad.Q.p, &base, true);
+    if (rc) return rc;
+    cudaStream_t st = piece[0]->stream;
+    run.mem.busy();
+    std::vector<SectorChains<T>> v;
+    for (size_t i = 0; i < piece.size(); ++i) {
+      const int64_t dim = piece[i]->plan.dim;
+      const T* Q = g_grad.Q.as<T>() + base[i];
+      T* AQ = op[i0 + i] ? g_grad.AQ.as<T>() + base[i] : nullptr;
+      // the operator on every stored vector: the planes of all steps are contiguous
+      if (AQ) CU_TRY(pl_apply(op[i0 + i]->dev, Q, AQ, M * planes, g_grad.flag.as<int>(), st));
+      v.push_back(SectorChains<T>{piece[i], R, Q, AQ, planes * dim, dim});
+    }
+    std::vector<ChainGrad> cg;
+    rc = chain_moments(v, M, bT, run.alpha, run.beta, run.used, run.scale, st, &cg);
+    if (rc) return rc;
+    run.mem.idle();
+    for (size_t i = 0; i < piece.size(); ++i)
+      (*out)[i0 + i].assign(cg.begin() + static_cast<long>(i) * R, cg.begin() + static_cast<long>(i + 1) * R);
+    i0 = i1;
+  }
+  return FTLM_OK;
+}
+
+// Chains of one sector on the whole GPU (planes.cu), replayed step by step with the vectors kept: the forward's groups and
+// kernels, so its alpha and beta.
+template <class T>
+int grad_planes(ftlm_sector* s, ftlm_sector* op, double bT, int R, int M, unsigned seed, int start_mode,
+                std::vector<ChainGrad>* out) {
+  constexpr bool c64 = std::is_same<T, float4>::value;
+  constexpr int kC = c64 ? 2 : 1;
   const int64_t dim = s->plan.dim;
+  const int most = (std::min(R, kBtChains) + kC - 1) / kC, group = pl_group(s->dev, c64, most);
+  const int64_t vs = dim * group;  // elements per stored vector of a group
+  std::lock_guard<std::mutex> lock(g_bt_mu);
+  CU_TRY(g_bt.ensure(0, M, pl_items_doubles(s->dev, c64, group)));
+  CU_TRY(g_grad.grow(g_grad.Q, g_grad.qcap, static_cast<size_t>(M + 1) * vs * sizeof(T)));
+  if (op) CU_TRY(g_grad.grow(g_grad.AQ, g_grad.acap, static_cast<size_t>(M) * vs * sizeof(T)));
+  if (!g_grad.flag.p) CU_TRY(g_grad.flag.alloc(sizeof(int)));
+  cudaStream_t st = s->stream;
+  T* Q = g_grad.Q.as<T>();
+  T* AQ = op ? g_grad.AQ.as<T>() : nullptr;
+  const size_t tab = static_cast<size_t>(M) * kBtChains;
+  std::vector<double> ha(tab), hb(tab), hs(kBtChains);  // hs: 1 / ||raw start||
+  std::vector<int> hu(kBtChains);
+  std::vector<std::complex<double>> start;
+  out->clear();
+  for (int r0 = 0; r0 < R;) {
+    // as the forward: blocks of 32 chains (complex64), groups of planes within them
+    const int left = c64 ? std::min(kBtChains - r0 % kBtChains, R - r0) : R - r0;
+    const int nc = std::min(group * kC, left), np = (nc + kC - 1) / kC;
+    const unsigned seed_g = seed + static_cast<unsigned>(r0) * 100003u;
+    const PlaneState z = g_bt.state(0);
+    CU_TRY(cudaMemsetAsync(z.alpha, 0, tab * sizeof(double), st));
+    CU_TRY(cudaMemsetAsync(z.beta, 0, tab * sizeof(double), st));
+    if constexpr (c64) {
+      CU_TRY(pl_start(s->dev, Q, np, seed_g, z, st));
+    } else {
+      const bool given = start_mode == FTLM_START_REFERENCE;
+      if (given) {
+        reference_normals(dim, np, seed_g, &start);
+        CU_TRY(cudaMemcpyAsync(Q, start.data(), start.size() * sizeof(double2), cudaMemcpyHostToDevice, st));
+      }
+      CU_TRY(pl_start(s->dev, Q, np, seed_g, given, z, st));
+    }
+    CU_TRY(cudaMemcpyAsync(hs.data(), z.st + kBtSin * kBtChains, kBtChains * sizeof(double), cudaMemcpyDeviceToHost, st));
+    const int64_t step = dim * np;
+    for (int k = 0; k < M; ++k)
+      CU_TRY(pl_step(s->dev, Q + k * step, Q + (k > 0 ? k - 1 : 0) * step, Q + (k + 1) * step, np, k, z, st));
+    CU_TRY(cudaMemcpyAsync(ha.data(), z.alpha, tab * sizeof(double), cudaMemcpyDeviceToHost, st));
+    CU_TRY(cudaMemcpyAsync(hb.data(), z.beta, tab * sizeof(double), cudaMemcpyDeviceToHost, st));
+    CU_TRY(cudaMemcpyAsync(hu.data(), z.used, hu.size() * sizeof(int), cudaMemcpyDeviceToHost, st));
+    CU_TRY(cudaStreamSynchronize(st));
+    if (op) CU_TRY(pl_apply(op->dev, Q, AQ, M * np, g_grad.flag.as<int>(), st));
+    // chain-major tables: alpha, beta, norms of the stored vectors (W_0 = ||raw|| q_0, W_i = beta_{i-1} q_i)
+    const size_t row = static_cast<size_t>(nc) * M;
+    std::vector<double> t(3 * row, 0.0);
+    std::vector<int> n(static_cast<size_t>(nc));
+    for (int c = 0; c < nc; ++c) {
+      n[static_cast<size_t>(c)] = hs[static_cast<size_t>(c)] > 0.0 ? hu[static_cast<size_t>(c)] : 0;
+      for (int k = 0; k < M; ++k) {
+        const size_t o = static_cast<size_t>(c) * M + k, h = static_cast<size_t>(k) * kBtChains + c;
+        t[o] = ha[h];
+        t[row + o] = hb[h];
+        double norm = 1.0;
+        if (k < n[static_cast<size_t>(c)]) norm = k == 0 ? 1.0 / hs[static_cast<size_t>(c)] : hb[h - kBtChains];
+        t[2 * row + o] = norm;
+      }
+    }
+    Scratch mem;
+    const size_t o_t = mem.array<double>(t.size()), o_n = mem.array<int>(n.size());
+    CU_TRY(mem.commit());
+    CU_TRY(cudaMemcpyAsync(mem.at<void>(o_t), t.data(), t.size() * sizeof(double), cudaMemcpyHostToDevice, st));
+    CU_TRY(cudaMemcpyAsync(mem.at<void>(o_n), n.data(), n.size() * sizeof(int), cudaMemcpyHostToDevice, st));
+    const double* dt = mem.at<double>(o_t);
+    std::vector<ChainGrad> cg;
+    const int rc = chain_moments<T>({SectorChains<T>{s, nc, Q, AQ, step, dim}}, M, bT, dt, dt + row, mem.at<int>(o_n),
+                                    dt + 2 * row, st, &cg);
+    if (rc) return rc;
+    mem.idle();
+    out->insert(out->end(), cg.begin(), cg.end());
+    r0 += nc;
+  }
+  return FTLM_OK;
+}
+
+// Complex128 chains one at a time with the sector's own H v (sectors without a gauge table).
+int grad_serial(ftlm_sector* s, ftlm_sector* op, double bT, int R, int M, unsigned seed, int start_mode,
+                std::vector<ChainGrad>* out) {
+  const int64_t dim = s->plan.dim;
+  std::lock_guard<std::mutex> lock(g_bt_mu);
   CU_TRY(g_grad.grow(g_grad.Q, g_grad.qcap, static_cast<size_t>(M) * dim * sizeof(double2)));
   if (op) CU_TRY(g_grad.grow(g_grad.AQ, g_grad.acap, static_cast<size_t>(M) * dim * sizeof(double2)));
   double2* Q = g_grad.Q.as<double2>();
   double2* AQ = op ? g_grad.AQ.as<double2>() : nullptr;
   out->assign(static_cast<size_t>(R), ChainGrad{});
-  std::vector<ChainGrad> one(1);
   for (int r = 0; r < R; ++r) {
     std::vector<double> a, b;
     int rc = run_lanczos(
@@ -112,105 +234,79 @@ int grad_plain(ftlm_sector* s, ftlm_sector* op, double bT, int R, int M, unsigne
     if (rc) return rc;
     const int n = static_cast<int>(a.size());
     if (n <= 0) continue;
-    std::vector<double> A(static_cast<size_t>(M), 0.0), B(static_cast<size_t>(M), 0.0);
-    std::copy(a.begin(), a.end(), A.begin());
-    std::copy(b.begin(), b.begin() + std::min<size_t>(b.size(), static_cast<size_t>(M)), B.begin());
     if (op)
       for (int i = 0; i < n; ++i) {
         rc = op->apply(Q + static_cast<int64_t>(i) * dim, AQ + static_cast<int64_t>(i) * dim, s->stream);
         if (rc) return rc;
       }
-    std::vector<std::vector<double>> scale(1, std::vector<double>(static_cast<size_t>(n), 1.0));
-    rc = fill_weights(s, 1, M, bT, std::vector<int>{n}, A, B, scale, &one);
+    std::vector<double> t(3 * static_cast<size_t>(M), 0.0);
+    std::copy(a.begin(), a.end(), t.begin());
+    std::copy(b.begin(), b.begin() + std::min<size_t>(b.size(), static_cast<size_t>(M)), t.begin() + M);
+    std::fill(t.begin() + 2 * M, t.end(), 1.0);
+    cudaStream_t st = s->stream;
+    Scratch mem;
+    const size_t o_t = mem.array<double>(t.size()), o_n = mem.array<int>(1);
+    CU_TRY(mem.commit());
+    CU_TRY(cudaMemcpyAsync(mem.at<void>(o_t), t.data(), t.size() * sizeof(double), cudaMemcpyHostToDevice, st));
+    CU_TRY(cudaMemcpyAsync(mem.at<void>(o_n), &n, sizeof(int), cudaMemcpyHostToDevice, st));
+    const double* dt = mem.at<double>(o_t);
+    std::vector<ChainGrad> cg;
+    rc = chain_moments<double2>({SectorChains<double2>{s, 1, Q, AQ, dim, dim}}, M, bT, dt, dt + M, mem.at<int>(o_n),
+                                dt + 2 * M, st, &cg);
     if (rc) return rc;
-    rc = run_moments<double2>(s, Q, AQ, dim, dim, 1, n, M, 1, &one);
-    if (rc) return rc;
-    (*out)[static_cast<size_t>(r)] = one[0];
+    mem.idle();
+    (*out)[static_cast<size_t>(r)] = cg[0];
   }
   return FTLM_OK;
 }
 
-// Batched path: complex64 32-chain blocks of ftlm_gpu_batched_ftlm_sector, replayed step by step.
-int grad_batched(ftlm_sector* s, ftlm_sector* op, double bT, int R, int M, unsigned seed, std::vector<ChainGrad>* out) {
-  const int64_t dim = s->plan.dim;
-  const int max_planes = (std::min(R, kBtChains) + 1) / 2, group = pl_group(s->dev, true, max_planes);
-  const int64_t vs = dim * max_planes;  // elements of two chains per stored vector
-  std::lock_guard<std::mutex> lock(g_bt_mu);
-  CU_TRY(g_bt.ensure(0, M, pl_items_doubles(s->dev, true, group)));
-  CU_TRY(g_grad.grow(g_grad.Q, g_grad.qcap, static_cast<size_t>(M + 1) * vs * sizeof(float4)));
-  if (op) CU_TRY(g_grad.grow(g_grad.AQ, g_grad.acap, static_cast<size_t>(M) * vs * sizeof(float4)));
-  if (!g_grad.zflag.p) {
-    CU_TRY(g_grad.zflag.alloc(sizeof(int)));
-    CU_TRY(cudaMemset(g_grad.zflag.p, 0, sizeof(int)));
+// ln Z = ln dim + log mean_r g_r, g_r = e^{-bT lmin_r} ghat_r; d ln Z = -sum_r e^{-bT lmin_r} m_r / sum_r g_r
+void sector_gradient(const std::vector<ChainGrad>& cg, int64_t dim, double bT, bool has_op, double* lnz, double* dlnz) {
+  double mx = -std::numeric_limits<double>::infinity();
+  int used = 0;
+  for (const auto& c : cg)
+    if (c.ok) {
+      mx = std::max(mx, -bT * c.lmin + std::log(c.g));
+      ++used;
+    }
+  dlnz[0] = dlnz[1] = dlnz[2] = 0.0;
+  if (used == 0) {
+    *lnz = -std::numeric_limits<double>::infinity();
+    return;
   }
-  cudaStream_t st = s->stream;
-  float4* Q = g_grad.Q.as<float4>();
-  float4* AQ = op ? g_grad.AQ.as<float4>() : nullptr;
-  double* sd = g_bt.st.as<double>();
-  double* al = g_bt.alpha.as<double>();
-  double* be = g_bt.beta.as<double>();
-  int* us = g_bt.used.as<int>();
-  out->assign(static_cast<size_t>(R), ChainGrad{});
-  std::vector<double> ha(static_cast<size_t>(M) * kBtChains), hb(static_cast<size_t>(M) * kBtChains),
-      hs(kBtChains);  // 1 / ||raw start||
-  std::vector<int> hu(kBtChains);
-  for (int blk = 0; blk * kBtChains < R; ++blk) {
-    const unsigned seed_b = seed + static_cast<unsigned>(blk * kBtChains) * 100003u;
-    CU_TRY(cudaMemsetAsync(al, 0, static_cast<size_t>(M) * kBtChains * sizeof(double), st));
-    CU_TRY(cudaMemsetAsync(be, 0, static_cast<size_t>(M) * kBtChains * sizeof(double), st));
-    const int nc = std::min(kBtChains, R - blk * kBtChains), planes = (nc + 1) / 2;
-    // the forward's groups and kernels; W_0's scale (st) is read before the steps overwrite it
-    for (int p0 = 0; p0 < planes; p0 += group) {
-      const int np = std::min(group, planes - p0);
-      const PlaneState z = g_bt.state(2 * p0);
-      float4* Qp = Q + p0 * dim;
-      CU_TRY(pl_start(s->dev, Qp, np, seed_b + static_cast<unsigned>(2 * p0) * 100003u, z, st));
-      CU_TRY(cudaMemcpyAsync(hs.data() + 2 * p0, sd + kBtSin * kBtChains + 2 * p0, 2 * np * sizeof(double),
-                             cudaMemcpyDeviceToHost, st));
-      for (int k = 0; k < M; ++k)
-        CU_TRY(pl_step(s->dev, Qp + k * vs, Qp + (k > 0 ? k - 1 : 0) * vs, Qp + (k + 1) * vs, np, k, z, st));
-    }
-    CU_TRY(cudaMemcpyAsync(ha.data(), al, ha.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
-    CU_TRY(cudaMemcpyAsync(hb.data(), be, hb.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
-    CU_TRY(cudaMemcpyAsync(hu.data(), us, hu.size() * sizeof(int), cudaMemcpyDeviceToHost, st));
-    CU_TRY(cudaStreamSynchronize(st));
-    std::vector<int> n(static_cast<size_t>(kBtChains), 0);
-    std::vector<double> A(static_cast<size_t>(kBtChains) * M, 0.0), B(static_cast<size_t>(kBtChains) * M, 0.0);
-    std::vector<std::vector<double>> scale(static_cast<size_t>(kBtChains));
-    int nmax = 0;
-    for (int c = 0; c < nc; ++c) {
-      const double sin0 = hs[static_cast<size_t>(c)];
-      const int nn = (sin0 > 0.0) ? hu[static_cast<size_t>(c)] : 0;
-      n[static_cast<size_t>(c)] = nn;
-      nmax = std::max(nmax, nn);
-      auto& sc = scale[static_cast<size_t>(c)];
-      sc.assign(static_cast<size_t>(std::max(nn, 1)), 1.0);
-      for (int k = 0; k < M; ++k) {
-        A[static_cast<size_t>(c) * M + k] = ha[static_cast<size_t>(k) * kBtChains + c];
-        B[static_cast<size_t>(c) * M + k] = hb[static_cast<size_t>(k) * kBtChains + c];
-      }
-      if (nn > 0) {  // W_0 = ||raw|| q_0, W_i = beta_{i-1} q_i
-        sc[0] = 1.0 / sin0;
-        for (int i = 1; i < nn; ++i) sc[static_cast<size_t>(i)] = B[static_cast<size_t>(c) * M + i - 1];
-      }
-    }
-    if (nmax == 0) continue;
-    if (op) {  // the operator on every stored vector: planes are contiguous over the vectors of a full store
-      if (planes == max_planes) {
-        CU_TRY(pl_apply(op->dev, Q, AQ, nmax * planes, g_grad.zflag.as<int>(), st));
-      } else {
-        for (int i = 0; i < nmax; ++i)
-          CU_TRY(pl_apply(op->dev, Q + i * vs, AQ + i * vs, planes, g_grad.zflag.as<int>(), st));
-      }
-    }
-    std::vector<ChainGrad> cg(static_cast<size_t>(kBtChains));
-    int rc = fill_weights(s, kBtChains, M, bT, n, A, B, scale, &cg);
-    if (rc) return rc;
-    rc = run_moments<float4>(s, Q, AQ, vs, dim, planes, nmax, M, kBtChains, &cg);
-    if (rc) return rc;
-    for (int c = 0; c < nc; ++c) (*out)[static_cast<size_t>(blk * kBtChains + c)] = cg[static_cast<size_t>(c)];
+  double zs = 0.0, d[3] = {0.0, 0.0, 0.0};
+  for (const auto& c : cg) {
+    if (!c.ok) continue;
+    const double w = std::exp(-bT * c.lmin - mx);
+    zs += w * c.g;
+    for (int q = 0; q < 3; ++q) d[q] -= w * c.m[q];
   }
-  return FTLM_OK;
+  *lnz = std::log(static_cast<double>(dim)) + mx + std::log(zs / static_cast<double>(used));
+  for (int q = 0; q < (has_op ? 3 : 2); ++q) dlnz[q] = d[q] / zs;
+}
+
+// The path of a sector's chains in the gradient, which is the forward's: fused, on planes, or (complex128 without a gauge
+// table) not available.
+bool grad_is_c64(const ftlm_sector* s, int M, int method) { return method == 1 && s->plan.dim > 2 * static_cast<int64_t>(M); }
+bool grad_is_fused(const ftlm_sector* s, bool c64) {
+  return s->plan.dim <= kFusedSweepMax && chain_rows(s->dev, c64, false) > 0 && s->plan.max_up_deg <= 120;
+}
+
+int grad_one(ftlm_sector* s, ftlm_sector* op, double bT, int R, int M, unsigned seed, int method, int start_mode,
+             std::vector<ChainGrad>* cg) {
+  const bool c64 = grad_is_c64(s, M, method);
+  const int mode = method == 1 ? FTLM_START_PHILOX : start_mode;
+  if (grad_is_fused(s, c64)) {
+    std::vector<std::vector<ChainGrad>> v;
+    const int rc = c64 ? grad_fused<float4>({s}, {op}, bT, R, M, seed, mode, &v)
+                       : grad_fused<double2>({s}, {op}, bT, R, M, seed, mode, &v);
+    if (!rc) *cg = v[0];
+    return rc;
+  }
+  if (c64) return grad_planes<float4>(s, op, bT, R, M, seed, mode, cg);
+  if (!pl_fits(s->dev, s->plan.max_up_deg) || (op && !pl_fits(op->dev, op->plan.max_up_deg)))
+    return grad_serial(s, op, bT, R, M, seed, mode, cg);
+  return grad_planes<double2>(s, op, bT, R, M, seed, mode, cg);
 }
 
 }  // namespace
@@ -231,39 +327,13 @@ int ftlm_gpu_grad_sector(ftlm_sector* s, ftlm_sector* op_tp, double bT, int R, i
   R = std::max(1, R);
   M = std::max(1, M);
   if (M > kMaxEig) return fail(FTLM_ERR_UNSUPPORTED, "more than 160 Lanczos steps for the GPU eigen-solver");
-  const int64_t dim = s->plan.dim;
+  if (method == 1 && s->plan.dim > 2 * static_cast<int64_t>(M) &&
+      (s->plan.max_up_deg > 120 || (op_tp && op_tp->plan.max_up_deg > 120)))
+    return fail(FTLM_ERR_UNSUPPORTED, "batched path: more than 120 up-hop sources per string");
   std::vector<ChainGrad> cg;
-  if (method == 1 && dim > 2 * static_cast<int64_t>(M)) {
-    if (s->plan.max_up_deg > 120 || (op_tp && op_tp->plan.max_up_deg > 120))
-      return fail(FTLM_ERR_UNSUPPORTED, "batched path: more than 120 up-hop sources per string");
-    rc = grad_batched(s, op_tp, bT, R, M, seed, &cg);
-  } else {
-    rc = grad_plain(s, op_tp, bT, R, M, seed, method == 1 ? FTLM_START_PHILOX : start_mode, &cg);
-  }
+  rc = grad_one(s, op_tp, bT, R, M, seed, method, start_mode, &cg);
   if (rc) return rc;
-  // ln Z = ln dim + log mean_r g_r, g_r = e^{-bT lmin_r} ghat_r; d ln Z = -sum_r e^{-bT lmin_r} m_r / sum_r g_r
-  double mx = -std::numeric_limits<double>::infinity();
-  int used = 0;
-  for (const auto& c : cg)
-    if (c.ok) {
-      mx = std::max(mx, -bT * c.lmin + std::log(c.g));
-      ++used;
-    }
-  if (used == 0) {
-    *lnz = -std::numeric_limits<double>::infinity();
-    dlnz[0] = dlnz[1] = dlnz[2] = 0.0;
-    return FTLM_OK;
-  }
-  double zs = 0.0, d[3] = {0.0, 0.0, 0.0};
-  for (const auto& c : cg) {
-    if (!c.ok) continue;
-    const double w = std::exp(-bT * c.lmin - mx);
-    zs += w * c.g;
-    for (int q = 0; q < 3; ++q) d[q] -= w * c.m[q];
-  }
-  *lnz = std::log(static_cast<double>(dim)) + mx + std::log(zs / static_cast<double>(used));
-  for (int q = 0; q < 3; ++q) dlnz[q] = d[q] / zs;
-  if (!op_tp) dlnz[2] = 0.0;
+  sector_gradient(cg, s->plan.dim, bT, op_tp != nullptr, lnz, dlnz);
   return FTLM_OK;
 }
 
@@ -416,6 +486,21 @@ int ftlm_gpu_gc_logz_grad(const ftlm_params* p, double mu, double bT, int R, int
   pop.U = 0.0;
   pop.V = 0.0;
   PlanParts parts(n), op_parts(n);
+  struct Term {
+    SectorPtr s, op;
+    size_t idx;
+    double w;
+  };
+  std::vector<Term> fused[2];  // small sectors, complex128 and complex64: their chains together
+  auto add = [&](const Term& t, const std::vector<ChainGrad>& cg) {
+    double lz = 0.0, g[3] = {0.0, 0.0, 0.0};
+    sector_gradient(cg, t.s->plan.dim, bT, true, &lz, g);
+    if (!(std::fabs(lz - lnz_s[t.idx]) <= 1e-9 * std::max(1.0, std::fabs(lz))))
+      return fail(FTLM_ERR_NUMERIC, "gradient replay of sector (" + std::to_string(t.s->plan.nu) + "," +
+                                        std::to_string(t.s->plan.nd) + ") did not reproduce the forward ln Z");
+    for (int q = 0; q < 3; ++q) d[q] += t.w * g[q];
+    return static_cast<int>(FTLM_OK);
+  };
   for (int nu = 0; nu <= n; ++nu)
     for (int nd = 0; nd <= n; ++nd) {
       const size_t idx = static_cast<size_t>(nu * (n + 1) + nd);
@@ -427,18 +512,35 @@ int ftlm_gpu_gc_logz_grad(const ftlm_params* p, double mu, double bT, int R, int
       ftlm_sector *rs = nullptr, *ro = nullptr;
       rc = sector_create(p, nu, nd, &parts, &rs);
       if (rc) return rc;
-      SectorPtr s(rs);
+      Term t{SectorPtr(rs), nullptr, idx, w};
       rc = sector_create(&pop, nu, nd, &op_parts, &ro);
       if (rc) return rc;
-      SectorPtr op(ro);
-      double lz = 0.0, g[3] = {0.0, 0.0, 0.0};
-      rc = ftlm_gpu_grad_sector(s.get(), op.get(), bT, R, M, seed, method, start_mode, &lz, g);
+      t.op.reset(ro);
+      const bool c64 = grad_is_c64(rs, M, method);
+      if (c64 && (rs->plan.max_up_deg > 120 || ro->plan.max_up_deg > 120))
+        return fail(FTLM_ERR_UNSUPPORTED, "batched path: more than 120 up-hop sources per string");
+      if (grad_is_fused(rs, c64)) {
+        fused[c64 ? 1 : 0].push_back(std::move(t));
+        continue;
+      }
+      std::vector<ChainGrad> cg;
+      rc = grad_one(rs, ro, bT, R, M, seed, method, start_mode, &cg);
+      if (!rc) rc = add(t, cg);
       if (rc) return rc;
-      if (!(std::fabs(lz - lnz_s[idx]) <= 1e-9 * std::max(1.0, std::fabs(lz))))
-        return fail(FTLM_ERR_NUMERIC, "gradient replay of sector (" + std::to_string(nu) + "," + std::to_string(nd) +
-                                          ") did not reproduce the forward ln Z");
-      for (int q = 0; q < 3; ++q) d[q] += w * g[q];
     }
+  for (int c64 = 0; c64 < 2; ++c64) {
+    std::vector<ftlm_sector*> hs, ho;
+    for (const Term& t : fused[c64]) {
+      hs.push_back(t.s.get());
+      ho.push_back(t.op.get());
+    }
+    if (hs.empty()) continue;
+    std::vector<std::vector<ChainGrad>> cg;
+    const int mode = method == 1 ? FTLM_START_PHILOX : start_mode;
+    rc = c64 ? grad_fused<float4>(hs, ho, bT, R, M, seed, mode, &cg) : grad_fused<double2>(hs, ho, bT, R, M, seed, mode, &cg);
+    for (size_t i = 0; !rc && i < hs.size(); ++i) rc = add(fused[c64][i], cg[i]);
+    if (rc) return rc;
+  }
   grad[0] = d[0];
   grad[1] = d[1];
   grad[2] = d[2];

@@ -359,14 +359,16 @@ int sector_create(const ftlm_params* p, int n_up, int n_dn, PlanParts* parts, ft
 extern BtWs g_bt;
 extern std::mutex g_bt_mu;
 
-// Krylov vector store of the gradient replay (grows to the largest sector seen).
+// Krylov vector store of the gradient replay (grows to the largest piece seen), kept between calls.
 struct GradWs {
-  DevBuf Q, AQ, Kp, part, zflag;
-  size_t qcap = 0, acap = 0, kcap = 0, pcap = 0;
+  DevBuf Q, AQ, flag;
+  size_t qcap = 0, acap = 0;
   cudaError_t grow(DevBuf& b, size_t& cap, size_t bytes) {
     if (bytes <= cap && b.p) return cudaSuccess;
-    cap = bytes;
-    return b.alloc(bytes);
+    cap = 0;
+    const cudaError_t e = b.alloc(bytes);
+    if (e == cudaSuccess) cap = bytes;
+    return e;
   }
   void release() {
     Q.alloc(0);

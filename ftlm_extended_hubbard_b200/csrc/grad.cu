@@ -41,17 +41,22 @@ struct Elem<double2> {  // one complex128 chain
 template <typename T>
 __global__ void __launch_bounds__(256) moments_kernel(DevSector S, const T* __restrict__ W, const T* __restrict__ AW,
                                                       int64_t vstride, int64_t pstride, const double* __restrict__ Kp,
-                                                      int n, int ld, int nc, int nb, double* __restrict__ partial) {
+                                                      const int* __restrict__ used, int chains, int ld, int nb,
+                                                      double* __restrict__ partial) {
   constexpr int kC = Elem<T>::kC;
   extern __shared__ __align__(16) unsigned char smraw[];
   const int E = blockDim.x;
-  T* Ws = reinterpret_cast<T*>(smraw);                                                    // [n][E]
-  double* Ks = reinterpret_cast<double*>(smraw + static_cast<size_t>(n) * E * sizeof(T));  // [n][kIB][kC]
   const int t = threadIdx.x;
   const int plane = blockIdx.x / nb, b = blockIdx.x - plane * nb;
+  int n = 0;  // the plane's longest chain
+#pragma unroll
+  for (int q = 0; q < kC; ++q)
+    if (plane * kC + q < chains) n = max(n, min(used[plane * kC + q], ld));
+  T* Ws = reinterpret_cast<T*>(smraw);                                                    // [n][E]
+  double* Ks = reinterpret_cast<double*>(smraw + static_cast<size_t>(n) * E * sizeof(T));  // [n][kIB][kC]
   const T* Wp = W + plane * pstride;
   const T* Ap = AW + plane * pstride;
-  const double* Kc = Kp + plane * kC;
+  const double* Kc = Kp + static_cast<int64_t>(plane) * kC * ld * ld;
   double accD[kC] = {}, accP[kC] = {}, accA[kC] = {};
   const int64_t nch = (S.dim + E - 1) / E;
   for (int64_t ch = b; ch < nch; ch += nb) {
@@ -71,8 +76,9 @@ __global__ void __launch_bounds__(256) moments_kernel(DevSector S, const T* __re
     for (int i0 = 0; i0 < n; i0 += kIB) {
       __syncthreads();
       for (int idx = t; idx < kIB * n * kC; idx += E) {
-        const int q = idx % kC, ib = idx / kC % kIB, l = idx / (kC * kIB);
-        Ks[idx] = (i0 + ib < n) ? Kc[(static_cast<int64_t>(i0 + ib) * ld + l) * nc + q] : 0.0;
+        const int l = idx % n, q = idx / n % kC, ib = idx / (n * kC);
+        Ks[(l * kIB + ib) * kC + q] =
+            (i0 + ib < n && plane * kC + q < chains) ? Kc[(static_cast<int64_t>(q) * ld + i0 + ib) * ld + l] : 0.0;
       }
       __syncthreads();
       if (!valid) continue;
@@ -125,14 +131,24 @@ __global__ void __launch_bounds__(256) moments_kernel(DevSector S, const T* __re
     double sum = 0.0;
     for (int j = lane; j < E; j += 32) sum += red[v * E + j];
     for (int o = 16; o > 0; o >>= 1) sum += __shfl_down_sync(0xffffffffu, sum, o);
-    if (lane == 0) partial[(static_cast<int64_t>(b) * nc + plane * kC + v / 3) * 3 + v % 3] = sum;
+    if (lane == 0 && plane * kC + v / 3 < chains) partial[(static_cast<int64_t>(b) * chains + plane * kC + v / 3) * 3 + v % 3] = sum;
   }
 }
 
+// out[v] = sum over the blocks of partial[block][v], in order.
+__global__ void sum_blocks_kernel(const double* __restrict__ partial, int blocks, int nv, double* __restrict__ out) {
+  const int v = blockIdx.x * blockDim.x + threadIdx.x;
+  if (v >= nv) return;
+  double s = 0.0;
+  for (int b = 0; b < blocks; ++b) s += partial[static_cast<int64_t>(b) * nv + v];
+  out[v] = s;
+}
+
 template <typename T>
-cudaError_t launch(const DevSector& S, const T* W, const T* AW, int64_t vstride, int64_t pstride, int planes,
-                   const double* Kp, int n, int ld, int nc, double* partial, int* blocks, cudaStream_t st) {
+cudaError_t launch(const DevSector& S, const T* W, const T* AW, int64_t vstride, int64_t pstride, int chains,
+                   const double* Kp, const int* used, int ld, double* partial, double* out, cudaStream_t st) {
   constexpr int kC = Elem<T>::kC;
+  const int planes = (chains + kC - 1) / kC, n = ld;
   int dev = 0, sms = 0, optin = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -153,23 +169,23 @@ cudaError_t launch(const DevSector& S, const T* W, const T* AW, int64_t vstride,
   const int per_sm = std::max(1, std::min(static_cast<int>(static_cast<size_t>(optin) / smem), 2048 / E));
   const int64_t cap = std::max<int64_t>(1, (static_cast<int64_t>(sms) * per_sm + planes - 1) / planes);
   const int nb = static_cast<int>(std::min<int64_t>({nch, cap, kGradMaxBlocks}));
-  *blocks = nb;
-  moments_kernel<T><<<nb * planes, E, smem, st>>>(S, W, AW, vstride, pstride, Kp, n, ld, nc, nb, partial);
+  moments_kernel<T><<<nb * planes, E, smem, st>>>(S, W, AW, vstride, pstride, Kp, used, chains, ld, nb, partial);
+  sum_blocks_kernel<<<(3 * chains + 63) / 64, 64, 0, st>>>(partial, nb, 3 * chains, out);
   return cudaGetLastError();
 }
 
 }  // namespace
 
 cudaError_t grad_moments(const DevSector& S, const float4* W, const float4* AW, int64_t vstride, int64_t pstride,
-                         int planes, const double* Kp, int n, int ld, int nc, double* partial, int* blocks,
+                         int chains, const double* Kp, const int* used, int ld, double* partial, double* out,
                          cudaStream_t st) {
-  return launch(S, W, AW, vstride, pstride, planes, Kp, n, ld, nc, partial, blocks, st);
+  return launch(S, W, AW, vstride, pstride, chains, Kp, used, ld, partial, out, st);
 }
 
 cudaError_t grad_moments(const DevSector& S, const double2* W, const double2* AW, int64_t vstride, int64_t pstride,
-                         int planes, const double* Kp, int n, int ld, int nc, double* partial, int* blocks,
+                         int chains, const double* Kp, const int* used, int ld, double* partial, double* out,
                          cudaStream_t st) {
-  return launch(S, W, AW, vstride, pstride, planes, Kp, n, ld, nc, partial, blocks, st);
+  return launch(S, W, AW, vstride, pstride, chains, Kp, used, ld, partial, out, st);
 }
 
 }  // namespace ftlm_b200

@@ -18,14 +18,14 @@ namespace ftlm_b200 {
 
 constexpr int64_t kGradMaxBlocks = 2048;
 
-// Kp: [n][ld][nc] (row i, column l, chain fastest), nc = the planes' chains.  partial: [blocks][nc][3] doubles, blocks
-// (<= kGradMaxBlocks) returned in *blocks.  Shared memory: the n vectors' entries of a block of 32 to 256 states;
-// cudaErrorInvalidValue when that does not fit.
+// Kp: [chains][ld][ld]; used [chains]: the vectors of each chain (those past a plane's longest chain are not read).
+// partial: scratch of kGradMaxBlocks * chains * 3 doubles; out: [chains][3].  Shared memory: the ld vectors' entries of a
+// block of 32 to 256 states; cudaErrorInvalidValue when that does not fit.
 cudaError_t grad_moments(const DevSector& S, const float4* W, const float4* AW, int64_t vstride, int64_t pstride,
-                         int planes, const double* Kp, int n, int ld, int nc, double* partial, int* blocks,
+                         int chains, const double* Kp, const int* used, int ld, double* partial, double* out,
                          cudaStream_t st);
 cudaError_t grad_moments(const DevSector& S, const double2* W, const double2* AW, int64_t vstride, int64_t pstride,
-                         int planes, const double* Kp, int n, int ld, int nc, double* partial, int* blocks,
+                         int chains, const double* Kp, const int* used, int ld, double* partial, double* out,
                          cudaStream_t st);
 
 }  // namespace ftlm_b200

@@ -562,6 +562,15 @@ cudaError_t step(const DevSector& S, const typename P::T* Wk, const typename P::
   return cudaGetLastError();
 }
 
+template <class P>
+cudaError_t apply(const DevSector& S, const typename P::T* X, typename P::T* Y, int planes, int* flag, cudaStream_t s) {
+  cudaError_t e = cudaMemsetAsync(flag, 0, sizeof(int), s);
+  if (e == cudaSuccess) e = launch_rows<P>(S, X, Y, planes, nullptr, flag, s);
+  if (e != cudaSuccess) return e;
+  launch_cols<P>(S, X, Y, planes, nullptr, nullptr, nullptr, flag, s);
+  return cudaGetLastError();
+}
+
 }  // namespace
 
 int pl_group(const DevSector& S, bool c64, int planes) {
@@ -598,11 +607,12 @@ cudaError_t pl_step(const DevSector& S, const double2* Wk, const double2* Wkm1, 
   return step<C128>(S, Wk, Wkm1, Y, planes, k, z, s);
 }
 
-cudaError_t pl_apply(const DevSector& S, const float4* X, float4* Y, int planes, int* zero_flag, cudaStream_t s) {
-  const cudaError_t e = launch_rows<C64>(S, X, Y, planes, nullptr, zero_flag, s);
-  if (e != cudaSuccess) return e;
-  launch_cols<C64>(S, X, Y, planes, nullptr, nullptr, nullptr, zero_flag, s);
-  return cudaGetLastError();
+cudaError_t pl_apply(const DevSector& S, const float4* X, float4* Y, int planes, int* flag, cudaStream_t s) {
+  return apply<C64>(S, X, Y, planes, flag, s);
+}
+
+cudaError_t pl_apply(const DevSector& S, const double2* X, double2* Y, int planes, int* flag, cudaStream_t s) {
+  return apply<C128>(S, X, Y, planes, flag, s);
 }
 
 }  // namespace ftlm_b200

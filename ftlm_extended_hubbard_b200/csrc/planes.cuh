@@ -47,8 +47,9 @@ cudaError_t pl_step(const DevSector& S, const float4* Wk, const float4* Wkm1, fl
                     const PlaneState& z, cudaStream_t s);
 cudaError_t pl_step(const DevSector& S, const double2* Wk, const double2* Wkm1, double2* Y, int planes, int k,
                     const PlaneState& z, cudaStream_t s);
-// Y = (G H G) X for any number of planes, without Lanczos bookkeeping; zero_flag points to an int 0 (no small-entry
-// filter).
-cudaError_t pl_apply(const DevSector& S, const float4* X, float4* Y, int planes, int* zero_flag, cudaStream_t s);
+// Y = (G H G) X for any number of planes, without Lanczos bookkeeping; flag: an int of scratch.  (complex64: no small-entry
+// filter.)
+cudaError_t pl_apply(const DevSector& S, const float4* X, float4* Y, int planes, int* flag, cudaStream_t s);
+cudaError_t pl_apply(const DevSector& S, const double2* X, double2* Y, int planes, int* flag, cudaStream_t s);
 
 }  // namespace ftlm_b200

@@ -362,14 +362,14 @@ __global__ void __launch_bounds__(kMaxEig) tql_vectors_kernel(const double* __re
   }
 }
 
-// K = Z P Z^T in the moment kernel's layout Kp[(i*ld + l)*nc + c] / (sc_i sc_l), with
+// K = Z P Z^T in the moment kernel's layout Kp[(c*ld + i)*ld + l] / (sc_i sc_l), 0 outside the chain's n rows, with
 // Z[i][j] = Vt[j][i] (ascending l_j); g = sum_j Z_0j^2 e^{-b (l_j - l_0)}, lmin = l_0.
 // P is formed once in shared memory (one expm1 and one division an entry); both products then read it and V.
 constexpr int kDuhThreads = 512;
 
 __global__ void __launch_bounds__(kDuhThreads) duhamel_kernel(const double* __restrict__ lam,
                                                               const double* __restrict__ vt,
-                                                              const int* __restrict__ nv, int ld, int nc, double bT,
+                                                              const int* __restrict__ nv, int ld, double bT,
                                                               const double* __restrict__ scale,
                                                               double* __restrict__ Y, double* __restrict__ Kp,
                                                               double* __restrict__ g_out,
@@ -378,7 +378,12 @@ __global__ void __launch_bounds__(kDuhThreads) duhamel_kernel(const double* __re
   const int ch = blockIdx.x;
   const int tid = threadIdx.x;
   const int n = nv[ch];
-  if (n <= 0 || n > ld) return;
+  double* Kc = Kp + static_cast<int64_t>(ch) * ld * ld;
+  if (n <= 0 || n > ld) {
+    for (int e = tid; e < ld * ld; e += kDuhThreads) Kc[e] = 0.0;
+    if (tid == 0) g_out[ch] = lmin_out[ch] = 0.0;
+    return;
+  }
   const double* l = lam + static_cast<int64_t>(ch) * ld;
   const double* V = vt + static_cast<int64_t>(ch) * ld * ld;  // V[j*ld + i] = Z[i][j]
   double* y = Y + static_cast<int64_t>(ch) * ld * ld;
@@ -407,13 +412,16 @@ __global__ void __launch_bounds__(kDuhThreads) duhamel_kernel(const double* __re
     y[static_cast<int64_t>(k) * ld + i] = acc * z0[k];
   }
   __syncthreads();
-  for (int e = tid; e < n * n; e += kDuhThreads) {
-    const int i = e / n, lq = e - i * n;
+  for (int e = tid; e < ld * ld; e += kDuhThreads) {
+    const int i = e / ld, lq = e - i * ld;
     double acc = 0.0;
+    if (i < n && lq < n) {
 #pragma unroll 4
-    for (int k = 0; k < n; ++k)
-      acc = fma(y[static_cast<int64_t>(k) * ld + i], V[static_cast<int64_t>(k) * ld + lq], acc);
-    Kp[(static_cast<int64_t>(i) * ld + lq) * nc + ch] = acc / (sc[i] * sc[lq]);
+      for (int k = 0; k < n; ++k)
+        acc = fma(y[static_cast<int64_t>(k) * ld + i], V[static_cast<int64_t>(k) * ld + lq], acc);
+      acc /= sc[i] * sc[lq];
+    }
+    Kc[e] = acc;
   }
   if (tid == 0) {
     double gs = 0.0;
@@ -481,7 +489,7 @@ cudaError_t duhamel_weights_dev(const double* lam, const double* vt, const int* 
   const size_t sm = static_cast<size_t>(ld) * ld * sizeof(double);
   const cudaError_t e = cudaFuncSetAttribute(duhamel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sm));
   if (e != cudaSuccess) return e;
-  duhamel_kernel<<<nc, kDuhThreads, sm, st>>>(lam, vt, n, ld, nc, bT, scale, Y, Kp, g, lmin);
+  duhamel_kernel<<<nc, kDuhThreads, sm, st>>>(lam, vt, n, ld, bT, scale, Y, Kp, g, lmin);
   return cudaGetLastError();
 }
 

@@ -19,9 +19,8 @@ cudaError_t symeig_dense(const double* A, const int* n, int nm, int ld, double* 
 // Real symmetric embedding [[Re H, -Im H], [Im H, Re H]] (2dk x 2dk, row-major) of a Hermitian
 // matrix given by its columns (column j at cols + j*dk).
 cudaError_t embed_hermitian(const double2* cols, int dk, double* R, cudaStream_t st);
-// Duhamel weights of nc chains from symeig_tridiag's lam / vt: Kp[(i*ld + l)*nc + c] =
-// K_il / (scale[c][i] scale[c][l]) for i, l < n[c] (other entries untouched: clear Kp first);
-// g[c] = sum_j Z_0j^2 e^{-bT (lam_j - lam_0)}, lmin[c] = lam_0.  Y: scratch [nc][ld][ld].
+// Duhamel weights of nc chains from symeig_tridiag's lam / vt: Kp[(c*ld + i)*ld + l] = K_il / (scale[c][i] scale[c][l]),
+// 0 where i or l >= n[c]; g[c] = sum_j Z_0j^2 e^{-bT (lam_j - lam_0)}, lmin[c] = lam_0.  Y: scratch [nc][ld][ld].
 cudaError_t duhamel_weights_dev(const double* lam, const double* vt, const int* n, int nc, int ld, double bT,
                                 const double* scale, double* Y, double* Kp, double* g, double* lmin, cudaStream_t st);
 

@@ -473,6 +473,7 @@ int ftlm_gpu_sector_diag(const ftlm_sector* s, long long index, double* value) {
 int ftlm_gpu_set_apply_path(ftlm_sector* s, int path) {
   if (!s || path < 0 || path > 3) return fail(FTLM_ERR_INVALID, "bad path");
   s->apply_path = path;
+  s->use_once = path == 0;
   return FTLM_OK;
 }
 
@@ -495,7 +496,11 @@ int ftlm_gpu_apply_profiled(ftlm_sector* s, const double* x, double* y, void* st
   cudaEvent_t ev[3];
   for (auto& e : ev) CU_TRY(cudaEventCreate(&e));
   CU_TRY(cudaEventRecord(ev[0], st));
-  if (path >= 2) {
+  const bool once = s->once();
+  if (once) {
+    CU_TRY(hv_launch_once(s->dev, reinterpret_cast<const double2*>(x), reinterpret_cast<double2*>(y), st));
+    CU_TRY(cudaEventRecord(ev[1], st));
+  } else if (path >= 2) {
     CU_TRY(hv_launch_pass(d, reinterpret_cast<const double2*>(x), reinterpret_cast<double2*>(y), 0, st,
                           s->cols_variant));
     CU_TRY(cudaEventRecord(ev[1], st));
@@ -509,7 +514,7 @@ int ftlm_gpu_apply_profiled(ftlm_sector* s, const double* x, double* y, void* st
   CU_TRY(cudaEventSynchronize(ev[2]));
   CU_TRY(cudaEventElapsedTime(&ms_passes[0], ev[0], ev[1]));
   *n_passes = 1;
-  if (path >= 2) {
+  if (path >= 2 && !once) {
     CU_TRY(cudaEventElapsedTime(&ms_passes[1], ev[1], ev[2]));
     *n_passes = 2;
   }
@@ -999,7 +1004,11 @@ int ftlm_gpu_autotune_apply(ftlm_sector* s, int reps, int* path, int* cols_varia
   const SectorPlan& P = s->plan;
   // one timing per sector shape and process
   static std::mutex mu;
-  static std::map<std::string, std::pair<int, int>> cache;
+  struct Choice {
+    int path, variant;
+    bool once;
+  };
+  static std::map<std::string, Choice> cache;
   char key[160];
   std::snprintf(key, sizeof(key), "%d/%d/%d/%zu/%zu/%d/%d", P.n, P.nu, P.nd, P.hu.size(), P.hd.size(), P.max_up_deg,
                 P.max_dn_deg);
@@ -1007,8 +1016,9 @@ int ftlm_gpu_autotune_apply(ftlm_sector* s, int reps, int* path, int* cols_varia
     std::lock_guard<std::mutex> lock(mu);
     auto it = cache.find(key);
     if (it != cache.end()) {
-      s->apply_path = it->second.first;
-      s->cols_variant = it->second.second;
+      s->apply_path = it->second.path;
+      s->cols_variant = it->second.variant;
+      s->use_once = it->second.once;
       if (path) *path = s->apply_path;
       if (cols_variant) *cols_variant = s->cols_variant;
       if (ms) *ms = -1.0f;
@@ -1029,17 +1039,24 @@ int ftlm_gpu_autotune_apply(ftlm_sector* s, int reps, int* path, int* cols_varia
   int best_p = 1, best_v = 0;
   float best = 3.4e38f;
   const bool fast = hv_fast_path_ok(s->dev_for(2), P.max_up_deg);
-  const int variants[10][2] = {{1, 0}, {2, 0}, {2, 1}, {2, 2}, {3, 0}, {3, 1}, {3, 2}, {3, 3}, {3, 4}, {3, 5}};
+  bool best_once = false;
+  const int variants[11][2] = {{0, 0}, {1, 0}, {2, 0}, {2, 1}, {2, 2}, {3, 0}, {3, 1}, {3, 2}, {3, 3}, {3, 4}, {3, 5}};
   cudaError_t ce = cudaSuccess;
   for (const auto& v : variants) {
+    const bool once = v[0] == 0;  // H v in one pass; reported as path 3, whose row pass it has
+    if (once && !hv_once_ok(s->dev, P.max_up_deg)) continue;
     if (v[0] >= 2 && !fast) continue;
     if (v[0] == 3 && !s->path_available(3)) continue;
     if (v[1] >= 3 && !s->dev.up_pk) continue;
     const DevSector d = s->dev_for(v[0], v[1]);
     const int lp = v[0] == 3 ? 2 : v[0];
-    ce = hv_launch(d, x.as<double2>(), y.as<double2>(), lp, st, v[1]);  // warm-up
+    auto run = [&]() {
+      return once ? hv_launch_once(s->dev, x.as<double2>(), y.as<double2>(), st)
+                  : hv_launch(d, x.as<double2>(), y.as<double2>(), lp, st, v[1]);
+    };
+    ce = run();  // warm-up
     if (ce == cudaSuccess) ce = cudaEventRecord(e0, st);
-    for (int r = 0; r < reps && ce == cudaSuccess; ++r) ce = hv_launch(d, x.as<double2>(), y.as<double2>(), lp, st, v[1]);
+    for (int r = 0; r < reps && ce == cudaSuccess; ++r) ce = run();
     if (ce == cudaSuccess) ce = cudaEventRecord(e1, st);
     if (ce == cudaSuccess) ce = cudaEventSynchronize(e1);
     float t = 0.0f;
@@ -1047,8 +1064,9 @@ int ftlm_gpu_autotune_apply(ftlm_sector* s, int reps, int* path, int* cols_varia
     if (ce != cudaSuccess) break;
     if (t < best) {
       best = t;
-      best_p = v[0];
+      best_p = once ? 3 : v[0];
       best_v = v[1];
+      best_once = once;
     }
   }
   cudaEventDestroy(e0);
@@ -1056,9 +1074,10 @@ int ftlm_gpu_autotune_apply(ftlm_sector* s, int reps, int* path, int* cols_varia
   CU_TRY(ce);
   s->apply_path = best_p;
   s->cols_variant = best_v;
+  s->use_once = best_once;
   {
     std::lock_guard<std::mutex> lock(mu);
-    cache[key] = {best_p, best_v};
+    cache[key] = Choice{best_p, best_v, best_once};
   }
   if (path) *path = best_p;
   if (cols_variant) *cols_variant = best_v;

@@ -306,6 +306,7 @@ struct ftlm_sector {
   size_t tables_bytes = 0;
   ftlm_b200::capi::BtWs planes;  // vectors and scalars of its complex128 Lanczos chains
   int apply_path = 0;    // 0 auto, 1 generic, 2 rows+cols, 3 rows (register coefficient classes)+cols
+  bool use_once = true;  // H v in one pass where it can be (until a path is set)
   int cols_variant = 0;  // column slab 256/128/512 (0/1/2); 3/4/5: the same over the packed up list (path 3)
   ftlm_b200::capi::LanczosWs ws;
   ftlm_b200::capi::DevBuf hx, hy;  // staging for the host-buffer apply
@@ -318,7 +319,7 @@ struct ftlm_sector {
   // Kernel choice for H·v: 1 = generic gather; 2 = row pass with the per-row coefficient table +
   // column-slab pass over the CSR up list; 3 = row pass in the gauge basis (register-held real
   // coefficients) + column-slab pass, over the packed up list when cols_variant >= 3 and the sector
-  // has one.  Automatic: 3, else 2, else 1.
+  // has one.  Automatic: one pass (hv_once) for small sectors, else 3, else 2, else 1.
   bool path_available(int path) const {
     if (path == 1) return true;
     if (path == 3 && !dev.dn_g.ent) return false;
@@ -338,7 +339,12 @@ struct ftlm_sector {
     if (path != 3 || cv < 3) d.up_pk = nullptr;
     return d;
   }
+  bool once() const { return use_once && ftlm_b200::hv_once_ok(dev, plan.max_up_deg); }
   int apply(const double2* x, double2* y, cudaStream_t st) {
+    if (once()) {
+      CU_TRY(ftlm_b200::hv_launch_once(dev, x, y, st));
+      return FTLM_OK;
+    }
     const int path = effective_path();
     const ftlm_b200::DevSector d = dev_for(path);
     if (path >= 2 && ftlm_b200::hv_rows_smem_bytes(d) > 227 * 1024)

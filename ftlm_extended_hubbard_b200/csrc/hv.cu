@@ -5,6 +5,8 @@
 //
 // Paths:
 //   hv_generic  one thread per output element, everything gathered from global memory.  Any size.
+//   hv_once     one pass for small sectors (the default there): a row staged in shared
+//               memory for the down hops, the up hops gathered from the other rows in L2.
 //   hv_rows     pass 1 of the fast path: persistent CTAs, one output row at a time; the input
 //               row is staged in shared memory (down hops gather inside it); writes
 //               y = diag o x + down part.  Requires a down row (+ coefficient table) to fit in SMEM.
@@ -216,10 +218,10 @@ __global__ void __launch_bounds__(kRowThreads, 1) hv_rows_gauge_kernel(DevSector
   const int Dd = static_cast<int>(S.Dd);
   double2* xs = reinterpret_cast<double2*>(smem_raw);
   double2* tab = xs + Dd + 8;
-  const int tid = threadIdx.x;
+  const int tid = threadIdx.x, nt = blockDim.x;
   const DevGauge G = S.dn_g;
   if (!kPhase)
-    for (int i = tid; i < G.nt * 8; i += kRowThreads) tab[i] = G.tab[i >> 3];
+    for (int i = tid; i < G.nt * 8; i += nt) tab[i] = G.tab[i >> 3];
   if (tid < 8) xs[Dd + tid] = make_double2(0.0, 0.0);  // zero sentinels for padding entries
   const double a0 = G.real2[0], a1 = G.real2[1];
   for (int64_t r = blockIdx.x; r < S.Du; r += gridDim.x) {
@@ -229,7 +231,7 @@ __global__ void __launch_bounds__(kRowThreads, 1) hv_rows_gauge_kernel(DevSector
     const uint4 w = S.wpl[r];
     const double2* xrow = x + r * S.Dd;
     int saw_tiny = 0;
-    for (int c = tid; c < Dd; c += kRowThreads) {
+    for (int c = tid; c < Dd; c += nt) {
       double2 v = xrow[c];
       if (tiny(v)) {
         saw_tiny |= (v.x != 0.0 || v.y != 0.0);
@@ -241,7 +243,7 @@ __global__ void __launch_bounds__(kRowThreads, 1) hv_rows_gauge_kernel(DevSector
     if (saw_tiny) atomicOr(S.flags, 1);
     __syncthreads();
     double2* yrow = y + r * S.Dd;
-    for (int c = tid; c < Dd; c += kRowThreads) {
+    for (int c = tid; c < Dd; c += nt) {
       const int d = gauge_string(G, c);  // table position c serves output string d
       const uint32_t dm = S.dmask[d];
       const double2 xv = xs[d];
@@ -250,6 +252,85 @@ __global__ void __launch_bounds__(kRowThreads, 1) hv_rows_gauge_kernel(DevSector
       gauge_hops<kPhase, kXor>(acc, G, c, smem_raw, tab, a0, a1);
       if (gauge_sign(u, dm)) acc = make_double2(-acc.x, -acc.y);
       yrow[d] = acc;
+    }
+    __syncthreads();
+  }
+}
+
+// One pass for small sectors: a block takes one output row, stages the input row in shared memory in
+// the spin-ordered basis for the down hops (the row pass), and adds the up hops straight from the other rows in L2 (the
+// column pass without its slabs) before the only write of y.  Against the two passes this saves a write and a read of y,
+// a launch and the flag's memset, and blocks as wide as a row fill an SM several at a time, so that staging overlaps the
+// hops of other blocks.  The skip rule is tested on every source, so no flag is needed.  Bound by the latency of its
+// gathers for small sectors and by the L1 data pipe for large ones: 4x2 (4,4) 12.3 us with the generic kernel, 6.4 here;
+// 3x3 (4,4) 18.9 and 8.2, 5x2 (5,5) 16.4 and 8.2.
+constexpr int kOnceThreads = 512;
+// Where one pass is the faster form: small sectors, and up to 64 MB of the 126 MB of L2 where the rows are short (their two
+// passes are mostly launches and idle lanes).  One pass / two passes: 4x3 (3,8), 108,900 states, 14.4 / 16.3 us; 4x3 (4,4),
+// 245,025 states, 22.8 / 22.6; 4x3 (6,6), 853,776 states, 77.5 / 57.2; 4x4 (8,2), rows of 120, 113 / 133.
+constexpr int64_t kOnceMaxDim = int64_t(1) << 17, kOnceShortRow = 256, kOnceShortDim = int64_t(1) << 22;
+constexpr size_t kOnceListBytes = kMaxUpDeg * 24;  // the row's source list
+
+template <bool kPhase, bool kXor>
+__global__ void __launch_bounds__(kOnceThreads, 2) hv_once_kernel(DevSector S, const double2* __restrict__ x,
+                                                                  double2* __restrict__ y) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ uint32_t s_off[kMaxUpDeg], s_lh[kMaxUpDeg];
+  __shared__ double2 s_coef[kMaxUpDeg];
+  const int Dd = static_cast<int>(S.Dd), Du = static_cast<int>(S.Du), nt = blockDim.x;
+  double2* xs = reinterpret_cast<double2*>(smem_raw);
+  double2* tab = xs + Dd + 8;
+  const int tid = threadIdx.x;
+  const DevGauge G = S.dn_g;
+  if (!kPhase)
+    for (int i = tid; i < G.nt * 8; i += nt) tab[i] = G.tab[i >> 3];
+  if (tid < 8) xs[Dd + tid] = make_double2(0.0, 0.0);  // zero sentinels for padding entries
+  const double a0 = G.real2[0], a1 = G.real2[1];
+  for (int r = blockIdx.x; r < Du; r += gridDim.x) {
+    const uint32_t u = S.umask[r];
+    const int cuu = S.cnt_uu[r];
+    const uint4 w = S.wpl[r];
+    const double2* xrow = x + static_cast<int64_t>(r) * Dd;
+    for (int c = tid; c < Dd; c += nt) {
+      double2 v = xrow[c];
+      if (tiny(v)) v = make_double2(0.0, 0.0);
+      if (gauge_sign(u, S.dmask[c])) v = make_double2(-v.x, -v.y);
+      xs[c] = v;
+    }
+    const int j0 = S.up_ptr[r], deg = S.up_ptr[r + 1] - j0;
+    for (int j = tid; j < deg; j += nt) {
+      s_off[j] = static_cast<uint32_t>(S.up_src[j0 + j]) * static_cast<uint32_t>(Dd);
+      s_coef[j] = S.up_coef[j0 + j];
+      s_lh[j] = S.up_lohi[j0 + j];
+    }
+    __syncthreads();
+    for (int c = tid; c < Dd; c += nt) {
+      const int d = gauge_string(G, c);  // table position c serves output string d
+      const uint32_t dm = S.dmask[d];
+      const double2 xv = xs[d];
+      const double dg = diag_value(S, u, dm, cuu, S.cnt_dd[d], w);
+      double2 acc = make_double2(dg * xv.x, dg * xv.y);
+      gauge_hops<kPhase, kXor>(acc, G, c, smem_raw, tab, a0, a1);
+      if (gauge_sign(u, dm)) acc = make_double2(-acc.x, -acc.y);
+      const uint32_t q = prefix_parity_shifted(dm);
+      const double2* col = x + d;
+      int j = 0;
+      for (; j + 4 <= deg; j += 4) {
+        double2 v[4];
+#pragma unroll
+        for (int t = 0; t < 4; ++t) v[t] = col[s_off[j + t]];
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+          const uint32_t lh = s_lh[j + t];
+          if (!tiny(v[t])) cmac_xor(acc, s_coef[j + t], v[t], ((q >> (lh & 255u)) ^ (q >> (lh >> 8))) & 1u);
+        }
+      }
+      for (; j < deg; ++j) {
+        const double2 v = col[s_off[j]];
+        const uint32_t lh = s_lh[j];
+        if (!tiny(v)) cmac_xor(acc, s_coef[j], v, ((q >> (lh & 255u)) ^ (q >> (lh >> 8))) & 1u);
+      }
+      y[static_cast<int64_t>(r) * Dd + d] = acc;
     }
     __syncthreads();
   }
@@ -443,6 +524,23 @@ cudaError_t launch_cols(const DevSector& S, const double2* x, double2* y, cudaSt
   return cudaGetLastError();
 }
 
+bool hv_once_ok(const DevSector& S, int max_up_deg) {
+  return S.dn_g.ent && S.dim <= (S.Dd <= kOnceShortRow ? kOnceShortDim : kOnceMaxDim) && max_up_deg <= kMaxUpDeg && hv_rows_smem_bytes(S) + kOnceListBytes <= 227 * 1024;
+}
+
+cudaError_t hv_launch_once(const DevSector& S, const double2* x, double2* y, cudaStream_t st) {
+  init_sm_count();
+  const size_t sm = hv_rows_smem_bytes(S);
+  const RowsKernel k = S.dn_g.phase ? (S.dn_g.xor_real ? hv_once_kernel<true, true> : hv_once_kernel<true, false>)
+                                    : (S.dn_g.xor_real ? hv_once_kernel<false, true> : hv_once_kernel<false, false>);
+  const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sm));
+  if (e != cudaSuccess) return e;
+  int threads = kOnceThreads;
+  while (threads > 64 && (threads / 2 >= S.Dd || (threads > 256 && S.Du > g_num_sms))) threads /= 2;
+  k<<<static_cast<unsigned>(S.Du), threads, sm, st>>>(S, x, y);
+  return cudaGetLastError();
+}
+
 cudaError_t hv_launch_pass(const DevSector& S, const double2* x, double2* y, int pass, cudaStream_t st,
                            int cols_variant) {
   if (S.dim <= 0) return cudaSuccess;
@@ -456,8 +554,15 @@ cudaError_t hv_launch_pass(const DevSector& S, const double2* x, double2* y, int
                                         : (S.dn_g.xor_real ? hv_rows_gauge_kernel<false, true> : hv_rows_gauge_kernel<false, false>);
     e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sm));
     if (e != cudaSuccess) return e;
-    const int grid_r = static_cast<int>(std::min<int64_t>(S.Du, g_num_sms));
-    k<<<grid_r, kRowThreads, sm, st>>>(S, x, y);
+    // Blocks as wide as a row needs, several on an SM where their rows fit: one block's staging overlaps another's hops.
+    int threads = kRowThreads, per_sm = 1;
+    if (S.dn_g.ent) {
+      const int fit = static_cast<int>((227 * 1024 + 1024) / (sm + 1024));
+      while (threads > 64 && (threads / 2 >= S.Dd || (threads > 256 && threads / 2 * fit >= kRowThreads))) threads /= 2;
+      per_sm = std::max(1, std::min(fit, kRowThreads / threads));
+    }
+    const int grid_r = static_cast<int>(std::min<int64_t>(S.Du, static_cast<int64_t>(g_num_sms) * per_sm));
+    k<<<grid_r, threads, sm, st>>>(S, x, y);
     return cudaGetLastError();
   }
   cols_variant %= 3;  // 3..5: the same slabs; the list form comes with S (S.up_pk)

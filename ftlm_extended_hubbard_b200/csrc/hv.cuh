@@ -13,6 +13,9 @@ namespace ftlm_b200 {
 // or 4) or 512 (2 or 5) columns.
 cudaError_t hv_launch(const DevSector& S, const double2* x, double2* y, int path, cudaStream_t st,
                       int cols_variant = 0);
+// H v in one pass: whether the sector takes it (small, with a gauge table), and the launch.
+bool hv_once_ok(const DevSector& S, int max_up_deg);
+cudaError_t hv_launch_once(const DevSector& S, const double2* x, double2* y, cudaStream_t st);
 // One pass of the fast path: 0 = row pass (diag + down hops), 1 = column-slab pass (up hops).
 cudaError_t hv_launch_pass(const DevSector& S, const double2* x, double2* y, int pass, cudaStream_t st,
                            int cols_variant = 0);

@@ -233,12 +233,13 @@ __global__ void __launch_bounds__(kScalarThreads) bt_scalar_kernel(const double*
   st[kBtSin * 32 + chain] = 1.0 / b;
 }
 
-// Orbit momentum block, 32 chains: Y[a, :] = H_K W[a, :] (complex64 block vectors over the
-// block's representatives) and the fused <W_k, Y> per chain.  Warp per representative: the lanes
-// walk the representative's sources in the sector's gather tables 32 at a time (table lookup and
-// coefficient <rep a|H|s> eta conj(chi(R)) sqrt|A_b| / sqrt|A_a| in FP64, rounded to complex64) and
-// compact the surviving ones into the warp's shared-memory list; then the half-warps gather the
-// 256-byte rows W[b, :] as in the column pass.  Same algebra as the complex128 apply_tables kernel.
+// Orbit momentum block, 32 chains: Y[a, :] = H_K W[a, :] (complex64 block vectors over the block's representatives) and
+// the fused <W_k, Y> per chain.  Warp per representative: its sources come from the block's list (orbit.cuh), or, where it
+// has none, from the sector's gather tables 32 at a time (a random 4-byte lookup per source), the surviving ones compacted
+// by ballot; coefficients <rep a|H|s> eta conj(chi(R)) sqrt|A_b| / sqrt|A_a| in FP64, rounded to complex64.  Then the
+// half-warps take every other source each and gather the 256-byte rows W[b, :].  Bound by instruction issue, about 900 per
+// representative (rows of 24 instead of 32 chains take as long): 4x4 (4,4), 207,000 representatives, 258 us with the table
+// lookups, 215 us with the lists.
 constexpr int kOrbTerms = 256;
 
 __device__ __forceinline__ void orb_push(bool ok, uint32_t off, float2 cf, int lane, int& cnt, uint32_t* s_off,
@@ -266,6 +267,9 @@ __global__ void __launch_bounds__(kBtThreads, kBtBlocksPerSm) bt_orbit_kernel(Or
   __shared__ uint32_t s_off[kBtWarps][kOrbTerms];
   __shared__ float2 s_cf[kBtWarps][kOrbTerms];
   __shared__ double sh[4 * kBtThreads];
+  __shared__ double2 s_dict[256];
+  if (A.list) s_dict[threadIdx.x] = A.dict[threadIdx.x];
+  __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int hv = lane >> 4, l = lane & 15;
   const bool filter = *flag != 0;
@@ -285,48 +289,59 @@ __global__ void __launch_bounds__(kBtThreads, kBtBlocksPerSm) bt_orbit_kernel(Or
     const double inv_sa = 1.0 / A.sqrtA[a];
     int cnt = 0;
     __syncwarp();
-    const uint32_t q = prefix_parity_shifted(d);
-    const int p1 = S.up_ptr[ru + 1];
-    for (int p0 = S.up_ptr[ru]; p0 < p1; p0 += 32) {
-      const int p = p0 + lane;
-      bool ok = false;
-      uint32_t o = 0;
-      float2 cf = make_float2(0.f, 0.f);
-      if (p < p1) {
-        const uint32_t e = __ldg(A.table + static_cast<int64_t>(S.up_src[p]) * Dd + rd);
-        if (e != kNone) {
-          const uint32_t lh = S.up_lohi[p];
-          double2 c = S.up_coef[p];
-          if (((q >> (lh & 255u)) ^ (q >> (lh >> 8))) & 1u) c = make_double2(-c.x, -c.y);
-          ok = true;
-          o = (e & 0xFFFFFFu) * 16u;
-          cf = orb_coef(A, c, e, inv_sa);
-        }
+    if (A.list) {
+      cnt = A.cnt[a];
+      const uint32_t* row = A.list + a * A.pitch;
+      for (int j = lane; j < cnt; j += 32) {
+        const uint32_t e = row[j];
+        const double2 c = s_dict[e >> 24];
+        off[j] = (e & 0xFFFFFFu) * 16u;
+        cfs[j] = make_float2(static_cast<float>(c.x * inv_sa), static_cast<float>(c.y * inv_sa));
       }
-      orb_push(ok, o, cf, lane, cnt, off, cfs);
-    }
-    const int64_t rowbase = static_cast<int64_t>(ru) * Dd;
-    const int64_t d1 = S.dn_csr_ptr[rd + 1];
-    for (int64_t p0 = S.dn_csr_ptr[rd]; p0 < d1; p0 += 32) {
-      const int64_t p = p0 + lane;
-      bool ok = false;
-      uint32_t o = 0;
-      float2 cf = make_float2(0.f, 0.f);
-      if (p < d1) {
-        const uint32_t ent = S.dn_csr_ent[p];
-        const int h = static_cast<int>((ent >> 1) & 255u);
-        if (h != S.n_dn_hops) {
-          const uint32_t e = __ldg(A.table + rowbase + (ent >> 9));
+    } else {
+      const uint32_t q = prefix_parity_shifted(d);
+      const int p1 = S.up_ptr[ru + 1];
+      for (int p0 = S.up_ptr[ru]; p0 < p1; p0 += 32) {
+        const int p = p0 + lane;
+        bool ok = false;
+        uint32_t o = 0;
+        float2 cf = make_float2(0.f, 0.f);
+        if (p < p1) {
+          const uint32_t e = __ldg(A.table + static_cast<int64_t>(S.up_src[p]) * Dd + rd);
           if (e != kNone) {
-            double2 c = S.dn_coef[h];
-            if ((ent & 1u) ^ (static_cast<uint32_t>(__popc(u & S.dn_nmask[h])) & 1u)) c = make_double2(-c.x, -c.y);
+            const uint32_t lh = S.up_lohi[p];
+            double2 c = S.up_coef[p];
+            if (((q >> (lh & 255u)) ^ (q >> (lh >> 8))) & 1u) c = make_double2(-c.x, -c.y);
             ok = true;
             o = (e & 0xFFFFFFu) * 16u;
             cf = orb_coef(A, c, e, inv_sa);
           }
         }
+        orb_push(ok, o, cf, lane, cnt, off, cfs);
       }
-      orb_push(ok, o, cf, lane, cnt, off, cfs);
+      const int64_t rowbase = static_cast<int64_t>(ru) * Dd;
+      const int64_t d1 = S.dn_csr_ptr[rd + 1];
+      for (int64_t p0 = S.dn_csr_ptr[rd]; p0 < d1; p0 += 32) {
+        const int64_t p = p0 + lane;
+        bool ok = false;
+        uint32_t o = 0;
+        float2 cf = make_float2(0.f, 0.f);
+        if (p < d1) {
+          const uint32_t ent = S.dn_csr_ent[p];
+          const int h = static_cast<int>((ent >> 1) & 255u);
+          if (h != S.n_dn_hops) {
+            const uint32_t e = __ldg(A.table + rowbase + (ent >> 9));
+            if (e != kNone) {
+              double2 c = S.dn_coef[h];
+              if ((ent & 1u) ^ (static_cast<uint32_t>(__popc(u & S.dn_nmask[h])) & 1u)) c = make_double2(-c.x, -c.y);
+              ok = true;
+              o = (e & 0xFFFFFFu) * 16u;
+              cf = orb_coef(A, c, e, inv_sa);
+            }
+          }
+        }
+        orb_push(ok, o, cf, lane, cnt, off, cfs);
+      }
     }
     const int deg8 = (cnt + 7) & ~7;
     for (int j = cnt + lane; j < deg8; j += 32) {  // padding: a valid row, zero coefficient

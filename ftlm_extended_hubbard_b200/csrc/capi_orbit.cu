@@ -29,6 +29,7 @@ struct ftlm_orbit {
   std::vector<int> stab;          // stabiliser size
   std::vector<int64_t> orbit_idx; // index among all representatives of the sector (ascending packed)
   DevBuf reps_dev, sqrtA, table, chi, xs;
+  DevBuf list, cnt, dict, lut;  // the block's source lists (null where their values have more than 255 codes)
   OrbitApplyDev app{};
   LanczosWs ws;
   DevBuf hx, hy;
@@ -159,6 +160,79 @@ int build_orbit_sector(ftlm_sector* s) {
   return FTLM_OK;
 }
 
+// The block's matrix as source lists (orbit.cuh): the values of the matrix elements, gathered up to rounding, become at
+// most 255 codes of 8 bits beside the 24 of a source's index.  Built once per block, for about two H_K v; each of these then
+// reads 4 bytes in order instead of 4 random ones per source.  Blocks with more values keep the tables.
+int build_lists(ftlm_orbit* o, const std::vector<double2>& chi) {
+  const SectorPlan& P = o->sector->plan;
+  OrbitApplyDev& A = o->app;
+  A.list = nullptr;
+  if (o->dk <= 0) return FTLM_OK;
+  OrbitCodes K{};
+  for (const auto* hops : {&P.hu, &P.hd})
+    for (const auto& h : *hops) {
+      bool known = false;
+      for (int i = 0; i < K.n_coef && !known; ++i)
+        known = (h.cre == K.coef[i].x && h.cim == K.coef[i].y) || (h.cre == -K.coef[i].x && h.cim == -K.coef[i].y);
+      if (known) continue;
+      if (K.n_coef == 16) return FTLM_OK;
+      K.coef[K.n_coef++] = make_double2(h.cre, h.cim);
+    }
+  for (int n = 1; n <= o->data->G; ++n) {  // |A| of a surviving representative is the size of its stabiliser
+    if (o->data->G % n != 0) continue;
+    if (K.n_a == 16) return FTLM_OK;
+    K.root[K.n_a++] = std::sqrt(static_cast<double>(n));
+  }
+  for (double a : o->absA) {
+    const double r = std::sqrt(a);
+    bool known = false;
+    for (int i = 0; i < K.n_a && !known; ++i) known = std::fabs(r - K.root[i]) <= 1e-12 * K.root[i];
+    if (!known) return FTLM_OK;
+  }
+  const int G = o->data->G;
+  std::vector<double2> dict(256, make_double2(0.0, 0.0));
+  std::vector<uint8_t> lut(static_cast<size_t>(std::max(1, K.n_coef)) * 2 * G * 2 * K.n_a, 0);
+  int n = 1;
+  for (int c = 0; c < K.n_coef; ++c)
+    for (int neg = 0; neg < 2; ++neg)
+      for (int R = 0; R < G; ++R)
+        for (int eta = 0; eta < 2; ++eta)
+          for (int a = 0; a < K.n_a; ++a) {
+            const double f = (neg != eta ? -1.0 : 1.0) * K.root[a];
+            const double2 cc = K.coef[c], ch = chi[static_cast<size_t>(R)];
+            const double2 v = make_double2(f * (cc.x * ch.x + cc.y * ch.y), f * (cc.y * ch.x - cc.x * ch.y));
+            const double size = std::hypot(v.x, v.y);
+            int code = 0;
+            for (int i = 1; i < n && !code; ++i)
+              if (std::fabs(dict[static_cast<size_t>(i)].x - v.x) <= 1e-14 * size && std::fabs(dict[static_cast<size_t>(i)].y - v.y) <= 1e-14 * size)
+                code = i;
+            if (!code) {
+              if (n == 256) return FTLM_OK;
+              code = n++;
+              dict[static_cast<size_t>(code)] = v;
+            }
+            lut[static_cast<size_t>((((c * 2 + neg) * G + R) * 2 + eta) * K.n_a + a)] = static_cast<uint8_t>(code);
+          }
+  const int pitch = (P.max_up_deg + P.max_dn_deg + 15) / 16 * 16;
+  if (pitch == 0 || pitch > 0xFFFF) return FTLM_OK;
+  if (o->list.alloc(static_cast<size_t>(o->dk) * pitch * sizeof(uint32_t)) != cudaSuccess) {  // no room: the tables do
+    cudaGetLastError();
+    o->list.p = nullptr;
+    return FTLM_OK;
+  }
+  CU_TRY(o->cnt.alloc(static_cast<size_t>(o->dk) * sizeof(uint16_t)));
+  CU_TRY(upload_to(o->dict, dict));
+  CU_TRY(upload_to(o->lut, lut));
+  K.lut = o->lut.as<uint8_t>();
+  CU_TRY(orbit_lists(A, K, o->list.as<uint32_t>(), o->cnt.as<uint16_t>(), pitch, o->sector->stream));
+  CU_TRY(cudaStreamSynchronize(o->sector->stream));
+  A.list = o->list.as<uint32_t>();
+  A.cnt = o->cnt.as<uint16_t>();
+  A.dict = o->dict.as<double2>();
+  A.pitch = pitch;
+  return FTLM_OK;
+}
+
 int orbit_apply_dev(ftlm_orbit* o, const double2* x, double2* y, cudaStream_t st) {
   CU_TRY(orbit_apply(o->app, x, y, st));
   return FTLM_OK;
@@ -281,6 +355,8 @@ int ftlm_gpu_orbit_create_ex(ftlm_sector* s, int kx, int ky, double survive_tol,
   CU_TRY(o->xs.alloc(static_cast<size_t>(std::max<int64_t>(o->dk, 1)) * sizeof(double2)));
   A.xs = o->xs.as<double2>();
   A.path = 1;
+  rc = build_lists(o.get(), chi);
+  if (rc) return rc;
   *out = o.release();
   return FTLM_OK;
 }

@@ -87,9 +87,27 @@ struct OrbitApplyDev {
   const uint32_t* dhop_own;
   const uint32_t* dhop_oth;
   int n_dhops;
+  // The block's matrix as source lists (null: not built): row a of list has cnt[a] entries beta | code<<24, in the order up
+  // sources, down sources, then zero entries (code 0) to a multiple of 16; dict[code] = <rep a|H|s> eta conj(chi(R)) sqrt|A_b|.
+  const uint32_t* list;
+  const uint16_t* cnt;
+  const double2* dict;       // [256]
+  int pitch;                 // entries per row
   double2* xs;               // [dk] workspace: sqrt(|A_b|) x_b, zero where |x_b|^2 < 1e-28
-  int path;                  // 0: hop list per representative; 1: sector gather tables (default)
+  int path;                  // 0: hop list per representative; 1: the source lists, or the sector's gather tables (default)
 };
+
+// What the codes of the lists stand for: code = lut[(((c * 2 + neg) * G + R) * 2 + eta) * n_a + a] for the hop coefficient
+// coef[c] (with the sign neg), translation R, sign eta and root[a] = sqrt|A_b|.
+struct OrbitCodes {
+  double2 coef[16];
+  double root[16];
+  int n_coef, n_a;
+  const uint8_t* lut;        // [n_coef * 2 * G * 2 * n_a]
+};
+// The source lists of a block (row length `pitch` >= every representative's sources, a multiple of 16).
+cudaError_t orbit_lists(const OrbitApplyDev& A, const OrbitCodes& codes, uint32_t* list, uint16_t* cnt, int pitch,
+                        cudaStream_t st);
 
 // red[full[b]] = b for b < n.
 cudaError_t orbit_scatter_index(const int64_t* full, int64_t n, int32_t* red, cudaStream_t st);

@@ -2,14 +2,19 @@
 //
 // One block per plane (chains.cuh) runs all M steps: a warp takes 32 output strings of one row, a lane one state, with
 // the row pass's gauge-table walk for the down hops and the row's source list (the same for the whole warp) for the up
-// hops; then the dot products, the update and the norm over the block's own vectors.  The vector that the hops gather
-// from is staged in shared memory where it fits (14,336 states with their padding); else the rows are, a block of rows at
-// a time, and the up hops read the block's scratch (32 lanes that gather at random within a row from global memory touch
-// a line each: 3x3 (4,4), 15,876 states, took 142 us a step that way).
-// Rows have a pitch of Dd + 8 elements whose last 8 stay zero: the target of the table's padding entries, and harmless
-// to the flat elementwise passes.  Bound by the latency of the gathers and of four block reductions a step; it exists
-// because a step of a small sector otherwise costs five kernel launches, whatever its size: 3x3
-// batched sweep (100 sectors, 60 steps) 336 -> 127 ms, most of that in the host's allocations.
+// hops.  The walk serves the 32 strings in the table's order, which spreads its gathers over the shared-memory banks;
+// the up hops read 32 neighbouring strings of a row, so they run in the strings' own order (of any 8
+// of them in the table's order about 2.5 share the fullest bank group) and the sums change lanes by a shuffle.  Their list is the packed one where
+// the sector has it: one word a source instead of three, two real FMAs a component instead of four.  Then the dot
+// products, the update and the norm over the block's own vectors.  The vector that the hops gather from is staged in
+// shared memory where it fits (14,336 states with their padding); else the rows are, a block of rows at a time, and the
+// up hops read the block's scratch (32 lanes that gather at random within a row from global memory touch a line each:
+// 3x3 (4,4), 15,876 states, took 142 us a step that way). Rows have a pitch of Dd + 8 elements whose last 8 stay zero:
+// the target of the table's padding entries, and harmless to the flat elementwise passes.  Bound by the shared-memory
+// pipe above 4,096 states (85 % of its wavefronts before the lane change and the packed list; 3x3 batched sweep, the
+// launch of 320 blocks, 13.4 -> 11.5 ms), by latency below; it exists because a step of a small sector otherwise costs
+// five kernel launches, whatever its size: 3x3 batched sweep (100 sectors, 60 steps) 336 -> 127 ms, most of that in the
+// host's allocations.
 // Same FP32 order of operations per element as planes.cu, so complex64 chains agree with that path up to the order of
 // the FP64 sums.  Sums are in a fixed order: bitwise repeatable.
 #include <algorithm>
@@ -60,8 +65,8 @@ __device__ __forceinline__ typename P::T list_hops(const DevSector& S, const typ
   return acc;
 }
 
-template <class P, bool kSmem, bool kPhase, bool kXor>
-__global__ void __launch_bounds__(1024, 1) chains_kernel(const DevSector* __restrict__ sectors,
+template <class P, int kMost, bool kSmem, bool kPhase, bool kXor>
+__global__ void __launch_bounds__(kMost, kMost == 1024 ? 1 : 2) chains_kernel(const DevSector* __restrict__ sectors,
                                                          const ChainDesc* __restrict__ descs, int M,
                                                          typename P::T* __restrict__ scratch,
                                                          const double2* __restrict__ init, double* __restrict__ alpha,
@@ -70,6 +75,8 @@ __global__ void __launch_bounds__(1024, 1) chains_kernel(const DevSector* __rest
   using T = typename P::T;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ double sh[2 * P::kC * 33];
+  __shared__ typename P::Cf uc[16];  // the packed up list's coefficients by its bits 28 to 31
+  using Coefs = RowCoefs<P, kXor>;
   const ChainDesc cd = descs[blockIdx.x];
   const DevSector S = sectors[cd.sector];
   const int Dd = static_cast<int>(S.Dd), Du = static_cast<int>(S.Du), pitch = Dd + 8;
@@ -82,7 +89,13 @@ __global__ void __launch_bounds__(1024, 1) chains_kernel(const DevSector* __rest
   const DevGauge G = S.dn_g;
   const size_t tab_bytes = kPhase ? 0 : (G.ent ? static_cast<size_t>(G.nt) * 8 * sizeof(typename P::Cf) : 0);
   T* xs = reinterpret_cast<T*>(smem_raw + ((tab_bytes + 15) & ~size_t(15)));
-  const RowCoefs<P, kXor> rc(G);
+  const Coefs rc(G);
+  const auto ua0 = P::coef(make_double2(S.up_real2[0], 0.0)).x, ua1 = P::coef(make_double2(S.up_real2[1], 0.0)).x;
+  if (tid < 16) {
+    const double cf = (tid & 8 ? -1.0 : 1.0) * (tid & 4 ? S.up_real2[1] : S.up_real2[0]);
+    const bool ph = tid & 2;
+    uc[tid] = P::coef(make_double2(ph ? cf * S.up_pc : cf, ph ? cf * (tid & 1 ? -S.up_ps : S.up_ps) : 0.0));
+  }
   if (!kPhase && G.ent)
     for (int i = tid; i < G.nt * 8; i += nt) tab[i] = P::coef(G.tab[i >> 3]);
   // padding: zero in every vector
@@ -157,21 +170,43 @@ __global__ void __launch_bounds__(1024, 1) chains_kernel(const DevSector* __rest
           acc = list_hops<P>(S, row, c, acc);
         }
         T up = P::zero();
-        const T* col = (kSmem ? xs : wk) + c;
-        auto source = [&](int j) {
-          const T v = col[S.up_src[j] * pitch];
+        const T* col = (kSmem ? xs : wk) + tp;
+        auto source = [&](int src) {
+          const T v = col[src * pitch];
           return kSmem ? v : P::filtered(v, s_in[0]);
         };
-        const int j1 = S.up_ptr[r + 1];
-        int j = S.up_ptr[r];
-        for (; j + 4 <= j1; j += 4) {
-          T v[4];
+        const int j0 = S.up_ptr[r], j1 = S.up_ptr[r + 1];
+        if (S.up_pk) {
+          auto term = [&](uint32_t e, T v) {
+            if (e & 0x20000000u)
+              P::cmac(up, uc[e >> 28], v);
+            else
+              Coefs::mac(up, Coefs::flip((e & 0x40000000u) ? ua1 : ua0, e & 0x80000000u), v);
+          };
+          int j = j0;
+          for (; j + 4 <= j1; j += 4) {
+            uint32_t e[4];
+            T v[4];
 #pragma unroll
-          for (int t = 0; t < 4; ++t) v[t] = source(j + t);
+            for (int t = 0; t < 4; ++t) e[t] = S.up_pk[j + t];
 #pragma unroll
-          for (int t = 0; t < 4; ++t) P::cmac(up, P::up_coef(S, j + t), v[t]);
+            for (int t = 0; t < 4; ++t) v[t] = source(e[t] & 0x3FFFu);
+#pragma unroll
+            for (int t = 0; t < 4; ++t) term(e[t], v[t]);
+          }
+          for (; j < j1; ++j) term(S.up_pk[j], source(S.up_pk[j] & 0x3FFFu));
+        } else {
+          int j = j0;
+          for (; j + 4 <= j1; j += 4) {
+            T v[4];
+#pragma unroll
+            for (int t = 0; t < 4; ++t) v[t] = source(S.up_src[j + t]);
+#pragma unroll
+            for (int t = 0; t < 4; ++t) P::cmac(up, P::up_coef(S, j + t), v[t]);
+          }
+          for (; j < j1; ++j) P::cmac(up, P::up_coef(S, j), source(S.up_src[j]));
         }
-        for (; j < j1; ++j) P::cmac(up, P::up_coef(S, j), source(j));
+        up = P::shuffle(up, rpw > 1 ? sub * Dd + c : c & 31);
         if (in) {
           const T v = P::add_scaled(acc, up, kSmem ? 1.0 : s_in[0]);
           y[r * pitch + c] = v;
@@ -251,6 +286,8 @@ __global__ void __launch_bounds__(1024, 1) chains_kernel(const DevSector* __rest
     for (int q = 0; q < P::kC && q < cd.chains; ++q) used[cd.out + q] = steps[q];
 }
 
+// Blocks of up to 256 threads have a kernel of their own with 128 registers a thread, without the spills of 64 (grad 3x2,
+// chains 1.46 -> 1.23 ms); with 512 or 768 threads and more registers the large classes are slower (27.9 -> 29.0 ms).
 constexpr int kClassThreads[4] = {1024, 512, 256, 64};
 
 }  // namespace
@@ -276,11 +313,14 @@ template <class P>
 cudaError_t launch(const ChainLaunch& L, cudaStream_t st) {
   using T = typename P::T;
   using K = void (*)(const DevSector*, const ChainDesc*, int, T*, const double2*, double*, double*, int*, double*, T*);
-  static const K kernels[8] = {chains_kernel<P, false, false, false>, chains_kernel<P, false, false, true>,
-                               chains_kernel<P, false, true, false>,  chains_kernel<P, false, true, true>,
-                               chains_kernel<P, true, false, false>,  chains_kernel<P, true, false, true>,
-                               chains_kernel<P, true, true, false>,   chains_kernel<P, true, true, true>};
-  const K k = kernels[(L.smem ? 4 : 0) + (L.phase ? 2 : 0) + (L.xor_real ? 1 : 0)];
+  static const K kernels[12] = {chains_kernel<P, 1024, false, false, false>, chains_kernel<P, 1024, false, false, true>,
+                                chains_kernel<P, 1024, false, true, false>,  chains_kernel<P, 1024, false, true, true>,
+                                chains_kernel<P, 1024, true, false, false>,  chains_kernel<P, 1024, true, false, true>,
+                                chains_kernel<P, 1024, true, true, false>,   chains_kernel<P, 1024, true, true, true>,
+                                chains_kernel<P, 256, true, false, false>,   chains_kernel<P, 256, true, false, true>,
+                                chains_kernel<P, 256, true, true, false>,    chains_kernel<P, 256, true, true, true>};
+  const int form = (L.phase ? 2 : 0) + (L.xor_real ? 1 : 0);
+  const K k = kernels[form + (!L.smem ? 0 : kClassThreads[L.size] > 256 ? 4 : 8)];
   const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(L.smem_bytes));
   if (e != cudaSuccess) return e;
   k<<<L.blocks, kClassThreads[L.size], L.smem_bytes, st>>>(L.sectors, L.descs, L.M, static_cast<T*>(L.scratch), L.init, L.alpha,

@@ -46,6 +46,10 @@ struct C64 {
     acc.w = fmaf(c.x, v.w, acc.w);
     acc.w = fmaf(c.y, v.z, acc.w);
   }
+  static __device__ __forceinline__ T shuffle(T v, int lane) {
+    return make_float4(__shfl_sync(0xffffffffu, v.x, lane), __shfl_sync(0xffffffffu, v.y, lane),
+                       __shfl_sync(0xffffffffu, v.z, lane), __shfl_sync(0xffffffffu, v.w, lane));
+  }
   // conj(w) y of the chains, (re, im) each
   static __device__ __forceinline__ void dot(double (&d)[4], T w, T y, double) {
     const double wx = w.x, wy = w.y, wz = w.z, ww = w.w;
@@ -87,6 +91,9 @@ struct C128 {
     acc.y = fma(c.x, v.y, acc.y);
     acc.y = fma(c.y, v.x, acc.y);
   }
+  static __device__ __forceinline__ T shuffle(T v, int lane) {
+    return make_double2(__shfl_sync(0xffffffffu, v.x, lane), __shfl_sync(0xffffffffu, v.y, lane));
+  }
   static __device__ __forceinline__ void dot(double (&d)[2], T w, T y, double s) {  // conj(s w) y
     const double x = s * w.x, z = s * w.y;
     d[0] += x * y.x + z * y.y;
@@ -124,9 +131,8 @@ struct RowCoefs<C64, kXor> {
       a1 = __double2float_rn(G.real2[1]);
     }
   }
-  __device__ __forceinline__ float pick(uint32_t e) const {
-    return __uint_as_float(__float_as_uint((e & cls) ? a1 : a0) ^ (e & 0x80000000u));
-  }
+  static __device__ __forceinline__ float flip(float v, uint32_t bits) { return __uint_as_float(__float_as_uint(v) ^ bits); }
+  __device__ __forceinline__ float pick(uint32_t e) const { return flip((e & cls) ? a1 : a0, e & 0x80000000u); }
   // Table-section entry in the phase form: real2[cls] (pc, +-ps), which is the table's value bit for bit.
   __device__ __forceinline__ float2 phase(uint32_t e) const {
     const float2 c = C64::signed_coef((e & 0x40000000u) ? p1 : p0, e);

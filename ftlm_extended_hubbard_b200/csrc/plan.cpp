@@ -543,7 +543,7 @@ void build_up_packed(SectorPlan* Pp) {
   int first = -1;
   for (int h = 0; h < nh && first < 0; ++h)
     if (P.hu[static_cast<size_t>(h)].cim != 0.0) first = h;
-  bool all = true;
+  bool all = first < 0;  // without a real hop there is no value to take a phase from
   for (int k0 = 0; k0 < 2 && first >= 0; ++k0) {
     const double a = P.up_real2[k0];
     if (a == 0.0) continue;

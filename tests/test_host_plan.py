@@ -327,3 +327,16 @@ def test_packed_up_list_reproduces_oracle_columns(c):
                 y[r] += colsign * cf * x[src * Dd + col]
         assert np.abs(y - ref).max() <= 1e-14 * np.abs(ref).max()
     _lib.lib().ftlm_gpu_sector_destroy(h)
+
+
+@pytest.mark.parametrize("phi,ok", [((0.31, -0.27), 0), ((0.31, 0.0), 1), ((0.0, 0.0), 1)])
+def test_packed_up_list_needs_a_real_hop(phi, ok):
+    """2x2 with a phase in both directions has complex hops only: no real value to take a phase from, so no packed list."""
+    hops, pairs = F.build_hubbard_geometry(F.HubbardParams(2, 2, 1.0, 0.0, 0.0, 0.0, *phi))
+    h = C.c_void_p()
+    _lib.call("ftlm_gpu_sector_create_host", 4, 2, 2, 0.0, 0.0, F.api._c_hops(hops), len(hops),
+              F.api._c_pairs(pairs), len(pairs), C.byref(h))
+    got, n = C.c_int(), C.c_longlong()
+    _lib.call("ftlm_gpu_sector_up_table_packed", h, C.byref(got), C.byref(n), None, None, None, None)
+    _lib.lib().ftlm_gpu_sector_destroy(h)
+    assert got.value == ok

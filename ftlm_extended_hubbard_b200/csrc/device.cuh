@@ -48,7 +48,7 @@ struct DevSector {
   const double2* dn_coef;  // [n_dn_hops+1]
   const uint32_t* dn_nmask;// [n_dn_hops+1]
   int n_dn_hops;           // == pad hop id
-  int* flags;              // [0]: input has a non-zero entry with |x|^2 < 1e-28
+  int* flags;              // between the passes of H v: does the input have a non-zero entry with |x|^2 < 1e-28 (hv.cu)
   // Gauge-basis down-hop table of the row pass (plan.hpp, GaugeTable); dn_g.ent == nullptr when the
   // sector has none or the launch uses the per-row table instead.
   DevGauge dn_g;

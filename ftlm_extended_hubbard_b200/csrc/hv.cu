@@ -46,6 +46,22 @@ __device__ __forceinline__ void prefetch_row_l2(const double2* row, int64_t n) {
   }
 }
 
+// DevSector::flags between the passes of one H v: [0] the last epoch whose input had an entry that is skipped as a source,
+// [1] the epoch of the last row pass, [2] of the last column pass.  A row pass reads [2] and writes [0] and [1], a column pass the
+// other way round, so no block meets a value that changes under it and nothing has to be cleared between calls (a memset
+// and its gap: 2.5 us).  A column pass without its row pass may filter for nothing, which gives the same sums.
+__device__ __forceinline__ int begin_epoch(int* flags) {
+  const int e = static_cast<int>(static_cast<unsigned>(flags[2]) + 1u);
+  if (blockIdx.x == 0 && threadIdx.x == 0) flags[1] = e;
+  return e;
+}
+
+__device__ __forceinline__ bool end_epoch(int* flags) {
+  const int e = flags[1];
+  if (blockIdx.x == 0 && threadIdx.x == 0) flags[2] = e;
+  return flags[0] == e;
+}
+
 __device__ __forceinline__ double flip_sign(double v, uint32_t neg) {
   return __hiloint2double(__double2hiint(v) ^ static_cast<int>(neg << 31), __double2loint(v));
 }
@@ -53,6 +69,7 @@ __device__ __forceinline__ double flip_sign(double v, uint32_t neg) {
 __global__ void __launch_bounds__(kRowThreads, 1) hv_rows_kernel(DevSector S, const double2* __restrict__ x,
                                                                    double2* __restrict__ y) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int epoch = begin_epoch(S.flags);
   const int Dd = static_cast<int>(S.Dd);
   double2* xs = reinterpret_cast<double2*>(smem_raw);
   double2* coef = xs + Dd;
@@ -83,7 +100,7 @@ __global__ void __launch_bounds__(kRowThreads, 1) hv_rows_kernel(DevSector S, co
       }
       coef[i] = cf;
     }
-    if (saw_tiny) atomicOr(S.flags, 1);
+    if (saw_tiny) S.flags[0] = epoch;
     __syncthreads();
     double2* yrow = y + r * S.Dd;
     for (int c = tid; c < Dd; c += kRowThreads) {
@@ -215,6 +232,7 @@ template <bool kPhase, bool kXor>
 __global__ void __launch_bounds__(kRowThreads, 1) hv_rows_gauge_kernel(DevSector S, const double2* __restrict__ x,
                                                                          double2* __restrict__ y) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int epoch = begin_epoch(S.flags);
   const int Dd = static_cast<int>(S.Dd);
   double2* xs = reinterpret_cast<double2*>(smem_raw);
   double2* tab = xs + Dd + 8;
@@ -240,7 +258,7 @@ __global__ void __launch_bounds__(kRowThreads, 1) hv_rows_gauge_kernel(DevSector
       if (gauge_sign(u, S.dmask[c])) v = make_double2(-v.x, -v.y);
       xs[c] = v;
     }
-    if (saw_tiny) atomicOr(S.flags, 1);
+    if (saw_tiny) S.flags[0] = epoch;
     __syncthreads();
     double2* yrow = y + r * S.Dd;
     for (int c = tid; c < Dd; c += nt) {
@@ -473,7 +491,7 @@ __global__ void __launch_bounds__(kColThreads, 896 / kColThreads) hv_cols_kernel
       s_lh[j] = S.up_lohi[j0 + j];
     }
   }
-  const bool filt = (*S.flags) != 0;
+  const bool filt = end_epoch(S.flags);
   __syncthreads();
   const int64_t c0 = chunk * kColChunk + threadIdx.x;
   if (c0 < S.Dd) {
@@ -546,18 +564,21 @@ cudaError_t hv_launch_pass(const DevSector& S, const double2* x, double2* y, int
   if (S.dim <= 0) return cudaSuccess;
   init_sm_count();
   if (pass == 0) {
-    cudaError_t e = cudaMemsetAsync(S.flags, 0, sizeof(int), st);
-    if (e != cudaSuccess) return e;
     const size_t sm = hv_rows_smem_bytes(S);
     const RowsKernel k = !S.dn_g.ent ? hv_rows_kernel
                          : S.dn_g.phase ? (S.dn_g.xor_real ? hv_rows_gauge_kernel<true, true> : hv_rows_gauge_kernel<true, false>)
                                         : (S.dn_g.xor_real ? hv_rows_gauge_kernel<false, true> : hv_rows_gauge_kernel<false, false>);
-    e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sm));
+    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sm));
     if (e != cudaSuccess) return e;
     // Blocks as wide as a row needs, several on an SM where their rows fit: one block's staging overlaps another's hops.
+    // Up to eight rows an SM run as one wave, the threads shared out among them.
     int threads = kRowThreads, per_sm = 1;
-    if (S.dn_g.ent) {
-      const int fit = static_cast<int>((227 * 1024 + 1024) / (sm + 1024));
+    const int fit = static_cast<int>((227 * 1024 + 1024) / (sm + 1024));
+    const int64_t wave = (S.Du + g_num_sms - 1) / g_num_sms;
+    if (S.dn_g.ent && wave <= std::min(fit, 8)) {
+      per_sm = static_cast<int>(wave);
+      threads = std::min(kRowThreads / per_sm, static_cast<int>(S.Dd) + 31) / 32 * 32;
+    } else if (S.dn_g.ent) {
       while (threads > 64 && (threads / 2 >= S.Dd || (threads > 256 && threads / 2 * fit >= kRowThreads))) threads /= 2;
       per_sm = std::max(1, std::min(fit, kRowThreads / threads));
     }

@@ -94,3 +94,35 @@ def test_fused_chains_in_both_list_forms(gpu, case):
     assert np.abs(a - a2).max() <= 1e-11 * scale
     A = s.batched_lanczos(3, 4, 5)[0]
     assert np.abs(A[0, :4] - a2[:4]).max() <= 1e-5 * scale
+
+
+def test_skip_rule_over_calls_of_one_sector(gpu):
+    """The two passes agree on each call's own input: with and without entries below the skip threshold in turn, launched and
+    replayed from a graph, one handle gives the bits of a fresh handle (an input with such an entry takes the filter)."""
+    import torch
+    p = F.HubbardParams(4, 3, 1.0, -0.25, 8.0, 1.0, 0.1, 0.0)
+    s = F.Sector(p, 4, 5)
+    s.set_apply_path(3)
+    gen = torch.Generator(device="cuda").manual_seed(4)
+    plain = torch.randn(s.dim(), dtype=torch.complex128, device="cuda", generator=gen)
+    small = plain.clone()
+    small[::7] = 5e-15
+    ref = []
+    for v in (plain, small):
+        f = F.Sector(p, 4, 5)
+        f.set_apply_path(3)
+        y = torch.empty_like(v)
+        f.apply(v, y)
+        ref.append(y)
+    x, y = plain.clone(), torch.empty_like(plain)
+    s.apply(x, y)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        s.apply(x, y, torch.cuda.current_stream().cuda_stream)
+    for k in (1, 0, 1, 1, 0, 0, 1):
+        x.copy_(small if k else plain)
+        for run in (lambda: s.apply(x, y), graph.replay):
+            y.zero_()
+            run()
+            assert torch.equal(y, ref[k])

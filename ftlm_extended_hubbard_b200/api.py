@@ -271,7 +271,7 @@ class Sector(_Handle):
 
 
     def batched_set_cols_variant(self, variant: int):
-        """Column-pass variant of the batched H·v: 0/1/2 = 16/8/4-column chunks."""
+        """Column-pass variant of the batched H·v: 0/1/2 = 256/128/512-column slabs."""
         call("ftlm_gpu_batched_set_cols_variant", self._h, variant)
 
     def batched_autotune(self, reps: int = 2):

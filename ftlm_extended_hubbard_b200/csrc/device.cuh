@@ -52,7 +52,7 @@ struct DevSector {
   // Gauge-basis down-hop table of the row pass (plan.hpp, GaugeTable); dn_g.ent == nullptr when the
   // sector has none or the launch uses the per-row table instead.
   DevGauge dn_g;
-  int bt_cols;              // batched column-pass variant: 0/1/2 = 16/8/4-column chunks
+  int bt_cols;              // column pass on planes: 0/1/2 = 256/128/512-column slabs
 };
 
 // The reference skips source columns with std::norm(x) < 1e-28

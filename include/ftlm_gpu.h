@@ -141,8 +141,9 @@ int ftlm_gpu_apply_profiled(ftlm_sector* s, const double* x_dev, double* y_dev, 
 /* Kernel selection for ftlm_gpu_apply: 0 = automatic, 1 = generic gather, 2 = row pass (per-row
  * coefficient table in shared memory) + column-slab pass, 3 = row pass in the gauge basis
  * (ftlm_gpu_sector_down_table_gauge: register-held real coefficients, one shared-memory load per
- * hop) + column-slab pass (where the sector has no gauge table, as 2).  Automatic picks 3, else 2,
- * else 1; ftlm_gpu_autotune_apply times them all.  All paths give the same matrix elements (sums may
+ * hop) + column-slab pass (where the sector has no gauge table, as 2).  Automatic takes small sectors with the
+ * gauge table in one pass (every output row's down and up hops in one block), else picks 3, else 2,
+ * else 1; ftlm_gpu_autotune_apply times them all (the one pass is reported as path 3).  All paths give the same matrix elements (sums may
  * differ in the last bits). */
 int ftlm_gpu_set_apply_path(ftlm_sector* s, int path);
 
@@ -225,11 +226,11 @@ int ftlm_gpu_gc_sweep(const ftlm_params* p, int R, int M, unsigned seed, int sta
 /* ---- batched complex64 FTLM (32 chains of a sector per block vector, FP64 scalars) ----
  * Chain r of a sector uses the Philox start vector of FTLM_START_PHILOX with seed + r*100003 (the
  * same vectors the complex128 path draws), rounded to complex64; H·v in FP32, dot products and
- * norms in compensated FP64; the M steps of each 32-chain block run as one CUDA graph.  Device
- * memory: 3 block vectors of dim*32 complex64 (127 GB at 4x4 (8,8)), kept between calls until
- * ftlm_gpu_batched_release(). */
-/* Column-pass variant of the batched H·v on this sector: 0/1/2 = 16/8/4-column chunks (the slab of
- * Du x chunk x 256 bytes that L2 keeps resident while every output row reads it).  Same terms in the
+ * norms in FP64.  Two chains share a plane of 16 bytes a state; the planes advance in groups, each step a
+ * few launches without a host round trip.  Device memory: 3 planes of 16*dim bytes for each plane of a group (at
+ * least 256 MB a vector, so one plane at 4x4 (8,8): 8 GB), kept between calls until ftlm_gpu_batched_release(). */
+/* Column-pass variant of the batched H·v on this sector: 0/1/2 = 256/128/512-column slabs (the slab of
+ * Du x columns x 16 bytes that L2 keeps resident while every output row reads it).  Same terms in the
  * same order per element: the variants give the same block vector. */
 int ftlm_gpu_batched_set_cols_variant(ftlm_sector* s, int variant);
 /* Times the batched H·v with each column-pass variant (CUDA events, reps launches after one warm-up,

@@ -22,6 +22,7 @@
 
 #include "device.cuh"
 #include "hv.cuh"
+#include "launch.cuh"
 
 namespace ftlm_b200 {
 
@@ -46,10 +47,11 @@ __device__ __forceinline__ void prefetch_row_l2(const double2* row, int64_t n) {
   }
 }
 
-// DevSector::flags between the passes of one H v: [0] the last epoch whose input had an entry that is skipped as a source,
-// [1] the epoch of the last row pass, [2] of the last column pass.  A row pass reads [2] and writes [0] and [1], a column pass the
-// other way round, so no block meets a value that changes under it and nothing has to be cleared between calls (a memset
-// and its gap: 2.5 us).  A column pass without its row pass may filter for nothing, which gives the same sums.
+// DevSector::flags between the passes of one H v: [0] the last epoch whose input had an entry that is skipped as a
+// source, [1] the epoch of the last row pass, [2] of the last column pass.  A row pass reads [2] and writes [0] and
+// [1], a column pass the other way round, so no block meets a value that changes under it and nothing has to be cleared
+// between calls (a memset and its gap: 2.5 us).  A column pass without its row pass may filter for nothing, which gives
+// the same sums.
 __device__ __forceinline__ int begin_epoch(int* flags) {
   const int e = static_cast<int>(static_cast<unsigned>(flags[2]) + 1u);
   if (blockIdx.x == 0 && threadIdx.x == 0) flags[1] = e;
@@ -66,9 +68,11 @@ __device__ __forceinline__ double flip_sign(double v, uint32_t neg) {
   return __hiloint2double(__double2hiint(v) ^ static_cast<int>(neg << 31), __double2loint(v));
 }
 
-__global__ void __launch_bounds__(kRowThreads, 1) hv_rows_kernel(DevSector S, const double2* __restrict__ x,
+template <bool kEarly>
+__global__ void __launch_bounds__(kRowThreads, 1) hv_rows_kernel(DevSector S, const double2* __restrict__ x_in,
                                                                    double2* __restrict__ y) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  const double2* x = follow<kEarly>(x_in);
   const int epoch = begin_epoch(S.flags);
   const int Dd = static_cast<int>(S.Dd);
   double2* xs = reinterpret_cast<double2*>(smem_raw);
@@ -228,10 +232,11 @@ __device__ __forceinline__ void gauge_hops(double2& acc, const DevGauge& G, int 
 // a small table copied once per CTA (8 copies, one per bank group).  Each hop then costs one 16-byte
 // shared load of x (plus one for table hops outside the phase form) instead of two.  Entries:
 // GaugeTable (plan.hpp).
-template <bool kPhase, bool kXor>
-__global__ void __launch_bounds__(kRowThreads, 1) hv_rows_gauge_kernel(DevSector S, const double2* __restrict__ x,
+template <bool kPhase, bool kXor, bool kEarly>
+__global__ void __launch_bounds__(kRowThreads, 1) hv_rows_gauge_kernel(DevSector S, const double2* __restrict__ x_in,
                                                                          double2* __restrict__ y) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  const double2* x = follow<kEarly>(x_in);
   const int epoch = begin_epoch(S.flags);
   const int Dd = static_cast<int>(S.Dd);
   double2* xs = reinterpret_cast<double2*>(smem_raw);
@@ -283,10 +288,11 @@ __global__ void __launch_bounds__(kRowThreads, 1) hv_rows_gauge_kernel(DevSector
 // gathers for small sectors and by the L1 data pipe for large ones: 4x2 (4,4) 12.3 us with the generic kernel, 6.4 here;
 // 3x3 (4,4) 18.9 and 8.2, 5x2 (5,5) 16.4 and 8.2.
 constexpr int kOnceThreads = 512;
-// Where one pass is the faster form: small sectors, and up to 64 MB of the 126 MB of L2 where the rows are short (their two
-// passes are mostly launches and idle lanes).  One pass / two passes: 4x3 (3,8), 108,900 states, 14.4 / 16.3 us; 4x3 (4,4),
-// 245,025 states, 22.8 / 22.6; 4x3 (6,6), 853,776 states, 77.5 / 57.2; 4x4 (8,2), rows of 120, 113 / 133.
-constexpr int64_t kOnceMaxDim = int64_t(1) << 17, kOnceShortRow = 256, kOnceShortDim = int64_t(1) << 22;
+// Where one pass is the faster form: small sectors, and up to 64 MB of the 126 MB of L2 where the rows are short.  One
+// pass / two passes: 4x4 (2,3), 67,200 states in rows of 560, 12.3 / 9.9 us; 4x3 (3,8), 108,900 in rows of 495, 14.4 /
+// 12.6; 4x3 (8,3), the same in rows of 220, 12.3 / 12.6; 4x4 (5,2), 524,160 in rows of 120, 41 / 45; 4x3 (6,6), rows of
+// 924, 77 / 54.
+constexpr int64_t kOnceMaxDim = int64_t(1) << 16, kOnceShortRow = 256, kOnceShortDim = int64_t(1) << 22;
 constexpr size_t kOnceListBytes = kMaxUpDeg * 24;  // the row's source list
 
 template <bool kPhase, bool kXor>
@@ -468,8 +474,8 @@ __device__ __forceinline__ void cols_body_packed(const DevSector& S, const doubl
 }
 
 // At least 896 resident threads per SM (28 warps): the L2 gathers need the bytes in flight.
-template <int kColThreads, bool kPacked>
-__global__ void __launch_bounds__(kColThreads, 896 / kColThreads) hv_cols_kernel(DevSector S, const double2* __restrict__ x,
+template <int kColThreads, bool kPacked, bool kEarly>
+__global__ void __launch_bounds__(kColThreads, 896 / kColThreads) hv_cols_kernel(DevSector S, const double2* __restrict__ x_in,
                                                               double2* __restrict__ y) {
   constexpr int kColChunk = 2 * kColThreads;
   constexpr int kListDeg = kPacked ? 4 : kMaxUpDeg;  // the list arrays of the form this launch does not use
@@ -491,6 +497,7 @@ __global__ void __launch_bounds__(kColThreads, 896 / kColThreads) hv_cols_kernel
       s_lh[j] = S.up_lohi[j0 + j];
     }
   }
+  const double2* x = follow<kEarly>(x_in);
   const bool filt = end_epoch(S.flags);
   __syncthreads();
   const int64_t c0 = chunk * kColChunk + threadIdx.x;
@@ -531,19 +538,26 @@ void init_sm_count() {
   }
 }
 
+template <bool kEarly>
+RowsKernel rows_kernel_of(const DevSector& S) {
+  if (!S.dn_g.ent) return hv_rows_kernel<kEarly>;
+  if (S.dn_g.phase) return S.dn_g.xor_real ? hv_rows_gauge_kernel<true, true, kEarly> : hv_rows_gauge_kernel<true, false, kEarly>;
+  return S.dn_g.xor_real ? hv_rows_gauge_kernel<false, true, kEarly> : hv_rows_gauge_kernel<false, false, kEarly>;
+}
+
 template <int kThreads>
 cudaError_t launch_cols(const DevSector& S, const double2* x, double2* y, cudaStream_t st) {
   const int64_t nchunks = (S.Dd + 2 * kThreads - 1) / (2 * kThreads);
   const unsigned grid = static_cast<unsigned>(nchunks * S.Du);
-  if (S.up_pk)
-    hv_cols_kernel<kThreads, true><<<grid, kThreads, 0, st>>>(S, x, y);
-  else
-    hv_cols_kernel<kThreads, false><<<grid, kThreads, 0, st>>>(S, x, y);
-  return cudaGetLastError();
+  const bool early = early_ok(S.dim, st);
+  const RowsKernel k = S.up_pk ? (early ? hv_cols_kernel<kThreads, true, true> : hv_cols_kernel<kThreads, true, false>)
+                               : (early ? hv_cols_kernel<kThreads, false, true> : hv_cols_kernel<kThreads, false, false>);
+  return launch_after(early, k, grid, kThreads, 0, st, S, x, y);
 }
 
 bool hv_once_ok(const DevSector& S, int max_up_deg) {
-  return S.dn_g.ent && S.dim <= (S.Dd <= kOnceShortRow ? kOnceShortDim : kOnceMaxDim) && max_up_deg <= kMaxUpDeg && hv_rows_smem_bytes(S) + kOnceListBytes <= 227 * 1024;
+  return S.dn_g.ent && S.dim <= (S.Dd <= kOnceShortRow ? kOnceShortDim : kOnceMaxDim) && max_up_deg <= kMaxUpDeg &&
+         hv_rows_smem_bytes(S) + kOnceListBytes <= 227 * 1024;
 }
 
 cudaError_t hv_launch_once(const DevSector& S, const double2* x, double2* y, cudaStream_t st) {
@@ -565,9 +579,8 @@ cudaError_t hv_launch_pass(const DevSector& S, const double2* x, double2* y, int
   init_sm_count();
   if (pass == 0) {
     const size_t sm = hv_rows_smem_bytes(S);
-    const RowsKernel k = !S.dn_g.ent ? hv_rows_kernel
-                         : S.dn_g.phase ? (S.dn_g.xor_real ? hv_rows_gauge_kernel<true, true> : hv_rows_gauge_kernel<true, false>)
-                                        : (S.dn_g.xor_real ? hv_rows_gauge_kernel<false, true> : hv_rows_gauge_kernel<false, false>);
+    const bool early = early_ok(S.dim, st);
+    const RowsKernel k = early ? rows_kernel_of<true>(S) : rows_kernel_of<false>(S);
     const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sm));
     if (e != cudaSuccess) return e;
     // Blocks as wide as a row needs, several on an SM where their rows fit: one block's staging overlaps another's hops.
@@ -583,8 +596,7 @@ cudaError_t hv_launch_pass(const DevSector& S, const double2* x, double2* y, int
       per_sm = std::max(1, std::min(fit, kRowThreads / threads));
     }
     const int grid_r = static_cast<int>(std::min<int64_t>(S.Du, static_cast<int64_t>(g_num_sms) * per_sm));
-    k<<<grid_r, threads, sm, st>>>(S, x, y);
-    return cudaGetLastError();
+    return launch_after(early, k, grid_r, threads, sm, st, S, x, y);
   }
   cols_variant %= 3;  // 3..5: the same slabs; the list form comes with S (S.up_pk)
   if (cols_variant == 1) return launch_cols<64>(S, x, y, st);

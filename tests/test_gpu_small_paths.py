@@ -126,3 +126,32 @@ def test_skip_rule_over_calls_of_one_sector(gpu):
             y.zero_()
             run()
             assert torch.equal(y, ref[k])
+
+
+@pytest.mark.parametrize("lat,nu,nd", [((4, 3), 3, 4), ((4, 3), 4, 5), ((4, 4), 2, 3), ((5, 3), 4, 4)])
+def test_calls_in_flight_keep_their_order(gpu, lat, nu, nd):
+    """Two-pass calls launched ahead of one another (67,200 to 1,863,225 states), each on the result of the one before with
+    an elementwise kernel between, on the default stream and on another one: the bits of the same calls one at a time."""
+    import torch
+    s = F.Sector(F.HubbardParams(*lat, 1.0, -0.25, 8.0, 1.0, 0.1, 0.0), nu, nd)
+    s.set_apply_path(3)
+    gen = torch.Generator(device="cuda").manual_seed(nu)
+    x0 = torch.randn(s.dim(), dtype=torch.complex128, device="cuda", generator=gen)
+
+    def chain(stream, wait):
+        with torch.cuda.stream(stream):
+            x, y = x0.clone(), torch.empty_like(x0)
+            for k in range(24):
+                s.apply(x, y, stream.cuda_stream)
+                if wait:
+                    torch.cuda.synchronize()
+                if k % 3:
+                    y.mul_(0.05)
+                x, y = y, x
+        torch.cuda.synchronize()
+        return x
+
+    ref = chain(torch.cuda.default_stream(), True)
+    for stream in (torch.cuda.default_stream(), torch.cuda.Stream()):
+        for _ in range(3):
+            assert torch.equal(chain(stream, False), ref)

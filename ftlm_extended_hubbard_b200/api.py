@@ -499,7 +499,7 @@ QUADRATURES = {"reference": 0, "converged": 1}
 
 def set_quadrature(mode: str) -> None:
     """Quadrature of the complex128 sector path: "reference" (default; the reference's rotation-capped
-    Jacobi, src/ftlm_thermo.cpp:83-146) or "converged" (the converged GPU Jacobi, which the batched
+    Jacobi, src/ftlm_thermo.cpp:83-146) or "converged" (implicit QL on the GPU, which the batched
     complex64 path always uses).  Process-wide."""
     call("ftlm_gpu_set_quadrature", QUADRATURES[mode])
 

@@ -52,10 +52,10 @@ __device__ __forceinline__ void prefetch_row_l2(const double2* row, int64_t n) {
 // [1], a column pass the other way round, so no block meets a value that changes under it and nothing has to be cleared
 // between calls (a memset and its gap: 2.5 us).  A column pass without its row pass may filter for nothing, which gives
 // the same sums.
-__device__ __forceinline__ int begin_epoch(int* flags) {
-  const int e = static_cast<int>(static_cast<unsigned>(flags[2]) + 1u);
-  if (blockIdx.x == 0 && threadIdx.x == 0) flags[1] = e;
-  return e;
+__device__ __forceinline__ int row_epoch(const int* flags) { return static_cast<int>(static_cast<unsigned>(flags[2]) + 1u); }
+
+__device__ __forceinline__ void begin_epoch(int* flags) {  // no block keeps it in a register: the row pass has none to spare
+  if (blockIdx.x == 0 && threadIdx.x == 0) flags[1] = row_epoch(flags);
 }
 
 __device__ __forceinline__ bool end_epoch(int* flags) {
@@ -73,7 +73,7 @@ __global__ void __launch_bounds__(kRowThreads, 1) hv_rows_kernel(DevSector S, co
                                                                    double2* __restrict__ y) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const double2* x = follow<kEarly>(x_in);
-  const int epoch = begin_epoch(S.flags);
+  begin_epoch(S.flags);
   const int Dd = static_cast<int>(S.Dd);
   double2* xs = reinterpret_cast<double2*>(smem_raw);
   double2* coef = xs + Dd;
@@ -104,7 +104,7 @@ __global__ void __launch_bounds__(kRowThreads, 1) hv_rows_kernel(DevSector S, co
       }
       coef[i] = cf;
     }
-    if (saw_tiny) S.flags[0] = epoch;
+    if (saw_tiny) S.flags[0] = row_epoch(S.flags);
     __syncthreads();
     double2* yrow = y + r * S.Dd;
     for (int c = tid; c < Dd; c += kRowThreads) {
@@ -237,7 +237,7 @@ __global__ void __launch_bounds__(kRowThreads, 1) hv_rows_gauge_kernel(DevSector
                                                                          double2* __restrict__ y) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const double2* x = follow<kEarly>(x_in);
-  const int epoch = begin_epoch(S.flags);
+  begin_epoch(S.flags);
   const int Dd = static_cast<int>(S.Dd);
   double2* xs = reinterpret_cast<double2*>(smem_raw);
   double2* tab = xs + Dd + 8;
@@ -263,7 +263,7 @@ __global__ void __launch_bounds__(kRowThreads, 1) hv_rows_gauge_kernel(DevSector
       if (gauge_sign(u, S.dmask[c])) v = make_double2(-v.x, -v.y);
       xs[c] = v;
     }
-    if (saw_tiny) S.flags[0] = epoch;
+    if (saw_tiny) S.flags[0] = row_epoch(S.flags);
     __syncthreads();
     double2* yrow = y + r * S.Dd;
     for (int c = tid; c < Dd; c += nt) {

@@ -202,7 +202,7 @@ int ftlm_gpu_ftlm_sector(ftlm_sector* s, const double* bts, int n_bt, int R, int
 /* Quadrature of the complex128 sector path (ftlm_gpu_ftlm_sector, ftlm_gpu_gc_sweep, orbit blocks):
  * FTLM_QUAD_REFERENCE (default) = the reference's classical Jacobi with max(3000, 120 n) rotations
  * (src/ftlm_thermo.cpp:83-146; for n ~ 100 at low temperature it stops unconverged, so its ln Z moves
- * by up to ~1e-5 under 1e-7 changes of alpha/beta); FTLM_QUAD_CONVERGED = the converged GPU Jacobi.
+ * by up to ~1e-5 under 1e-7 changes of alpha/beta); FTLM_QUAD_CONVERGED = implicit QL on the GPU.
  * The batched complex64 path always uses the converged quadrature.  Process-wide setting. */
 #define FTLM_QUAD_REFERENCE 0
 #define FTLM_QUAD_CONVERGED 1

@@ -308,7 +308,7 @@ int ftlm_gpu_orbit_entries(const ftlm_orbit* o, uint32_t* rep_packed, double* ab
 int ftlm_gpu_orbit_entries_ex(const ftlm_orbit* o, uint32_t* rep_packed, double* A, double* absA, int* orbit_size,
                               int* stabilizer_size, long long* orbit_index);
 int ftlm_gpu_orbit_apply(ftlm_orbit* o, const double* x_dev, double* y_dev, void* stream);
-/* 0: hop list scan per representative; 1 (default): the sector's gather tables, batched gathers.
+/* 0: hop list scan per representative; 1 (default): the block's source lists, or the sector's gather tables without them.
  * No reference counterpart (both compute apply_orbit_k_block). */
 int ftlm_gpu_orbit_set_apply_path(ftlm_orbit* o, int path);
 int ftlm_gpu_orbit_apply_host(ftlm_orbit* o, const double* x_host, double* y_host);

@@ -37,11 +37,13 @@ struct ftlm_orbit {
 
 namespace {
 
+// Copies v to the device on the stream that reads it.  A copy on the legacy stream would not do: from pageable memory it
+// may return before the bytes have arrived, and the sectors' non-blocking streams do not wait for that stream.
 template <class T>
-cudaError_t upload_to(DevBuf& b, const std::vector<T>& v) {
+cudaError_t upload_to(DevBuf& b, const std::vector<T>& v, cudaStream_t st) {
   cudaError_t e = b.alloc(std::max<size_t>(v.size(), 1) * sizeof(T));
   if (e != cudaSuccess || v.empty()) return e;
-  return cudaMemcpy(b.p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice);
+  return cudaMemcpyAsync(b.p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, st);
 }
 
 int build_orbit_sector(ftlm_sector* s) {
@@ -76,11 +78,11 @@ int build_orbit_sector(ftlm_sector* s) {
   std::vector<int32_t> rku(65536, -1), rkd(65536, -1);
   for (int64_t i = 0; i < P.up.D; ++i) rku[P.up.masks[static_cast<size_t>(i)]] = static_cast<int32_t>(i);
   for (int64_t i = 0; i < P.dn.D; ++i) rkd[P.dn.masks[static_cast<size_t>(i)]] = static_cast<int32_t>(i);
-  CU_TRY(upload_to(D->tlut, tl));
-  CU_TRY(upload_to(D->tsite, ts));
-  CU_TRY(upload_to(D->rorder, ro));
-  CU_TRY(upload_to(D->rank_u, rku));
-  CU_TRY(upload_to(D->rank_d, rkd));
+  CU_TRY(upload_to(D->tlut, tl, s->stream));
+  CU_TRY(upload_to(D->tsite, ts, s->stream));
+  CU_TRY(upload_to(D->rorder, ro, s->stream));
+  CU_TRY(upload_to(D->rank_u, rku, s->stream));
+  CU_TRY(upload_to(D->rank_d, rkd, s->stream));
   OrbitDev& O = D->dev;
   O.n = n;
   O.Lx = Lx;
@@ -110,8 +112,8 @@ int build_orbit_sector(ftlm_sector* s) {
     std::sort(inv_d.begin(), inv_d.end(),
               [&P](int32_t a, int32_t b) { return P.dn.masks[static_cast<size_t>(a)] < P.dn.masks[static_cast<size_t>(b)]; });
     DevBuf iu, id, counts;
-    CU_TRY(upload_to(iu, inv_u));
-    CU_TRY(upload_to(id, inv_d));
+    CU_TRY(upload_to(iu, inv_u, s->stream));
+    CU_TRY(upload_to(id, inv_d, s->stream));
     CU_TRY(counts.alloc(static_cast<size_t>(orbit_compact_counts(P.dim)) * sizeof(int32_t)));
     CU_TRY(orbit_count_reps(O, D->rep_full.as<int32_t>(), iu.as<int32_t>(), id.as<int32_t>(), counts.as<int32_t>(),
                             &D->nreps, s->stream));
@@ -133,11 +135,11 @@ int build_orbit_sector(ftlm_sector* s) {
     oth.push_back(h.other_mask);
   }
   D->n_uh = static_cast<int>(f.size());
-  CU_TRY(upload_to(D->uh_from, f));
-  CU_TRY(upload_to(D->uh_to, t));
-  CU_TRY(upload_to(D->uh_c, c));
-  CU_TRY(upload_to(D->uh_own, own));
-  CU_TRY(upload_to(D->uh_oth, oth));
+  CU_TRY(upload_to(D->uh_from, f, s->stream));
+  CU_TRY(upload_to(D->uh_to, t, s->stream));
+  CU_TRY(upload_to(D->uh_c, c, s->stream));
+  CU_TRY(upload_to(D->uh_own, own, s->stream));
+  CU_TRY(upload_to(D->uh_oth, oth, s->stream));
   f.clear();
   t.clear();
   c.clear();
@@ -151,11 +153,12 @@ int build_orbit_sector(ftlm_sector* s) {
     oth.push_back(h.other_mask);
   }
   D->n_dh = static_cast<int>(f.size());
-  CU_TRY(upload_to(D->dh_from, f));
-  CU_TRY(upload_to(D->dh_to, t));
-  CU_TRY(upload_to(D->dh_c, c));
-  CU_TRY(upload_to(D->dh_own, own));
-  CU_TRY(upload_to(D->dh_oth, oth));
+  CU_TRY(upload_to(D->dh_from, f, s->stream));
+  CU_TRY(upload_to(D->dh_to, t, s->stream));
+  CU_TRY(upload_to(D->dh_c, c, s->stream));
+  CU_TRY(upload_to(D->dh_own, own, s->stream));
+  CU_TRY(upload_to(D->dh_oth, oth, s->stream));
+  CU_TRY(cudaStreamSynchronize(s->stream));  // a caller's stream reads them too
   s->orbit_data = D;
   return FTLM_OK;
 }
@@ -221,8 +224,8 @@ int build_lists(ftlm_orbit* o, const std::vector<double2>& chi) {
     return FTLM_OK;
   }
   CU_TRY(o->cnt.alloc(static_cast<size_t>(o->dk) * sizeof(uint16_t)));
-  CU_TRY(upload_to(o->dict, dict));
-  CU_TRY(upload_to(o->lut, lut));
+  CU_TRY(upload_to(o->dict, dict, o->sector->stream));
+  CU_TRY(upload_to(o->lut, lut, o->sector->stream));
   K.lut = o->lut.as<uint8_t>();
   CU_TRY(orbit_lists(A, K, o->list.as<uint32_t>(), o->cnt.as<uint16_t>(), pitch, o->sector->stream));
   CU_TRY(cudaStreamSynchronize(o->sector->stream));
@@ -280,7 +283,7 @@ int ftlm_gpu_orbit_create_ex(ftlm_sector* s, int kx, int ky, double survive_tol,
                             static_cast<double>(ky * dy) / static_cast<double>(s->Ly));
       chi[static_cast<size_t>(dy * s->Lx + dx)] = make_double2(std::cos(theta), std::sin(theta));
     }
-  CU_TRY(upload_to(o->chi, chi));
+  CU_TRY(upload_to(o->chi, chi, s->stream));
   const int64_t nreps = D.nreps;
   DevBuf absA, Adev, sdev, counts;
   CU_TRY(absA.alloc(std::max<int64_t>(nreps, 1) * sizeof(double)));

@@ -83,53 +83,84 @@ int chain_moments(const std::vector<SectorChains<T>>& v, int ld, double bT, cons
   return FTLM_OK;
 }
 
+// Bytes of stored vectors (and as many of their images under the operator) of one piece of a replay.  A replay whose
+// device memory does not suffice is tried again with half, down to one plane.
+constexpr size_t kGradStore = size_t(6) << 30;
+
+// One piece of grad_fused: chains r0 .. r0 + R - 1 of the sectors, their vectors at the elements `base` of the store of
+// `total` elements; out: [sector][R].
+template <class T>
+int grad_piece(const std::vector<ftlm_sector*>& secs, const std::vector<ftlm_sector*>& op, double bT, int r0, int R, int M,
+               unsigned seed, int start_mode, const std::vector<int64_t>& base, int64_t total, std::vector<ChainGrad>* out) {
+  constexpr bool c64 = std::is_same<T, float4>::value;
+  const int planes = c64 ? (R + 1) / 2 : R;
+  CU_TRY(g_grad.grow(g_grad.Q, g_grad.qcap, static_cast<size_t>(total) * sizeof(T)));
+  CU_TRY(g_grad.grow(g_grad.AQ, g_grad.acap, static_cast<size_t>(total) * sizeof(T)));
+  ChainRun run;
+  const unsigned seed0 = seed + static_cast<unsigned>(r0) * 100003u;
+  int rc = chains_run(secs, R, M, seed0, start_mode, c64, &run, g_grad.Q.p, &base, true);
+  if (rc) return rc;
+  cudaStream_t st = secs[0]->stream;
+  run.mem.busy();
+  std::vector<SectorChains<T>> v;
+  for (size_t i = 0; i < secs.size(); ++i) {
+    const int64_t dim = secs[i]->plan.dim;
+    const T* Q = g_grad.Q.as<T>() + base[i];
+    T* AQ = op[i] ? g_grad.AQ.as<T>() + base[i] : nullptr;
+    // the operator on every stored vector: the planes of all steps are contiguous
+    if (AQ) CU_TRY(pl_apply(op[i]->dev, Q, AQ, M * planes, g_grad.flag.as<int>(), st));
+    v.push_back(SectorChains<T>{secs[i], R, Q, AQ, planes * dim, dim});
+  }
+  rc = chain_moments(v, M, bT, run.alpha, run.beta, run.used, run.scale, st, out);
+  if (!rc) run.mem.idle();
+  return rc;
+}
+
 // Chains of small sectors (chains_run), replayed with their vectors kept; op[i] (may be null) is the operator's sector.
-// Sectors go in pieces whose stored vectors fit a bounded store.  out: [sector][R].
+// Pieces of a bounded store: several whole sectors, or a range of one sector's chains where all of them do not fit (a
+// plane's two complex64 chains stay together, so each chain is the forward's).  out: [sector][R].
 template <class T>
 int grad_fused(const std::vector<ftlm_sector*>& secs, const std::vector<ftlm_sector*>& op, double bT, int R, int M,
                unsigned seed, int start_mode, std::vector<std::vector<ChainGrad>>* out) {
-  constexpr bool c64 = sizeof(T) == sizeof(float4) && std::is_same<T, float4>::value;
-  constexpr size_t kStore = size_t(6) << 30;
-  const int planes = c64 ? (R + 1) / 2 : R;
+  constexpr int kC = std::is_same<T, float4>::value ? 2 : 1;
   out->assign(secs.size(), {});
   std::lock_guard<std::mutex> lock(g_bt_mu);
   if (!g_grad.flag.p) CU_TRY(g_grad.flag.alloc(sizeof(int)));
+  size_t store = kGradStore;
+  auto vectors = [&](size_t i, int chains) {  // elements of the stored vectors of so many chains
+    return static_cast<int64_t>(M) * ((chains + kC - 1) / kC) * secs[i]->plan.dim;
+  };
+  const size_t weights = static_cast<size_t>(M) * M * sizeof(double) * 3;  // of a chain, at most half a store of them
   for (size_t i0 = 0; i0 < secs.size();) {
-    std::vector<ftlm_sector*> piece;
-    std::vector<int64_t> base;
-    int64_t at = 0;
-    size_t i1 = i0;
-    for (; i1 < secs.size(); ++i1) {
-      const int64_t add = static_cast<int64_t>(M) * planes * secs[i1]->plan.dim;
-      const size_t weights = (piece.size() + 1) * R * static_cast<size_t>(M) * M * sizeof(double) * 3;
-      if (!piece.empty() && (static_cast<size_t>(at + add) * sizeof(T) > kStore || weights > kStore / 2)) break;
-      piece.push_back(secs[i1]);
-      base.push_back(at);
-      at += add;
-    }
-    CU_TRY(g_grad.grow(g_grad.Q, g_grad.qcap, static_cast<size_t>(at) * sizeof(T)));
-    CU_TRY(g_grad.grow(g_grad.AQ, g_grad.acap, static_cast<size_t>(at) * sizeof(T)));
-    ChainRun run;
-    int rc = chains_run(piece, R, M, seed, start_mode, c64, &run, g_grad.Q.p, &base, true);
-    if (rc) return rc;
-    cudaStream_t st = piece[0]->stream;
-    run.mem.busy();
-    std::vector<SectorChains<T>> v;
-    for (size_t i = 0; i < piece.size(); ++i) {
-      const int64_t dim = piece[i]->plan.dim;
-      const T* Q = g_grad.Q.as<T>() + base[i];
-      T* AQ = op[i0 + i] ? g_grad.AQ.as<T>() + base[i] : nullptr;
-      // the operator on every stored vector: the planes of all steps are contiguous
-      if (AQ) CU_TRY(pl_apply(op[i0 + i]->dev, Q, AQ, M * planes, g_grad.flag.as<int>(), st));
-      v.push_back(SectorChains<T>{piece[i], R, Q, AQ, planes * dim, dim});
-    }
+    const int r0 = static_cast<int>((*out)[i0].size());
+    const size_t plane = static_cast<size_t>(vectors(i0, 1)) * sizeof(T);
+    const int64_t most = std::max<int64_t>(1, std::min<int64_t>(store / plane, store / 2 / (weights * kC)));  // planes
+    const int n = static_cast<int>(std::min<int64_t>(R - r0, most * kC));
+    std::vector<ftlm_sector*> piece{secs[i0]}, ops{op[i0]};
+    std::vector<int64_t> base{0};
+    int64_t total = vectors(i0, n);
+    size_t i1 = i0 + 1;
+    if (n == R)
+      for (; i1 < secs.size(); ++i1) {
+        const int64_t add = vectors(i1, R);
+        if (static_cast<size_t>(total + add) * sizeof(T) > store || (piece.size() + 1) * R * weights > store / 2) break;
+        piece.push_back(secs[i1]);
+        ops.push_back(op[i1]);
+        base.push_back(total);
+        total += add;
+      }
     std::vector<ChainGrad> cg;
-    rc = chain_moments(v, M, bT, run.alpha, run.beta, run.used, run.scale, st, &cg);
+    const int rc = grad_piece<T>(piece, ops, bT, r0, n, M, seed, start_mode, base, total, &cg);
+    if (rc == FTLM_ERR_NOMEM && store > plane) {
+      cudaGetLastError();
+      g_grad.release();
+      store /= 2;
+      continue;
+    }
     if (rc) return rc;
-    run.mem.idle();
     for (size_t i = 0; i < piece.size(); ++i)
-      (*out)[i0 + i].assign(cg.begin() + static_cast<long>(i) * R, cg.begin() + static_cast<long>(i + 1) * R);
-    i0 = i1;
+      (*out)[i0 + i].insert((*out)[i0 + i].end(), cg.begin() + static_cast<long>(i) * n, cg.begin() + static_cast<long>(i + 1) * n);
+    if (r0 + n == R) i0 = i1;
   }
   return FTLM_OK;
 }
@@ -142,13 +173,29 @@ int grad_planes(ftlm_sector* s, ftlm_sector* op, double bT, int R, int M, unsign
   constexpr bool c64 = std::is_same<T, float4>::value;
   constexpr int kC = c64 ? 2 : 1;
   const int64_t dim = s->plan.dim;
-  const int most = (std::min(R, kBtChains) + kC - 1) / kC, group = pl_group(s->dev, c64, most);
-  const int64_t vs = dim * group;  // elements per stored vector of a group
+  const int most = (std::min(R, kBtChains) + kC - 1) / kC;
+  int group = pl_group(s->dev, c64, most);
+  // Complex64 chains replay in the forward's groups, at most a block's 16 planes: a group of another size adds its sums
+  // in another order, which their FP32 vectors do not forgive.  Complex128 chains take as many as the store holds.
+  if (!c64)
+    group = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(group, kGradStore / ((M + 1) * dim * sizeof(T)))));
   std::lock_guard<std::mutex> lock(g_bt_mu);
-  CU_TRY(g_bt.ensure(0, M, pl_items_doubles(s->dev, c64, group)));
-  CU_TRY(g_grad.grow(g_grad.Q, g_grad.qcap, static_cast<size_t>(M + 1) * vs * sizeof(T)));
-  if (op) CU_TRY(g_grad.grow(g_grad.AQ, g_grad.acap, static_cast<size_t>(M) * vs * sizeof(T)));
-  if (!g_grad.flag.p) CU_TRY(g_grad.flag.alloc(sizeof(int)));
+  auto room = [&]() -> int {
+    const size_t vector = static_cast<size_t>(dim) * group * sizeof(T);
+    CU_TRY(g_bt.ensure(0, M, pl_items_doubles(s->dev, c64, group)));
+    CU_TRY(g_grad.grow(g_grad.Q, g_grad.qcap, static_cast<size_t>(M + 1) * vector));
+    if (op) CU_TRY(g_grad.grow(g_grad.AQ, g_grad.acap, static_cast<size_t>(M) * vector));
+    if (!g_grad.flag.p) CU_TRY(g_grad.flag.alloc(sizeof(int)));
+    return FTLM_OK;
+  };
+  for (;;) {
+    const int rc = room();
+    if (!rc) break;
+    if (rc != FTLM_ERR_NOMEM || c64 || group == 1) return rc;
+    cudaGetLastError();
+    g_grad.release();
+    group = (group + 1) / 2;
+  }
   cudaStream_t st = s->stream;
   T* Q = g_grad.Q.as<T>();
   T* AQ = op ? g_grad.AQ.as<T>() : nullptr;

@@ -507,7 +507,7 @@ int launch_cols_t(const DevSector& S, const typename P::T* W, typename P::T* Y, 
   const int64_t grid = std::min<int64_t>({per * planes, static_cast<int64_t>(sm_count()) * (P::kColThreads / kT), kPlMaxBlocks});
   // From 8 items of a plane for each block of the persistent grid, one block per item: 4x4 (6,6) complex128 2.19 -> 1.86 ms,
   // 4x4 (5,6) complex64 1.09 -> 0.97 ms a plane; below, the persistent grid's prefetched lists: 4x3 (4,5) 40 us, 44 by items.
-  if (per >= 8 * grid && per * planes <= INT32_MAX) {
+  if (per >= 8 * grid) {
     const unsigned n = static_cast<unsigned>(per * planes);
     if (!partial) {
       cols_items_kernel<P, kT, false><<<n, kT, 0, s>>>(S, W, Y, static_cast<uint32_t>(per), st, nullptr, flag);
@@ -545,6 +545,12 @@ cudaError_t start(const DevSector& S, typename P::T* W, int planes, unsigned see
   return cudaGetLastError();
 }
 
+// The row and column passes number their work items in 32 bits.
+bool items_fit(const DevSector& S, int planes) {
+  const int64_t kT = S.bt_cols == 1 ? 64 : S.bt_cols == 2 ? 256 : 128;
+  return (S.Dd + 2 * kT - 1) / (2 * kT) * S.Du <= (INT32_MAX - 65536) / std::max(1, planes);
+}
+
 template <class P>
 cudaError_t step(const DevSector& S, const typename P::T* Wk, const typename P::T* Wkm1, typename P::T* Y, int planes,
                  int k, const PlaneState& z, cudaStream_t s) {
@@ -552,6 +558,7 @@ cudaError_t step(const DevSector& S, const typename P::T* Wk, const typename P::
   // alpha scalars' kernel.  C128: flags[0], written by the row pass and cleared by that kernel.
   int* fin = z.flags + (P::kScaled ? 0 : (k & 1));
   int* fout = z.flags + (P::kScaled ? 0 : ((k + 1) & 1));
+  if (!items_fit(S, planes)) return cudaErrorInvalidValue;
   const cudaError_t e = launch_rows<P>(S, Wk, Y, planes, z.st, fin, s);
   if (e != cudaSuccess) return e;
   const int nc = launch_cols<P>(S, Wk, Y, planes, z.st, z.partial, z.items, fin, s);
@@ -564,6 +571,7 @@ cudaError_t step(const DevSector& S, const typename P::T* Wk, const typename P::
 
 template <class P>
 cudaError_t apply(const DevSector& S, const typename P::T* X, typename P::T* Y, int planes, int* flag, cudaStream_t s) {
+  if (!items_fit(S, planes)) return cudaErrorInvalidValue;
   cudaError_t e = cudaMemsetAsync(flag, 0, sizeof(int), s);
   if (e == cudaSuccess) e = launch_rows<P>(S, X, Y, planes, nullptr, flag, s);
   if (e != cudaSuccess) return e;

@@ -36,3 +36,40 @@ def test_momentum_blocks_built_while_copies_are_queued(gpu, lat, nu, nd):
         ref = o.apply_host(x)
         assert np.abs(y - ref).max() <= 1e-13 * max(1.0, np.abs(ref).max())
     torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("method,R", [("plain", 1400), ("batched", 2800)])
+def test_gradient_of_more_chains_than_a_store_holds(gpu, method, R):
+    """60 vectors of 4,900 states for each of R chains are more than one 6 GB store: the gradient of all R chains is that of
+    the two halves, each within a store, put together (ln Z is the log of a mean over chains, its gradient weighted by the
+    means)."""
+    lat = (4, 2)
+    s = F.Sector(F.HubbardParams(*lat, 1.0, -0.2, 4.0, 1.0), 4, 4)
+    op = F.Sector(F.HubbardParams(*lat, 0.0, 1.0, 0.0, 0.0), 4, 4)
+    beta, M, seed, h = 2.0, 60, 11, R // 2
+    kw = dict(op_tp=op, method=method, start="philox")
+    lz, g = s.ftlm_grad(beta, R, M, seed, **kw)
+    l1, g1 = s.ftlm_grad(beta, h, M, seed, **kw)
+    l2, g2 = s.ftlm_grad(beta, h, M, seed + h * 100003, **kw)
+    w1, w2 = np.exp(l1 - np.logaddexp(l1, l2)), np.exp(l2 - np.logaddexp(l1, l2))
+    assert abs(lz - (np.logaddexp(l1, l2) - np.log(2.0))) <= 1e-11 * abs(lz)
+    want = w1 * np.asarray(g1) + w2 * np.asarray(g2)
+    assert np.abs(np.asarray(g) - want).max() <= 1e-9 * np.abs(want).max()
+    F.api.batched_release()
+
+
+def test_gradient_of_many_chains_with_short_rows(gpu):
+    """Rows of one string, 12,870 of them, 160 vectors of each of 1,050 chains: more (row, vector) pairs than 31 bits
+    number.  The gradient is that of five fifths of the chains put together; without down electrons dH/dU is zero."""
+    s = F.Sector(F.HubbardParams(4, 4, 1.0, -0.2, 4.0, 0.0), 8, 0)
+    op = F.Sector(F.HubbardParams(4, 4, 0.0, 1.0, 0.0, 0.0), 8, 0)
+    beta, M = 0.5, 160
+    lz, g = s.ftlm_grad(beta, 1050, M, 3, op_tp=op, start="philox")
+    part = [s.ftlm_grad(beta, 210, M, 3 + 210 * 100003 * i, op_tp=op, start="philox") for i in range(5)]
+    l = np.array([p[0] for p in part])
+    w = np.exp(l - l.max())
+    assert abs(lz - (l.max() + np.log(w.mean()))) <= 1e-11 * abs(lz)
+    want = (w[:, None] * np.array([p[1] for p in part])).sum(0) / w.sum()
+    assert g[0] == 0.0 and abs(g[2]) > 1e-3
+    assert np.abs(np.asarray(g) - want).max() <= 1e-9 * np.abs(want).max()
+    F.api.batched_release()

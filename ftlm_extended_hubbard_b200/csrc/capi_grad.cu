@@ -335,7 +335,8 @@ void sector_gradient(const std::vector<ChainGrad>& cg, int64_t dim, double bT, b
 // The path of a sector's chains in the gradient, which is the forward's: fused, on planes, or (complex128 without a gauge
 // table) not available.
 bool grad_is_c64(const ftlm_sector* s, int M, int method) { return method == 1 && s->plan.dim > 2 * static_cast<int64_t>(M); }
-bool grad_is_fused(const ftlm_sector* s, bool c64) {
+bool grad_is_fused(const ftlm_sector* s, const ftlm_sector* op, bool c64) {
+  if (op && !c64 && !pl_fits(op->dev, op->plan.max_up_deg)) return false;  // complex128 planes of it do not run
   return s->plan.dim <= kFusedSweepMax && chain_rows(s->dev, c64, false) > 0 && s->plan.max_up_deg <= 120;
 }
 
@@ -343,7 +344,7 @@ int grad_one(ftlm_sector* s, ftlm_sector* op, double bT, int R, int M, unsigned 
              std::vector<ChainGrad>* cg) {
   const bool c64 = grad_is_c64(s, M, method);
   const int mode = method == 1 ? FTLM_START_PHILOX : start_mode;
-  if (grad_is_fused(s, c64)) {
+  if (grad_is_fused(s, op, c64)) {
     std::vector<std::vector<ChainGrad>> v;
     const int rc = c64 ? grad_fused<float4>({s}, {op}, bT, R, M, seed, mode, &v)
                        : grad_fused<double2>({s}, {op}, bT, R, M, seed, mode, &v);
@@ -566,7 +567,7 @@ int ftlm_gpu_gc_logz_grad(const ftlm_params* p, double mu, double bT, int R, int
       const bool c64 = grad_is_c64(rs, M, method);
       if (c64 && (rs->plan.max_up_deg > 120 || ro->plan.max_up_deg > 120))
         return fail(FTLM_ERR_UNSUPPORTED, "batched path: more than 120 up-hop sources per string");
-      if (grad_is_fused(rs, c64)) {
+      if (grad_is_fused(rs, ro, c64)) {
         fused[c64 ? 1 : 0].push_back(std::move(t));
         continue;
       }

@@ -73,3 +73,26 @@ def test_gradient_of_many_chains_with_short_rows(gpu):
     assert g[0] == 0.0 and abs(g[2]) > 1e-3
     assert np.abs(np.asarray(g) - want).max() <= 1e-9 * np.abs(want).max()
     F.api.batched_release()
+
+
+def test_gradient_with_an_operator_whose_row_does_not_fit(gpu):
+    """A row of 12,870 strings fits shared memory, with a table of 240 different complex coefficients it does not: the
+    derivative with respect to such an operator against the central difference of H + h * operator (1e-6, as the error of
+    the difference at h = 1e-4)."""
+    hops, pairs = F.build_hubbard_geometry(F.HubbardParams(4, 4, 1.0, -0.2, 0.0, 0.0))
+    rng = np.random.default_rng(2)
+    extra = []
+    for i in range(16):
+        for j in range(i):
+            c = complex(0.1 + rng.random(), rng.standard_normal()) * 0.2
+            extra += [F.SpinfulHopping(i, j, 1, c), F.SpinfulHopping(j, i, 1, c.conjugate())]
+
+    def sector(h):
+        more = [F.SpinfulHopping(e.from_, e.to, e.spin, h * e.coeff) for e in extra]
+        return F.Sector(None, 0, 8, hops=list(hops) + more if h else hops, pairs=pairs, n_sites=16, U=0.0, V=0.0)
+
+    op = F.Sector(None, 0, 8, hops=extra, pairs=pairs, n_sites=16, U=0.0, V=0.0)
+    lz, g = sector(0.0).ftlm_grad(1.0, 2, 30, 5, op_tp=op, start="philox")
+    h = 1e-4
+    l1, l2 = (sector(x).ftlm(1.0, 2, 30, 5, start="philox")[0][0] for x in (h, -h))
+    assert abs(g[2] - (l1 - l2) / (2 * h)) <= 1e-6 * max(1.0, abs(g[2]))

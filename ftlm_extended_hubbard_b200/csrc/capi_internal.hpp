@@ -113,12 +113,13 @@ struct DevBuf {
   DevBuf() = default;
   DevBuf(const DevBuf&) = delete;
   DevBuf& operator=(const DevBuf&) = delete;
-  ~DevBuf() {
-    if (p) cudaFree(p);
-  }
-  cudaError_t alloc(size_t bytes) {
+  ~DevBuf() { free(); }
+  void free() {
     if (p) cudaFree(p);
     p = nullptr;
+  }
+  cudaError_t alloc(size_t bytes) {
+    free();
     cudaError_t e = cudaMalloc(&p, std::max<size_t>(bytes, 16));
     if (e == cudaErrorMemoryAllocation) {
       cudaGetLastError();

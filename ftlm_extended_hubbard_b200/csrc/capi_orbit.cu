@@ -163,6 +163,10 @@ int build_orbit_sector(ftlm_sector* s) {
   return FTLM_OK;
 }
 
+// Share of the free device memory that one block's lists may take: 4x4 (8,8) needs 3.3 of 180 GB, and 16 blocks held at
+// once leave at least 60 % to everything else.
+constexpr size_t kListShare = 32;
+
 // The block's matrix as source lists (orbit.cuh): the values of the matrix elements, gathered up to rounding, become at
 // most 255 codes of 8 bits beside the 24 of a source's index.  Built once per block, for about two H_K v; each of these then
 // reads 4 bytes in order instead of 4 random ones per source.  Blocks with more values keep the tables.
@@ -218,17 +222,30 @@ int build_lists(ftlm_orbit* o, const std::vector<double2>& chi) {
           }
   const int pitch = (P.max_up_deg + P.max_dn_deg + 15) / 16 * 16;
   if (pitch == 0 || pitch > 0xFFFF) return FTLM_OK;
-  if (o->list.alloc(static_cast<size_t>(o->dk) * pitch * sizeof(uint32_t)) != cudaSuccess) {  // no room: the tables do
+  // The lists only save time, so they take a small share of the free memory and none that is not there: what has to be
+  // allocated after them (vectors, other blocks) then finds as good as what it did without them.
+  const size_t bytes = static_cast<size_t>(o->dk) * pitch * sizeof(uint32_t);
+  size_t free_bytes = 0, total_bytes = 0;
+  CU_TRY(cudaMemGetInfo(&free_bytes, &total_bytes));
+  if (bytes > free_bytes / kListShare) return FTLM_OK;
+  cudaStream_t st = o->sector->stream;
+  cudaError_t e = o->list.alloc(bytes);
+  if (e == cudaSuccess) e = o->cnt.alloc(static_cast<size_t>(o->dk) * sizeof(uint16_t));
+  if (e == cudaSuccess) e = upload_to(o->dict, dict, st);
+  if (e == cudaSuccess) e = upload_to(o->lut, lut, st);
+  if (e == cudaErrorMemoryAllocation) {  // the tables do
     cudaGetLastError();
-    o->list.p = nullptr;
+    o->list.free();
+    o->cnt.free();
+    o->dict.free();
+    o->lut.free();
     return FTLM_OK;
   }
-  CU_TRY(o->cnt.alloc(static_cast<size_t>(o->dk) * sizeof(uint16_t)));
-  CU_TRY(upload_to(o->dict, dict, o->sector->stream));
-  CU_TRY(upload_to(o->lut, lut, o->sector->stream));
+  CU_TRY(e);
   K.lut = o->lut.as<uint8_t>();
-  CU_TRY(orbit_lists(A, K, o->list.as<uint32_t>(), o->cnt.as<uint16_t>(), pitch, o->sector->stream));
-  CU_TRY(cudaStreamSynchronize(o->sector->stream));
+  CU_TRY(orbit_lists(A, K, o->list.as<uint32_t>(), o->cnt.as<uint16_t>(), pitch, st));
+  CU_TRY(cudaStreamSynchronize(st));
+  o->lut.free();
   A.list = o->list.as<uint32_t>();
   A.cnt = o->cnt.as<uint16_t>();
   A.dict = o->dict.as<double2>();
@@ -355,11 +372,13 @@ int ftlm_gpu_orbit_create_ex(ftlm_sector* s, int kx, int ky, double survive_tol,
   A.dhop_own = D.dh_own.as<uint32_t>();
   A.dhop_oth = D.dh_oth.as<uint32_t>();
   A.n_dhops = D.n_dh;
-  CU_TRY(o->xs.alloc(static_cast<size_t>(std::max<int64_t>(o->dk, 1)) * sizeof(double2)));
-  A.xs = o->xs.as<double2>();
   A.path = 1;
   rc = build_lists(o.get(), chi);
   if (rc) return rc;
+  if (!A.list) {  // only the table form has use for it
+    CU_TRY(o->xs.alloc(static_cast<size_t>(std::max<int64_t>(o->dk, 1)) * sizeof(double2)));
+    A.xs = o->xs.as<double2>();
+  }
   *out = o.release();
   return FTLM_OK;
 }

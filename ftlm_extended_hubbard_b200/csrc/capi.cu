@@ -178,6 +178,7 @@ int upload_plan(ftlm_sector* s) {
   const SectorPlan& P = s->plan;
   DevSector& D = s->dev;
   CU_TRY(cudaGetDevice(&s->device));
+  s->stream.set_device(s->device);
   D.n = P.n;
   D.Du = P.up.D;
   D.Dd = P.dn.D;

@@ -20,6 +20,7 @@
 #include "chains.cuh"
 #include "grad.cuh"
 #include "hv.cuh"
+#include "lazy_stream.hpp"
 #include "orbit.cuh"
 #include "planes.cuh"
 #include "plan.hpp"
@@ -132,24 +133,6 @@ struct DevBuf {
   T* as() const {
     return static_cast<T*>(p);
   }
-};
-
-// A non-blocking stream, created when it is first asked for: a sweep's sectors mostly share one launch and need none.
-class LazyStream {
- public:
-  LazyStream() = default;
-  LazyStream(const LazyStream&) = delete;
-  LazyStream& operator=(const LazyStream&) = delete;
-  ~LazyStream() {
-    if (s_) cudaStreamDestroy(s_);
-  }
-  operator cudaStream_t() {  // the legacy default stream where none can be created
-    if (!s_ && cudaStreamCreateWithFlags(&s_, cudaStreamNonBlocking) != cudaSuccess) s_ = nullptr;
-    return s_;
-  }
-
- private:
-  cudaStream_t s_ = nullptr;
 };
 
 // Plans of a sweep's sectors by N_up and by N_down, whose tables of that species the other sectors copy (build_plan).

@@ -118,3 +118,25 @@ def test_momentum_block_lists_leave_the_memory_to_others(gpu):
     torch.cuda.empty_cache()
     assert used < 45 << 20  # 13 MB table, 8 MB of entries, 3 MB workspace, in blocks of 2 MB
     assert np.abs(y - y2).max() <= 1e-13 * np.abs(y).max()
+
+
+def test_threads_share_a_fresh_handle(gpu):
+    """Eight threads make the first calls of one handle at once: each gets the chains of a handle of its own."""
+    import threading
+    p = F.HubbardParams(3, 3, 1.0, -0.25, 8.0, 1.0)
+    ref = F.Sector(p, 4, 4).batched_lanczos(4, 6, 3)
+    for _ in range(5):
+        s, out = F.Sector(p, 4, 4), [None] * 8
+        ready = threading.Barrier(8)
+
+        def work(i):
+            ready.wait()
+            out[i] = s.batched_lanczos(4, 6, 3)
+
+        pool = [threading.Thread(target=work, args=(i,)) for i in range(8)]
+        for t in pool:
+            t.start()
+        for t in pool:
+            t.join()
+        for o in out:
+            assert all(np.array_equal(a, b) for a, b in zip(o, ref))

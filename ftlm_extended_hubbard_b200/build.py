@@ -28,7 +28,7 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr"] + ARCH
 CXX_FLAGS = ["-O3", "-std=c++17", "-fPIC"]
 CU_SOURCES = ["hv.cu", "lanczos.cu", "quad.cu", "capi.cu", "capi_batched.cu", "capi_chains.cu", "capi_grad.cu", "capi_orbit.cu", "noalloc.cu", "batched.cu", "planes.cu", "orbit.cu", "grad.cu", "chains.cu", "symeig.cu"]
-CXX_SOURCES = ["plan.cpp", "tridiag.cpp"]
+CXX_SOURCES = ["plan.cpp", "pool.cpp", "tridiag.cpp"]
 
 
 def _nvcc() -> str:
@@ -77,7 +77,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
         o = os.path.join(BUILD, src + ".o")
         objs.append(o)
         if force or _stale(o, [s] + hdrs):
-            jobs.append([cxx, *CXX_FLAGS, "-I", CSRC, "-c", s, "-o", o])
+            jobs.append([cxx, *CXX_FLAGS, "-I", CSRC, "-I", os.path.join(_cuda_home(), "include"), "-c", s, "-o", o])
     if jobs:
         with ThreadPoolExecutor(max_workers=min(8, len(jobs))) as ex:
             list(ex.map(_run, jobs))

@@ -3,8 +3,8 @@
 // kernels of hv.cu / lanczos.cu / quad.cu.  No exception crosses the ABI.  The batched path,
 // the parameter gradient and the momentum blocks are in capi_batched.cu, capi_grad.cu and
 // capi_orbit.cu.
-#include <map>
 #include <atomic>
+#include <map>
 
 #include "capi_internal.hpp"
 
@@ -24,97 +24,6 @@ int ftlm_b200::capi::fail(int code, const std::string& msg) {
 }
 
 int ftlm_b200::set_error(int code, const char* msg) { return fail(code, msg); }
-
-namespace {
-
-struct PoolBlock {
-  void* p;
-  size_t bytes;
-};
-struct Pool {
-  std::mutex mu;
-  std::map<int, std::vector<PoolBlock>> free;  // by device
-  std::map<void*, int> device;                 // of every block taken or kept
-  size_t kept = 0;
-};
-Pool& pool() {
-  static Pool* p = new Pool;  // not destroyed: its blocks end with the context
-  return *p;
-}
-
-}  // namespace
-
-cudaError_t ftlm_b200::capi::pool_take(size_t bytes, void** p, size_t* got) {
-  *p = nullptr;
-  *got = 0;
-  bytes = std::max<size_t>(bytes, 256);
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  Pool& P = pool();
-  {
-    std::lock_guard<std::mutex> lock(P.mu);
-    auto& v = P.free[dev];
-    size_t best = v.size();
-    for (size_t i = 0; i < v.size(); ++i)  // the smallest that fits, unless most of it would lie idle
-      if (v[i].bytes >= bytes && v[i].bytes <= 8 * bytes + (size_t(1) << 20) && (best == v.size() || v[i].bytes < v[best].bytes))
-        best = i;
-    if (best < v.size()) {
-      *p = v[best].p;
-      *got = v[best].bytes;
-      P.kept -= v[best].bytes;
-      v[best] = v.back();
-      v.pop_back();
-      return cudaSuccess;
-    }
-  }
-  size_t want = bytes;  // rounded up to an eighth of its power of two, so that blocks fit each other's uses
-  size_t unit = 256;
-  while (unit * 16 < bytes) unit *= 2;
-  want = (bytes + unit - 1) / unit * unit;
-  e = cudaMalloc(p, want);
-  if (e == cudaErrorMemoryAllocation) {
-    cudaGetLastError();
-    pool_trim();
-    e = cudaMalloc(p, want);
-  }
-  if (e != cudaSuccess) return e;
-  *got = want;
-  std::lock_guard<std::mutex> lock(P.mu);
-  P.device[*p] = dev;
-  return cudaSuccess;
-}
-
-void ftlm_b200::capi::pool_give(void* p, size_t got) {
-  if (!p) return;
-  Pool& P = pool();
-  {
-    std::lock_guard<std::mutex> lock(P.mu);
-    auto it = P.device.find(p);
-    if (it != P.device.end() && P.kept + got <= kPoolKeep) {
-      P.free[it->second].push_back(PoolBlock{p, got});
-      P.kept += got;
-      return;
-    }
-    if (it != P.device.end()) P.device.erase(it);
-  }
-  cudaFree(p);
-}
-
-void ftlm_b200::capi::pool_trim() {
-  Pool& P = pool();
-  std::vector<PoolBlock> all;
-  {
-    std::lock_guard<std::mutex> lock(P.mu);
-    for (auto& d : P.free) {
-      all.insert(all.end(), d.second.begin(), d.second.end());
-      d.second.clear();
-    }
-    for (const PoolBlock& b : all) P.device.erase(b.p);
-    P.kept = 0;
-  }
-  for (const PoolBlock& b : all) cudaFree(b.p);
-}
 
 namespace ftlm_b200 {
 namespace capi {

@@ -23,6 +23,7 @@
 #include "lazy_stream.hpp"
 #include "orbit.cuh"
 #include "planes.cuh"
+#include "pool.hpp"
 #include "plan.hpp"
 #include "symeig.cuh"
 #include "tridiag.hpp"
@@ -40,73 +41,6 @@ int fail(int code, const std::string& msg);
       return ::ftlm_b200::capi::fail(e_ == cudaErrorMemoryAllocation ? FTLM_ERR_NOMEM : FTLM_ERR_CUDA,   \
                   std::string(#expr) + ": " + cudaGetErrorString(e_));                                   \
   } while (0)
-
-// Device blocks kept between calls, for workspaces and tables that live for one call or one small sector: cudaMalloc and
-// cudaFree cost tens of microseconds to milliseconds each, more than many of the calls.  Per device, at most kPoolKeep
-// bytes stay here (given back by ftlm_gpu_batched_release, or when device memory runs out); thread-safe.  A block is
-// given only when no work on it is in flight.
-constexpr size_t kPoolKeep = size_t(1) << 30;
-cudaError_t pool_take(size_t bytes, void** p, size_t* got);
-void pool_give(void* p, size_t got);
-void pool_trim();
-
-// One array in a block of the pool; its owner gives it back when no work on it is in flight.
-struct PoolBuf {
-  void* p = nullptr;
-  size_t got = 0;
-  PoolBuf() = default;
-  PoolBuf(const PoolBuf&) = delete;
-  PoolBuf& operator=(const PoolBuf&) = delete;
-  ~PoolBuf() { free(); }
-  void free() {
-    if (p) pool_give(p, got);
-    p = nullptr;
-    got = 0;
-  }
-  cudaError_t alloc(size_t bytes) {
-    free();
-    return pool_take(bytes, &p, &got);
-  }
-  template <class T>
-  T* as() const {
-    return static_cast<T*>(p);
-  }
-};
-
-// One block of the pool, laid out by add() and obtained by commit().  idle() says that the work on it has ended; without
-// it (an error on the way) the block is given back after the device has.
-class Scratch {
- public:
-  Scratch() = default;
-  Scratch(const Scratch&) = delete;
-  Scratch& operator=(const Scratch&) = delete;
-  ~Scratch() {
-    if (!p_) return;
-    if (busy_) cudaDeviceSynchronize();
-    pool_give(p_, got_);
-  }
-  size_t add(size_t bytes) {
-    const size_t at = size_;
-    size_ += (std::max<size_t>(bytes, 1) + 255) / 256 * 256;
-    return at;
-  }
-  template <class T>
-  size_t array(size_t n) {
-    return add(n * sizeof(T));
-  }
-  cudaError_t commit() { return pool_take(size_, &p_, &got_); }
-  template <class T>
-  T* at(size_t off) const {
-    return reinterpret_cast<T*>(static_cast<char*>(p_) + off);
-  }
-  void idle() { busy_ = false; }
-  void busy() { busy_ = true; }
-
- private:
-  void* p_ = nullptr;
-  size_t size_ = 0, got_ = 0;
-  bool busy_ = true;
-};
 
 // Device buffer that frees itself.
 struct DevBuf {
@@ -271,6 +205,12 @@ struct BtWs {
     for (auto& b : buf) b.free();
     cap = 0;
   }
+  void free_all(bool idle) {
+    for (PoolBuf* b : {&buf[0], &buf[1], &buf[2], &st, &partial, &items, &alpha, &beta, &used, &flags}) b->free(idle);
+    cap = 0;
+    mcap = 0;
+    icap = 0;
+  }
 };
 
 }  // namespace capi
@@ -297,8 +237,10 @@ struct ftlm_sector {
   ftlm_b200::capi::LazyStream stream;
   ~ftlm_sector() {
     if (!tables) return;
-    cudaDeviceSynchronize();  // as a free would: a caller's H v may still read the tables (and before `planes` goes back)
-    ftlm_b200::capi::pool_give(tables, tables_bytes);
+    // as a free would wait: a caller's H v may still read the tables
+    const bool idle = ftlm_b200::capi::device_idle(device);
+    ftlm_b200::capi::pool_give(tables, tables_bytes, idle);
+    planes.free_all(idle);
   }
   // Kernel choice for H·v: 1 = generic gather; 2 = row pass with the per-row coefficient table +
   // column-slab pass over the CSR up list; 3 = row pass in the gauge basis (register-held real

@@ -140,3 +140,28 @@ def test_threads_share_a_fresh_handle(gpu):
             t.join()
         for o in out:
             assert all(np.array_equal(a, b) for a, b in zip(o, ref))
+
+
+def test_handle_goes_while_its_call_is_in_flight(gpu):
+    """A handle is dropped right after an asynchronous H v and another of the same shape takes its tables' place: both
+    results are those of calls one at a time."""
+    torch = gpu
+    a, b = F.HubbardParams(4, 3, 1.0, -0.25, 8.0, 1.0), F.HubbardParams(4, 3, 0.5, 0.3, 2.0, 0.0)
+    x = torch.randn(245025, dtype=torch.complex128, device="cuda")
+    ref = []
+    for p in (a, b):
+        y = torch.empty_like(x)
+        F.Sector(p, 4, 4).apply(x, y)
+        torch.cuda.synchronize()
+        ref.append(y)
+    side = torch.cuda.Stream()
+    for _ in range(10):
+        out = [torch.empty_like(x) for _ in range(2)]
+        torch.cuda.synchronize()
+        for p, y in zip((a, b), out):
+            s = F.Sector(p, 4, 4)
+            for _ in range(20):
+                s.apply(x, y, side.cuda_stream)
+            s.close()
+        torch.cuda.synchronize()
+        assert torch.equal(out[0], ref[0]) and torch.equal(out[1], ref[1])

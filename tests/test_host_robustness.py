@@ -21,6 +21,6 @@ def _run_program(tmp_path, name, *sources):
     assert r.returncode == 0, r.stderr
 
 
-@pytest.mark.parametrize("name", ["host_lazy_stream"])
-def test_host_classes(tmp_path, name):
-    _run_program(tmp_path, name)
+@pytest.mark.parametrize("name,sources", [("host_lazy_stream", []), ("host_pool", ["pool.cpp"])])
+def test_host_classes(tmp_path, name, sources):
+    _run_program(tmp_path, name, *(os.path.join(CSRC, s) for s in sources))

@@ -161,17 +161,24 @@ int create_common(int n_sites, int n_up, int n_dn, double U, double V, const ftl
   *out = nullptr;
   if (n_hops < 0 || n_pairs < 0 || (n_hops > 0 && !hops) || (n_pairs > 0 && !pairs))
     return fail(FTLM_ERR_INVALID, "bad hopping/pair arrays");
-  std::vector<HopIn> hv(static_cast<size_t>(n_hops));
-  for (int i = 0; i < n_hops; ++i) hv[i] = HopIn{hops[i].from, hops[i].to, hops[i].spin, hops[i].coeff_re, hops[i].coeff_im};
-  std::vector<PairIn> pv(static_cast<size_t>(n_pairs));
-  for (int i = 0; i < n_pairs; ++i) pv[i] = PairIn{pairs[i].i, pairs[i].j};
   auto* s = new (std::nothrow) ftlm_sector();
   if (!s) return fail(FTLM_ERR_NOMEM, "host allocation failed");
   std::string err;
   try {
+    std::vector<HopIn> hv(static_cast<size_t>(n_hops));
+    for (int i = 0; i < n_hops; ++i) hv[i] = HopIn{hops[i].from, hops[i].to, hops[i].spin, hops[i].coeff_re, hops[i].coeff_im};
+    std::vector<PairIn> pv(static_cast<size_t>(n_pairs));
+    for (int i = 0; i < n_pairs; ++i) pv[i] = PairIn{pairs[i].i, pairs[i].j};
     err = build_plan(n_sites, n_up, n_dn, U, V, hv, pv, &s->plan, parts ? parts->find(parts->up, n_up) : nullptr,
                      parts ? parts->find(parts->dn, n_dn) : nullptr);
     if (parts && err.empty()) parts->keep(s->plan);
+    if (device && err.empty()) {
+      const int rc = upload_plan(s);
+      if (rc != FTLM_OK) {
+        delete s;
+        return rc;
+      }
+    }
   } catch (const std::bad_alloc&) {
     delete s;
     return fail(FTLM_ERR_NOMEM, "host allocation failed while building the sector plan");
@@ -180,13 +187,6 @@ int create_common(int n_sites, int n_up, int n_dn, double U, double V, const ftl
     delete s;
     const bool unsup = err.find("not supported") != std::string::npos || err.find("2^31") != std::string::npos;
     return fail(unsup ? FTLM_ERR_UNSUPPORTED : FTLM_ERR_INVALID, err);
-  }
-  if (device) {
-    const int rc = upload_plan(s);
-    if (rc != FTLM_OK) {
-      delete s;
-      return rc;
-    }
   }
   *out = s;
   return FTLM_OK;

@@ -3,6 +3,7 @@
 #include <thread>
 
 #include "capi_internal.hpp"
+#include "workers.hpp"
 
 using namespace ftlm_b200;
 using namespace ftlm_b200::capi;
@@ -15,27 +16,16 @@ namespace capi {
 void reference_normals(int64_t dim, int R, unsigned seed, std::vector<std::complex<double>>* out) {
   out->resize(static_cast<size_t>(R) * dim);
   const int hw = static_cast<int>(std::max(1u, std::min(32u, std::thread::hardware_concurrency())));
-  auto work = [&](int w, int n) {
-    for (int r = w; r < R; r += n) {
-      std::mt19937 rng(seed + static_cast<unsigned>(r) * 100003u);
-      std::normal_distribution<double> gauss(0.0, 1.0);
-      std::complex<double>* v = out->data() + static_cast<size_t>(r) * dim;
-      for (int64_t i = 0; i < dim; ++i) {
-        const double re = gauss(rng);
-        const double im = gauss(rng);
-        v[i] = {re, im};
-      }
+  share_out(static_cast<int64_t>(R) * dim < 4096 ? 1 : hw, R, [&](int64_t r) {
+    std::mt19937 rng(seed + static_cast<unsigned>(r) * 100003u);
+    std::normal_distribution<double> gauss(0.0, 1.0);
+    std::complex<double>* v = out->data() + static_cast<size_t>(r) * dim;
+    for (int64_t i = 0; i < dim; ++i) {
+      const double re = gauss(rng);
+      const double im = gauss(rng);
+      v[i] = {re, im};
     }
-  };
-  const int n = std::min(hw, R);
-  if (n <= 1 || static_cast<int64_t>(R) * dim < 4096) {
-    work(0, 1);
-    return;
-  }
-  std::vector<std::thread> pool;
-  for (int w = 1; w < n; ++w) pool.emplace_back(work, w, n);
-  work(0, n);
-  for (auto& th : pool) th.join();
+  });
 }
 
 int chains_run(const std::vector<ftlm_sector*>& secs, int R, int M, unsigned seed, int start_mode, bool c64,

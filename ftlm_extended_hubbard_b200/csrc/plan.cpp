@@ -7,8 +7,9 @@
 #include <complex>
 #include <cstring>
 #include <map>
-#include <thread>
 #include <utility>
+
+#include "workers.hpp"
 
 namespace ftlm_b200 {
 
@@ -378,16 +379,7 @@ void build_gauge_table(const SpinSpace& sp, const std::vector<MergedHop>& hops, 
   };
   const int nthreads = static_cast<int>(
       std::max<int64_t>(1, std::min<int64_t>({static_cast<int64_t>(std::thread::hardware_concurrency()), 16, ngroups / 16})));
-  if (nthreads == 1) {
-    for (int64_t g = 0; g < ngroups; ++g) build_group(g);
-  } else {
-    std::vector<std::thread> pool;
-    for (int w = 0; w < nthreads; ++w)
-      pool.emplace_back([&, w]() {
-        for (int64_t g = w; g < ngroups; g += nthreads) build_group(g);
-      });
-    for (auto& t : pool) t.join();
-  }
+  share_out(nthreads, ngroups, build_group);
   for (const Group& R : groups) {
     const size_t off = G.ent.size();
     if (!R.ok || off + R.ent.size() > static_cast<size_t>(INT32_MAX) || R.KR0 > 0xFFFF || R.KT0 > 0x7FFF) {

@@ -23,6 +23,20 @@ int ftlm_b200::capi::fail(int code, const std::string& msg) {
   return code;
 }
 
+int ftlm_b200::capi::caught() noexcept {
+  try {
+    try {
+      throw;
+    } catch (const std::bad_alloc&) {
+      return fail(FTLM_ERR_NOMEM, "host allocation failed");
+    } catch (const std::exception& e) {  // a size that no vector can have
+      return fail(FTLM_ERR_NOMEM, e.what());
+    }
+  } catch (...) {  // not even the message
+  }
+  return FTLM_ERR_NOMEM;
+}
+
 int ftlm_b200::set_error(int code, const char* msg) { return fail(code, msg); }
 
 namespace ftlm_b200 {
@@ -238,7 +252,7 @@ int ftlm_gpu_device_count(int* n) {
 }
 
 int ftlm_gpu_build_geometry(const ftlm_params* p, ftlm_hop* hops, int max_hops, int* n_hops, ftlm_pair* pairs,
-                            int max_pairs, int* n_pairs) {
+                            int max_pairs, int* n_pairs) try {
   if (!p || !n_hops || !n_pairs) return fail(FTLM_ERR_INVALID, "null argument");
   if (p->Lx <= 0 || p->Ly <= 0) return fail(FTLM_ERR_INVALID, "Lx, Ly must be positive");
   std::vector<HopIn> hv;
@@ -250,6 +264,8 @@ int ftlm_gpu_build_geometry(const ftlm_params* p, ftlm_hop* hops, int max_hops, 
     hops[i] = ftlm_hop{hv[i].from, hv[i].to, hv[i].spin, hv[i].cre, hv[i].cim};
   for (int i = 0; i < *n_pairs && i < max_pairs && pairs; ++i) pairs[i] = ftlm_pair{pv[i].i, pv[i].j};
   return FTLM_OK;
+} catch (...) {
+  return caught();
 }
 
 int ftlm_gpu_sector_create_hops(int n_sites, int n_up, int n_dn, double U, double V, const ftlm_hop* hops, int n_hops,
@@ -262,8 +278,10 @@ int ftlm_gpu_sector_create_host(int n_sites, int n_up, int n_dn, double U, doubl
   return create_common(n_sites, n_up, n_dn, U, V, hops, n_hops, pairs, n_pairs, false, out);
 }
 
-int ftlm_gpu_sector_create(const ftlm_params* p, int n_up, int n_dn, ftlm_sector** out) {
+int ftlm_gpu_sector_create(const ftlm_params* p, int n_up, int n_dn, ftlm_sector** out) try {
   return sector_create(p, n_up, n_dn, nullptr, out);
+} catch (...) {
+  return caught();
 }
 
 int ftlm_gpu_sector_destroy(ftlm_sector* s) {
@@ -517,7 +535,7 @@ void trim_chain(int n, std::vector<double>* a, std::vector<double>* b) {
 extern "C" {
 
 int ftlm_gpu_lanczos(ftlm_sector* s, int max_steps, unsigned seed, int start_mode, double* alpha, double* beta,
-                     int* n_beta, int* used) {
+                     int* n_beta, int* used) try {
   int rc = need_device(s);
   if (rc) return rc;
   std::vector<double> a, b;
@@ -549,6 +567,8 @@ int ftlm_gpu_lanczos(ftlm_sector* s, int max_steps, unsigned seed, int start_mod
   if (n_beta) *n_beta = static_cast<int>(b.size());
   if (used) *used = static_cast<int>(a.size());
   return FTLM_OK;
+} catch (...) {
+  return caught();
 }
 
 int ftlm_gpu_lanczos_op(long long dim, ftlm_apply_fn fn, void* ctx, int max_steps, unsigned seed, int start_mode,
@@ -604,7 +624,7 @@ int ftlm_gpu_lanczos_host_op(long long dim, ftlm_host_apply_fn fn, void* ctx, in
 }
 
 int ftlm_gpu_ftlm_combine(const double* logq, const double* energy_r, const int* used, int R, int n_bt, double log_dim,
-                          double* lnz, double* energy) {
+                          double* lnz, double* energy) try {
   if (R <= 0 || n_bt < 0 || !logq || !energy_r || !used || !lnz || !energy) return fail(FTLM_ERR_INVALID, "bad arguments");
   if (n_bt == 0) return FTLM_OK;
   const size_t qb = static_cast<size_t>(R) * n_bt * sizeof(double);
@@ -621,10 +641,12 @@ int ftlm_gpu_ftlm_combine(const double* logq, const double* energy_r, const int*
   CU_TRY(cudaMemcpy(energy, mem.at<void>(o_den), n_bt * sizeof(double), cudaMemcpyDeviceToHost));
   mem.idle();
   return FTLM_OK;
+} catch (...) {
+  return caught();
 }
 
 int ftlm_gpu_tridiag_eig(const double* alpha, const double* beta, const int* n, int nc, int ld, int max_rot, double tol,
-                         double* lam, double* w0) {
+                         double* lam, double* w0) try {
   if (nc < 0 || ld <= 0 || !alpha || !beta || !n || !lam || !w0) return fail(FTLM_ERR_INVALID, "bad arguments");
   if (ld > 160) return fail(FTLM_ERR_UNSUPPORTED, "tridiagonal size > 160 is not supported by the on-chip Jacobi");
   for (int c = 0; c < nc; ++c)
@@ -644,10 +666,12 @@ int ftlm_gpu_tridiag_eig(const double* alpha, const double* beta, const int* n, 
   CU_TRY(cudaMemcpy(w0, mem.at<void>(o_dw), mat, cudaMemcpyDeviceToHost));
   mem.idle();
   return FTLM_OK;
+} catch (...) {
+  return caught();
 }
 
 int ftlm_gpu_tridiag_quadrature(const double* alpha, const double* beta, const int* n, int nc, int ld,
-                                const double* bts, int n_bt, double* logq, double* energy) {
+                                const double* bts, int n_bt, double* logq, double* energy) try {
   if (nc < 0 || ld <= 0 || n_bt < 0 || !alpha || !beta || !n || !bts || !logq || !energy)
     return fail(FTLM_ERR_INVALID, "bad arguments");
   if (ld > 160) return fail(FTLM_ERR_UNSUPPORTED, "tridiagonal size > 160 is not supported by the on-chip Jacobi");
@@ -674,9 +698,11 @@ int ftlm_gpu_tridiag_quadrature(const double* alpha, const double* beta, const i
   CU_TRY(cudaMemcpy(energy, mem.at<void>(o_de), outb, cudaMemcpyDeviceToHost));
   mem.idle();
   return FTLM_OK;
+} catch (...) {
+  return caught();
 }
 
-int ftlm_gpu_ritz_values(const double* alpha, const double* beta, int n, int k, double* ritz) {
+int ftlm_gpu_ritz_values(const double* alpha, const double* beta, int n, int k, double* ritz) try {
   if (n <= 0 || k <= 0 || !alpha || !ritz || (n > 1 && !beta)) return fail(FTLM_ERR_INVALID, "bad arguments");
   k = std::min(k, n);
   Scratch mem;
@@ -689,10 +715,12 @@ int ftlm_gpu_ritz_values(const double* alpha, const double* beta, int n, int k, 
   CU_TRY(cudaMemcpy(ritz, mem.at<void>(o_dr), k * sizeof(double), cudaMemcpyDeviceToHost));
   mem.idle();
   return FTLM_OK;
+} catch (...) {
+  return caught();
 }
 
 int ftlm_gpu_lanczos_extrema(ftlm_sector* s, int max_steps, unsigned seed, int start_mode, double* mn, double* mx,
-                             int* steps_used) {
+                             int* steps_used) try {
   if (!mn || !mx) return fail(FTLM_ERR_INVALID, "null output");
   *mn = 0.0;
   *mx = 0.0;
@@ -719,6 +747,8 @@ int ftlm_gpu_lanczos_extrema(ftlm_sector* s, int max_steps, unsigned seed, int s
   *mn = *std::min_element(lam.begin(), lam.end());
   *mx = *std::max_element(lam.begin(), lam.end());
   return FTLM_OK;
+} catch (...) {
+  return caught();
 }
 
 int ftlm_gpu_set_quadrature(int mode) {
@@ -728,8 +758,10 @@ int ftlm_gpu_set_quadrature(int mode) {
 }
 
 int ftlm_gpu_ftlm_sector(ftlm_sector* s, const double* bts, int n_bt, int R, int M, unsigned seed, int start_mode,
-                         double* lnz, double* energy) {
+                         double* lnz, double* energy) try {
   return plain_sector_ftlm(s, bts, n_bt, R, M, seed, start_mode, plain_quadrature_converged(), lnz, energy);
+} catch (...) {
+  return caught();
 }
 
 }  // extern "C"
@@ -807,7 +839,7 @@ bool plain_quadrature_converged() { return g_quad_converged.load(); }
 extern "C" {
 
 int ftlm_gpu_gc_reduce(const double* lnz_s, const double* e_s, const int* N_s, int n_sec, const double* bts, int n_bt,
-                       const double* mus, int n_mu, int n_sites, double* lnz_gc, double* n_avg, double* e_avg) {
+                       const double* mus, int n_mu, int n_sites, double* lnz_gc, double* n_avg, double* e_avg) try {
   if (n_sec < 0 || n_bt < 0 || n_mu < 0 || !lnz_s || !e_s || !N_s || !bts || !mus || !lnz_gc || !n_avg || !e_avg)
     return fail(FTLM_ERR_INVALID, "bad arguments");
   if (n_bt == 0 || n_mu == 0) return FTLM_OK;
@@ -832,6 +864,8 @@ int ftlm_gpu_gc_reduce(const double* lnz_s, const double* e_s, const int* N_s, i
   CU_TRY(cudaMemcpy(e_avg, mem.at<void>(o_o3), gb, cudaMemcpyDeviceToHost));
   mem.idle();
   return FTLM_OK;
+} catch (...) {
+  return caught();
 }
 
 }  // extern "C"
@@ -863,7 +897,7 @@ int fused_sectors_ftlm(const std::vector<ftlm_sector*>& secs, const std::vector<
 extern "C" {
 
 int ftlm_gpu_lanczos_sectors(ftlm_sector* const* secs, int n_sectors, int R, int M, unsigned seed, int start_mode,
-                             double* alpha, double* beta, int* used) {
+                             double* alpha, double* beta, int* used) try {
   if (!secs || n_sectors < 0 || R <= 0 || M <= 0 || !alpha || !beta || !used) return fail(FTLM_ERR_INVALID, "bad arguments");
   // Sectors far beyond the fused path's range, or with rows too long for it, run their chains one at a time.
   constexpr int64_t kFusedMost = int64_t(1) << 22;
@@ -899,6 +933,8 @@ int ftlm_gpu_lanczos_sectors(ftlm_sector* const* secs, int n_sectors, int R, int
     CU_TRY(cudaMemcpy(used + o, run.used + i * rows, rows * sizeof(int), cudaMemcpyDeviceToHost));
   }
   return FTLM_OK;
+} catch (...) {
+  return caught();
 }
 
 int ftlm_gpu_set_cols_variant(ftlm_sector* s, int variant) {
@@ -907,7 +943,7 @@ int ftlm_gpu_set_cols_variant(ftlm_sector* s, int variant) {
   return FTLM_OK;
 }
 
-int ftlm_gpu_autotune_apply(ftlm_sector* s, int reps, int* path, int* cols_variant, float* ms) {
+int ftlm_gpu_autotune_apply(ftlm_sector* s, int reps, int* path, int* cols_variant, float* ms) try {
   int rc = need_device(s);
   if (rc) return rc;
   reps = std::max(1, reps);
@@ -993,6 +1029,8 @@ int ftlm_gpu_autotune_apply(ftlm_sector* s, int reps, int* path, int* cols_varia
   if (cols_variant) *cols_variant = best_v;
   if (ms) *ms = best / static_cast<float>(reps);
   return FTLM_OK;
+} catch (...) {
+  return caught();
 }
 
 int ftlm_gpu_set_fused_max_dim(long long max_dim) {
@@ -1003,27 +1041,23 @@ int ftlm_gpu_set_fused_max_dim(long long max_dim) {
 
 int ftlm_gpu_gc_sweep(const ftlm_params* p, int R, int M, unsigned seed, int start_mode, const double* bts, int n_bt,
                       const double* mus, int n_mu, double* lnz_s, double* e_s, double* lnz_gc, double* n_avg,
-                      double* e_avg) {
+                      double* e_avg) try {
   if (!p || !lnz_s || !e_s) return fail(FTLM_ERR_INVALID, "null argument");
   const int n = p->Lx * p->Ly;
   if (n <= 0 || n > 32) return fail(FTLM_ERR_INVALID, "FockBasis: require 1 <= n_sites <= 32 (bit packing)");
   const int nsec = (n + 1) * (n + 1);
   std::vector<int> N(static_cast<size_t>(nsec));
   PlanParts parts(n);
-  std::vector<ftlm_sector*> small;  // sectors for the fused small-sector launch
+  OwnedSectors owned;
+  std::vector<ftlm_sector*>& small = owned.v;  // sectors for the fused small-sector launch
   std::vector<int> small_idx;
-  auto clear_and = [](std::vector<ftlm_sector*>& v, int rc) {
-    for (ftlm_sector* x : v) ftlm_gpu_sector_destroy(x);
-    v.clear();
-    return rc;
-  };
   for (int nu = 0; nu <= n; ++nu)
     for (int nd = 0; nd <= n; ++nd) {
       const int idx = nu * (n + 1) + nd;  // benchmarks/bench_ftlm_nmu_rect.cpp:62
       N[static_cast<size_t>(idx)] = nu + nd;
       ftlm_sector* s = nullptr;
       int rc = sector_create(p, nu, nd, &parts, &s);
-      if (rc) return clear_and(small, rc);
+      if (rc) return rc;
       if (s->plan.dim >= 2 && s->plan.dim <= g_fused_max_dim && M <= 160 && chain_rows(s->dev, false, false) > 0) {  // fused below
         small.push_back(s);
         small_idx.push_back(idx);
@@ -1032,15 +1066,16 @@ int ftlm_gpu_gc_sweep(const ftlm_params* p, int R, int M, unsigned seed, int sta
       rc = ftlm_gpu_ftlm_sector(s, bts, n_bt, R, M, seed, start_mode, lnz_s + static_cast<size_t>(idx) * n_bt,
                                 e_s + static_cast<size_t>(idx) * n_bt);
       ftlm_gpu_sector_destroy(s);
-      if (rc) return clear_and(small, rc);
+      if (rc) return rc;
     }
   const int rcf = fused_sectors_ftlm(small, small_idx, std::max(1, R), std::max(1, M), seed, start_mode, false, bts, n_bt,
                                      lnz_s, e_s, plain_quadrature_converged());
-  clear_and(small, FTLM_OK);
   if (rcf) return rcf;
   if (lnz_gc && n_avg && e_avg)
     return ftlm_gpu_gc_reduce(lnz_s, e_s, N.data(), nsec, bts, n_bt, mus, n_mu, n, lnz_gc, n_avg, e_avg);
   return FTLM_OK;
+} catch (...) {
+  return caught();
 }
 
 }  // extern "C"

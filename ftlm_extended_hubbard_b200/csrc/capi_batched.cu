@@ -72,7 +72,7 @@ int ftlm_gpu_batched_set_cols_variant(ftlm_sector* s, int variant) {
   return FTLM_OK;
 }
 
-int ftlm_gpu_batched_autotune(ftlm_sector* s, int reps, int* variant, float* ms) {
+int ftlm_gpu_batched_autotune(ftlm_sector* s, int reps, int* variant, float* ms) try {
   int rc = need_device(s);
   if (rc) return rc;
   if (s->plan.max_up_deg > 120)
@@ -137,9 +137,11 @@ int ftlm_gpu_batched_autotune(ftlm_sector* s, int reps, int* variant, float* ms)
   if (variant) *variant = best_v;
   if (ms) *ms = best / static_cast<float>(reps);
   return FTLM_OK;
+} catch (...) {
+  return caught();
 }
 
-int ftlm_gpu_batched_lanczos(ftlm_sector* s, int R, int M, unsigned seed, double* alpha, double* beta, int* used) {
+int ftlm_gpu_batched_lanczos(ftlm_sector* s, int R, int M, unsigned seed, double* alpha, double* beta, int* used) try {
   int rc = need_device(s);
   if (rc) return rc;
   if (s->plan.max_up_deg > 120)
@@ -153,6 +155,8 @@ int ftlm_gpu_batched_lanczos(ftlm_sector* s, int R, int M, unsigned seed, double
   std::copy(B.begin(), B.end(), beta);
   std::copy(u.begin(), u.end(), used);
   return FTLM_OK;
+} catch (...) {
+  return caught();
 }
 
 namespace {
@@ -211,14 +215,18 @@ int batched_sector(ftlm_sector* s, const double* bts, int n_bt, int R, int M, un
 }  // namespace
 
 int ftlm_gpu_batched_ftlm_sector(ftlm_sector* s, const double* bts, int n_bt, int R, int M, unsigned seed, double* lnz,
-                                 double* energy) {
+                                 double* energy) try {
   return batched_sector(s, bts, n_bt, R, M, seed, 0, lnz, energy, nullptr);
+} catch (...) {
+  return caught();
 }
 
 int ftlm_gpu_batched_ftlm_sector_checked(ftlm_sector* s, const double* bts, int n_bt, int R, int M, unsigned seed,
-                                         int n_check, double* lnz, double* energy, double* lnz_err) {
+                                         int n_check, double* lnz, double* energy, double* lnz_err) try {
   if (n_check < 1) return fail(FTLM_ERR_INVALID, "n_check must be >= 1");
   return batched_sector(s, bts, n_bt, R, M, seed, n_check, lnz, energy, lnz_err);
+} catch (...) {
+  return caught();
 }
 
 namespace {
@@ -231,14 +239,16 @@ int batched_sweep(const ftlm_params* p, int R, int M, unsigned seed, const doubl
 
 int ftlm_gpu_batched_sweep(const ftlm_params* p, int R, int M, unsigned seed, const double* bts, int n_bt,
                            const double* mus, int n_mu, double* lnz_s, double* e_s, double* lnz_gc, double* n_avg,
-                           double* e_avg) {
+                           double* e_avg) try {
   return batched_sweep(p, R, M, seed, bts, n_bt, mus, n_mu, 0, lnz_s, e_s, lnz_gc, n_avg, e_avg, nullptr);
+} catch (...) {
+  return caught();
 }
 
 int ftlm_gpu_batched_sweep_checked(const ftlm_params* p, int R, int M, unsigned seed, const double* bts, int n_bt,
                                    const double* mus, int n_mu, int n_check, double* lnz_s, double* e_s, double* lnz_gc,
                                    double* n_avg, double* e_avg, double* lnz_s_err, double* lnz_gc_err,
-                                   double* n_err) {
+                                   double* n_err) try {
   if (n_check < 1) return fail(FTLM_ERR_INVALID, "n_check must be >= 1");
   if (!p || !lnz_s_err || !lnz_gc || !n_avg || !e_avg || !lnz_gc_err || !n_err)
     return fail(FTLM_ERR_INVALID, "null argument");
@@ -265,6 +275,8 @@ int ftlm_gpu_batched_sweep_checked(const ftlm_params* p, int R, int M, unsigned 
       n_err[o] = en;
     }
   return FTLM_OK;
+} catch (...) {
+  return caught();
 }
 
 namespace {
@@ -280,22 +292,16 @@ int batched_sweep(const ftlm_params* p, int R, int M, unsigned seed, const doubl
   // small sectors go to fused launches: those the batched path runs in complex128 (dim <= 2M, Philox starts), and
   // those whose complex64 chains need no check against complex128
   PlanParts parts(n);
-  std::vector<ftlm_sector*> small, mid;
+  OwnedSectors owned[2];
+  std::vector<ftlm_sector*>&small = owned[0].v, &mid = owned[1].v;
   std::vector<int> small_idx, mid_idx;
-  auto clear_and = [&small, &mid](int rc) {
-    for (ftlm_sector* x : small) ftlm_gpu_sector_destroy(x);
-    for (ftlm_sector* x : mid) ftlm_gpu_sector_destroy(x);
-    small.clear();
-    mid.clear();
-    return rc;
-  };
   for (int nu = 0; nu <= n; ++nu)
     for (int nd = 0; nd <= n; ++nd) {
       const int idx = nu * (n + 1) + nd;
       N[static_cast<size_t>(idx)] = nu + nd;
       ftlm_sector* s = nullptr;
       int rc = sector_create(p, nu, nd, &parts, &s);
-      if (rc) return clear_and(rc);
+      if (rc) return rc;
       if (s->plan.dim >= 2 && s->plan.dim <= 2 * static_cast<int64_t>(std::max(1, M)) && M <= 160) {  // a row fits: <= 320
         small.push_back(s);
         small_idx.push_back(idx);
@@ -311,14 +317,13 @@ int batched_sweep(const ftlm_params* p, int R, int M, unsigned seed, const doubl
                           e_s + static_cast<size_t>(idx) * n_bt,
                           lnz_s_err ? lnz_s_err + static_cast<size_t>(idx) * n_bt : nullptr);
       ftlm_gpu_sector_destroy(s);
-      if (rc) return clear_and(rc);
+      if (rc) return rc;
     }
   int rcf = fused_sectors_ftlm(small, small_idx, std::max(1, R), std::max(1, M), seed, FTLM_START_PHILOX, false, bts, n_bt,
                                lnz_s, e_s, true);
   if (!rcf)
     rcf = fused_sectors_ftlm(mid, mid_idx, std::max(1, R), std::max(1, M), seed, FTLM_START_PHILOX, true, bts, n_bt, lnz_s,
                              e_s, true);
-  clear_and(FTLM_OK);
   if (rcf) return rcf;
   if (lnz_s_err)  // the fused small sectors ran in complex128
     for (int i : small_idx) std::fill(lnz_s_err + static_cast<size_t>(i) * n_bt, lnz_s_err + static_cast<size_t>(i + 1) * n_bt, 0.0);
@@ -329,12 +334,14 @@ int batched_sweep(const ftlm_params* p, int R, int M, unsigned seed, const doubl
 
 }  // namespace
 
-int ftlm_gpu_batched_release(void) {
+int ftlm_gpu_batched_release(void) try {
   std::lock_guard<std::mutex> lock(g_bt_mu);
   g_bt.release();
   g_grad.release();
   pool_trim();
   return FTLM_OK;
+} catch (...) {
+  return caught();
 }
 
 }  // extern "C"

@@ -362,7 +362,7 @@ int grad_one(ftlm_sector* s, ftlm_sector* op, double bT, int R, int M, unsigned 
 extern "C" {
 
 int ftlm_gpu_grad_sector(ftlm_sector* s, ftlm_sector* op_tp, double bT, int R, int M, unsigned seed, int method,
-                         int start_mode, double* lnz, double* dlnz) {
+                         int start_mode, double* lnz, double* dlnz) try {
   int rc = need_device(s);
   if (rc) return rc;
   if (op_tp) {
@@ -383,6 +383,8 @@ int ftlm_gpu_grad_sector(ftlm_sector* s, ftlm_sector* op_tp, double bT, int R, i
   if (rc) return rc;
   sector_gradient(cg, s->plan.dim, bT, op_tp != nullptr, lnz, dlnz);
   return FTLM_OK;
+} catch (...) {
+  return caught();
 }
 
 // ---- differentiable grand-canonical ln Z at one (T, mu) ----------------------------------------
@@ -435,7 +437,7 @@ double gc_lse(const std::vector<double>& x) {
 }  // namespace
 
 int ftlm_gpu_gc_logz(const ftlm_params* p, double mu, double bT, int R, int M, unsigned seed, int method,
-                     int start_mode, double* lnz_s, double* e_s, double* lnz_gc) {
+                     int start_mode, double* lnz_s, double* e_s, double* lnz_gc) try {
   int rc = gc_check(p, bT, R, M, method, start_mode);
   if (rc) return rc;
   if (!lnz_s || !e_s || !lnz_gc) return fail(FTLM_ERR_INVALID, "null output");
@@ -509,10 +511,12 @@ int ftlm_gpu_gc_logz(const ftlm_params* p, double mu, double bT, int R, int M, u
     }
   *lnz_gc = gc_lse(x);
   return FTLM_OK;
+} catch (...) {
+  return caught();
 }
 
 int ftlm_gpu_gc_logz_grad(const ftlm_params* p, double mu, double bT, int R, int M, unsigned seed, int method,
-                          int start_mode, const double* lnz_s, const double* e_s, double* grad) {
+                          int start_mode, const double* lnz_s, const double* e_s, double* grad) try {
   int rc = gc_check(p, bT, R, M, method, start_mode);
   if (rc) return rc;
   if (!lnz_s || !e_s || !grad) return fail(FTLM_ERR_INVALID, "null argument");
@@ -595,13 +599,15 @@ int ftlm_gpu_gc_logz_grad(const ftlm_params* p, double mu, double bT, int R, int
   grad[3] = dmu;
   grad[4] = dbeta;
   return FTLM_OK;
+} catch (...) {
+  return caught();
 }
 
 // Per-chain log quadrature and energy ratio with a converged eigen-decomposition (implicit QL
 // on the GPU, symeig.cu), the quadrature the gradient differentiates; same layout as
 // ftlm_gpu_tridiag_quadrature.
 int ftlm_gpu_tridiag_quadrature_exact(const double* alpha, const double* beta, const int* n, int nc, int ld,
-                                      const double* bts, int n_bt, double* logq, double* energy) {
+                                      const double* bts, int n_bt, double* logq, double* energy) try {
   if (nc < 0 || ld <= 0 || n_bt < 0 || !alpha || !beta || !n || (n_bt > 0 && (!bts || !logq || !energy)))
     return fail(FTLM_ERR_INVALID, "bad arguments");
   if (ld > kMaxEig) return fail(FTLM_ERR_UNSUPPORTED, "tridiagonal size > 160 is not supported by the GPU eigen-solver");
@@ -632,23 +638,29 @@ int ftlm_gpu_tridiag_quadrature_exact(const double* alpha, const double* beta, c
   CU_TRY(cudaMemcpy(energy, mem.at<void>(o_de), outb, cudaMemcpyDeviceToHost));
   mem.idle();
   return FTLM_OK;
+} catch (...) {
+  return caught();
 }
 
 // Host-only helper exposed for tests: eigenvalues/eigenvectors of a symmetric tridiagonal.
-int ftlm_gpu_tridiag_eigvec(const double* alpha, const double* beta, int n, double* lam, double* Z) {
+int ftlm_gpu_tridiag_eigvec(const double* alpha, const double* beta, int n, double* lam, double* Z) try {
   if (n < 0 || (n > 0 && (!alpha || !lam || !Z || (n > 1 && !beta)))) return fail(FTLM_ERR_INVALID, "bad arguments");
   const std::string err = tridiag_eigvec(n, alpha, beta, lam, Z);
   if (!err.empty()) return fail(FTLM_ERR_NUMERIC, err);
   return FTLM_OK;
+} catch (...) {
+  return caught();
 }
 
 // Host-only helper exposed for tests: the Duhamel weight matrix of one tridiagonal.
 int ftlm_gpu_duhamel_weights(const double* alpha, const double* beta, int n, double bT, double* K, double* g,
-                             double* lam_min) {
+                             double* lam_min) try {
   if (n < 0 || (n > 0 && (!alpha || !K || !g || (n > 1 && !beta)))) return fail(FTLM_ERR_INVALID, "bad arguments");
   const std::string err = duhamel_weights(n, alpha, beta, bT, K, g, lam_min);
   if (!err.empty()) return fail(FTLM_ERR_NUMERIC, err);
   return FTLM_OK;
+} catch (...) {
+  return caught();
 }
 
 }  // extern "C"

@@ -33,6 +33,8 @@ namespace capi {
 
 // Records msg for ftlm_gpu_last_error() (per host thread) and returns code.
 int fail(int code, const std::string& msg);
+// The error code of the exception in flight (in a handler): no exception crosses the C ABI.
+int caught() noexcept;
 
 #define CU_TRY(expr)                                                                                     \
   do {                                                                                                   \
@@ -284,6 +286,16 @@ namespace ftlm_b200 {
 namespace capi {
 
 int need_device(const ftlm_sector* s);
+// Sectors that go with the scope.
+struct OwnedSectors {
+  std::vector<ftlm_sector*> v;
+  OwnedSectors() = default;
+  OwnedSectors(const OwnedSectors&) = delete;
+  OwnedSectors& operator=(const OwnedSectors&) = delete;
+  ~OwnedSectors() {
+    for (ftlm_sector* s : v) delete s;
+  }
+};
 // ftlm_gpu_sector_create, with the tables that a sweep's sectors share (parts may be null).
 int sector_create(const ftlm_params* p, int n_up, int n_dn, PlanParts* parts, ftlm_sector** out);
 

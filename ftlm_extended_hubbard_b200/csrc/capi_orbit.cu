@@ -262,8 +262,10 @@ int orbit_apply_dev(ftlm_orbit* o, const double2* x, double2* y, cudaStream_t st
 
 extern "C" {
 
-int ftlm_gpu_orbit_create(ftlm_sector* s, int kx, int ky, ftlm_orbit** out) {
+int ftlm_gpu_orbit_create(ftlm_sector* s, int kx, int ky, ftlm_orbit** out) try {
   return ftlm_gpu_orbit_create_ex(s, kx, ky, 1e-12, out);
+} catch (...) {
+  return caught();
 }
 
 int ftlm_gpu_sector_set_lattice(ftlm_sector* s, int Lx, int Ly) {
@@ -276,7 +278,7 @@ int ftlm_gpu_sector_set_lattice(ftlm_sector* s, int Lx, int Ly) {
   return FTLM_OK;
 }
 
-int ftlm_gpu_orbit_create_ex(ftlm_sector* s, int kx, int ky, double survive_tol, ftlm_orbit** out) {
+int ftlm_gpu_orbit_create_ex(ftlm_sector* s, int kx, int ky, double survive_tol, ftlm_orbit** out) try {
   int rc = need_device(s);
   if (rc) return rc;
   if (!out) return fail(FTLM_ERR_INVALID, "null output");
@@ -381,6 +383,8 @@ int ftlm_gpu_orbit_create_ex(ftlm_sector* s, int kx, int ky, double survive_tol,
   }
   *out = o.release();
   return FTLM_OK;
+} catch (...) {
+  return caught();
 }
 
 int ftlm_gpu_orbit_destroy(ftlm_orbit* o) {
@@ -449,7 +453,7 @@ int ftlm_gpu_orbit_apply_host(ftlm_orbit* o, const double* x, double* y) {
 }
 
 int ftlm_gpu_orbit_ftlm(ftlm_orbit* o, const double* bts, int n_bt, int R, int M, unsigned seed, int start_mode,
-                        double* lnz, double* energy) {
+                        double* lnz, double* energy) try {
   if (!o) return fail(FTLM_ERR_INVALID, "null orbit");
   if (n_bt < 0 || (n_bt > 0 && (!bts || !lnz || !energy))) return fail(FTLM_ERR_INVALID, "bad arguments");
   R = std::max(1, R);
@@ -491,12 +495,14 @@ int ftlm_gpu_orbit_ftlm(ftlm_orbit* o, const double* bts, int n_bt, int R, int M
                             plain_quadrature_converged());
   if (rc) return rc;
   return ftlm_gpu_ftlm_combine(lq.data(), eq.data(), nv.data(), R, n_bt, std::log(static_cast<double>(dk)), lnz, energy);
+} catch (...) {
+  return caught();
 }
 
 // Batched complex64 FTLM of one block: 32-chain blocks of bt_orbit_step (Philox starts, as the
 // sector path); blocks with dim <= 2M use the complex128 Philox path.
 int ftlm_gpu_orbit_batched_ftlm(ftlm_orbit* o, const double* bts, int n_bt, int R, int M, unsigned seed, double* lnz,
-                                double* energy) {
+                                double* energy) try {
   if (!o) return fail(FTLM_ERR_INVALID, "null orbit");
   if (n_bt < 0 || (n_bt > 0 && (!bts || !lnz || !energy))) return fail(FTLM_ERR_INVALID, "bad arguments");
   R = std::max(1, R);
@@ -521,6 +527,8 @@ int ftlm_gpu_orbit_batched_ftlm(ftlm_orbit* o, const double* bts, int n_bt, int 
   rc = chain_quadrature(A.data(), B.data(), used.data(), R, M, bts, n_bt, lq.data(), eq.data(), true);
   if (rc) return rc;
   return ftlm_gpu_ftlm_combine(lq.data(), eq.data(), used.data(), R, n_bt, std::log(static_cast<double>(dk)), lnz, energy);
+} catch (...) {
+  return caught();
 }
 
 // Exact ln Tr e^{-bT H_K} of a small block (the k-bench's exact_log_partition_small_complex,
@@ -628,14 +636,18 @@ static int orbit_sector_impl(ftlm_sector* s, const double* bts, int n_bt, int R,
 
 int ftlm_gpu_orbit_sector_ftlm(ftlm_sector* s, const double* bts, int n_bt, int R, int M, unsigned seed,
                                int sector_index, int start_mode, int ed_cutoff, double* lnz, double* energy,
-                               long long* dims_k) {
+                               long long* dims_k) try {
   return orbit_sector_impl(s, bts, n_bt, R, M, seed, sector_index, start_mode, ed_cutoff, false, lnz, energy, dims_k);
+} catch (...) {
+  return caught();
 }
 
 int ftlm_gpu_orbit_sector_batched_ftlm(ftlm_sector* s, const double* bts, int n_bt, int R, int M, unsigned seed,
-                                       int sector_index, int ed_cutoff, double* lnz, double* energy, long long* dims_k) {
+                                       int sector_index, int ed_cutoff, double* lnz, double* energy, long long* dims_k) try {
   return orbit_sector_impl(s, bts, n_bt, R, M, seed, sector_index, FTLM_START_PHILOX, ed_cutoff, true, lnz, energy,
                            dims_k);
+} catch (...) {
+  return caught();
 }
 
 }  // extern "C"

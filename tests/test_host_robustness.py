@@ -77,3 +77,25 @@ def test_plan_without_a_further_thread():
     r = subprocess.run([sys.executable, "-c", _NO_THREADS], capture_output=True, text=True, timeout=300, preexec_fn=stack,
                        cwd=os.path.dirname(HERE))
     assert r.returncode == 0, r.stderr
+
+
+_NO_MEMORY = '''
+import resource
+import numpy as np
+from ftlm_extended_hubbard_b200 import _lib
+n = 40000  # the n x n matrices take 13 GB
+a, lam, z = np.ones(n), np.empty(n), np.empty(1)
+with open("/proc/self/statm") as f:
+    size = int(f.read().split()[0]) * resource.getpagesize()
+resource.setrlimit(resource.RLIMIT_AS, (size + (1 << 30),) * 2)
+p = [v.ctypes.data for v in (a, a, lam, z)]
+L = _lib.lib()
+assert L.ftlm_gpu_duhamel_weights(p[0], p[1], n, 1.0, p[2], p[2], p[2]) == 3
+assert b"allocation" in L.ftlm_gpu_last_error()
+'''
+
+
+def test_no_exception_crosses_the_c_interface():
+    """Host memory that does not suffice is an error code (3)."""
+    r = subprocess.run([sys.executable, "-c", _NO_MEMORY], capture_output=True, text=True, timeout=300, cwd=os.path.dirname(HERE))
+    assert r.returncode == 0, r.stderr

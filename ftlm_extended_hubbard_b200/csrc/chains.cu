@@ -20,6 +20,7 @@
 #include <algorithm>
 
 #include "chains.cuh"
+#include "launch.cuh"
 #include "philox.cuh"
 #include "planes_dev.cuh"
 
@@ -27,7 +28,7 @@ namespace ftlm_b200 {
 
 namespace {
 
-constexpr size_t kMaxSmem = 227 * 1024;
+constexpr size_t kMaxSmem = 227 * 1024, kOwnSmem = 2048;  // of which the reductions' own
 
 // Totals of NV doubles over the block, in every thread.
 template <int NV>
@@ -300,7 +301,7 @@ size_t chain_smem_bytes(const DevSector& S, bool c64, bool phase, int rows) {
 }
 
 int chain_rows(const DevSector& S, bool c64, bool phase) {
-  const size_t most = kMaxSmem - 2048;  // 2048: the reductions' own
+  const size_t most = kMaxSmem - kOwnSmem;
   if (chain_smem_bytes(S, c64, phase, static_cast<int>(S.Du)) <= most) return static_cast<int>(S.Du);
   const size_t base = chain_smem_bytes(S, c64, phase, 0), line = static_cast<size_t>(S.Dd + 8) * 16;
   if (base + line > most) return 0;
@@ -321,7 +322,7 @@ cudaError_t launch(const ChainLaunch& L, cudaStream_t st) {
                                 chains_kernel<P, 256, true, true, false>,    chains_kernel<P, 256, true, true, true>};
   const int form = (L.phase ? 2 : 0) + (L.xor_real ? 1 : 0);
   const K k = kernels[form + (!L.smem ? 0 : kClassThreads[L.size] > 256 ? 4 : 8)];
-  const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(L.smem_bytes));
+  const cudaError_t e = allow_shared(k, L.smem_bytes, kOwnSmem);
   if (e != cudaSuccess) return e;
   k<<<L.blocks, kClassThreads[L.size], L.smem_bytes, st>>>(L.sectors, L.descs, L.M, static_cast<T*>(L.scratch), L.init, L.alpha,
                                                     L.beta, L.used, L.scale, static_cast<T*>(L.store));

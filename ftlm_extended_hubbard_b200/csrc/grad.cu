@@ -10,6 +10,7 @@
 #include <algorithm>
 
 #include "grad.cuh"
+#include "launch.cuh"
 
 namespace ftlm_b200 {
 
@@ -162,8 +163,7 @@ cudaError_t launch(const DevSector& S, const T* W, const T* AW, int64_t vstride,
   while (E > 32 && (bytes(E) > static_cast<size_t>(optin) || E / 2 >= S.dim)) E /= 2;
   const size_t smem = bytes(E);
   if (n <= 0 || smem > static_cast<size_t>(optin)) return cudaErrorInvalidValue;
-  cudaError_t e = cudaFuncSetAttribute(moments_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       static_cast<int>(smem));
+  const cudaError_t e = allow_shared(moments_kernel<T>, smem);
   if (e != cudaSuccess) return e;
   const int64_t nch = (S.dim + E - 1) / E;
   const int per_sm = std::max(1, std::min(static_cast<int>(static_cast<size_t>(optin) / smem), 2048 / E));

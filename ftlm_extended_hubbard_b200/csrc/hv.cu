@@ -565,7 +565,7 @@ cudaError_t hv_launch_once(const DevSector& S, const double2* x, double2* y, cud
   const size_t sm = hv_rows_smem_bytes(S);
   const RowsKernel k = S.dn_g.phase ? (S.dn_g.xor_real ? hv_once_kernel<true, true> : hv_once_kernel<true, false>)
                                     : (S.dn_g.xor_real ? hv_once_kernel<false, true> : hv_once_kernel<false, false>);
-  const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sm));
+  const cudaError_t e = allow_shared(k, sm, kOnceListBytes);
   if (e != cudaSuccess) return e;
   int threads = kOnceThreads;
   while (threads > 64 && (threads / 2 >= S.Dd || (threads > 256 && S.Du > g_num_sms))) threads /= 2;
@@ -581,7 +581,7 @@ cudaError_t hv_launch_pass(const DevSector& S, const double2* x, double2* y, int
     const size_t sm = hv_rows_smem_bytes(S);
     const bool early = early_ok(S.dim, st);
     const RowsKernel k = early ? rows_kernel_of<true>(S) : rows_kernel_of<false>(S);
-    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sm));
+    const cudaError_t e = allow_shared(k, sm);
     if (e != cudaSuccess) return e;
     // Blocks as wide as a row needs, several on an SM where their rows fit: one block's staging overlaps another's hops.
     // Up to eight rows an SM run as one wave, the threads shared out among them.

@@ -1,3 +1,5 @@
+// Launches: the shared memory a kernel may use, and kernels without the gap of a launch between them.
+//
 // Kernels that follow one another on a stream without the gap of a launch (programmatic dependent launch).  A kernel
 // that starts with x = follow<true>(x) may be launched with early = true: its blocks are then placed while the kernel
 // before it drains, and wait in follow() until that kernel has ended and its writes are visible, so the order of all
@@ -12,6 +14,16 @@
 #include <cstdint>
 
 namespace ftlm_b200 {
+
+// Allows a kernel `bytes` of dynamic shared memory, beside `own` of its static.  The limit is a property of the kernel that
+// all threads share, so it is always set to the same value, the most there is: a call that set it to its own size could
+// lower it between another thread's call and launch.
+constexpr size_t kBlockShared = 227 * 1024;
+template <class K>
+cudaError_t allow_shared(K kernel, size_t bytes, size_t own = 0) {
+  if (bytes + own > kBlockShared) return cudaErrorInvalidValue;
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kBlockShared - own));
+}
 
 constexpr int64_t kEarlyStates = int64_t(1) << 21;  // 16-byte elements of a vector: 32 MB
 

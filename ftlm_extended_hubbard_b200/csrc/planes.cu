@@ -18,6 +18,7 @@
 
 #include "batched.cuh"
 #include "device.cuh"
+#include "launch.cuh"
 #include "philox.cuh"
 #include "planes.cuh"
 #include "planes_dev.cuh"
@@ -463,7 +464,7 @@ cudaError_t launch_rows_p(const DevSector& S, const typename P::T* W, typename P
                           int* flag, cudaStream_t s) {
   const auto k = rows_kernel<P, kP, kPhase, kXor>;
   const size_t sm = static_cast<size_t>(kP) * (S.Dd + 8) * 16 + (kPhase ? 0 : S.dn_g.nt * 8 * sizeof(typename P::Cf));
-  const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sm));
+  const cudaError_t e = allow_shared(k, sm);
   if (e != cudaSuccess) return e;
   const int per_smem = std::max<int>(1, static_cast<int>((kMaxSmem + 1024) / (sm + 1024)));
   int threads = 1024;

@@ -13,6 +13,7 @@
 #include <math_constants.h>
 
 #include "hv.cuh"
+#include "launch.cuh"
 
 namespace ftlm_b200 {
 
@@ -410,7 +411,7 @@ cudaError_t quad_jacobi(const double* alpha, const double* beta, const int* n, i
                                          jacobi_kernel<5>};
   const K k = kernels[(ld - 1) / 32];
   const size_t sm = (static_cast<size_t>(ld) * (ld - 1) / 2 + 2 * static_cast<size_t>(ld)) * sizeof(double);
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sm));
+  const cudaError_t e = allow_shared(k, sm);
   if (e != cudaSuccess) return e;
   k<<<nc, 32, sm, st>>>(alpha, beta, n, ld, max_rot, tol, lam, w0, bad);
   return cudaGetLastError();

@@ -20,6 +20,7 @@
 // k-resolved path (reference benchmarks/bench_ftlm_nmu_4x4_k.cpp:249-336 restated).
 #include <cfloat>
 
+#include "launch.cuh"
 #include "symeig.cuh"
 
 namespace ftlm_b200 {
@@ -27,6 +28,7 @@ namespace ftlm_b200 {
 namespace {
 
 constexpr int kEigThreads = 256;
+constexpr size_t kEigOwn = 2560;  // static shared memory of the kernels here, at most
 
 // Pair k of round r of the circle method for m (even) players: player m-1 is fixed.
 __device__ __forceinline__ void rr_pair(int r, int k, int m, int* p, int* q) {
@@ -461,8 +463,7 @@ cudaError_t symeig_tridiag(const double* alpha, const double* beta, const int* n
   if (vt) {
     const int threads = (ld + 31) / 32 * 32;
     const size_t sm = (static_cast<size_t>(2) * ld * (threads / 32) + static_cast<size_t>(ld) * threads) * sizeof(double);
-    const cudaError_t e = cudaFuncSetAttribute(tql_vectors_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               static_cast<int>(sm));
+    const cudaError_t e = allow_shared(tql_vectors_kernel, sm);
     if (e != cudaSuccess) return e;
     tql_vectors_kernel<<<nm, threads, sm, st>>>(alpha, beta, n, ld, lam, vt, info);
   } else {
@@ -477,7 +478,7 @@ cudaError_t symeig_dense(const double* A, const int* n, int nm, int ld, double* 
   if (ld > kMaxEig || ld <= 0) return cudaErrorInvalidValue;
   const int m = ld + (ld & 1);
   const size_t sm = (static_cast<size_t>(m) * (m + 1) + m) * sizeof(double);
-  cudaError_t e = cudaFuncSetAttribute(symeig_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sm));
+  const cudaError_t e = allow_shared(symeig_kernel, sm, kEigOwn);
   if (e != cudaSuccess) return e;
   symeig_kernel<<<nm, kEigThreads, sm, st>>>(A, n, ld, lam, info);
   return cudaGetLastError();
@@ -487,7 +488,7 @@ cudaError_t duhamel_weights_dev(const double* lam, const double* vt, const int* 
                                 const double* scale, double* Y, double* Kp, double* g, double* lmin, cudaStream_t st) {
   if (nc <= 0) return cudaSuccess;
   const size_t sm = static_cast<size_t>(ld) * ld * sizeof(double);
-  const cudaError_t e = cudaFuncSetAttribute(duhamel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sm));
+  const cudaError_t e = allow_shared(duhamel_kernel, sm, kEigOwn);
   if (e != cudaSuccess) return e;
   duhamel_kernel<<<nc, kDuhThreads, sm, st>>>(lam, vt, n, ld, bT, scale, Y, Kp, g, lmin);
   return cudaGetLastError();

@@ -165,3 +165,36 @@ def test_handle_goes_while_its_call_is_in_flight(gpu):
             s.close()
         torch.cuda.synchronize()
         assert torch.equal(out[0], ref[0]) and torch.equal(out[1], ref[1])
+
+
+@pytest.mark.parametrize("path", [0, 3])
+def test_threads_on_handles_of_different_sizes(gpu, path):
+    """Two threads, each with a handle and a stream of its own and rows of 70 and 4,368 (one pass) or 924 and 11,440 strings
+    (two passes): no call of one takes the shared memory that the other's kernel needs."""
+    import threading
+    torch = gpu
+    shapes = [((4, 2), 4, 4), ((4, 4), 0, 5)] if path == 0 else [((4, 3), 6, 6), ((4, 4), 2, 7)]
+    out, errors = [], []
+
+    def work(lat, nu, nd):
+        s = F.Sector(F.HubbardParams(*lat, 1.0, -0.25, 8.0, 1.0), nu, nd)
+        s.set_apply_path(path)
+        st = torch.cuda.Stream()
+        with torch.cuda.stream(st):
+            x = torch.randn(s.dim(), dtype=torch.complex128, device="cuda")
+            y, ref = torch.empty_like(x), torch.empty_like(x)
+            s.apply(x, ref, st.cuda_stream)
+            try:
+                for _ in range(4000):
+                    s.apply(x, y, st.cuda_stream)
+            except F.FtlmError as e:
+                errors.append(e)
+            st.synchronize()
+            out.append(torch.equal(y, ref))
+
+    pool = [threading.Thread(target=work, args=c) for c in shapes]
+    for t in pool:
+        t.start()
+    for t in pool:
+        t.join()
+    assert not errors and out == [True, True]

@@ -401,6 +401,7 @@ int ftlm_gpu_sector_diag(const ftlm_sector* s, long long index, double* value) {
 int ftlm_gpu_set_apply_path(ftlm_sector* s, int path) {
   if (!s || path < 0 || path > 3) return fail(FTLM_ERR_INVALID, "bad path");
   s->apply_path = path;
+  s->pinned = path != 0;
   s->use_once = path == 0;
   return FTLM_OK;
 }
@@ -477,7 +478,7 @@ int ftlm_b200::capi::planes_lanczos(ftlm_sector* s, int R, int M, unsigned seed,
   B->assign(static_cast<size_t>(R) * M, 0.0);
   used->assign(static_cast<size_t>(R), 0);
   const int64_t dim = s->plan.dim;
-  const DevSector& S = s->dev;
+  const DevSector S = s->planes_dev();
   cudaStream_t st = s->stream;
   BtWs& ws = s->planes;
   const int group = pl_group(S, false, std::min(R, kBtChains));
@@ -539,7 +540,7 @@ int ftlm_gpu_lanczos(ftlm_sector* s, int max_steps, unsigned seed, int start_mod
   int rc = need_device(s);
   if (rc) return rc;
   std::vector<double> a, b;
-  if (s->apply_path == 0 && fused_alone(s->dev) && max_steps > 0) {
+  if (s->chains() == ftlm_sector::Chains::fused && max_steps > 0) {
     // few states: all steps in one kernel
     ChainRun run;
     rc = chains_run({s}, 1, max_steps, seed, start_mode, false, &run);
@@ -551,7 +552,7 @@ int ftlm_gpu_lanczos(ftlm_sector* s, int max_steps, unsigned seed, int start_mod
     CU_TRY(cudaMemcpy(a.data(), run.alpha, a.size() * sizeof(double), cudaMemcpyDeviceToHost));
     CU_TRY(cudaMemcpy(b.data(), run.beta, b.size() * sizeof(double), cudaMemcpyDeviceToHost));
     trim_chain(n, &a, &b);
-  } else if (s->apply_path != 1 && max_steps > 0 && pl_fits(s->dev, s->plan.max_up_deg)) {
+  } else if (s->chains() == ftlm_sector::Chains::planes && max_steps > 0) {
     std::vector<int> u;
     rc = planes_lanczos(s, 1, max_steps, seed, start_mode, &a, &b, &u);
     if (rc) return rc;
@@ -789,11 +790,11 @@ int plain_sector_ftlm(ftlm_sector* s, const double* bts, int n_bt, int R, int M,
     }
     return FTLM_OK;
   }
-  if (s->apply_path == 0 && fused_alone(s->dev))
+  if (s->chains() == ftlm_sector::Chains::fused)
     return chains_ftlm({s}, R, M, seed, start_mode, false, bts, n_bt, converged, lnz, energy);
   std::vector<double> A(static_cast<size_t>(R) * M, 0.0), B(static_cast<size_t>(R) * M, 0.0);
   std::vector<int> nv(static_cast<size_t>(R), 0);
-  if (s->apply_path != 1 && pl_fits(s->dev, s->plan.max_up_deg)) {
+  if (s->chains() == ftlm_sector::Chains::planes) {
     rc = planes_lanczos(s, R, M, seed, start_mode, &A, &B, &nv);
     if (rc) return rc;
   } else {
@@ -940,6 +941,7 @@ int ftlm_gpu_lanczos_sectors(ftlm_sector* const* secs, int n_sectors, int R, int
 int ftlm_gpu_set_cols_variant(ftlm_sector* s, int variant) {
   if (!s || variant < 0 || variant > 5) return fail(FTLM_ERR_INVALID, "cols variant must be in [0, 6)");
   s->cols_variant = variant;
+  s->cols_chosen = true;
   return FTLM_OK;
 }
 
@@ -955,6 +957,13 @@ int ftlm_gpu_autotune_apply(ftlm_sector* s, int reps, int* path, int* cols_varia
     bool once;
   };
   static std::map<std::string, Choice> cache;
+  auto take = [s](const Choice& c) {
+    s->apply_path = c.path;
+    s->cols_variant = c.variant;
+    s->use_once = c.once;
+    s->pinned = false;
+    s->cols_chosen = c.path >= 2 && !c.once;  // else no slab was timed
+  };
   char key[160];
   std::snprintf(key, sizeof(key), "%d/%d/%d/%zu/%zu/%d/%d", P.n, P.nu, P.nd, P.hu.size(), P.hd.size(), P.max_up_deg,
                 P.max_dn_deg);
@@ -962,9 +971,7 @@ int ftlm_gpu_autotune_apply(ftlm_sector* s, int reps, int* path, int* cols_varia
     std::lock_guard<std::mutex> lock(mu);
     auto it = cache.find(key);
     if (it != cache.end()) {
-      s->apply_path = it->second.path;
-      s->cols_variant = it->second.variant;
-      s->use_once = it->second.once;
+      take(it->second);
       if (path) *path = s->apply_path;
       if (cols_variant) *cols_variant = s->cols_variant;
       if (ms) *ms = -1.0f;
@@ -1018,9 +1025,7 @@ int ftlm_gpu_autotune_apply(ftlm_sector* s, int reps, int* path, int* cols_varia
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   CU_TRY(ce);
-  s->apply_path = best_p;
-  s->cols_variant = best_v;
-  s->use_once = best_once;
+  take(Choice{best_p, best_v, best_once});
   {
     std::lock_guard<std::mutex> lock(mu);
     cache[key] = Choice{best_p, best_v, best_once};

@@ -232,6 +232,7 @@ struct ftlm_sector {
   size_t tables_bytes = 0;
   ftlm_b200::capi::BtWs planes;  // vectors and scalars of its complex128 Lanczos chains
   int apply_path = 0;    // 0 auto, 1 generic, 2 rows+cols, 3 rows (register coefficient classes)+cols
+  bool pinned = false;   // apply_path comes from ftlm_gpu_set_apply_path: the chains keep to it too
   bool use_once = true;  // H v in one pass where it can be (until a path is set)
   int cols_variant = 0;  // column slab 256/128/512 (0/1/2); 3/4/5: the same over the packed up list (path 3)
   ftlm_b200::capi::LanczosWs ws;
@@ -268,6 +269,16 @@ struct ftlm_sector {
     return d;
   }
   bool once() const { return use_once && ftlm_b200::hv_once_ok(dev, plan.max_up_deg); }
+  bool cols_chosen = false;  // cols_variant was set or timed: the slab of the complex128 chains on planes, too
+  // How complex128 chains run: all steps in one kernel, on planes (gauge row pass + column slabs, so also where path 3 is
+  // pinned), or step by step on apply().
+  enum class Chains { fused, planes, steps };
+  Chains chains() const;
+  ftlm_b200::DevSector planes_dev() const {
+    ftlm_b200::DevSector d = dev;
+    if (cols_chosen) d.bt_cols = cols_variant % 3;
+    return d;
+  }
   int apply(const double2* x, double2* y, cudaStream_t st) {
     if (once()) {
       CU_TRY(ftlm_b200::hv_launch_once(dev, x, y, st));
@@ -426,6 +437,18 @@ inline bool fused_alone(const DevSector& S) {  // and a row of it fits (chain_ro
   const int64_t lanes = S.Dd <= 16 ? S.Du / (32 / S.Dd) * 32 : S.Du * ((S.Dd + 31) / 32 * 32);
   return lanes <= 8192 && chain_rows(S, false, false) > 0;
 }
+}  // namespace capi
+}  // namespace ftlm_b200
+
+inline ftlm_sector::Chains ftlm_sector::chains() const {
+  if (!pinned && ftlm_b200::capi::fused_alone(dev)) return Chains::fused;
+  if ((!pinned || effective_path() == 3) && ftlm_b200::pl_fits(dev, plan.max_up_deg)) return Chains::planes;
+  return Chains::steps;
+}
+
+namespace ftlm_b200 {
+namespace capi {
+
 // Largest sector that joins the fused launch of a sweep; a larger one fills the GPU by itself.
 constexpr int64_t kFusedSweepMax = 1 << 14;
 

@@ -198,3 +198,30 @@ def test_threads_on_handles_of_different_sizes(gpu, path):
     for t in pool:
         t.join()
     assert not errors and out == [True, True]
+
+
+@pytest.mark.parametrize("lat,nu,nd", [((3, 3), 4, 4), ((4, 2), 4, 4), ((4, 3), 4, 5)])
+def test_chains_of_a_tuned_handle(gpu, lat, nu, nd):
+    """Timing the H v variants leaves a small sector's chains in their fused kernel (the bits of an untuned handle) and a
+    larger one's on planes, with the timed column slab (the dot products' order)."""
+    p = F.HubbardParams(*lat, 1.0, -0.25, 8.0, 1.0, 0.1, 0.0)
+    s, t = F.Sector(p, nu, nd), F.Sector(p, nu, nd)
+    t.autotune(2)
+    a, b = s.lanczos(12, 5, start="philox"), t.lanczos(12, 5, start="philox")
+    if s.dim() < 20000:
+        assert all(np.array_equal(x, y) for x, y in zip(a[:2], b[:2]))
+        assert np.array_equal(s.ftlm([0.5, 2.0], 3, 20, 5, start="philox")[0], t.ftlm([0.5, 2.0], 3, 20, 5, start="philox")[0])
+    else:  # rounding grows by about two a step
+        assert np.abs(a[0] - b[0]).max() <= 1e-11 * np.abs(a[0]).max()
+
+
+def test_chains_keep_to_a_set_path(gpu):
+    """A handle set to path 2 runs its chains on that path: the bits of the general recurrence on its own apply."""
+    torch = gpu
+    s = F.Sector(F.HubbardParams(4, 3, 1.0, -0.25, 8.0, 1.0), 4, 4)
+    n = s.dim()
+    for path in (1, 2):
+        s.set_apply_path(path)
+        a, b, _ = s.lanczos(8, 5, start="philox")
+        a2, b2 = F.lanczos_tridiagonal(n, lambda x, y: s.apply(x, y), 8, 5, start="philox")[:2]
+        assert np.array_equal(a, a2) and np.array_equal(b, b2)

@@ -186,7 +186,7 @@ __global__ void __launch_bounds__(kScalarThreads) bt_scalar_kernel(const double*
                                                                    int mode, int k, double* __restrict__ st,
                                                                    double* __restrict__ alpha, double* __restrict__ beta,
                                                                    int* __restrict__ used, int* __restrict__ clear,
-                                                                   bool scaled) {
+                                                                   int* __restrict__ live, bool scaled) {
   const int chain = blockIdx.x;
   if (mode == 1) {
     double z[2];
@@ -210,6 +210,7 @@ __global__ void __launch_bounds__(kScalarThreads) bt_scalar_kernel(const double*
     st[kBtSin * 32 + chain] = (n0 < 1e-18) ? 0.0 : 1.0 / n0;
     st[kBtC2 * 32 + chain] = 0.0;
     st[kBtActive * 32 + chain] = (n0 < 1e-18) ? 0.0 : 1.0;
+    if (live && !(n0 < 1e-18)) atomicAdd(live, 1);
     used[chain] = 0;
     return;
   }
@@ -225,6 +226,7 @@ __global__ void __launch_bounds__(kScalarThreads) bt_scalar_kernel(const double*
     st[kBtActive * 32 + chain] = 0.0;
     st[kBtSin * 32 + chain] = 0.0;
     st[kBtC2 * 32 + chain] = 0.0;
+    if (live) atomicSub(live, 1);
     return;
   }
   const double b = sqrt(n2);
@@ -391,8 +393,8 @@ __global__ void __launch_bounds__(kBtThreads, kBtBlocksPerSm) bt_orbit_kernel(Or
 }  // namespace
 
 void bt_scalars(const double* partial, int nblocks, int mode, int k, int lanes, bool scaled, double* st, double* alpha,
-                double* beta, int* used, int* clear, cudaStream_t s) {
-  bt_scalar_kernel<<<lanes, kScalarThreads, 0, s>>>(partial, nblocks, mode, k, st, alpha, beta, used, clear, scaled);
+                double* beta, int* used, int* clear, int* live, cudaStream_t s) {
+  bt_scalar_kernel<<<lanes, kScalarThreads, 0, s>>>(partial, nblocks, mode, k, st, alpha, beta, used, clear, live, scaled);
 }
 
 cudaError_t bt_start(float2* W, int64_t dim, unsigned seed, double* st, double* partial, int* used, int* flags,
@@ -400,7 +402,7 @@ cudaError_t bt_start(float2* W, int64_t dim, unsigned seed, double* st, double* 
   cudaError_t e = cudaMemsetAsync(flags, 0, 2 * sizeof(int), s);
   if (e != cudaSuccess) return e;
   bt_start_kernel<<<kBtBlocks, kBtThreads, 0, s>>>(W, dim, seed, partial, flags);
-  bt_scalars(partial, kBtBlocks, 0, 0, 32, false, st, nullptr, nullptr, used, nullptr, s);
+  bt_scalars(partial, kBtBlocks, 0, 0, 32, false, st, nullptr, nullptr, used, nullptr, nullptr, s);
   return cudaGetLastError();
 }
 
@@ -410,9 +412,9 @@ cudaError_t bt_orbit_step(const OrbitApplyDev& A, const float2* Wk, const float2
   int* fin = flags + (k & 1);
   int* fout = flags + ((k + 1) & 1);
   bt_orbit_kernel<<<kBtBlocks, kBtThreads, 0, s>>>(A, Wk, Y, st, partial, fin);
-  bt_scalars(partial, kBtBlocks, 1, k, 32, false, st, alpha, beta, used, fout, s);
+  bt_scalars(partial, kBtBlocks, 1, k, 32, false, st, alpha, beta, used, fout, nullptr, s);
   bt_update_kernel<<<kBtBlocks, kBtThreads, 0, s>>>(Y, Wk, Wkm1, A.dk, st, k > 0, partial, fout);
-  bt_scalars(partial, kBtBlocks, 2, k, 32, false, st, alpha, beta, used, nullptr, s);
+  bt_scalars(partial, kBtBlocks, 2, k, 32, false, st, alpha, beta, used, nullptr, nullptr, s);
   return cudaGetLastError();
 }
 

@@ -35,9 +35,10 @@ __device__ __forceinline__ bool tinyf(float2 v) { return fmaf(v.x, v.x, v.y * v.
 
 // Totals of nblocks partial sums per chain (partial[(block * 32 + chain) * values]) and the recurrence's scalars for
 // the first `lanes` chains.  mode 0: start norms; 1: dot products, alpha_k; 2: norms, beta_k and breakdown.  scaled:
-// the dot products are of H q_k (complex128 chains) instead of H W_k.  clear (mode 1): set to 0.
+// the dot products are of H q_k (complex128 chains) instead of H W_k.  clear (mode 1): set to 0.  live (or null): counts the
+// chains that have not ended, from 0 before mode 0.
 void bt_scalars(const double* partial, int nblocks, int mode, int k, int lanes, bool scaled, double* st, double* alpha,
-                double* beta, int* used, int* clear, cudaStream_t s);
+                double* beta, int* used, int* clear, int* live, cudaStream_t s);
 
 // W <- complex64 Philox start vectors of the block's representatives (chain r: key seed + r*100003), norms -> scalar
 // state.  flags: 2 ints (tiny-entry flags of the current and next vector, cleared here).

@@ -230,7 +230,9 @@ int grad_planes(ftlm_sector* s, ftlm_sector* op, double bT, int R, int M, unsign
     CU_TRY(cudaMemcpyAsync(hb.data(), z.beta, tab * sizeof(double), cudaMemcpyDeviceToHost, st));
     CU_TRY(cudaMemcpyAsync(hu.data(), z.used, hu.size() * sizeof(int), cudaMemcpyDeviceToHost, st));
     CU_TRY(cudaStreamSynchronize(st));
-    if (op) CU_TRY(pl_apply(op->dev, Q, AQ, M * np, g_grad.flag.as<int>(), st));
+    int steps = 0;  // of the group's longest chain: no vector is written after it
+    for (int c = 0; c < nc; ++c) steps = std::max(steps, hu[static_cast<size_t>(c)]);
+    if (op && steps > 0) CU_TRY(pl_apply(op->dev, Q, AQ, steps * np, g_grad.flag.as<int>(), st));
     // chain-major tables: alpha, beta, norms of the stored vectors (W_0 = ||raw|| q_0, W_i = beta_{i-1} q_i)
     const size_t row = static_cast<size_t>(nc) * M;
     std::vector<double> t(3 * row, 0.0);

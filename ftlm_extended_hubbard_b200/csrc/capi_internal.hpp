@@ -187,7 +187,7 @@ struct BtWs {
     if (!st.p) {
       if ((e = partial.alloc(std::max<int64_t>(kBtPartialDoubles, kPlPartialDoubles) * sizeof(double))) != cudaSuccess) return e;
       if ((e = used.alloc(kBtChains * sizeof(int))) != cudaSuccess) return e;
-      if ((e = flags.alloc(2 * sizeof(int))) != cudaSuccess) return e;
+      if ((e = flags.alloc(kPlFlags * sizeof(int))) != cudaSuccess) return e;
       if ((e = st.alloc(kBtFields * kBtChains * sizeof(double))) != cudaSuccess) return e;
     }
     if (M > mcap) {

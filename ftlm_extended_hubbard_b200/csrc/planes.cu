@@ -32,6 +32,11 @@ constexpr int kMaxDeg = 128;       // up sources of a string
 constexpr int kStreamBlocks = 592; // start / update: blocks over all planes (4 per SM of 148, a multiple of 16)
 constexpr size_t kMaxSmem = 227 * 1024;
 
+// Whether every chain of the group has ended (live: the count of those that have not; null outside a chain).  The steps
+// that are still to come then cost their launches alone: a Hamiltonian with few levels ends all chains early, and the
+// host does not wait to learn of it.
+__device__ __forceinline__ bool all_ended(const int* live) { return live && *live == 0; }
+
 // Start vectors: given ones (in W already, in the sector's order), or chain c of the group uses Philox4x32-10 with key seed + c*100003 and counter = state index, the
 // stream of FTLM_START_PHILOX, rounded to the chains' type and expressed in the gauge basis (W = G r).
 template <class P>
@@ -88,8 +93,10 @@ __device__ __forceinline__ void prefetch_l2(const void* from, uint32_t bytes) {
 template <class P, int kP, bool kPhase, bool kXor>
 __global__ void __launch_bounds__(1024, 1) rows_kernel(DevSector S, const typename P::T* __restrict__ W,
                                                        typename P::T* __restrict__ Y, int planes,
-                                                       const double* __restrict__ st, int* __restrict__ flag) {
+                                                       const double* __restrict__ st, int* __restrict__ flag,
+                                                       const int* __restrict__ live) {
   using T = typename P::T;
+  if (all_ended(live)) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int Dd = static_cast<int>(S.Dd), Du = static_cast<int>(S.Du), nt = blockDim.x;
   const uint32_t line = static_cast<uint32_t>(Dd + 8) * 16u;
@@ -160,9 +167,11 @@ __global__ void __launch_bounds__(1024, 1) rows_kernel(DevSector S, const typena
 template <class P>
 __global__ void __launch_bounds__(kThreads) rows_gather_kernel(DevSector S, const typename P::T* __restrict__ W,
                                                                typename P::T* __restrict__ Y, int planes,
-                                                               const int* __restrict__ flag) {
+                                                               const int* __restrict__ flag,
+                                                               const int* __restrict__ live) {
   static_assert(!P::kScaled, "complex128 chains without the gauge table run on the H v kernels of hv.cu");
   using T = typename P::T;
+  if (all_ended(live)) return;
   const bool filter = *flag != 0;
   const int64_t total = S.dim * planes;
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * kThreads + threadIdx.x; i < total;
@@ -224,8 +233,9 @@ template <class P, int kT, bool kDot>
 __global__ void __launch_bounds__(kT, P::kColThreads / kT) cols_kernel(DevSector S, const typename P::T* __restrict__ W,
                                                              typename P::T* __restrict__ Y, int planes,
                                                              const double* __restrict__ st, double* __restrict__ partial,
-                                                             const int* __restrict__ flag) {
+                                                             const int* __restrict__ flag, const int* __restrict__ live) {
   using T = typename P::T;
+  if (all_ended(live)) return;
   constexpr int kPer = (kMaxDeg + kT - 1) / kT;  // list entries per thread
   __shared__ uint32_t s_off[2][kMaxDeg];
   __shared__ __align__(16) typename P::Cf s_cf[2][kMaxDeg];
@@ -314,8 +324,10 @@ __global__ void __launch_bounds__(kT, P::kColThreads / kT) cols_items_kernel(Dev
                                                                              typename P::T* __restrict__ Y, uint32_t per,
                                                                              const double* __restrict__ st,
                                                                              double* __restrict__ items,
-                                                                             const int* __restrict__ flag) {
+                                                                             const int* __restrict__ flag,
+                                                                             const int* __restrict__ live) {
   using T = typename P::T;
+  if (all_ended(live)) return;
   __shared__ uint32_t s_off[kMaxDeg];
   __shared__ __align__(16) typename P::Cf s_cf[kMaxDeg];
   __shared__ double sh[2 * P::kC * kT / 32];
@@ -388,8 +400,10 @@ __global__ void __launch_bounds__(kThreads, 4) update_kernel(typename P::T* __re
                                                              const typename P::T* __restrict__ Wk,
                                                              const typename P::T* __restrict__ Wkm1, int64_t dim, int nb,
                                                              const double* __restrict__ st, int use_prev,
-                                                             double* __restrict__ partial, int* __restrict__ flag) {
+                                                             double* __restrict__ partial, int* __restrict__ flag,
+                                                             const int* __restrict__ live) {
   using T = typename P::T;
+  if (all_ended(live)) return;
   __shared__ double sh[P::kC * kThreads / 32];
   const int plane = blockIdx.x / nb, b = blockIdx.x - plane * nb;
   double s_in[P::kC], c1r[P::kC], c1i[P::kC], c2[P::kC];
@@ -461,7 +475,7 @@ int row_planes(const DevSector& S) {
 // 1024-thread block leaves the SM idle while it stages, and most of its threads where a row is short).
 template <class P, int kP, bool kPhase, bool kXor>
 cudaError_t launch_rows_p(const DevSector& S, const typename P::T* W, typename P::T* Y, int planes, const double* st,
-                          int* flag, cudaStream_t s) {
+                          int* flag, const int* live, cudaStream_t s) {
   const auto k = rows_kernel<P, kP, kPhase, kXor>;
   const size_t sm = static_cast<size_t>(kP) * (S.Dd + 8) * 16 + (kPhase ? 0 : S.dn_g.nt * 8 * sizeof(typename P::Cf));
   const cudaError_t e = allow_shared(k, sm);
@@ -472,38 +486,38 @@ cudaError_t launch_rows_p(const DevSector& S, const typename P::T* W, typename P
   const int per_sm = std::max(1, std::min(per_smem, 1024 / threads));
   const int64_t items = S.Du * ((planes + kP - 1) / kP);
   const int grid = static_cast<int>(std::min<int64_t>(items, static_cast<int64_t>(sm_count()) * per_sm));
-  k<<<grid, threads, sm, s>>>(S, W, Y, planes, st, flag);
+  k<<<grid, threads, sm, s>>>(S, W, Y, planes, st, flag, live);
   return cudaGetLastError();
 }
 
 template <class P, int kP>
 cudaError_t launch_rows_n(const DevSector& S, const typename P::T* W, typename P::T* Y, int planes, const double* st,
-                          int* flag, cudaStream_t s) {
+                          int* flag, const int* live, cudaStream_t s) {
   if (S.dn_g.phase)
-    return S.dn_g.xor_real ? launch_rows_p<P, kP, true, true>(S, W, Y, planes, st, flag, s)
-                           : launch_rows_p<P, kP, true, false>(S, W, Y, planes, st, flag, s);
-  return S.dn_g.xor_real ? launch_rows_p<P, kP, false, true>(S, W, Y, planes, st, flag, s)
-                         : launch_rows_p<P, kP, false, false>(S, W, Y, planes, st, flag, s);
+    return S.dn_g.xor_real ? launch_rows_p<P, kP, true, true>(S, W, Y, planes, st, flag, live, s)
+                           : launch_rows_p<P, kP, true, false>(S, W, Y, planes, st, flag, live, s);
+  return S.dn_g.xor_real ? launch_rows_p<P, kP, false, true>(S, W, Y, planes, st, flag, live, s)
+                         : launch_rows_p<P, kP, false, false>(S, W, Y, planes, st, flag, live, s);
 }
 
 template <class P>
 cudaError_t launch_rows(const DevSector& S, const typename P::T* W, typename P::T* Y, int planes, const double* st,
-                        int* flag, cudaStream_t s) {
+                        int* flag, const int* live, cudaStream_t s) {
   const int rp = row_planes<P>(S);
-  if (rp == 2 && planes > 1) return launch_rows_n<P, 2>(S, W, Y, planes, st, flag, s);
-  if (rp > 0) return launch_rows_n<P, 1>(S, W, Y, planes, st, flag, s);
+  if (rp == 2 && planes > 1) return launch_rows_n<P, 2>(S, W, Y, planes, st, flag, live, s);
+  if (rp > 0) return launch_rows_n<P, 1>(S, W, Y, planes, st, flag, live, s);
   if constexpr (P::kScaled) {
     return cudaErrorNotSupported;  // pl_fits
   } else {
     const int64_t blocks = std::min<int64_t>((S.dim * planes + kThreads - 1) / kThreads, static_cast<int64_t>(sm_count()) * 16);
-    rows_gather_kernel<P><<<static_cast<unsigned>(blocks), kThreads, 0, s>>>(S, W, Y, planes, flag);
+    rows_gather_kernel<P><<<static_cast<unsigned>(blocks), kThreads, 0, s>>>(S, W, Y, planes, flag, live);
     return cudaGetLastError();
   }
 }
 
 template <class P, int kT>
 int launch_cols_t(const DevSector& S, const typename P::T* W, typename P::T* Y, int planes, const double* st,
-                  double* partial, double* items, const int* flag, cudaStream_t s) {
+                  double* partial, double* items, const int* flag, const int* live, cudaStream_t s) {
   const int64_t per = (S.Dd + 2 * kT - 1) / (2 * kT) * S.Du;
   const int64_t grid = std::min<int64_t>({per * planes, static_cast<int64_t>(sm_count()) * (P::kColThreads / kT), kPlMaxBlocks});
   // From 8 items of a plane for each block of the persistent grid, one block per item: 4x4 (6,6) complex128 2.19 -> 1.86 ms,
@@ -511,38 +525,38 @@ int launch_cols_t(const DevSector& S, const typename P::T* W, typename P::T* Y, 
   if (per >= 8 * grid) {
     const unsigned n = static_cast<unsigned>(per * planes);
     if (!partial) {
-      cols_items_kernel<P, kT, false><<<n, kT, 0, s>>>(S, W, Y, static_cast<uint32_t>(per), st, nullptr, flag);
+      cols_items_kernel<P, kT, false><<<n, kT, 0, s>>>(S, W, Y, static_cast<uint32_t>(per), st, nullptr, flag, live);
       return 0;
     }
-    cols_items_kernel<P, kT, true><<<n, kT, 0, s>>>(S, W, Y, static_cast<uint32_t>(per), st, items, flag);
+    cols_items_kernel<P, kT, true><<<n, kT, 0, s>>>(S, W, Y, static_cast<uint32_t>(per), st, items, flag, live);
     const int nb = std::max(1, kStreamBlocks / planes);
     fold_kernel<P::kC><<<nb * planes, kThreads, 0, s>>>(items, static_cast<uint32_t>(per), nb, partial);
     return nb;
   }
   if (partial)
-    cols_kernel<P, kT, true><<<static_cast<unsigned>(grid), kT, 0, s>>>(S, W, Y, planes, st, partial, flag);
+    cols_kernel<P, kT, true><<<static_cast<unsigned>(grid), kT, 0, s>>>(S, W, Y, planes, st, partial, flag, live);
   else
-    cols_kernel<P, kT, false><<<static_cast<unsigned>(grid), kT, 0, s>>>(S, W, Y, planes, st, partial, flag);
+    cols_kernel<P, kT, false><<<static_cast<unsigned>(grid), kT, 0, s>>>(S, W, Y, planes, st, partial, flag, live);
   return static_cast<int>(grid);
 }
 
 // Returns the grid: the number of partials per chain.
 template <class P>
 int launch_cols(const DevSector& S, const typename P::T* W, typename P::T* Y, int planes, const double* st,
-                double* partial, double* items, const int* flag, cudaStream_t s) {
-  if (S.bt_cols == 1) return launch_cols_t<P, 64>(S, W, Y, planes, st, partial, items, flag, s);
-  if (S.bt_cols == 2) return launch_cols_t<P, 256>(S, W, Y, planes, st, partial, items, flag, s);
-  return launch_cols_t<P, 128>(S, W, Y, planes, st, partial, items, flag, s);
+                double* partial, double* items, const int* flag, const int* live, cudaStream_t s) {
+  if (S.bt_cols == 1) return launch_cols_t<P, 64>(S, W, Y, planes, st, partial, items, flag, live, s);
+  if (S.bt_cols == 2) return launch_cols_t<P, 256>(S, W, Y, planes, st, partial, items, flag, live, s);
+  return launch_cols_t<P, 128>(S, W, Y, planes, st, partial, items, flag, live, s);
 }
 
 template <class P>
 cudaError_t start(const DevSector& S, typename P::T* W, int planes, unsigned seed, bool given, const PlaneState& z,
                   cudaStream_t s) {
-  const cudaError_t e = cudaMemsetAsync(z.flags, 0, 2 * sizeof(int), s);
+  const cudaError_t e = cudaMemsetAsync(z.flags, 0, kPlFlags * sizeof(int), s);
   if (e != cudaSuccess) return e;
   const int nb = std::max(1, kStreamBlocks / planes);
   start_kernel<P><<<nb * planes, kThreads, 0, s>>>(W, S.dim, seed, nb, z.partial, z.flags, S.umask, S.dmask, S.Dd, given);
-  bt_scalars(z.partial, nb, 0, 0, P::kC * planes, P::kScaled, z.st, nullptr, nullptr, z.used, nullptr, s);
+  bt_scalars(z.partial, nb, 0, 0, P::kC * planes, P::kScaled, z.st, nullptr, nullptr, z.used, nullptr, z.flags + 2, s);
   return cudaGetLastError();
 }
 
@@ -555,18 +569,19 @@ bool items_fit(const DevSector& S, int planes) {
 template <class P>
 cudaError_t step(const DevSector& S, const typename P::T* Wk, const typename P::T* Wkm1, typename P::T* Y, int planes,
                  int k, const PlaneState& z, cudaStream_t s) {
-  // C64: flags[k % 2]: W_k has a tiny non-zero entry, written with W_k; flags[(k+1) % 2] is cleared for W_{k+1} by the
+  // flags[2]: the live chains.  C64: flags[k % 2]: W_k has a tiny non-zero entry, written with W_k; flags[(k+1) % 2] is cleared for W_{k+1} by the
   // alpha scalars' kernel.  C128: flags[0], written by the row pass and cleared by that kernel.
   int* fin = z.flags + (P::kScaled ? 0 : (k & 1));
   int* fout = z.flags + (P::kScaled ? 0 : ((k + 1) & 1));
   if (!items_fit(S, planes)) return cudaErrorInvalidValue;
-  const cudaError_t e = launch_rows<P>(S, Wk, Y, planes, z.st, fin, s);
+  int* live = z.flags + 2;
+  const cudaError_t e = launch_rows<P>(S, Wk, Y, planes, z.st, fin, live, s);
   if (e != cudaSuccess) return e;
-  const int nc = launch_cols<P>(S, Wk, Y, planes, z.st, z.partial, z.items, fin, s);
-  bt_scalars(z.partial, nc, 1, k, P::kC * planes, P::kScaled, z.st, z.alpha, z.beta, z.used, fout, s);
+  const int nc = launch_cols<P>(S, Wk, Y, planes, z.st, z.partial, z.items, fin, live, s);
+  bt_scalars(z.partial, nc, 1, k, P::kC * planes, P::kScaled, z.st, z.alpha, z.beta, z.used, fout, nullptr, s);
   const int nb = std::max(1, kStreamBlocks / planes);
-  update_kernel<P><<<nb * planes, kThreads, 0, s>>>(Y, Wk, Wkm1, S.dim, nb, z.st, k > 0, z.partial, fout);
-  bt_scalars(z.partial, nb, 2, k, P::kC * planes, P::kScaled, z.st, z.alpha, z.beta, z.used, nullptr, s);
+  update_kernel<P><<<nb * planes, kThreads, 0, s>>>(Y, Wk, Wkm1, S.dim, nb, z.st, k > 0, z.partial, fout, live);
+  bt_scalars(z.partial, nb, 2, k, P::kC * planes, P::kScaled, z.st, z.alpha, z.beta, z.used, nullptr, live, s);
   return cudaGetLastError();
 }
 
@@ -574,9 +589,9 @@ template <class P>
 cudaError_t apply(const DevSector& S, const typename P::T* X, typename P::T* Y, int planes, int* flag, cudaStream_t s) {
   if (!items_fit(S, planes)) return cudaErrorInvalidValue;
   cudaError_t e = cudaMemsetAsync(flag, 0, sizeof(int), s);
-  if (e == cudaSuccess) e = launch_rows<P>(S, X, Y, planes, nullptr, flag, s);
+  if (e == cudaSuccess) e = launch_rows<P>(S, X, Y, planes, nullptr, flag, nullptr, s);
   if (e != cudaSuccess) return e;
-  launch_cols<P>(S, X, Y, planes, nullptr, nullptr, nullptr, flag, s);
+  launch_cols<P>(S, X, Y, planes, nullptr, nullptr, nullptr, flag, nullptr, s);
   return cudaGetLastError();
 }
 

@@ -20,7 +20,8 @@ namespace ftlm_b200 {
 int pl_group(const DevSector& S, bool c64, int planes);
 
 // Per-chain scalar state and results of a group (kBt* fields of batched.cuh, stride 32), the partial sums of one step
-// (kPlPartialDoubles; of large planes also one per item of the column pass, pl_items_doubles) and two tiny-entry flags.
+// (kPlPartialDoubles; of large planes also one per item of the column pass, pl_items_doubles), two tiny-entry flags and the
+// number of chains that have not ended (kPlFlags ints).
 struct PlaneState {
   double* st;
   double* partial;
@@ -31,6 +32,7 @@ struct PlaneState {
   int* flags;
 };
 int64_t pl_items_doubles(const DevSector& S, bool c64, int planes);
+constexpr int kPlFlags = 3;
 constexpr int64_t kPlMaxBlocks = 2560;
 constexpr int64_t kPlPartialDoubles = kPlMaxBlocks * 32 * 2;
 

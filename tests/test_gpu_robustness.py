@@ -225,3 +225,39 @@ def test_chains_keep_to_a_set_path(gpu):
         a, b, _ = s.lanczos(8, 5, start="philox")
         a2, b2 = F.lanczos_tridiagonal(n, lambda x, y: s.apply(x, y), 8, 5, start="philox")[:2]
         assert np.array_equal(a, a2) and np.array_equal(b, b2)
+
+
+def test_chains_that_end_early_do_no_further_work(gpu):
+    """Without hopping a 4x4 (5,6) sector has the six levels 0, 8 .. 40, so its chains end after six steps, and 300 steps asked
+    for take less time than 30 steps of a chain that goes on.  The chain is right, and so are complex64 chains and the
+    gradient (d ln Z/dU of independent doublons is that of the levels' estimate)."""
+    import time
+    p = F.HubbardParams(4, 4, 0.0, 0.0, 8.0, 0.0)
+    s, go = F.Sector(p, 5, 6), F.Sector(F.HubbardParams(4, 4, 1.0, -0.25, 8.0, 1.0), 5, 6)
+
+    def seconds(h, steps):
+        h.lanczos(2, 1, start="philox")
+        t = time.perf_counter()
+        out = h.lanczos(steps, 1, start="philox")
+        return time.perf_counter() - t, out
+
+    on, _ = seconds(go, 30)
+    ended, (a, b, used) = seconds(s, 300)
+    assert ended < on
+    assert used == a.size <= 8
+    ritz = F.ritz_values(a, b[:used - 1], used)
+    assert all(np.abs(ritz - v).min() <= 1e-8 for v in 8.0 * np.arange(6))
+    A, B, u = s.batched_lanczos(3, 40, 1)
+    assert np.abs(A[0, :5] - a[:5]).max() <= 1e-4 and np.isfinite(A).all()
+
+
+def test_gradient_of_chains_that_end_early(gpu):
+    """d ln Z/dU of the 4x3 (4,4) sector without hopping, chains on planes that end after five steps, against the central
+    difference (1e-6 at h = 1e-4)."""
+    def at(U):
+        return F.Sector(F.HubbardParams(4, 3, 0.0, 0.0, U, 0.0), 4, 4)
+
+    op = F.Sector(F.HubbardParams(4, 3, 0.0, 1.0, 0.0, 0.0), 4, 4)
+    lz, g = at(4.0).ftlm_grad(0.7, 3, 60, 5, op_tp=op, start="philox")
+    l1, l2 = (at(u).ftlm(0.7, 3, 60, 5, start="philox")[0][0] for u in (4.0 + 1e-4, 4.0 - 1e-4))
+    assert abs(g[0] - (l1 - l2) / 2e-4) <= 1e-6 * max(1.0, abs(g[0])) and np.isfinite(g).all()

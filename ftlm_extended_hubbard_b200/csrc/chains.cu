@@ -105,7 +105,8 @@ __global__ void __launch_bounds__(kMost, kMost == 1024 ? 1 : 2) chains_kernel(co
     wk[o] = y[o] = wkm1[o] = P::zero();
   }
   // start vector: Philox (chain q: key seed + q * 100003) or the caller's, in the gauge basis
-  double n0[P::kC] = {};
+  double n0[P::kC];
+  typename P::Norm acc0[P::kC];
   for (int i = tid; i < dim; i += nt) {
     const uint32_t r = static_cast<uint32_t>(i) / static_cast<uint32_t>(Dd), c = static_cast<uint32_t>(i) - r * Dd;
     const double g = gauge_sign(S.umask[r], S.dmask[c]) ? -1.0 : 1.0;
@@ -114,10 +115,12 @@ __global__ void __launch_bounds__(kMost, kMost == 1024 ? 1 : 2) chains_kernel(co
     for (int q = 0; q < P::kC; ++q) {
       const double2 n = init ? init[cd.init + i] : philox_normal(i, cd.seed + static_cast<unsigned>(q) * 100003u);
       z[q] = P::narrow(g * n.x, g * n.y);
-      n0[q] += static_cast<double>(z[q].x) * z[q].x + static_cast<double>(z[q].y) * z[q].y;
+      acc0[q].add(static_cast<double>(z[q].x) * z[q].x + static_cast<double>(z[q].y) * z[q].y);
     }
     wk[r * pitch + c] = P::make(z);
   }
+#pragma unroll
+  for (int q = 0; q < P::kC; ++q) n0[q] = acc0[q].value();
   all_totals<P::kC>(n0, sh);
   double s_in[P::kC], c2[P::kC];
   bool active[P::kC];
@@ -225,7 +228,8 @@ __global__ void __launch_bounds__(kMost, kMost == 1024 ? 1 : 2) chains_kernel(co
       c1i[q] = zi * s_in[q];
       if (active[q] && tid == 0 && q < cd.chains) alpha[static_cast<int64_t>(cd.out + q) * M + k] = zr;
     }
-    double n2[P::kC] = {};
+    double n2[P::kC];
+    typename P::Norm acc2[P::kC];
     constexpr int kBatch = P::kC == 1 ? 2 : 1;  // two complex64 chains need the registers
     for (int i0 = tid; i0 < V; i0 += kBatch * nt) {
       T yv[kBatch], av[kBatch], pv[kBatch];
@@ -249,11 +253,13 @@ __global__ void __launch_bounds__(kMost, kMost == 1024 ? 1 : 2) chains_kernel(co
           wr -= c2[q] * pp.x;
           wi -= c2[q] * pp.y;
           w[q] = P::narrow(wr, wi);
-          n2[q] += static_cast<double>(w[q].x) * w[q].x + static_cast<double>(w[q].y) * w[q].y;
+          acc2[q].add(static_cast<double>(w[q].x) * w[q].x + static_cast<double>(w[q].y) * w[q].y);
         }
         y[i0 + t * nt] = P::make(w);
       }
     }
+#pragma unroll
+    for (int q = 0; q < P::kC; ++q) n2[q] = acc2[q].value();
     all_totals<P::kC>(n2, sh);
     bool any = false;
 #pragma unroll

@@ -12,6 +12,7 @@ namespace ftlm_b200 {
 struct C64 {
   using T = float4;
   using Cf = float2;
+  using Norm = Neu;  // a thread's share of a squared norm: compensated, as in every complex64 chain
   static constexpr int kC = 2;
   static constexpr bool kScaled = false;
   static constexpr int kColThreads = 1024;  // resident threads per SM of the column pass (registers)
@@ -68,9 +69,16 @@ struct C64 {
   }
 };
 
+struct Plain {
+  double s = 0.0;
+  __device__ __forceinline__ void add(double v) { s += v; }
+  __device__ __forceinline__ double value() const { return s; }
+};
+
 struct C128 {
   using T = double2;
   using Cf = double2;
+  using Norm = Plain;
   static constexpr int kC = 1;
   static constexpr bool kScaled = true;
   static constexpr int kColThreads = 896;  // 4x4 (6,6): 2.19 ms, 2.33 with 1024

@@ -226,8 +226,8 @@ int ftlm_gpu_gc_sweep(const ftlm_params* p, int R, int M, unsigned seed, int sta
 /* ---- batched complex64 FTLM (32 chains of a sector per block vector, FP64 scalars) ----
  * Chain r of a sector uses the Philox start vector of FTLM_START_PHILOX with seed + r*100003 (the
  * same vectors the complex128 path draws), rounded to complex64; H·v in FP32, dot products and
- * norms in FP64.  Two chains share a plane of 16 bytes a state; the planes advance in groups, each step a
- * few launches without a host round trip.  Device memory: 3 planes of 16*dim bytes for each plane of a group (at
+ * norms in FP64 (norms compensated).  Two chains share a plane of 16 bytes a state; the planes
+ * advance in groups, each step a few launches without a host round trip.  Device memory: 3 planes of 16*dim bytes for each plane of a group (at
  * least 256 MB a vector, so one plane at 4x4 (8,8): 8 GB), kept between calls until ftlm_gpu_batched_release(). */
 /* Column-pass variant of the batched H·v on this sector: 0/1/2 = 256/128/512-column slabs (the slab of
  * Du x columns x 16 bytes that L2 keeps resident while every output row reads it).  Same terms in the

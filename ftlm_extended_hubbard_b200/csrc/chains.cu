@@ -149,12 +149,22 @@ __global__ void __launch_bounds__(kMost, kMost == 1024 ? 1 : 2) chains_kernel(co
     for (int rb = 0; rb < Du; rb += cd.rows) {  // all rows at once where the whole vector is staged
       const int nr = min(cd.rows, Du - rb);
       if (rb > 0) __syncthreads();
+      bool saw = false;
       for (int i = tid; i < nr * pitch; i += nt) {
         T v = wk[rb * pitch + i];
-        if (P::kScaled) v = P::times(s_in[0], v);
+        if constexpr (P::kScaled) {
+          v = P::times(s_in[0], v);
+          saw = saw || P::small(v);
+        }
         xs[i] = P::filtered(v, 1.0);
       }
-      __syncthreads();
+      // Where an entry is skipped as a source the dot product takes it from the vector itself (complex128; beside the
+      // rounding of FP32 vectors it is nothing).
+      bool filtered = false;
+      if constexpr (P::kScaled)
+        filtered = __syncthreads_or(saw);
+      else
+        __syncthreads();
       const int items = (nr + rpw - 1) / rpw * ng;
       for (int it = warp; it < items; it += nw) {
         const int rl = it / ng * rpw + sub, pos = (it - it / ng * ng) * 32 + pos0;
@@ -214,7 +224,10 @@ __global__ void __launch_bounds__(kMost, kMost == 1024 ? 1 : 2) chains_kernel(co
         if (in) {
           const T v = P::add_scaled(acc, up, kSmem ? 1.0 : s_in[0]);
           y[r * pitch + c] = v;
-          P::dot(d, row[c], v, 1.0);
+          T left = row[c];
+          if constexpr (P::kScaled)
+            if (filtered) left = P::times(s_in[0], wk[r * pitch + c]);
+          P::dot(d, left, v, 1.0);
         }
       }
     }

@@ -167,10 +167,24 @@ int build_orbit_sector(ftlm_sector* s) {
 // once leave at least 60 % to everything else.
 constexpr size_t kListShare = 32;
 
-// The block's matrix as source lists (orbit.cuh): the values of the matrix elements, gathered up to rounding, become at
-// most 255 codes of 8 bits beside the 24 of a source's index.  Built once per block, for about two H_K v; each of these then
+// e^{2 pi i m / n} (0 <= m < n) rounded once from extended precision, so that values which are equal up to sign or an
+// exchange of their parts are so bit for bit.
+void unit_root(int m, int n, long double* re, long double* im) {
+  const int q = 4 * m / n, r = 4 * m - q * n;  // quadrant, and the angle within it: (pi / 2) r / n
+  const long double quarter = std::acos(-1.0L) / 2.0L;
+  const bool low = 2 * r <= n;
+  const long double x = quarter * static_cast<long double>(low ? r : n - r) / static_cast<long double>(n);
+  const long double c = static_cast<double>(low ? std::cos(x) : std::sin(x));
+  const long double s = static_cast<double>(low ? std::sin(x) : std::cos(x));
+  *re = q == 0 ? c : q == 1 ? -s : q == 2 ? -c : s;
+  *im = q == 0 ? s : q == 1 ? c : q == 2 ? -s : -c;
+}
+
+// The block's matrix as source lists (orbit.cuh): the values of the matrix elements become at most 255 codes of 8 bits
+// beside the 24 of a source's index.  A value is rounded to double once, from the exact character and root, and only equal
+// doubles share a code, so no element is further off than the product of its rounded factors.  Built once per block, for about two H_K v; each of these then
 // reads 4 bytes in order instead of 4 random ones per source.  Blocks with more values keep the tables.
-int build_lists(ftlm_orbit* o, const std::vector<double2>& chi) {
+int build_lists(ftlm_orbit* o) {
   const SectorPlan& P = o->sector->plan;
   OrbitApplyDev& A = o->app;
   A.list = nullptr;
@@ -185,10 +199,13 @@ int build_lists(ftlm_orbit* o, const std::vector<double2>& chi) {
       if (K.n_coef == 16) return FTLM_OK;
       K.coef[K.n_coef++] = make_double2(h.cre, h.cim);
     }
+  long double root[16];
   for (int n = 1; n <= o->data->G; ++n) {  // |A| of a surviving representative is the size of its stabiliser
     if (o->data->G % n != 0) continue;
     if (K.n_a == 16) return FTLM_OK;
-    K.root[K.n_a++] = std::sqrt(static_cast<double>(n));
+    root[K.n_a] = std::sqrt(static_cast<long double>(n));
+    K.root[K.n_a] = static_cast<double>(root[K.n_a]);
+    ++K.n_a;
   }
   for (double a : o->absA) {
     const double r = std::sqrt(a);
@@ -196,7 +213,7 @@ int build_lists(ftlm_orbit* o, const std::vector<double2>& chi) {
     for (int i = 0; i < K.n_a && !known; ++i) known = std::fabs(r - K.root[i]) <= 1e-12 * K.root[i];
     if (!known) return FTLM_OK;
   }
-  const int G = o->data->G;
+  const int G = o->data->G, Lx = o->sector->Lx, Ly = o->sector->Ly;
   std::vector<double2> dict(256, make_double2(0.0, 0.0));
   std::vector<uint8_t> lut(static_cast<size_t>(std::max(1, K.n_coef)) * 2 * G * 2 * K.n_a, 0);
   int n = 1;
@@ -205,14 +222,14 @@ int build_lists(ftlm_orbit* o, const std::vector<double2>& chi) {
       for (int R = 0; R < G; ++R)
         for (int eta = 0; eta < 2; ++eta)
           for (int a = 0; a < K.n_a; ++a) {
-            const double f = (neg != eta ? -1.0 : 1.0) * K.root[a];
-            const double2 cc = K.coef[c], ch = chi[static_cast<size_t>(R)];
-            const double2 v = make_double2(f * (cc.x * ch.x + cc.y * ch.y), f * (cc.y * ch.x - cc.x * ch.y));
-            const double size = std::hypot(v.x, v.y);
+            const long double f = (neg != eta ? -1.0L : 1.0L) * root[a], cx = K.coef[c].x, cy = K.coef[c].y;
+            // conj(chi(R)): chi = e^{-2 pi i (kx dx / Lx + ky dy / Ly)}
+            long double wx, wy;
+            unit_root((o->kx * (R % Lx) * Ly + o->ky * (R / Lx) * Lx) % G, G, &wx, &wy);
+            const double2 v = make_double2(static_cast<double>(f * (cx * wx - cy * wy)), static_cast<double>(f * (cy * wx + cx * wy)));
             int code = 0;
             for (int i = 1; i < n && !code; ++i)
-              if (std::fabs(dict[static_cast<size_t>(i)].x - v.x) <= 1e-14 * size && std::fabs(dict[static_cast<size_t>(i)].y - v.y) <= 1e-14 * size)
-                code = i;
+              if (dict[static_cast<size_t>(i)].x == v.x && dict[static_cast<size_t>(i)].y == v.y) code = i;
             if (!code) {
               if (n == 256) return FTLM_OK;
               code = n++;
@@ -375,7 +392,7 @@ int ftlm_gpu_orbit_create_ex(ftlm_sector* s, int kx, int ky, double survive_tol,
   A.dhop_oth = D.dh_oth.as<uint32_t>();
   A.n_dhops = D.n_dh;
   A.path = 1;
-  rc = build_lists(o.get(), chi);
+  rc = build_lists(o.get());
   if (rc) return rc;
   if (!A.list) {  // only the table form has use for it
     CU_TRY(o->xs.alloc(static_cast<size_t>(std::max<int64_t>(o->dk, 1)) * sizeof(double2)));

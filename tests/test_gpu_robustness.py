@@ -261,3 +261,19 @@ def test_gradient_of_chains_that_end_early(gpu):
     lz, g = at(4.0).ftlm_grad(0.7, 3, 60, 5, op_tp=op, start="philox")
     l1, l2 = (at(u).ftlm(0.7, 3, 60, 5, start="philox")[0][0] for u in (4.0 + 1e-4, 4.0 - 1e-4))
     assert abs(g[0] - (l1 - l2) / 2e-4) <= 1e-6 * max(1.0, abs(g[0])) and np.isfinite(g).all()
+
+
+@pytest.mark.parametrize("k", [(0, 0), (2, 0)])
+def test_momentum_block_values_that_almost_agree(gpu, k):
+    """Hops of 1 and of 1 + 8e-15 are two values of the source lists: columns of H_K against the hop scan, to 9 ulp (a few
+    products and square roots)."""
+    s = F.Sector(F.HubbardParams(4, 3, 1.0, 1.0 + 8e-15, 4.0, 0.0), 2, 2)
+    o = s.orbit_block(*k)
+    for j in range(0, o.dim, 17):
+        x = np.zeros(o.dim, complex)
+        x[j] = 1.0
+        o.set_apply_path(1)
+        y = o.apply_host(x)
+        o.set_apply_path(0)
+        ref = o.apply_host(x)
+        assert np.abs(y - ref).max() <= 2e-15 * np.abs(ref).max()

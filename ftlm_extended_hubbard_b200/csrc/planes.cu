@@ -327,12 +327,11 @@ __global__ void __launch_bounds__(kT, P::kColThreads / kT) cols_items_kernel(Dev
                                                                              const int* __restrict__ flag,
                                                                              const int* __restrict__ live) {
   using T = typename P::T;
-  if (all_ended(live)) return;
   __shared__ uint32_t s_off[kMaxDeg];
   __shared__ __align__(16) typename P::Cf s_cf[kMaxDeg];
   __shared__ double sh[2 * P::kC * kT / 32];
   const int t = threadIdx.x;
-  const bool filter = *flag != 0;
+  const bool filter = *flag != 0, ended = all_ended(live);  // tested late: the list loads need not wait for it
   const uint32_t Dd = static_cast<uint32_t>(S.Dd), Du = static_cast<uint32_t>(S.Du);
   const uint32_t p = blockIdx.x / per, it = blockIdx.x - p * per, chunk = it / Du, r = it - chunk * Du;
   const int j0 = S.up_ptr[r], deg = S.up_ptr[r + 1] - j0;
@@ -346,7 +345,7 @@ __global__ void __launch_bounds__(kT, P::kColThreads / kT) cols_items_kernel(Dev
   const uint32_t c0 = chunk * (2 * kT) + t, c1 = c0 + kT;
   double d[2 * P::kC] = {};
   __syncthreads();
-  if (c0 < Dd) {
+  if (c0 < Dd && !ended) {
     const bool has1 = c1 < Dd;
     const uint32_t c1s = has1 ? c1 : c0;
     T a0, a1;

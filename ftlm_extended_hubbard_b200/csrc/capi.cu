@@ -520,6 +520,10 @@ int ftlm_b200::capi::planes_lanczos(ftlm_sector* s, int R, int M, unsigned seed,
       }
     }
   }
+  // A handle keeps the three vectors of one chain, or what L2 holds of several (given back and taken again, those cost
+  // 4x3 (4,5) with four chains 0.4 % of a call); more goes back to the pool, which ftlm_gpu_batched_release empties.
+  constexpr size_t kHandleKeep = size_t(40) << 20;  // a vector
+  if (group > 1 && ws.cap > kHandleKeep) ws.release();
   return FTLM_OK;
 }
 

@@ -277,3 +277,17 @@ def test_momentum_block_values_that_almost_agree(gpu, k):
         o.set_apply_path(0)
         ref = o.apply_host(x)
         assert np.abs(y - ref).max() <= 2e-15 * np.abs(ref).max()
+
+
+def test_handles_keep_the_vectors_of_one_chain(gpu):
+    """After 32 chains at once (376 MB of vectors) a handle holds those of one chain; what the library keeps for the
+    next call goes back with batched_release."""
+    torch = gpu
+    F.api.batched_release()
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    hold = [F.Sector(F.HubbardParams(4, 3, 1.0, -0.25, 8.0, 1.0), 4, 4) for _ in range(3)]
+    for s in hold:
+        s.ftlm([1.0], 32, 4, 1, start="philox")
+    F.api.batched_release()
+    assert free - torch.cuda.mem_get_info()[0] < 100 << 20  # tables, scalars and at most 12 MB of vectors each

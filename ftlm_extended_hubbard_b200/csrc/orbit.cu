@@ -330,8 +330,8 @@ __global__ void __launch_bounds__(256) list_kernel(OrbitApplyDev A, OrbitCodes K
 // y = H_K x over the source lists: 8 lanes per representative, each two entries of every 16, so that a round loads 64
 // contiguous bytes of the list and has 64 gathers of x in flight per warp; coefficients from the dictionary in shared
 // memory.  The table form above looks every source up in the dim-long state table first (4 random bytes, a 32-byte sector,
-// before each gather) and multiplies the coefficient out.  Bound by the L2's rate of random 32-byte sectors (190 G/s): 4x4 (6,6),
-// 4.0 million representatives, 1.67 ms with the tables, 1.17 ms here.
+// before each gather) and multiplies the coefficient out.  Bound by its random gathers: 4x4 (6,6), 4.0 million
+// representatives, 1.67 ms with the tables, 1.01 ms here (1.15 with the rows' padding gathered too, 7.5 of 58 entries).
 __global__ void __launch_bounds__(256) apply_list_kernel(OrbitApplyDev A, const double2* __restrict__ x,
                                                          double2* __restrict__ y) {
   __shared__ double2 dict[256];
@@ -354,12 +354,14 @@ __global__ void __launch_bounds__(256) apply_list_kernel(OrbitApplyDev A, const 
       acc.y = fma(c.x, v.y, acc.y);
       acc.y = fma(c.y, v.x, acc.y);
     };
+    // padding (code 0) is not read: 0 times an entry that is not finite would be NaN
+    auto source = [&](uint32_t e) { return e >= (1u << 24) ? x[e & 0xFFFFFFu] : make_double2(0.0, 0.0); };
     int k = 0;
     for (; k + 2 <= n; k += 2) {
       const uint2 e0 = *reinterpret_cast<const uint2*>(row + 16 * k);
       const uint2 e1 = *reinterpret_cast<const uint2*>(row + 16 * k + 16);
-      const double2 v0 = x[e0.x & 0xFFFFFFu], v1 = x[e0.y & 0xFFFFFFu];
-      const double2 v2 = x[e1.x & 0xFFFFFFu], v3 = x[e1.y & 0xFFFFFFu];
+      const double2 v0 = source(e0.x), v1 = source(e0.y);
+      const double2 v2 = source(e1.x), v3 = source(e1.y);
       term(e0.x, v0);
       term(e0.y, v1);
       term(e1.x, v2);
@@ -367,7 +369,7 @@ __global__ void __launch_bounds__(256) apply_list_kernel(OrbitApplyDev A, const 
     }
     if (k < n) {
       const uint2 e0 = *reinterpret_cast<const uint2*>(row + 16 * k);
-      const double2 v0 = x[e0.x & 0xFFFFFFu], v1 = x[e0.y & 0xFFFFFFu];
+      const double2 v0 = source(e0.x), v1 = source(e0.y);
       term(e0.x, v0);
       term(e0.y, v1);
     }

@@ -291,3 +291,22 @@ def test_handles_keep_the_vectors_of_one_chain(gpu):
         s.ftlm([1.0], 32, 4, 1, start="philox")
     F.api.batched_release()
     assert free - torch.cuda.mem_get_info()[0] < 100 << 20  # tables, scalars and at most 12 MB of vectors each
+
+
+def test_momentum_block_apply_of_entries_that_are_not_finite(gpu):
+    """An infinite entry gives infinities and NaN where the hop scan has them: padding of the source lists adds nothing."""
+    s = F.Sector(F.HubbardParams(4, 3, 1.0, -0.25, 4.0, 0.5), 2, 2)
+    o = s.orbit_block(0, 0)
+    rng = np.random.default_rng(8)
+    for bad in (np.inf, -np.inf):
+        x = rng.standard_normal(o.dim) + 1j * rng.standard_normal(o.dim)
+        x[o.dim // 3] = bad
+        o.set_apply_path(1)
+        y = o.apply_host(x)
+        o.set_apply_path(0)
+        ref = o.apply_host(x)
+        for part in (np.real, np.imag):
+            a, b = part(y), part(ref)
+            assert np.array_equal(np.isnan(a), np.isnan(b)) and np.array_equal(np.isinf(a), np.isinf(b))
+            ok = np.isfinite(b)
+            assert np.abs(a[ok] - b[ok]).max() <= 1e-12

@@ -529,10 +529,10 @@ int ftlm_b200::capi::planes_lanczos(ftlm_sector* s, int R, int M, unsigned seed,
 
 namespace {
 
-// A chain's alpha and beta without their padding: one that ended has no last beta.
+// A chain's alpha and beta without their padding: one that ended has no last beta (0; one that is not a number counts).
 void trim_chain(int n, std::vector<double>* a, std::vector<double>* b) {
   a->resize(static_cast<size_t>(n));
-  b->resize(static_cast<size_t>(n > 0 && (*b)[static_cast<size_t>(n) - 1] > 0.0 ? n : std::max(0, n - 1)));
+  b->resize(static_cast<size_t>(n > 0 && (*b)[static_cast<size_t>(n) - 1] != 0.0 ? n : std::max(0, n - 1)));
 }
 
 }  // namespace

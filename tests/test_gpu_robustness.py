@@ -310,3 +310,16 @@ def test_momentum_block_apply_of_entries_that_are_not_finite(gpu):
             assert np.array_equal(np.isnan(a), np.isnan(b)) and np.array_equal(np.isinf(a), np.isinf(b))
             ok = np.isfinite(b)
             assert np.abs(a[ok] - b[ok]).max() <= 1e-12
+
+
+@pytest.mark.parametrize("lat,nu,nd", [((3, 3), 4, 4), ((4, 3), 4, 4)])
+def test_chains_of_numbers_that_are_not_finite(gpu, lat, nu, nd):
+    """An interaction that is not a number gives a chain of as many alphas and betas as steps, fused and on planes, as the
+    step-by-step recurrence does."""
+    s = F.Sector(F.HubbardParams(*lat, 1.0, -0.25, float("nan"), 1.0), nu, nd)
+    g = F.Sector(F.HubbardParams(*lat, 1.0, -0.25, float("nan"), 1.0), nu, nd)
+    g.set_apply_path(1)
+    a, b, used = s.lanczos(5, 1, start="philox")
+    a2, b2, used2 = g.lanczos(5, 1, start="philox")
+    assert used == used2 == 5 and a.size == a2.size == 5 and b.size == b2.size == 5
+    assert np.isnan(b).all() and np.isnan(b2).all()

@@ -323,3 +323,46 @@ def test_chains_of_numbers_that_are_not_finite(gpu, lat, nu, nd):
     a2, b2, used2 = g.lanczos(5, 1, start="philox")
     assert used == used2 == 5 and a.size == a2.size == 5 and b.size == b2.size == 5
     assert np.isnan(b).all() and np.isnan(b2).all()
+
+
+@pytest.mark.parametrize("lat,nu,nd,path", [((3, 3), 4, 4, 0), ((4, 2), 4, 4, 0), ((4, 4), 2, 2, 0), ((4, 3), 4, 4, 0), ((4, 3), 4, 4, 1),
+                                            ((4, 3), 4, 4, 2), ((4, 3), 4, 4, 3)])
+def test_entries_below_the_threshold_are_no_sources(gpu, lat, nu, nd, path):
+    """Entries with |x|^2 < 1e-28 contribute nothing: a vector of such entries gives exact zeros, and beside others they leave
+    the bits of the vector with zeros in their place (one pass and two, a row of the block and other rows)."""
+    torch = gpu
+    s = F.Sector(F.HubbardParams(*lat, 1.0, -0.25, 8.0, 1.0, 0.1, 0.0), nu, nd)
+    s.set_apply_path(path)
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    small = torch.randn(s.dim(), dtype=torch.complex128, device="cuda", generator=gen)
+    small = 9e-15 * small / small.abs()
+    y, ref = torch.empty_like(small), torch.empty_like(small)
+    s.apply(small, y)
+    assert not y.any()
+    for every in (2, 37, s.dim()):
+        x, x0 = small.clone(), torch.zeros_like(small)
+        x[::every] = x0[::every] = 1.0 + 0.5j
+        s.apply(x, y)
+        s.apply(x0, ref)
+        assert torch.equal(y, ref) and ref.any()
+
+
+@pytest.mark.parametrize("lat,nu,nd,k", [((4, 3), 3, 3, (1, 1)), ((3, 3), 4, 2, (0, 0)), ((4, 4), 3, 2, (2, 1))])
+@pytest.mark.parametrize("path", [0, 1])
+def test_entries_below_the_threshold_in_a_momentum_block(gpu, lat, nu, nd, k, path):
+    """The same in a momentum block, from its source lists and by the hop scan."""
+    torch = gpu
+    o = F.Sector(F.HubbardParams(*lat, 1.0, -0.25, 6.0, 0.5), nu, nd).orbit_block(*k)
+    o.set_apply_path(path)
+    gen = torch.Generator(device="cuda").manual_seed(6)
+    small = torch.randn(o.dim, dtype=torch.complex128, device="cuda", generator=gen)
+    small = 9e-15 * small / small.abs()
+    y, ref = torch.empty_like(small), torch.empty_like(small)
+    o.apply(small, y)
+    assert not y.any()
+    for every in (2, 37, o.dim):
+        x, x0 = small.clone(), torch.zeros_like(small)
+        x[::every] = x0[::every] = 1.0 + 0.5j
+        o.apply(x, y)
+        o.apply(x0, ref)
+        assert torch.equal(y, ref) and ref.any()

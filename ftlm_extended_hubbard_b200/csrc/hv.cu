@@ -293,6 +293,11 @@ constexpr int kOnceThreads = 512;
 // 12.6; 4x3 (8,3), the same in rows of 220, 12.3 / 12.6; 4x4 (5,2), 524,160 in rows of 120, 41 / 45; 4x3 (6,6), rows of
 // 924, 77 / 54.
 constexpr int64_t kOnceMaxDim = int64_t(1) << 16, kOnceShortRow = 256, kOnceShortDim = int64_t(1) << 22;
+// Where it is slower than the generic kernel, whose threads know no rows: rows that keep one block long (one pass / generic,
+// rows of 1,820: 16.8 / 20.6 us; 3,003: 24.7 / 22.6; 4,368: 24.7 / 20.6; 12,870: 66 / 23), and many rows that fill a fraction
+// of a warp (rows of 1 or 16, 3,003 of them: 14.5 to 16.4 / 14.4 to 18.5; 4,368: 16.5 to 18.5 / 15.6 to 18.5; 5,005: 20.6 to 22.7 /
+// 16.5 to 18.5; 12,870: 45 to 49 / 20 to 25).
+constexpr int64_t kOnceLongRow = 2048, kOnceThinRow = 32, kOnceThinRows = 4096;
 constexpr size_t kOnceListBytes = kMaxUpDeg * 24;  // the row's source list
 
 template <bool kPhase, bool kXor>
@@ -556,6 +561,7 @@ cudaError_t launch_cols(const DevSector& S, const double2* x, double2* y, cudaSt
 }
 
 bool hv_once_ok(const DevSector& S, int max_up_deg) {
+  if (S.Dd > kOnceLongRow || (S.Dd < kOnceThinRow && S.Du > kOnceThinRows)) return false;
   return S.dn_g.ent && S.dim <= (S.Dd <= kOnceShortRow ? kOnceShortDim : kOnceMaxDim) && max_up_deg <= kMaxUpDeg &&
          hv_rows_smem_bytes(S) + kOnceListBytes <= 227 * 1024;
 }

@@ -366,3 +366,31 @@ def test_entries_below_the_threshold_in_a_momentum_block(gpu, lat, nu, nd, k, pa
         o.apply(x, y)
         o.apply(x0, ref)
         assert torch.equal(y, ref) and ref.any()
+
+
+@pytest.mark.parametrize("nu,nd", [(0, 8), (8, 0), (8, 1), (1, 5), (5, 1), (4, 1), (0, 4)])
+def test_default_apply_of_thin_sectors(gpu, nu, nd):
+    """Sectors with few strings of one species: the default H v is the faster of the one pass and the generic kernel (to 30 %,
+    which a wrong choice exceeds by far), and gives its sums (1e-13 of the largest)."""
+    torch = gpu
+    s = F.Sector(F.HubbardParams(4, 4, 1.0, -0.25, 8.0, 1.0, 0.1, 0.0), nu, nd)
+    x = torch.randn(s.dim(), dtype=torch.complex128, device="cuda")
+    y, ref = torch.empty_like(x), torch.empty_like(x)
+
+    def us(path, out):
+        s.set_apply_path(path)
+        best = 1e9
+        for _ in range(5):
+            a, b = torch.cuda.Event(True), torch.cuda.Event(True)
+            s.apply(x, out)
+            a.record()
+            for _ in range(50):
+                s.apply(x, out)
+            b.record()
+            b.synchronize()
+            best = min(best, a.elapsed_time(b) * 20.0)
+        return best
+
+    generic, default = us(1, ref), us(0, y)
+    assert default <= 1.3 * generic
+    assert (y - ref).abs().max() <= 1e-13 * ref.abs().max()

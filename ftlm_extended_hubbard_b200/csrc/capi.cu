@@ -544,7 +544,7 @@ int ftlm_gpu_lanczos(ftlm_sector* s, int max_steps, unsigned seed, int start_mod
   int rc = need_device(s);
   if (rc) return rc;
   std::vector<double> a, b;
-  if (s->chains() == ftlm_sector::Chains::fused && max_steps > 0) {
+  if (s->chains(1) == ftlm_sector::Chains::fused && max_steps > 0) {
     // few states: all steps in one kernel
     ChainRun run;
     rc = chains_run({s}, 1, max_steps, seed, start_mode, false, &run);
@@ -556,7 +556,7 @@ int ftlm_gpu_lanczos(ftlm_sector* s, int max_steps, unsigned seed, int start_mod
     CU_TRY(cudaMemcpy(a.data(), run.alpha, a.size() * sizeof(double), cudaMemcpyDeviceToHost));
     CU_TRY(cudaMemcpy(b.data(), run.beta, b.size() * sizeof(double), cudaMemcpyDeviceToHost));
     trim_chain(n, &a, &b);
-  } else if (s->chains() == ftlm_sector::Chains::planes && max_steps > 0) {
+  } else if (s->chains(1) == ftlm_sector::Chains::planes && max_steps > 0) {
     std::vector<int> u;
     rc = planes_lanczos(s, 1, max_steps, seed, start_mode, &a, &b, &u);
     if (rc) return rc;
@@ -794,11 +794,11 @@ int plain_sector_ftlm(ftlm_sector* s, const double* bts, int n_bt, int R, int M,
     }
     return FTLM_OK;
   }
-  if (s->chains() == ftlm_sector::Chains::fused)
+  if (s->chains(R) == ftlm_sector::Chains::fused)
     return chains_ftlm({s}, R, M, seed, start_mode, false, bts, n_bt, converged, lnz, energy);
   std::vector<double> A(static_cast<size_t>(R) * M, 0.0), B(static_cast<size_t>(R) * M, 0.0);
   std::vector<int> nv(static_cast<size_t>(R), 0);
-  if (s->chains() == ftlm_sector::Chains::planes) {
+  if (s->chains(R) == ftlm_sector::Chains::planes) {
     rc = planes_lanczos(s, R, M, seed, start_mode, &A, &B, &nv);
     if (rc) return rc;
   } else {

@@ -478,7 +478,7 @@ int ftlm_gpu_gc_logz(const ftlm_params* p, double mu, double bT, int R, int M, u
         rc = bt_run_chains(s.get(), R, M, seed, &A, &B, &used);
         if (rc) return rc;
       } else {
-        if (s->chains() == ftlm_sector::Chains::planes) {
+        if (s->chains(R) == ftlm_sector::Chains::planes) {
           rc = planes_lanczos(s.get(), R, M, seed, st_mode, &A, &B, &used);
           if (rc) return rc;
         } else {

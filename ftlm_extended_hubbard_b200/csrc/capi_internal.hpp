@@ -273,7 +273,7 @@ struct ftlm_sector {
   // How complex128 chains run: all steps in one kernel, on planes (gauge row pass + column slabs, so also where path 3 is
   // pinned), or step by step on apply().
   enum class Chains { fused, planes, steps };
-  Chains chains() const;
+  Chains chains(int R) const;  // of R of them
   ftlm_b200::DevSector planes_dev() const {
     ftlm_b200::DevSector d = dev;
     if (cols_chosen) d.bt_cols = cols_variant % 3;
@@ -430,18 +430,26 @@ int fused_sectors_ftlm(const std::vector<ftlm_sector*>& secs, const std::vector<
                        unsigned seed, int start_mode, bool c64, const double* bts, int n_bt, double* lnz_s, double* e_s,
                        bool converged);
 
-// Whether a single sector's own chains run fused, by the lanes that a step of its block has to go through: a step takes
-// about 20 us at 8192 lanes, what the kernels of a step on the whole GPU take for their launches alone (3x3 (5,4), 15,876
-// states, one chain: 180 us a step fused).
-inline bool fused_alone(const DevSector& S) {  // and a row of it fits (chain_rows)
+// Whether a single sector's own chains run fused, by the lanes that a step of its block has to go through.  A step on planes
+// takes 27 us for sectors of any shape up to 50,000 states; fused, 28 us at 3,456 lanes, 37 at 6,336, 55 at 8,064 (3x3
+// (2,3), 4x3 (2,2), 3x3 (3,3), complex128).  Sectors of one row are slower on planes (47 us at 5,005 strings, 58 at 8,008; fused 31 and
+// 48).  A vector that is not staged whole is read from the block's scratch: 4x4 (6,0), 8,008 rows of one string and 8 of padding,
+// 275 us a step fused, 52 on planes.
+inline bool fused_alone(const DevSector& S) {
   const int64_t lanes = S.Dd <= 16 ? S.Du / (32 / S.Dd) * 32 : S.Du * ((S.Dd + 31) / 32 * 32);
-  return lanes <= 8192 && chain_rows(S, false, false) > 0;
+  return lanes <= (S.Du == 1 ? 8192 : 4096) && chain_rows(S, false, false) == S.Du;
 }
+// Sectors with very few strings of one species and many of the other: few or short work items for the passes on planes.
+inline bool thin_sector(const DevSector& S) { return std::min(S.Du, S.Dd) <= 16 && std::max(S.Du, S.Dd) > 10000; }
+
 }  // namespace capi
 }  // namespace ftlm_b200
 
-inline ftlm_sector::Chains ftlm_sector::chains() const {
+inline ftlm_sector::Chains ftlm_sector::chains(int R) const {
   if (!pinned && ftlm_b200::capi::fused_alone(dev)) return Chains::fused;
+  // one chain of a thin sector whose H v is the generic kernel (by rule or by timing): 4x4 (0,8) 64 us a step, 82 on planes;
+  // (8,1) 66 and 76; (1,8) timed 78 and 88.  From two chains on the planes share their launches: 82 us a step of both.
+  if (!pinned && R == 1 && ftlm_b200::capi::thin_sector(dev) && effective_path() == 1 && !once()) return Chains::steps;
   if ((!pinned || effective_path() == 3) && ftlm_b200::pl_fits(dev, plan.max_up_deg)) return Chains::planes;
   return Chains::steps;
 }

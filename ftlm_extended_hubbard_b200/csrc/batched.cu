@@ -239,9 +239,9 @@ __global__ void __launch_bounds__(kScalarThreads) bt_scalar_kernel(const double*
 // the fused <W_k, Y> per chain.  Warp per representative: its sources come from the block's list (orbit.cuh), or, where it
 // has none, from the sector's gather tables 32 at a time (a random 4-byte lookup per source), the surviving ones compacted
 // by ballot; coefficients <rep a|H|s> eta conj(chi(R)) sqrt|A_b| / sqrt|A_a| in FP64, rounded to complex64.  Then the
-// half-warps take every other source each and gather the 256-byte rows W[b, :].  Bound by instruction issue, about 900 per
-// representative (rows of 24 instead of 32 chains take as long): 4x4 (4,4), 207,000 representatives, 258 us with the table
-// lookups, 215 us with the lists.
+// half-warps take every other source each and gather the 256-byte rows W[b, :].  Bound by the L1 pipe (71 % of its
+// wavefronts) and instruction issue (64 %; 745 warp instructions a representative; rows of 24 instead of 32 chains take as
+// long): 4x4 (4,4), 207,000 representatives, 258 us with the table lookups, 215 us with the lists.
 constexpr int kOrbTerms = 256;
 
 __device__ __forceinline__ void orb_push(bool ok, uint32_t off, float2 cf, int lane, int& cnt, uint32_t* s_off,

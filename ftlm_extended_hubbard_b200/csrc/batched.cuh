@@ -1,4 +1,5 @@
-// Batched complex64 FTLM kernels (batched.cu): 32 chains of one sector per block vector.
+// Complex64 Lanczos of a momentum block (batched.cu): 32 chains of the block per vector; the chains' scalars, which the
+// planes of a sector (planes.cu) share.
 #pragma once
 
 #include <cuda_runtime.h>

@@ -64,7 +64,6 @@ void reference_start(int64_t dim, unsigned seed, std::vector<std::complex<double
   }
 }
 
-// Device Lanczos workspace.
 }  // namespace capi
 }  // namespace ftlm_b200
 

@@ -8,13 +8,12 @@
 // the sector has it: one word a source instead of three, two real FMAs a component instead of four.  Then the dot
 // products, the update and the norm over the block's own vectors.  The vector that the hops gather from is staged in
 // shared memory where it fits (14,336 states with their padding); else the rows are, a block of rows at a time, and the
-// up hops read the block's scratch (32 lanes that gather at random within a row from global memory touch a line each:
-// 3x3 (4,4), 15,876 states, took 142 us a step that way). Rows have a pitch of Dd + 8 elements whose last 8 stay zero:
+// up hops read the block's scratch: 3x3 (4,4), 15,876 states, 146 us a step of one complex128 chain. Rows have a pitch of Dd + 8 elements whose last 8 stay zero:
 // the target of the table's padding entries, and harmless to the flat elementwise passes.  Bound by the shared-memory
-// pipe above 4,096 states (85 % of its wavefronts before the lane change and the packed list; 3x3 batched sweep, the
-// launch of 320 blocks, 13.4 -> 11.5 ms), by latency below; it exists because a step of a small sector otherwise costs
-// five kernel launches, whatever its size: 3x3 batched sweep (100 sectors, 60 steps) 336 -> 127 ms, most of that in the
-// host's allocations.
+// pipe and instruction issue above 4,096 states (60 and 64 % in the 3x3 batched sweep's launch of 320 blocks; 85 % of the
+// wavefronts before the lane change and the packed list, 13.4 -> 11.5 ms), by latency below; it exists because a step of a small sector otherwise costs
+// five kernel launches, whatever its size: 3x3 batched sweep (100 sectors, 60 steps) 336 ms without it, 27.2 now, the host's
+// allocations and tables included.
 // Same FP32 order of operations per element as planes.cu, so complex64 chains agree with that path up to the order of
 // the FP64 sums.  Sums are in a fixed order: bitwise repeatable.
 #include <algorithm>

@@ -97,7 +97,7 @@ __device__ __forceinline__ void cmac(double2& acc, double2 c, double2 v, uint32_
 
 // (H x)[idx] in gather form from the sector tables: diagonal, down hops (ELL group of the column,
 // sources in the same row), up hops (CSR of the row, sources in the same column), with the
-// reference's source-skip rule.  The generic H·v kernel and the fused small-sector Lanczos use it.
+// reference's source-skip rule.  The generic H·v kernel.
 __device__ __forceinline__ double2 hv_element(const DevSector& S, const double2* __restrict__ x, int64_t idx) {
   const int64_t r = idx / S.Dd;
   const int64_t c = idx - r * S.Dd;

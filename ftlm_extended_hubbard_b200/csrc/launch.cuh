@@ -5,7 +5,7 @@
 // before it drains, and wait in follow() until that kernel has ended and its writes are visible, so the order of all
 // reads and writes is that of an ordinary launch.  Every thread of every block passes follow(), so the kernel's end
 // implies that of all before it. Only where the vectors stay in L2 (kEarlyStates): there the gap is a large part of a
-// kernel (two-pass H v, 4x3 (5,6): 55.3 -> 50.8 us back to back; 4x3 (4,4): 22.6 -> 19.2), while waiting blocks cost
+// kernel (two-pass H v, a call: 4x3 (5,6) 55.3 -> 51.6 us, 4x3 (4,4) 21.4 -> 17.2), while waiting blocks cost
 // large sectors 1 to 2 % (5x3 (5,5) 506 -> 514 us).  Under stream capture the launches are ordinary ones.
 #pragma once
 

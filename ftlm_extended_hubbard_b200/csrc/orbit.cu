@@ -330,8 +330,9 @@ __global__ void __launch_bounds__(256) list_kernel(OrbitApplyDev A, OrbitCodes K
 // y = H_K x over the source lists: 8 lanes per representative, each two entries of every 16, so that a round loads 64
 // contiguous bytes of the list and has 64 gathers of x in flight per warp; coefficients from the dictionary in shared
 // memory.  The table form above looks every source up in the dim-long state table first (4 random bytes, a 32-byte sector,
-// before each gather) and multiplies the coefficient out.  Bound by its random gathers: 4x4 (6,6), 4.0 million
-// representatives, 1.67 ms with the tables, 1.01 ms here (1.15 with the padding gathered too, 6 entries beside 64 sources).
+// before each gather) and multiplies the coefficient out.  Bound by the L1 pipe, whose wavefronts are 94 % busy (every lane
+// gathers from a line of its own): 4x4 (6,6), 4.0 million representatives, 1.67 ms with the tables, 1.01 ms here (1.15 with
+// the padding gathered too, 6 entries beside 64 sources).
 __global__ void __launch_bounds__(256) apply_list_kernel(OrbitApplyDev A, const double2* __restrict__ x,
                                                          double2* __restrict__ y) {
   __shared__ double2 dict[256];

@@ -6,8 +6,8 @@
 //                   stride m+1 so that column accesses of a warp fall in distinct bank pairs):
 //                   eigenvalues of a dense matrix in ascending order.
 //   tql_weights_kernel, tql_vectors_kernel
-//                   implicit QL iteration of a tridiagonal matrix (Bowdler, Martin, Reinsch and
-//                   Wilkinson, Numer. Math. 11, 293 (1968)): eigenvalues in ascending order with the
+//                   implicit QL iteration of a tridiagonal matrix (Dubrulle, Martin and Wilkinson,
+//                   Numer. Math. 12, 377 (1968)): eigenvalues in ascending order with the
 //                   squared first row of the eigenvector matrix (the quadrature weights), or with all
 //                   eigenvectors (row j of Vt = eigenvector j).
 //   duhamel_kernel  the Duhamel weight matrix of one Lanczos chain from its eigen-decomposition:

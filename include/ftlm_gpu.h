@@ -142,9 +142,11 @@ int ftlm_gpu_apply_profiled(ftlm_sector* s, const double* x_dev, double* y_dev, 
  * coefficient table in shared memory) + column-slab pass, 3 = row pass in the gauge basis
  * (ftlm_gpu_sector_down_table_gauge: register-held real coefficients, one shared-memory load per
  * hop) + column-slab pass (where the sector has no gauge table, as 2).  Automatic takes small sectors with the
- * gauge table in one pass (every output row's down and up hops in one block), else picks 3, else 2,
- * else 1; ftlm_gpu_autotune_apply times them all (the one pass is reported as path 3).  All paths give the same matrix elements (sums may
- * differ in the last bits). */
+ * gauge table in one pass (every output row's down and up hops in one block) unless they have very long or very
+ * many very short rows, else picks 3, else 2, else 1; ftlm_gpu_autotune_apply times them all (the one pass is
+ * reported as path 3).  All paths give the same matrix elements (sums may differ in the last bits).
+ * The complex128 chains (ftlm_gpu_lanczos, ftlm_gpu_ftlm_sector) keep to a path set to 1 or 2; set to 0 or 3, or
+ * on a timed handle, they run in their own kernels, whose form depends on the sector's shape. */
 int ftlm_gpu_set_apply_path(ftlm_sector* s, int path);
 
 /* lanczos_tridiagonal on the sector operator.  alpha/beta: host arrays of max_steps entries;
@@ -289,7 +291,9 @@ int ftlm_gpu_lanczos_sectors(ftlm_sector* const* secs, int n_sectors, int R, int
 /* ---- translation-orbit momentum blocks (sectors built from lattice parameters, n_sites <= 16) ----
  * Basis: canonical orbit representatives (smallest packed up<<16|dn) whose fermionic stabiliser sum
  * |A(K)| > 1e-12, ascending packed order (OrbitKBlockBasis::build, src/orbit_k_block_basis.cpp:70-117).
- * Apply: apply_orbit_k_block (src/orbit_k_block_basis.cpp:151-220) on reduced complex128 vectors. */
+ * Apply: apply_orbit_k_block (src/orbit_k_block_basis.cpp:151-220) on reduced complex128 vectors.
+ * Device memory of a block: 4 bytes per state of the sector, 12 per representative, and its source lists (4 bytes per
+ * source; 3.3 GB at 4x4 (8,8)) where they take at most a 32nd of the free memory when it is created. */
 typedef struct ftlm_orbit ftlm_orbit;
 int ftlm_gpu_orbit_create(ftlm_sector* s, int kx, int ky, ftlm_orbit** out);
 /* Same with the survival threshold of OrbitKBlockBasis::build(fb, K, survive_tol)
@@ -339,8 +343,9 @@ int ftlm_gpu_orbit_sector_batched_ftlm(ftlm_sector* s, const double* bts, int n_
  *   dlnz[3]  d lnZ/dU, d lnZ/dV, d lnZ/dt' of that estimate with the start vectors fixed: per
  *            chain the Duhamel derivative -sum_il K_il <q_i|dH/dtheta|q_l> of e_1^T e^{-bT T} e_1.
  * op_tp is a sector of the same (n_sites, N_up, N_dn) built with t = 0, t' = 1, U = V = 0 (the
- * operator dH/dt'), or NULL (dlnz[2] = 0).  Device memory: M (M+1 for method 1) vectors of the
- * sector, twice with op_tp; released by ftlm_gpu_batched_release. */
+ * operator dH/dt'), or NULL (dlnz[2] = 0).  Device memory, twice with op_tp: the M vectors of as many chains as 6 GB
+ * hold (fewer where memory is short, at least one plane), M + 1 of a block's 32 chains for method 1 on large
+ * sectors; released by ftlm_gpu_batched_release. */
 int ftlm_gpu_grad_sector(ftlm_sector* s, ftlm_sector* op_tp, double bT, int R, int M, unsigned seed, int method,
                          int start_mode, double* lnz, double* dlnz);
 /* Differentiable grand-canonical ln Z at one point (no reference counterpart; the combination is the

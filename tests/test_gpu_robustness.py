@@ -416,3 +416,35 @@ def test_chain_of_a_small_or_thin_sector(gpu, lat, nu, nd):
     (general, a1), (default, a0) = run(1), run(0)
     assert default <= 1.15 * general
     assert np.abs(a0[:8] - a1[:8]).max() <= 1e-11 * np.abs(a1).max()
+
+
+def test_column_pass_by_items_and_on_the_persistent_grid(gpu):
+    """5x3 (3,6): slabs of 256 and 128 columns run one block per item, 512 columns the persistent grid (a plane has 9,100, 18,200
+    and 4,550 items). One chain with each, against the general recurrence (rounding grows by about two a step)."""
+    from ftlm_extended_hubbard_b200 import _lib
+    s = F.Sector(F.HubbardParams(5, 3, 1.0, -0.25, 8.0, 1.0, 0.1, 0.0), 3, 6)
+    s.set_apply_path(1)
+    a1, b1, _ = s.lanczos(8, 3, start="philox")
+    s.set_apply_path(0)
+    for v in (0, 1, 2):
+        _lib.call("ftlm_gpu_set_cols_variant", s.handle, v)
+        a, b, _ = s.lanczos(8, 3, start="philox")
+        assert np.abs(a - a1).max() <= 1e-12 * np.abs(a1).max() and np.abs(b - b1).max() <= 1e-12 * np.abs(b1).max()
+
+
+@pytest.mark.parametrize("lat,nu,nd,method", [((3, 3), 3, 2, "plain"), ((3, 3), 4, 5, "batched"), ((4, 3), 4, 4, "plain"), ((4, 3), 4, 4, "batched")])
+def test_gradient_of_an_odd_number_of_planes(gpu, lat, nu, nd, method):
+    """25 vectors of each of three or five chains: an odd number of planes, of which the operator's row pass takes two at a
+    time.  The gradient is that of the chains one by one (complex64: two by two and one) put together."""
+    s = F.Sector(F.HubbardParams(*lat, 1.0, -0.2, 4.0, 1.0), nu, nd)
+    op = F.Sector(F.HubbardParams(*lat, 0.0, 1.0, 0.0, 0.0), nu, nd)
+    kw = dict(op_tp=op, method=method, start="philox")
+    R, M, beta, seed = (3, 25, 1.5, 7) if method == "plain" else (5, 25, 1.5, 7)
+    parts = [(r, 1) for r in range(R)] if method == "plain" else [(0, 2), (2, 2), (4, 1)]
+    lz, g = s.ftlm_grad(beta, R, M, seed, **kw)
+    p = [(n,) + s.ftlm_grad(beta, n, M, seed + r * 100003, **kw) for r, n in parts]
+    w = np.array([n * np.exp(l - lz) for n, l, _ in p]) / R
+    tol = 1e-10 if method == "plain" else 1e-6
+    assert abs(w.sum() - 1.0) <= tol
+    want = (w[:, None] * np.array([q[2] for q in p])).sum(0) / w.sum()
+    assert np.abs(np.asarray(g) - want).max() <= 10 * tol * np.abs(want).max()

@@ -97,7 +97,7 @@ __global__ void __launch_bounds__(1024, 1) rows_kernel(DevSector S, const typena
                                                        const double* __restrict__ st, int* __restrict__ flag,
                                                        const int* __restrict__ live) {
   using T = typename P::T;
-  if (all_ended(live)) return;
+  const bool ended = all_ended(live);  // tested after the first row's loads, which need not wait for it
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int Dd = static_cast<int>(S.Dd), Du = static_cast<int>(S.Du), nt = blockDim.x;
   const uint32_t line = static_cast<uint32_t>(Dd + 8) * 16u;
@@ -146,6 +146,7 @@ __global__ void __launch_bounds__(1024, 1) rows_kernel(DevSector S, const typena
     }
     if (P::kScaled && saw) *flag = 1;
     __syncthreads();
+    if (ended) return;
     for (int c = tid; c < Dd; c += nt) {
       const int d = gauge_string(G, c);  // table position c serves output string d
       const double dg = diag_value(S, u, S.dmask[d], cuu, S.cnt_dd[d], wp);
@@ -237,13 +238,12 @@ __global__ void __launch_bounds__(kT, P::kColThreads / kT) cols_kernel(DevSector
                                                              const double* __restrict__ st, double* __restrict__ partial,
                                                              const int* __restrict__ flag, const int* __restrict__ live) {
   using T = typename P::T;
-  if (all_ended(live)) return;
   constexpr int kPer = (kMaxDeg + kT - 1) / kT;  // list entries per thread
   __shared__ uint32_t s_off[2][kMaxDeg];
   __shared__ __align__(16) typename P::Cf s_cf[2][kMaxDeg];
   __shared__ double sh[2 * P::kC * kT / 32];
   const int t = threadIdx.x;
-  const bool filter = *flag != 0;
+  const bool filter = *flag != 0, ended = all_ended(live);
   const uint32_t Dd = static_cast<uint32_t>(S.Dd), Du = static_cast<uint32_t>(S.Du);
   const uint32_t per = (Dd + 2 * kT - 1) / (2 * kT) * Du, total = per * static_cast<uint32_t>(planes);
   uint32_t off[kPer];
@@ -274,6 +274,7 @@ __global__ void __launch_bounds__(kT, P::kColThreads / kT) cols_kernel(DevSector
     place(0, deg);
   }
   __syncthreads();
+  if (ended) return;
   for (int p = 0; p < planes; ++p) {
     double d[2 * P::kC] = {};
     const uint32_t end = per * static_cast<uint32_t>(p + 1);
@@ -404,7 +405,7 @@ __global__ void __launch_bounds__(kThreads, 4) update_kernel(typename P::T* __re
                                                              double* __restrict__ partial, int* __restrict__ flag,
                                                              const int* __restrict__ live) {
   using T = typename P::T;
-  if (all_ended(live)) return;
+  const bool ended = all_ended(live);
   __shared__ double sh[P::kC * kThreads / 32];
   const int plane = blockIdx.x / nb, b = blockIdx.x - plane * nb;
   double s_in[P::kC], c1r[P::kC], c1i[P::kC], c2[P::kC];
@@ -416,6 +417,7 @@ __global__ void __launch_bounds__(kThreads, 4) update_kernel(typename P::T* __re
     c1i[q] = st[kBtC1i * 32 + ch];
     c2[q] = use_prev ? st[kBtC2 * 32 + ch] : 0.0;
   }
+  if (ended) return;
   Neu acc[P::kC];
   const int64_t base = static_cast<int64_t>(plane) * dim, stride = static_cast<int64_t>(nb) * kThreads;
   for (int64_t i0 = static_cast<int64_t>(b) * kThreads + threadIdx.x; i0 < dim; i0 += 2 * stride) {
@@ -575,7 +577,9 @@ cudaError_t step(const DevSector& S, const typename P::T* Wk, const typename P::
   int* fin = z.flags + (P::kScaled ? 0 : (k & 1));
   int* fout = z.flags + (P::kScaled ? 0 : ((k + 1) & 1));
   if (!items_fit(S, planes)) return cudaErrorInvalidValue;
-  int* live = z.flags + 2;
+  // Below this a step is its launches, with work or without, and the reads of the count cost it 0.65 of 24 us (3x3 (4,4)).
+  constexpr int64_t kCounted = int64_t(1) << 18;
+  int* live = S.dim * planes >= kCounted ? z.flags + 2 : nullptr;
   const cudaError_t e = launch_rows<P>(S, Wk, Y, planes, z.st, fin, live, s);
   if (e != cudaSuccess) return e;
   const int nc = launch_cols<P>(S, Wk, Y, planes, z.st, z.partial, z.items, fin, live, s);
